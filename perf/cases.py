@@ -15,6 +15,7 @@ The forward pass is the only direction there is.  Shapes are those of the benchm
 """
 import math
 
+import numpy as np
 import torch
 
 import shflbw_sparse_nn_b200 as sb
@@ -164,6 +165,67 @@ def run(s):
     else:
         s["net"].forward(torch.cuda.current_stream())
     return s["net"].y
+
+
+# --------------------------------------------------------------------- the same in 64 bits --
+
+def _dense64(m):
+    """The dense matrix that a sparse operand's arrays describe, rows in logical order."""
+    rows = torch.from_numpy(np.asarray(m.row_permute_ids).copy() if m.row_permute else np.arange(m.nrow)).cuda().long()
+    per_block = torch.from_numpy(np.diff(np.asarray(m.indptr)).astype(np.int64)).cuda()
+    block = torch.repeat_interleave(torch.arange(len(per_block), device="cuda"), per_block)
+    cols = torch.from_numpy(np.asarray(m.indices).astype(np.int64)).cuda()
+    values = torch.from_numpy(np.asarray(m.values).view(np.float16).copy()).cuda().double().reshape(-1, m.brow)
+    d = torch.zeros((m.nrow, m.ncol), dtype=torch.float64, device="cuda")
+    d[rows.reshape(-1, m.brow)[block], cols[:, None]] = values
+    return d
+
+
+def _conv64(x, f, stride):
+    """x [B][H][W][C] and a filter whose columns are (r * R + s) * C + c; padding R // 2, outputs ceil(H / stride)."""
+    B, H, W, ch = x.shape
+    Ho, Wo, R = -(-H // stride), -(-W // stride), f.R
+    w = _dense64(f).reshape(f.F, R, R, ch)
+    p = torch.nn.functional.pad(x, (0, 0, R // 2, R // 2, R // 2, R // 2))
+    out = torch.zeros((B, Ho, Wo, f.F), dtype=torch.float64, device="cuda")
+    for r in range(R):
+        for c in range(R):
+            tap = p[:, r:r + (Ho - 1) * stride + 1:stride, c:c + (Wo - 1) * stride + 1:stride]
+            out += tap @ w[:, r, c].t()
+    return out
+
+
+def exact(case, seed):
+    s = prepare(case, seed)
+    kind = case["kind"]
+    if kind == "spmm":
+        y = case["alpha"] * (_dense64(s["mat"]) @ s["B"].double())
+        return y + case["beta"] * s["C"].double() if case["beta"] != 0.0 else y
+    if kind == "spmm_host":
+        return (_dense64(s["mat"]) @ s["B"].cuda().double()).cpu()
+    if kind == "linear":
+        y = s["x"].double() @ _dense64(s["layer"].spmat).t()
+        return y + s["layer"].bias.double() if case["bias"] else y
+    if kind == "spconv":
+        return _conv64(s["x"].double(), s["filter"], case["stride"])
+    if kind == "conv2d":
+        y = _conv64(s["x"].permute(0, 2, 3, 1).double(), s["layer"].spfilter, case["stride"])
+        return (y + s["layer"].bias.double() if case["bias"] else y).permute(0, 3, 1, 2)
+    net = s["net"]
+    outs = {-1: net.x.double()}
+    last_use = {}
+    for i, sp in enumerate(net.specs):
+        for j in (sp.src, sp.residual):
+            if j is not None:
+                last_use[j] = i
+    for i, sp in enumerate(net.specs):
+        y = net.alphas[i] * _conv64(outs[sp.src], net.filters[i], sp.stride)
+        if sp.residual is not None:
+            y = y + outs[sp.residual]
+        outs[i] = y.clamp_(min=0) if sp.relu else y
+        for j in [j for j in outs if last_use.get(j, len(net.specs)) <= i]:
+            del outs[j]
+    return outs[len(net.specs) - 1]
 
 
 # -------------------------------------------------------------------------------- cost --
