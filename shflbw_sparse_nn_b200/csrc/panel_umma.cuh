@@ -24,8 +24,8 @@
 // One CTA per SM loops over items (item = blockIdx.x + i*gridDim.x, decoded block-major or
 // tile-major, PanelParams::tile_major); their extents are read once into a shared-memory table.
 // Warp roles (warp w issues from scheduler partition w % 4; EW = 8 or 16 epilogue warps):
-//   warps 0..EW-1    epilogue.  Warp w reads TMEM lane quadrant w % 4 and part w / 4 of the
-//                    accumulator columns.  Tokens in lanes: TMEM -> registers -> fp16 -> transpose
+//   warps 0..EW-1    epilogue.  Warp w reads TMEM lane quadrant w % 4 and half w / 4 % 2 of the
+//                    accumulator columns; sixteen warps are two sets that take the items in turn.  Tokens in lanes: TMEM -> registers -> fp16 -> transpose
 //                    of 32-row chunks through shared memory -> 16-byte global stores (inverse row
 //                    permutation fused for SpMM).  Rows in lanes: stores straight from registers.
 //   warp  EW         allocates TMEM; its lane 0 issues tcgen05.mma, releases stages and
@@ -149,10 +149,11 @@ constexpr int kPanelSpmm = 0, kPanelConv = 1, kPanelConvChain = 2, kPanelSpmmRow
 //                   step; row ids travel in registers (loaded two stages ahead).
 constexpr int kGatherCpAsync = 0, kGatherTma = 1, kGatherCpAsyncArrive = 2;
 
-// EW: epilogue warps, 8 or 16.  A warp can read only the TMEM lane quadrant warp % 4, so the
+// EW: epilogue warps, 8 or 16.  A warp can read only the TMEM lane quadrant warp % 4, so the two
 // warps of a quadrant split the accumulator columns between them.  Items with few non-zero
 // columns are all epilogue, and one warp's chain (TMEM read, convert, transpose, store) is
-// latency-bound: sixteen warps keep four such chains per scheduler in flight instead of two.
+// latency-bound: sixteen warps, as two sets on alternate items, keep four such chains per
+// scheduler in flight instead of two.
 template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int LAG_ = 1, int GATHER_ = kGatherCpAsync,
           int EW_ = 8>
 struct PanelCfg {
@@ -200,13 +201,16 @@ struct PanelCfg {
     // rows / filters through 2 KB so that its global stores are 16 bytes per lane and 64-byte
     // runs.  With rows in lanes the stores go straight from registers.
     static constexpr int OUT_BYTES = (MODE == kPanelSpmmRows || MODE == kPanelConvChainRows) ? 0 : EW * 2048;
+    // With sixteen epilogue warps the addend of an item (C, or a chained layer's residual) is copied to
+    // shared memory an item ahead: each lane's own 16-byte pieces, 64 rows x 32 tokens per warp.
+    static constexpr int RES_BYTES = EW == 16 ? EW * 4096 : 0;
     static constexpr int BAR_BYTES = (STAGES * 2 + 12) * 8;  // mbarriers (ring, up to 4 + 4 accumulator, drain) + tmem slot + abort flag
     static constexpr int TAB_BYTES = 512 * 8;               // per-CTA item table (kPanelMaxItemsPerCta entries)
     static constexpr int IDX_AHEAD = LAG + 1;              // a group fetches row ids this many of its stages ahead
     static constexpr int IDX_RING = (IDX_AHEAD + 1) * GROUPS <= 8 ? 8 : 16;   // stages of row ids kept in shared memory
     static_assert((IDX_AHEAD + 1) * GROUPS <= IDX_RING, "row-id ring too small");
     static constexpr int IDX_BYTES = (TMA || ARRIVE) ? 0 : IDX_RING * KS * 4;   // (the TMA gather loads its row ids straight into registers)
-    static constexpr int SMEM_BYTES = PIPE_BYTES + OUT_BYTES + BAR_BYTES + TAB_BYTES + IDX_BYTES + 1024;  // + align slack
+    static constexpr int SMEM_BYTES = PIPE_BYTES + OUT_BYTES + RES_BYTES + BAR_BYTES + TAB_BYTES + IDX_BYTES + 1024;  // + align slack
     static constexpr bool SWAP = MODE == kPanelSpmmRows || MODE == kPanelConvChainRows;
     static constexpr int KG_BYTES = SWAP ? T * 16 : 2048;   // 8 gathered rows (one K group) of the token tile
     static constexpr uint32_t ACC_COLS = SWAP ? T : TM * V; // fp32 columns of one accumulator set
@@ -215,6 +219,9 @@ struct PanelCfg {
     // four with sixteen epilogue warps, whose items are so short that the hand-over itself
     // (commit -> barrier -> poll -> TMEM read -> release -> poll -> issue) is what two sets
     // cannot hide.
+    // Sixteen epilogue warps work as two sets of eight that take the items in turn, so that the chains
+    // of two items (accumulator wait, TMEM read, transpose, stores) overlap.
+    static constexpr int ESETS = EW / 8;
     static constexpr int NBUF = (EW == 16 && ACC_COLS * 4 <= 512) ? 4 : 2;
     static constexpr uint32_t TMEM_COLS = NBUF * ACC_COLS < 32 ? 32 : NBUF * ACC_COLS;
     static_assert(V == 16 || V == 32 || V == 64 || V == 128, "row-block height");
@@ -259,7 +266,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     extern __shared__ uint8_t smem_raw[];
     // 1024-byte alignment: swizzle atoms are addressed by absolute shared-memory address bits.
     uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-    uint8_t* bar_area = smem + Cfg::PIPE_BYTES + Cfg::OUT_BYTES;
+    uint8_t* bar_area = smem + Cfg::PIPE_BYTES + Cfg::OUT_BYTES + Cfg::RES_BYTES;
     uint64_t* full_bar = (uint64_t*)bar_area;          // [STAGES] producers -> MMA
     uint64_t* empty_bar = full_bar + STAGES;           // [STAGES] MMA -> producers
     constexpr int NBUF = Cfg::NBUF;
@@ -304,7 +311,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         }
         for (int b = 0; b < NBUF; ++b) {
             sm100::mbar_init(&acc_full[b], 1);
-            sm100::mbar_init(&acc_empty[b], EW);  // one arrival per epilogue warp
+            sm100::mbar_init(&acc_empty[b], EW / Cfg::ESETS);  // one arrival per epilogue warp of the set that reads it
         }
         sm100::mbar_init(drain_bar, 1);
         *cta_abort = 0;
@@ -910,13 +917,14 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         if (lane == 0) CTRACE(3);
     } else {
         // -------------------------------------------------------------- epilogue ----
-        // Warp w reads TMEM lane quadrant w % 4 (tokens) and part w / 4 of the accumulator
-        // columns (the block's output rows / filters): halves with eight warps, quarters with
-        // sixteen.
+        // Warp w reads TMEM lane quadrant w % 4 (tokens) and half w / 4 % 2 of the accumulator
+        // columns (the block's output rows / filters).  Sixteen warps are two sets of eight that take
+        // the items in turn: against all sixteen on one item (a quarter of the columns each), 108 ->
+        // 93 us on 56x56x64 -> 256 at batch 256, since an item's chain of waits is most of its time.
         sm100::grid_dependency_wait();
-        const int quad = warp & 3, half_id = warp >> 2;
+        const int quad = warp & 3, half_id = (warp >> 2) & 1;
         // (a single 16- or 32-column accumulator is not split; two 16-column accumulators go to the two halves)
-        constexpr int HALVES = (Cfg::ACC_COLS >= 64 || (V == 16 && TM == 2)) ? EW / 4 : 1;
+        constexpr int HALVES = (Cfg::ACC_COLS >= 64 || (V == 16 && TM == 2)) ? 2 : 1;
         constexpr int COLS = Cfg::ACC_COLS / HALVES;          // fp32 columns handled by this warp
         constexpr int CW = COLS < 32 ? COLS : 32;             // columns per pass through the 2 KB tile
         const bool reads = half_id < HALVES;
@@ -925,7 +933,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 #ifdef SHFLBW_COUNTERS
         long long ec_wait = 0, ec_t0 = clock64();
 #endif
-        for (int li = 0; li < nloc; ++li) {
+        bool res_primed = false;               // addend copies (RES_BYTES) run an item ahead
+        for (int li = Cfg::ESETS > 1 ? warp >> 3 : 0; li < nloc; li += Cfg::ESETS) {
 #ifdef SHFLBW_COUNTERS
             const long long ew0 = clock64();
 #endif
@@ -1142,29 +1151,61 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             __half* const obase = MODE == kPanelSpmm ? p.D : p.out;
             const __half2 zero2 = __float2half2_rn(0.f);
             // What gets added to the product (beta * C, or the residual of a chained layer) does not
-            // depend on the accumulator: the addends of the item's first two chunks are requested
-            // BEFORE waiting for it, each later chunk's two chunks ahead, so that their global-memory
-            // latency is off the critical path (these layers are often all epilogue).  (Requesting
-            // the NEXT item's addend a whole item ahead was measured 3-5 % slower on the residual
-            // layers of the ResNet stack, which run at ~4.1 TB/s of HBM traffic either way.)
+            // depend on the accumulator and is requested early, so that its global-memory latency is off
+            // the critical path (these layers are often all epilogue).
+            //   Sixteen epilogue warps: an item ahead, by cp.async into the lane's own slots in shared
+            // memory.  Ordinary loads would need an L1 line per piece until it arrives, and beside a
+            // block's shared memory the L1 holds about 28 KB, less than one item's 32 KB: with them more
+            // requests in flight made these layers slower (56x56x64 -> 256 with residual, batch 256:
+            // 214 us with loads before the accumulator wait, 230 with two items' loads in flight, 187 with
+            // the copies; the same product without a residual takes 93).
+            //   Eight: into registers, the first two chunks before the accumulator wait, each later
+            // chunk's two chunks ahead.
             constexpr int NCH = COLS / CW;
+            constexpr bool RES_AHEAD = Cfg::RES_BYTES > 0;
             const bool add_res = MODE == kPanelConvChain && p.res != nullptr;
             const bool need_add = ok_g && (use_c || add_res);
-            uint4 addend[NCH > 1 ? 2 : 1][4];
+            auto addend_at = [&](int blk_, uint32_t goff_, int cc, int i) -> const __half* {
+                const int m = mbase + cc + slot_row(i);
+                if (use_c) {
+                    const int row = (p.perm && !(ablate & 1024)) ? __ldg(p.perm + blk_ * V + m) : blk_ * V + m;
+                    return p.C + (size_t)((uint32_t)row * (uint32_t)p.N) + (size_t)goff_;
+                }
+                const uint32_t rr = (uint32_t)(p.res_map ? __ldg(p.res_map + blk_ * V + m) : blk_ * V + m) * (uint32_t)p.out_plane;
+                return p.res + (size_t)rr + (size_t)goff_;
+            };
+            uint4 addend[NCH > 1 && !RES_AHEAD ? 2 : 1][4];
             auto fetch_addend = [&](int blk_, uint32_t goff_, int cc, uint4 (&dst)[4]) {
 #pragma unroll
-                for (int i = 0; i < NSLOT; ++i) {
-                    const int m = mbase + cc + slot_row(i);
-                    if (use_c) {
-                        const int row = (p.perm && !(ablate & 1024)) ? __ldg(p.perm + blk_ * V + m) : blk_ * V + m;
-                        dst[i] = *(const uint4*)(p.C + (size_t)((uint32_t)row * (uint32_t)p.N) + (size_t)goff_);
-                    } else {
-                        const uint32_t rr = (uint32_t)(p.res_map ? __ldg(p.res_map + blk_ * V + m) : blk_ * V + m) * (uint32_t)p.out_plane;
-                        dst[i] = *(const uint4*)(p.res + (size_t)rr + (size_t)goff_);
+                for (int i = 0; i < NSLOT; ++i) dst[i] = *(const uint4*)addend_at(blk_, goff_, cc, i);
+            };
+            uint8_t* const my_res = smem + Cfg::PIPE_BYTES + Cfg::OUT_BYTES + warp * 4096 + lane * 16;   // slot (chunk, i): + (chunk*4 + i) * 512
+            static_assert(!RES_AHEAD || NCH * NSLOT * 512 <= 4096, "addend slots");
+            auto copy_addend = [&](int blk_, uint32_t goff_, bool ok_, int ch_) {   // one cp.async group per chunk, empty or not
+                if (ok_) {
+#pragma unroll
+                    for (int i = 0; i < NSLOT; ++i)
+                        sm100::cp_async_16(sm100::smem_u32(my_res + (ch_ * 4 + i) * 512), addend_at(blk_, goff_, ch_ * CW, i), 16u);
+                }
+                sm100::cp_async_commit();
+            };
+            int blk_next = 0;                     // this warp's next item: block, group offset, anything to copy
+            uint32_t goff_next = 0;
+            bool ok_next = false;
+            if constexpr (RES_AHEAD) {
+                if (use_c || add_res) {
+                    if (!res_primed) {            // the warp's first item: nothing was copied ahead
+#pragma unroll
+                        for (int ch = 0; ch < NCH; ++ch) copy_addend(blk, goff, ok_g, ch);
+                        res_primed = true;
+                    }
+                    if (li + Cfg::ESETS < nloc) {
+                        const int item_next = (int)blockIdx.x + (li + Cfg::ESETS) * (int)gridDim.x;
+                        blk_next = item_block(item_next);
+                        goff_next = group_offset(item_tile(item_next) * T, ok_next);
                     }
                 }
-            };
-            if (need_add) {
+            } else if (need_add) {
                 fetch_addend(blk, goff, 0, addend[0]);
                 if constexpr (NCH > 1) fetch_addend(blk, goff, CW, addend[1]);
             }
@@ -1210,6 +1251,13 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     }
                 }
                 __syncwarp();
+                if constexpr (RES_AHEAD) {
+                    if (use_c || add_res) {
+                        sm100::cp_async_wait<NCH - 1>();     // this chunk's copies (each lane reads only its own)
+#pragma unroll
+                        for (int i = 0; i < NSLOT; ++i) addend[0][i] = *(const uint4*)(my_res + (ch * 4 + i) * 512);
+                    }
+                }
                 if (!(ablate & 512)) {
 #pragma unroll
                     for (int k = 0; k < NSLOT / 2; ++k) {
@@ -1227,14 +1275,14 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                             const size_t off = (size_t)roff[i] + (size_t)goff;
                             if (use_c) {
                                 __half* h = (__half*)&v;
-                                const __half* cadd = (const __half*)&addend[NCH > 1 ? (ch & 1) : 0][i];
+                                const __half* cadd = (const __half*)&addend[NCH > 1 && !RES_AHEAD ? (ch & 1) : 0][i];
 #pragma unroll
                                 for (int e = 0; e < 8; ++e) h[e] = __hfma(h[e], alpha1, __hmul(cadd[e], beta1));
                             }
                             if constexpr (MODE == kPanelConvChain) {   // out = relu(alpha * conv + residual), fp16
                                 __half2* h = (__half2*)&v;
                                 if (add_res) {
-                                    const __half2* rh = (const __half2*)&addend[NCH > 1 ? (ch & 1) : 0][i];
+                                    const __half2* rh = (const __half2*)&addend[NCH > 1 && !RES_AHEAD ? (ch & 1) : 0][i];
 #pragma unroll
                                     for (int e = 0; e < 4; ++e) h[e] = __hadd2(h[e], rh[e]);
                                 }
@@ -1248,7 +1296,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     }
                     }
                 }
-                if constexpr (NCH > 2) { if (need_add && ch + 2 < NCH) fetch_addend(blk, goff, cc + 2 * CW, addend[ch & 1]); }
+                if constexpr (RES_AHEAD) { if (use_c || add_res) copy_addend(blk_next, goff_next, ok_next, ch); }
+                else if constexpr (NCH > 2) { if (need_add && ch + 2 < NCH) fetch_addend(blk, goff, cc + 2 * CW, addend[ch & 1]); }
                 __syncwarp();
             }
             } else {
@@ -1298,6 +1347,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             }
             if (tid == 0) TRACE(2, li, 3);
         }
+        if constexpr (Cfg::RES_BYTES > 0) sm100::cp_async_wait<0>();   // nothing of this warp is in flight when the block ends
 #ifdef SHFLBW_COUNTERS
         if (lane == 0 && p.trace != nullptr && warp < 8) {   // per epilogue warp: cycles waiting for an accumulator, cycles in the role
             unsigned long long* o = p.trace + 148 * 48 + (blockIdx.x * 8 + warp) * 2;

@@ -198,10 +198,11 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         // Shallow items (at most 64 non-zero columns): sixteen epilogue warps and three producer
         // warps, each a group of its own (20 warps: 96 registers per thread); stages of 32 columns,
-        // eight of them beside the 32 KB of epilogue tiles, so that up to eight items' inputs are
-        // in flight from HBM.  Built for 64-row blocks.
+        // six of them beside the 32 KB of epilogue tiles and the 64 KB of addend slots, so that up to
+        // six items' inputs are in flight from HBM (five: 37.5 -> 40.5 us on 14x14x256 -> 1024 at batch
+        // 256, the rest equal).  Built for 64-row blocks.
         if (wide_epilogue && tile == 256 && V == 64) {
-            *out = choice<64, 2, 32, 8, 3, MODE, 3, 1, shflbw::kGatherCpAsync, 16>();
+            *out = choice<64, 2, 32, 6, 3, MODE, 3, 1, shflbw::kGatherCpAsync, 16>();
             return true;
         }
     }
@@ -968,6 +969,18 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     if (!f || !st || !st->init_success || !st->chain || !res_chain) return SHFLBW_ERR_INVALID_ARG;
     if (!on_current_device(*f) || st->blk_ptr != f->d_kptr) return SHFLBW_ERR_INVALID_ARG;
     if ((uintptr_t)res_chain & 15) return SHFLBW_ERR_UNSUPPORTED;
+    // The sixteen-epilogue-warp kernel copies the residual an item ahead, which pays up to two stages of
+    // columns per block (7x7x512 -> 2048 with residual, batch 256: 38 -> 31 us); without a residual the
+    // limit is one stage (pick_panel).
+    if (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
+        (f->kptr.empty() ? 0 : f->kptr.back()) <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count()) {
+        PanelChoice ch;
+        if (lookup<shflbw::kPanelConvChain>(64, 256, &ch, shflbw::kGatherCpAsync, true)) {
+            const int rc = allow_smem(ch.fn, ch.smem);
+            if (rc != SHFLBW_OK) return rc;
+            st->variant = 2; st->stages = ch.stages; st->producer_warps = ch.pw; st->block_x = ch.threads; st->shared_mem_size = ch.smem;
+        }
+    }
     // A map buffer made by an earlier call for this state is one of the handle's retired buffers.
     const int* prev_map = nullptr;
     for (void* r : f->retired) if (r == (const void*)st->residual_map) prev_map = st->residual_map;
