@@ -200,6 +200,15 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
  * (a cudaStream_t; NULL = default stream).  Returns launch errors only. */
 int shflbw_spmm_exec(const shflbw_spmm_state_t* st, void* stream);
 
+/* A sparse linear layer, y = x W^T + bias, with W the sparse operand: x[tokens][K] (token-major, any
+ * alignment) is transposed into xt[K][N] with zeros beyond `tokens`, and out[M][N] (feature-major) =
+ * W . xt + bias[M] is formed with the bias added to the fp16 product in the kernel's epilogue.  x == NULL:
+ * xt holds the operand already.  bias may be NULL.  xt and out are caller-owned device buffers,
+ * 16-byte aligned, N % 8 == 0, N >= tokens.  Asynchronous on `stream`; two launches.  No counterpart in
+ * the reference (its operator takes the feature-major operand only). */
+int shflbw_linear_exec(const shflbw_matrix_t* m, int tokens, const void* x, const void* bias, void* xt, int N,
+                       void* out, void* stream);
+
 /* Reads (and clears) the device status word of the matrix used by `st`; synchronises the
  * device.  SHFLBW_OK or SHFLBW_ERR_DEVICE_TIMEOUT. */
 int shflbw_matrix_device_status(const shflbw_matrix_t* m);

@@ -257,6 +257,12 @@ def SpmmBlockwiseExecFn(state: SpmmBlockwiseOp, stream=None) -> None:
     state(stream)
 
 
+def linear_exec(spmat: BlockwiseSpMatrix, tokens: int, x, bias, xt, N: int, out, stream=None) -> None:
+    """out[M][N] = W . xt + bias[M], x[tokens][K] transposed into xt[K][N] first (x None: xt is the operand)."""
+    check(_cabi.lib().shflbw_linear_exec(spmat._h, tokens, _ptr(x), _ptr(bias), _ptr(xt), N, _ptr(out), _stream_ptr(stream)),
+          "linear_exec")
+
+
 def spmm_host(spmat: BlockwiseSpMatrix, N: int, B_host: np.ndarray, D_host: np.ndarray, alpha=1.0,
               C_host: Optional[np.ndarray] = None, beta=0.0) -> None:
     """End-to-end call with HOST buffers (numpy arrays or pinned torch CPU tensors)."""

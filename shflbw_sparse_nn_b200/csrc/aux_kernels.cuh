@@ -79,6 +79,47 @@ relayout_nhwc_to_chwn(const __half* __restrict__ in, __half* __restrict__ Xs, in
     }
 }
 
+// x[t][k] (tokens x K) -> xt[k][Np]: token-major activations to the feature-major operand of an SpMM,
+// tokens padded with zeros to Np (a multiple of 8).  One block: 64 tokens x 64 features through 8 KB of
+// shared memory; 16-byte loads of 8 features of one token, 2-byte scatters into [feature][token] (8-token
+// groups XOR-swizzled by the feature group: no bank conflicts), 16-byte stores of 8 tokens of one feature.
+// vec: K % 8 == 0 and x 16-byte aligned; otherwise the loads are 2 bytes each.  Bound by launch latency at
+// decode sizes (37 x 4096: 1.7 us, against 4.2 us for a fill and a strided copy).
+__global__ void __launch_bounds__(256)
+transpose_tokens(const __half* __restrict__ x, __half* __restrict__ xt, int tokens, int K, int Np, int vec) {
+    __shared__ __align__(16) __half tile[64 * 64];
+    grid_dep_launch();
+    grid_dep_wait();                                     // x may be the previous kernel's output
+    const int k_tiles = (K + 63) / 64;
+    const int k0 = (blockIdx.x % k_tiles) * 64, t0 = (blockIdx.x / k_tiles) * 64;
+    const int c = threadIdx.x & 7, r0 = threadIdx.x >> 3;   // 16-byte chunk, row of the pass
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const int r = r0 + 32 * pass;                    // token of the tile
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        __half* h = (__half*)&v;
+        if (t0 + r < tokens) {
+            const int k = k0 + c * 8;
+            const __half* src = x + (size_t)(t0 + r) * K + k;
+            if (vec) { if (k < K) v = *(const uint4*)src; }
+            else
+#pragma unroll
+                for (int j = 0; j < 8; ++j) if (k + j < K) h[j] = src[j];
+        }
+        const int col = (((r >> 3) ^ c) << 3) | (r & 7);    // feature group c: token group XOR c
+#pragma unroll
+        for (int j = 0; j < 8; ++j) tile[(c * 8 + j) * 64 + col] = h[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const int f = r0 + 32 * pass;                    // feature of the tile
+        if (k0 + f < K && t0 + c * 8 < Np)
+            *(uint4*)(xt + (size_t)(k0 + f) * Np + t0 + c * 8) =
+                *(const uint4*)(tile + f * 64 + ((c ^ ((f >> 3) & 7)) << 3));
+    }
+}
+
 // out[q][perm[f]] = staged[q][f] for every output position q.  G = clamp(F/8, 8, 64) threads
 // share one position (each moves 8 filters at a time with 16-byte global accesses), so a block
 // of 256 threads handles 256/G positions at once: 4 for F >= 512 (two warps each -- the kernel

@@ -113,6 +113,7 @@ struct alignas(64) PanelParams {
     const __half* B;         // [K][N]
     const __half* C;         // [M][N] or nullptr
     __half* D;               // [M][N]
+    int c_row;               // C is one value per output row ([M], a bias) instead of a matrix
     int N;                   // dense columns (SpMM) / Ho*Wo*Bp (SpConv)
     // SpConv (input staged channel-major, batch innermost, with a zero halo:
     // Xs[c][Hp][Wp][Bp], Hp = Hin + R - 1, Wp = Win + S - 1, image origin at (R/2, S/2))
@@ -248,6 +249,12 @@ __device__ __forceinline__ uint32_t tile128_off(int r, int c) {
 }
 __device__ __forceinline__ uint32_t tile64_off(int r, int c) { return (uint32_t)(r * 128 + ((c ^ (r & 7)) << 4)); }
 __device__ __forceinline__ uint32_t tile32_off(int r, int c) { return (uint32_t)(r * 64 + ((c ^ ((r >> 1) & 3)) << 4)); }
+
+// The value at p in all eight halves of 16 bytes.
+__device__ __forceinline__ uint4 broadcast8(const __half* p) {
+    const uint32_t h = __ldg((const unsigned short*)p) * 0x10001u;
+    return make_uint4(h, h, h, h);
+}
 
 constexpr int kPanelMaxItemsPerCta = 512;  // capacity of the per-CTA item table
 
@@ -1058,7 +1065,9 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                             for (int c = 0; c < 4; ++c) {
                                 if (tok0 + c * 8 < p.N) {                // N % 8 == 0: 8 tokens are valid as a whole
                                     if (use_c) {                         // (the rare beta != 0 case pays the load's latency here)
-                                        const uint4 cv = *(const uint4*)(p.C + roff + tok0 + c * 8);
+                                        uint4 cv;
+                                        if (p.c_row) cv = broadcast8(p.C + (p.perm ? __ldg(p.perm + blk * V + m) : blk * V + m));
+                                        else cv = *(const uint4*)(p.C + roff + tok0 + c * 8);
                                         __half* h = (__half*)&v[c];
                                         const __half* ch = (const __half*)&cv;
 #pragma unroll
@@ -1163,12 +1172,14 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             // chunk's two chunks ahead.
             constexpr int NCH = COLS / CW;
             constexpr bool RES_AHEAD = Cfg::RES_BYTES > 0;
+            const bool ahead = RES_AHEAD && ((use_c && !p.c_row) || (MODE == kPanelConvChain && p.res != nullptr));
             const bool add_res = MODE == kPanelConvChain && p.res != nullptr;
             const bool need_add = ok_g && (use_c || add_res);
             auto addend_at = [&](int blk_, uint32_t goff_, int cc, int i) -> const __half* {
                 const int m = mbase + cc + slot_row(i);
                 if (use_c) {
                     const int row = (p.perm && !(ablate & 1024)) ? __ldg(p.perm + blk_ * V + m) : blk_ * V + m;
+                    if (p.c_row) return p.C + row;
                     return p.C + (size_t)((uint32_t)row * (uint32_t)p.N) + (size_t)goff_;
                 }
                 const uint32_t rr = (uint32_t)(p.res_map ? __ldg(p.res_map + blk_ * V + m) : blk_ * V + m) * (uint32_t)p.out_plane;
@@ -1177,7 +1188,11 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             uint4 addend[NCH > 1 && !RES_AHEAD ? 2 : 1][4];
             auto fetch_addend = [&](int blk_, uint32_t goff_, int cc, uint4 (&dst)[4]) {
 #pragma unroll
-                for (int i = 0; i < NSLOT; ++i) dst[i] = *(const uint4*)addend_at(blk_, goff_, cc, i);
+                for (int i = 0; i < NSLOT; ++i) {
+                    const __half* src = addend_at(blk_, goff_, cc, i);
+                    if (MODE == kPanelSpmm && p.c_row) dst[i] = broadcast8(src);
+                    else dst[i] = *(const uint4*)src;
+                }
             };
             uint8_t* const my_res = smem + Cfg::PIPE_BYTES + Cfg::OUT_BYTES + warp * 4096 + lane * 16;   // slot (chunk, i): + (chunk*4 + i) * 512
             static_assert(!RES_AHEAD || NCH * NSLOT * 512 <= 4096, "addend slots");
@@ -1193,7 +1208,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             uint32_t goff_next = 0;
             bool ok_next = false;
             if constexpr (RES_AHEAD) {
-                if (use_c || add_res) {
+                if (ahead) {
                     if (!res_primed) {            // the warp's first item: nothing was copied ahead
 #pragma unroll
                         for (int ch = 0; ch < NCH; ++ch) copy_addend(blk, goff, ok_g, ch);
@@ -1252,10 +1267,12 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 }
                 __syncwarp();
                 if constexpr (RES_AHEAD) {
-                    if (use_c || add_res) {
+                    if (ahead) {
                         sm100::cp_async_wait<NCH - 1>();     // this chunk's copies (each lane reads only its own)
 #pragma unroll
                         for (int i = 0; i < NSLOT; ++i) addend[0][i] = *(const uint4*)(my_res + (ch * 4 + i) * 512);
+                    } else if (need_add) {
+                        fetch_addend(blk, goff, cc, addend[0]);
                     }
                 }
                 if (!(ablate & 512)) {
@@ -1296,7 +1313,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     }
                     }
                 }
-                if constexpr (RES_AHEAD) { if (use_c || add_res) copy_addend(blk_next, goff_next, ok_next, ch); }
+                if constexpr (RES_AHEAD) { if (ahead) copy_addend(blk_next, goff_next, ok_next, ch); }
                 else if constexpr (NCH > 2) { if (need_add && ch + 2 < NCH) fetch_addend(blk, goff, cc + 2 * CW, addend[ch & 1]); }
                 __syncwarp();
             }

@@ -504,7 +504,8 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
     return SHFLBW_OK;
 }
 
-int shflbw_spmm_exec(const shflbw_spmm_state_t* st, void* stream) {
+// bias: nullptr, or one value per output row, added to the fp16 product (state without C; tensor-core kernels).
+static int spmm_exec_impl(const shflbw_spmm_state_t* st, const void* bias, void* stream) {
     if (!st || !st->init_success) return SHFLBW_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     if (st->kernel == SHFLBW_KERNEL_SIMT) {
@@ -523,6 +524,7 @@ int shflbw_spmm_exec(const shflbw_spmm_state_t* st, void* stream) {
         p.perm = st->perm; p.status_word = st->status_word; p.alpha = st->alpha; p.beta = st->beta;
         p.wait_limit = g_wait_limit; p.inject_from = g_inject_from; p.idx_limit = (unsigned)(st->K - 1);
         p.B = (const __half*)st->B; p.C = (const __half*)st->C; p.D = (__half*)st->D; p.N = st->N;
+        if (bias) { p.C = (const __half*)bias; p.beta = 1.f; p.c_row = 1; }
         p.wide_stores = (st->N % 16 == 0) && (((uintptr_t)st->D & 31) == 0);
         if (ch.gather != st->gather) return SHFLBW_ERR_INVALID_ARG;
         if (st->gather == shflbw::kGatherTma) std::memcpy(p.tmap_b, st->tmap_b, sizeof p.tmap_b);
@@ -541,6 +543,24 @@ int shflbw_spmm_exec(const shflbw_spmm_state_t* st, void* stream) {
     }
     CK(cudaGetLastError());
     return SHFLBW_OK;
+}
+
+int shflbw_spmm_exec(const shflbw_spmm_state_t* st, void* stream) { return spmm_exec_impl(st, nullptr, stream); }
+
+int shflbw_linear_exec(const shflbw_matrix_t* m, int tokens, const void* x, const void* bias, void* xt, int N, void* out,
+                       void* stream) {
+    if (!m || !xt || !out || N <= 0 || tokens > N || (x && tokens <= 0)) return SHFLBW_ERR_INVALID_ARG;
+    if (((uintptr_t)x | (uintptr_t)bias) & 1) return SHFLBW_ERR_UNSUPPORTED;
+    shflbw_spmm_state_t st;
+    const int rc = shflbw_spmm_init(m, N, xt, 1.f, nullptr, 0.f, out, SHFLBW_KERNEL_AUTO, &st);   // (asks for 16-byte aligned xt, out and N % 8)
+    if (rc != SHFLBW_OK) return rc;
+    if (x) {
+        const long long tiles = (long long)((m->ncol + 63) / 64) * ((N + 63) / 64);   // < 2^31: ncol * N < 2^40 or refused above
+        if (tiles >= (1ll << 31)) return SHFLBW_ERR_UNSUPPORTED;
+        CK(launch(shflbw::transpose_tokens, dim3((unsigned)tiles), dim3(256), 0, (cudaStream_t)stream, (const __half*)x, (__half*)xt, tokens,
+                  m->ncol, N, (int)(m->ncol % 8 == 0 && ((uintptr_t)x & 15) == 0)));
+    }
+    return spmm_exec_impl(&st, bias, stream);
 }
 
 int shflbw_spmm_launches_per_exec(const shflbw_spmm_state_t* st) { return st && st->init_success ? 1 : 0; }

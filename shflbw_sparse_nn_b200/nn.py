@@ -13,6 +13,8 @@ library's SpMM / SpConv kernel.  fp16 inference only; there is no backward pass.
 """
 from __future__ import annotations
 
+from contextlib import nullcontext
+
 import numpy as np
 import torch
 from torch import nn
@@ -26,13 +28,19 @@ def _require_cuda_half(x: torch.Tensor, what: str):
         raise TypeError(f"{what}: expected a CUDA float16 tensor, got {x.device} {x.dtype}")
 
 
+def _on_device(device: torch.device):
+    """Makes `device` current where it is not."""
+    return nullcontext() if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
 class ShflBWLinear(nn.Module):
     """y = x @ W_pruned^T + b with W in the Shfl-BW format.
 
     The SpMM computes D[out][tokens] = A[out][in] . B[in][tokens], i.e. it wants activations
-    feature-major (tokens contiguous).  `forward` takes the usual [..., in_features] tensor and
-    pays one transpose each way; `forward_feature_major` takes [in_features][tokens] and returns
-    [out_features][tokens] with no copies (tokens a multiple of 8)."""
+    feature-major (tokens contiguous).  `forward` takes the usual [..., in_features] tensor,
+    pays one transpose kernel and returns a view of the feature-major result;
+    `forward_feature_major` takes [in_features][tokens] and returns [out_features][tokens] with no
+    copies (tokens a multiple of 8).  The bias is added in the SpMM kernel."""
 
     def __init__(self, spmat: bw.BlockwiseSpMatrix, bias: torch.Tensor | None, info: dict | None = None):
         super().__init__()
@@ -53,29 +61,33 @@ class ShflBWLinear(nn.Module):
                 self.spmat.transform_and_sync_device()
             self._uploaded_on = device
 
+    def _run(self, x, tokens: int, xt: torch.Tensor, n: int) -> torch.Tensor:
+        """out[M][n] = W . xt + bias; x (token-major, or None when xt holds the operand) is transposed into xt first."""
+        dev = xt.device
+        self._upload(dev)
+        out = torch.empty((self.out_features, n), dtype=torch.float16, device=dev)
+        bias = None if self.bias is None else self.bias.to(dev)
+        fused = bias is not None and bias.dtype == torch.float16 and bias.shape == (self.out_features,) and bias.is_contiguous()
+        with _on_device(dev):
+            bw.linear_exec(self.spmat, tokens, x, bias if fused else None, xt, n, out, torch.cuda.current_stream(dev))
+        if bias is not None and not fused:
+            out += bias[:, None]
+        return out
+
     def forward_feature_major(self, xt: torch.Tensor) -> torch.Tensor:
         _require_cuda_half(xt, "ShflBWLinear")
         if xt.dim() != 2 or xt.shape[0] != self.in_features or xt.shape[1] % 8 or not xt.is_contiguous():
             raise ValueError("expected a contiguous [in_features][tokens] tensor with tokens % 8 == 0")
-        self._upload(xt.device)
-        n = xt.shape[1]
-        out = torch.empty((self.out_features, n), dtype=torch.float16, device=xt.device)
-        with torch.cuda.device(xt.device):
-            op = bw.SpmmBlockwiseOp().initialize(self.spmat, n, xt, out)
-            op(torch.cuda.current_stream(xt.device))
-        if self.bias is not None:
-            out += self.bias.to(xt.device)[:, None]
-        return out
+        return self._run(None, xt.shape[1], xt, xt.shape[1])
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         _require_cuda_half(x, "ShflBWLinear")
         lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
+        x2 = x.reshape(-1, self.in_features).contiguous()
         tokens = x2.shape[0]
         padded = -(-tokens // 8) * 8
-        xt = torch.zeros((self.in_features, padded), dtype=torch.float16, device=x.device)
-        xt[:, :tokens] = x2.t()
-        yt = self.forward_feature_major(xt)
+        xt = torch.empty((self.in_features, padded), dtype=torch.float16, device=x.device)
+        yt = self._run(x2, tokens, xt, padded)
         return yt[:, :tokens].t().reshape(*lead, self.out_features)
 
     def dense_weight(self) -> torch.Tensor:

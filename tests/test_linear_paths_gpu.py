@@ -1,0 +1,68 @@
+"""ShflBWLinear: the transpose kernel and the bias added in the SpMM epilogue, against the plain
+operator on a transposed copy and torch's fp16 add.  Both round the product to fp16 and then the
+sum, so the results are the same bits."""
+import pytest
+import torch
+
+import shflbw_sparse_nn_b200 as sb
+from gpu_util import epilogue_warps, operand_swap, tile
+from shflbw_sparse_nn_b200.nn import ShflBWLinear
+
+pytestmark = pytest.mark.gpu
+
+
+def _plain(m, x2, bias):
+    """[tokens][M] from SpmmBlockwiseOp on a padded transposed copy, bias added by torch."""
+    n = -(-x2.shape[0] // 8) * 8
+    xt = torch.zeros((m.ncol, n), dtype=torch.float16, device="cuda")
+    xt[:, :x2.shape[0]] = x2.t()
+    out = torch.empty((m.nrow, n), dtype=torch.float16, device="cuda")
+    sb.SpmmBlockwiseOp().initialize(m, n, xt, out)(torch.cuda.current_stream())
+    if bias is not None:
+        out += bias[:, None]
+    return out[:, :x2.shape[0]].t()
+
+
+@pytest.mark.parametrize("V,K,tokens,swap,ew,t", [
+    (64, 320, 1, None, None, None), (64, 320, 37, 1, None, 128), (64, 328, 65, 0, None, 128), (128, 320, 63, 1, None, 128),
+    (32, 203, 8, None, None, None),                  # K % 8 != 0: 2-byte loads
+    (64, 203, 300, 1, None, 256), (16, 77, 130, None, None, None),
+    (64, 200, 256 * 40 + 5, 0, 16, 256),             # sixteen epilogue warps
+    (64, 640, 256 * 40 + 13, 1, None, 256),          # TMA gather
+])
+@pytest.mark.parametrize("bias", [True, False])
+def test_forward_equals_operator_plus_bias_bit_for_bit(V, K, tokens, swap, ew, t, bias):
+    m = sb.BlockwiseSpMatrix().init_random(512, K, V, 1, 0.3, True, 17, values="uniform")
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    b = (torch.rand(512, generator=g, device="cuda") * 2 - 1).half() if bias else None
+    x = (torch.rand(tokens, K, generator=g, device="cuda") * 2 - 1).half()
+    lin = ShflBWLinear(m, b).cuda()
+    with operand_swap(swap), epilogue_warps(ew), tile(t):
+        y = lin(x)
+        want = _plain(m, x, b)
+        xt = torch.zeros((K, -(-tokens // 8) * 8), dtype=torch.float16, device="cuda")
+        xt[:, :tokens] = x.t()
+        yt = lin.forward_feature_major(xt)
+    torch.cuda.synchronize()
+    m.device_status()
+    assert y.shape == (tokens, 512) and torch.equal(y, want) and torch.equal(yt[:, :tokens].t(), want)
+
+
+def test_inputs_that_are_not_contiguous_or_aligned():
+    K, M = 256, 256
+    m = sb.BlockwiseSpMatrix().init_random(M, K, 64, 1, 0.3, True, 18, values="uniform")
+    lin = ShflBWLinear(m, torch.ones(M)).cuda()
+    base = (torch.rand(41 * K + 3, device="cuda") * 2 - 1).half()
+    x = base[3:].view(41, K)                              # 2-byte aligned only
+    b = lin.bias
+    assert torch.equal(lin(x), _plain(m, x, b))
+    xs = (torch.rand(20, 2 * K, device="cuda") * 2 - 1).half()[:, ::2]      # strided
+    assert torch.equal(lin(xs), _plain(m, xs, b))
+    x3 = xs.reshape(4, 5, K)
+    assert torch.equal(lin(x3), _plain(m, xs, b).reshape(4, 5, M))
+    lin.bias = torch.rand(M, device="cuda")               # a bias that is not fp16 is added by torch
+    assert torch.equal(lin(x), _plain(m, x, lin.bias))
+    with pytest.raises(sb.ShflbwError):
+        lin(x[:0])
+    torch.cuda.synchronize()
+    m.device_status()
