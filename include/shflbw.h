@@ -280,6 +280,9 @@ int shflbw_spconv_init(shflbw_matrix_t* filter, int B, int Hin, int Win, int str
 /* Replaces SpconvBlockwiseOp::operator() / SpconvBlockwiseExecFn
  * (block_sparse/spconv/blockwise_op.h:148-153, 177-187). */
 int shflbw_spconv_exec(const shflbw_spconv_state_t* st, void* stream);
+/* The same with bias[F] (logical channel order, 16-byte aligned device pointer; NULL: none) added to the
+ * fp16 result by the last pass of the call.  Not for chained states or the plain kernel. */
+int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, void* stream);
 
 /* End-to-end conv with HOST NHWC buffers.  Batches of 32 images or more move in up to four
  * chunks of whole 8-image groups through the same three streams as shflbw_spmm_host (copy in,

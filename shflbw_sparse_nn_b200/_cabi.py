@@ -106,6 +106,7 @@ _PROTOS = {
     "shflbw_spconv_init": (C.c_int, [_H, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p,
                                      C.c_float, C.c_int, C.POINTER(SpconvState)]),
     "shflbw_spconv_exec": (C.c_int, [C.POINTER(SpconvState), C.c_void_p]),
+    "shflbw_spconv_exec_bias": (C.c_int, [C.POINTER(SpconvState), C.c_void_p, C.c_void_p]),
     "shflbw_spconv_host": (C.c_int, [_H, C.c_int, C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_float]),
     "shflbw_spconv_launches_per_exec": (C.c_int, [C.POINTER(SpconvState)]),
     "shflbw_chain_buffer_elems": (C.c_size_t, [C.c_int] * 6),

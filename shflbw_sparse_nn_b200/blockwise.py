@@ -293,6 +293,10 @@ class SpconvBlockwiseOp:
     def __call__(self, stream=None):
         check(_cabi.lib().shflbw_spconv_exec(C.byref(self._state), _stream_ptr(stream)), "SpconvBlockwiseOp()")
 
+    def run_with_bias(self, bias, stream=None):
+        """As a call, with bias[F] (fp16, 16-byte aligned; None: none) added to the fp16 result."""
+        check(_cabi.lib().shflbw_spconv_exec_bias(C.byref(self._state), _ptr(bias), _stream_ptr(stream)), "SpconvBlockwiseOp()")
+
     @property
     def launches_per_exec(self) -> int:
         return _cabi.lib().shflbw_spconv_launches_per_exec(C.byref(self._state))

@@ -12,6 +12,7 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include "panel_umma.cuh"
 #include "shflbw_internal.hpp"
 
 namespace shflbw {
@@ -24,14 +25,16 @@ __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol
 // buffer with a zero halo: hp = hi + ph in [0, Hp), wp = wi + pw in [0, Wp); images n >= Bn and
 // halo pixels are written as zero, so every filter tap of every output pixel reads a valid
 // address and the gather needs no bounds logic.
+// step > 1 (1x1 filters, no halo): only the pixels that the stride visits are staged, hi = hp * step, and
+// Hp x Wp is the output's size -- a quarter of the bytes and of the blocks at stride 2.
 // One block: 64 channels x 128 (padded pixel, image) slots, images fastest.  Both global
 // accesses are 16 bytes per thread (8 channels in, 8 images out); the transpose happens in
 // shared memory, whose 8-slot groups are XOR-swizzled by the channel group so that neither
 // the 2-byte scatter nor the 16-byte read-back has bank conflicts.  C % 8 == 0, Bp % 8 == 0.
 constexpr int kRelayoutC = 64, kRelayoutSlots = 128;
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 8)
 relayout_nhwc_to_chwn(const __half* __restrict__ in, __half* __restrict__ Xs, int Bn, int Bp, int Hin, int Win,
-                      int Hp, int Wp, int ph, int pw, int C) {
+                      int Hp, int Wp, int ph, int pw, int C, int step) {
     __shared__ __align__(16) __half tile[kRelayoutC * kRelayoutSlots];
     grid_dep_launch();                       // the consumer may set itself up while this kernel runs
     grid_dep_wait();                         // the staging buffer may still be read by the previous call's kernels
@@ -49,7 +52,7 @@ relayout_nhwc_to_chwn(const __half* __restrict__ in, __half* __restrict__ Xs, in
         const int chunk = e & 7, slot = e >> 3;
         const int pl = slot / NT, nl = slot - pl * NT;
         const int pp = p0 + pl, n = nb + nl;
-        const int hp = pp / Wp, hi = hp - ph, wi = pp - hp * Wp - pw;
+        const int hp = pp / Wp, hi = hp * step - ph, wi = (pp - hp * Wp) * step - pw;
         v[i] = make_uint4(0u, 0u, 0u, 0u);
         if (pl < PT && pp < PP && n < Bn && c0 + chunk * 8 < C && (unsigned)hi < (unsigned)Hin &&
             (unsigned)wi < (unsigned)Win)
@@ -120,10 +123,21 @@ transpose_tokens(const __half* __restrict__ x, __half* __restrict__ xt, int toke
     }
 }
 
-// out[q][perm[f]] = staged[q][f] for every output position q.  G = clamp(F/8, 8, 64) threads
-// share one position (each moves 8 filters at a time with 16-byte global accesses), so a block
+// Adds the bias of 8 consecutive channels (16-byte aligned) to 8 fp16 results.
+__device__ __forceinline__ uint4 add_bias8(uint4 v, const uint4& b) {
+    __half2* h = (__half2*)&v;
+    const __half2* bh = (const __half2*)&b;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) h[e] = __hadd2(h[e], bh[e]);
+    return v;
+}
+
+// out[q][perm[f]] = staged[q][f] (+ bias[perm[f]]) for every output position q.  G = clamp(F/8, 8, 64)
+// threads share one position (each moves 8 filters at a time with 16-byte global accesses), so a block
 // of 256 threads handles 256/G positions at once: 4 for F >= 512 (two warps each -- the kernel
-// is latency-bound and more warps per position shorten it) up to 32 for F = 64.  The
+// is latency-bound and more warps per position shorten it) up to 32 for F = 64.  (Four positions' pieces
+// loaded before the first is used were slower, 2.8 -> 3.8 us for 980 positions of 512 filters: fewer
+// blocks.)  The
 // permutation sits in shared memory as 16-bit ids (read once per block); values are scattered
 // into the position's F-vector in shared memory with 2-byte stores and leave as 16-byte stores.
 // Dynamic shared memory: F*2 bytes (perm) + (256/G)*F*2 bytes.  F % 8 == 0, F <= 65536.
@@ -135,7 +149,7 @@ __host__ __device__ inline int unperm_threads_per_pos(int F) {
 }
 __global__ void __launch_bounds__(kUnpermThreads)
 unpermute_filters(const __half* __restrict__ staged, __half* __restrict__ out, const int* __restrict__ perm,
-                  int num_pos, int F) {
+                  const __half* __restrict__ bias, int num_pos, int F) {
     extern __shared__ __align__(16) uint8_t unperm_smem[];
     unsigned short* sperm = (unsigned short*)unperm_smem;        // [F]
     __half* vec = (__half*)(unperm_smem + (size_t)F * 2);        // [positions per block][F]
@@ -163,76 +177,97 @@ unpermute_filters(const __half* __restrict__ staged, __half* __restrict__ out, c
         if (q < num_pos) {
             __half* dst = out + (size_t)q * F;
 #pragma unroll 4
-            for (int f8 = t * 8; f8 < F; f8 += G * 8) *(uint4*)(dst + f8) = *(const uint4*)(mine + f8);
+            for (int f8 = t * 8; f8 < F; f8 += G * 8) {
+                uint4 v = *(const uint4*)(mine + f8);
+                if (bias) v = add_bias8(v, __ldg((const uint4*)(bias + f8)));
+                *(uint4*)(dst + f8) = v;
+            }
         }
     }
 }
 
-// Chain buffer -> NHWC: out[n][h][w][perm[f]] = buf[f][h + ph][w + pw][n] (perm == nullptr:
-// channels stay in stored order).  One block: one pixel x 8 images x all F filters; reads are
-// 16 bytes (8 images of one (filter, pixel)), the F-vectors of the 8 images are assembled in
-// shared memory with 2-byte stores and leave as 16-byte stores.  Dynamic shared memory:
-// 8 * F * 2 bytes.  F % 8 == 0, Bp % 8 == 0.
+// Channel-major planes -> NHWC: out[n][h][w][c] = planes[f][h + ph][w + pw][n] (+ bias[c]), where plane f
+// holds logical channel c = perm[f] (perm == nullptr: c = f).  Used for the output of an NHWC call computed
+// as planes (perm == nullptr, no halo) and to export a chain buffer.  Bound by HBM / L2 bandwidth: both
+// sides should move whole lines.  One block owns 64 channels and moves them 64 tokens (tok = pixel * Bp + n)
+// at a time through 8 KB of shared memory: 16-byte loads of 8 tokens of one plane, 2-byte scatters into
+// [token][channel] (8-channel groups XOR-swizzled by the token group, so neither side has bank conflicts),
+// 16-byte stores of 8 channels of one token -- 128-byte runs in global memory on both sides; the loads of
+// the next 64 tokens are issued before the current ones are stored.  The planes of the block's channels
+// are found once, by a scan of perm.  (One pixel x 8 images x all channels per block, 16-byte reads of
+// scattered lines: 52 us for 256 x 7 x 7 x 2048, 103 MB; this kernel: 21 us.)  F % 8 == 0, Bp % 8 == 0;
+// images n >= Bn are padding.  A launch covers pixels pix0 .. pix0 + npix of out_pix.
+// PLAIN (plane c of channel c, no halo): a token's place in its plane is its index, and a block moves one
+// 64 x 64 tile; the general form's start-up and registers cost 1.1 us of 4.8 at 3136 tokens x 2048 filters.
+template <bool PLAIN>
 __global__ void __launch_bounds__(256)
-chain_export_nhwc(const __half* __restrict__ buf, __half* __restrict__ out, const int* __restrict__ perm,
-                  int Bn, int Bp, int H, int W, int Hp, int Wp, int ph, int pw, int F) {
-    extern __shared__ __align__(16) uint8_t export_smem[];
-    __half* vec = (__half*)export_smem;                  // [8 images][F]
-    grid_dep_launch();
-    grid_dep_wait();                                     // the planes are complete only when their producer is
-    const int groups = Bp / 8;
-    const int pix = blockIdx.x / groups, n0 = (blockIdx.x % groups) * 8;
-    const int h = pix / W, w = pix - h * W;
-    const size_t plane = (size_t)Hp * Wp * Bp;
-    const __half* src = buf + ((size_t)(h + ph) * Wp + (w + pw)) * Bp + n0;
-    for (int f = threadIdx.x; f < F; f += 256) {
-        const uint4 v = *(const uint4*)(src + (size_t)f * plane);
-        const __half* hv = (const __half*)&v;
-        const int c = perm ? __ldg(perm + f) : f;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) vec[j * F + c] = hv[j];
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < F; e += 256) {         // e = (image j, 8-channel chunk)
-        const int j = e / (F / 8), c8 = (e - j * (F / 8)) * 8;
-        if (n0 + j < Bn)
-            *(uint4*)(out + (((size_t)(n0 + j) * H + h) * W + w) * F + c8) = *(const uint4*)(vec + j * F + c8);
-    }
-}
-
-// planes[f][tok] -> out[n][pix][f]: the output of an NHWC call computed as planes (one row of
-// tok = pix * Bp + n tokens per LOGICAL filter f) transposed to NHWC.  One block moves a tile of
-// 64 filters x 64 tokens through 8 KB of shared memory: 16-byte loads of 8 tokens of one
-// filter, 2-byte scatters into [token][filter] (8-filter groups XOR-swizzled by the token group,
-// so neither side has bank conflicts), 16-byte stores of 8 filters of one token -- 128-byte runs
-// in global memory on both sides.  F % 64 == 0, Bp % 8 == 0; images n >= Bn are padding.
-__global__ void __launch_bounds__(256)
-planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, int Bn, int Bp, int npix, int F) {
+planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, const int* __restrict__ perm,
+               const __half* __restrict__ bias, int Bn, int Bp, int pix0, int npix, int out_pix, int W, int Wp, int ph, int pw,
+               size_t plane, int F, FastDiv div_bp, FastDiv div_w) {
     __shared__ __align__(16) __half tile[64 * 64];
+    __shared__ int plane_of[64];                         // of the block's channels
     grid_dep_launch();
+    const int f0 = blockIdx.y * 64, nf = min(64, F - f0);
+    if constexpr (!PLAIN) {
+    if (perm) {
+        for (int f = threadIdx.x; f < F; f += 256) {     // a permutation: every channel is found exactly once
+            const int c = __ldg(perm + f) - f0;
+            if ((unsigned)c < 64u) plane_of[c] = f;
+        }
+    } else if (threadIdx.x < 64) plane_of[threadIdx.x] = f0 + threadIdx.x;
+    __syncthreads();
+    }
     grid_dep_wait();                                     // the planes are complete only when the panel kernel is
     const int ntok = npix * Bp;
-    const int tok0 = blockIdx.x * 64, f0 = blockIdx.y * 64;
     const int c = threadIdx.x & 7, r0 = threadIdx.x >> 3;   // 16-byte chunk, row of the pass
+    const __half* src[2];
 #pragma unroll
     for (int pass = 0; pass < 2; ++pass) {
-        const int r = r0 + 32 * pass;                    // filter of the tile
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (tok0 + c * 8 < ntok) v = *(const uint4*)(planes + (size_t)(f0 + r) * ntok + tok0 + c * 8);
-        const __half* h = (const __half*)&v;
-        const int col = (((r >> 3) ^ c) << 3) | (r & 7);    // token group c: filter group XOR c
-#pragma unroll
-        for (int j = 0; j < 8; ++j) tile[(c * 8 + j) * 64 + col] = h[j];
+        const int r = r0 + 32 * pass;
+        src[pass] = r < nf ? planes + (size_t)(PLAIN ? f0 + r : plane_of[r]) * plane : nullptr;
     }
-    __syncthreads();
+    uint4 v[2];
+    auto load = [&](int tok0) {
+        const int tok = tok0 + c * 8;
+        size_t off = 0;
+        if (PLAIN) off = (size_t)pix0 * Bp + tok;
+        else if (tok < ntok) {
+            const int lpix = fast_div(tok, div_bp), n = tok - lpix * Bp, pix = pix0 + lpix;
+            const int h = fast_div(pix, div_w), w = pix - h * W;
+            off = ((size_t)(h + ph) * Wp + w + pw) * Bp + n;
+        }
 #pragma unroll
-    for (int pass = 0; pass < 2; ++pass) {
-        const int t = r0 + 32 * pass;                    // token of the tile
-        const int tok = tok0 + t;
-        const int pix = tok / Bp, n = tok - pix * Bp;
-        if (tok < ntok && n < Bn)
-            *(uint4*)(out + ((size_t)n * npix + pix) * F + f0 + c * 8) =
-                *(const uint4*)(tile + t * 64 + ((c ^ ((t >> 3) & 7)) << 3));
+        for (int pass = 0; pass < 2; ++pass) {
+            v[pass] = make_uint4(0u, 0u, 0u, 0u);
+            if (tok < ntok && src[pass]) v[pass] = *(const uint4*)(src[pass] + off);
+        }
+    };
+    int tok0 = blockIdx.x * 64;
+    load(tok0);
+    for (; tok0 < ntok; tok0 += gridDim.x * 64) {
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass) {
+            const int r = r0 + 32 * pass;                    // channel of the tile
+            const __half* h = (const __half*)&v[pass];
+            const int col = (((r >> 3) ^ c) << 3) | (r & 7);    // token group c: channel group XOR c
+#pragma unroll
+            for (int j = 0; j < 8; ++j) tile[(c * 8 + j) * 64 + col] = h[j];
+        }
+        __syncthreads();
+        if constexpr (!PLAIN) load(tok0 + gridDim.x * 64);
+#pragma unroll
+        for (int pass = 0; pass < 2; ++pass) {
+            const int t = r0 + 32 * pass;                    // token of the tile
+            const int tok = tok0 + t;
+            const int pix = fast_div(tok, div_bp), n = tok - pix * Bp;
+            if (tok < ntok && n < Bn && c * 8 < nf) {
+                uint4 o = *(const uint4*)(tile + t * 64 + ((c ^ ((t >> 3) & 7)) << 3));
+                if (bias) o = add_bias8(o, __ldg((const uint4*)(bias + f0 + c * 8)));
+                *(uint4*)(out + ((size_t)n * out_pix + pix0 + pix) * F + f0 + c * 8) = o;
+            }
+        }
+        if constexpr (PLAIN) return;
+        __syncthreads();
     }
 }
 

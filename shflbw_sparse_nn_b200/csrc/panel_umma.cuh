@@ -111,7 +111,7 @@ struct alignas(64) PanelParams {
     int ablate;              // tuning builds only (-DSHFLBW_ABLATE): 1 no MMA, 2 no gather, 4 no value copies, 8 no stores
     // SpMM
     const __half* B;         // [K][N]
-    const __half* C;         // [M][N] or nullptr
+    const __half* C;         // [M][N] or nullptr; SpConv writing NHWC: bias[F] or nullptr
     __half* D;               // [M][N]
     int c_row;               // C is one value per output row ([M], a bias) instead of a matrix
     int N;                   // dense columns (SpMM) / Ho*Wo*Bp (SpConv)
@@ -1355,7 +1355,14 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int row = i * 8 + (lane >> 2), c = lane & 3;
-                        const uint4 v = *(const uint4*)(my_tile + row * 64 + ((c ^ ((row >> 1) & 3)) << 4));
+                        uint4 v = *(const uint4*)(my_tile + row * 64 + ((c ^ ((row >> 1) & 3)) << 4));
+                        if (p.C != nullptr && c < CW / 8) {              // bias (stored order is logical order here)
+                            const uint4 bv = __ldg((const uint4*)(p.C + blk * V + mbase + cc + c * 8));
+                            __half2* h = (__half2*)&v;
+                            const __half2* bh = (const __half2*)&bv;
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) h[e] = __hadd2(h[e], bh[e]);
+                        }
                         if (row_off[i] != 0xffffffffu && c < CW / 8) *(uint4*)(p.out + (size_t)row_off[i] + cc + c * 8) = v;
                     }
                 }

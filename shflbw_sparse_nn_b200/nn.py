@@ -132,11 +132,14 @@ class ShflBWConv2d(nn.Module):
         x_nhwc = x.permute(0, 2, 3, 1).contiguous()          # a view when x is channels-last
         ho, wo = -(-h // self.stride), -(-w // self.stride)
         out = torch.empty((n, ho, wo, self.out_channels), dtype=torch.float16, device=x.device)
-        with torch.cuda.device(x.device):
+        bias = None if self.bias is None else self.bias.to(x.device)
+        fused = bias is not None and bias.dtype == torch.float16 and bias.shape == (self.out_channels,) and \
+            bias.is_contiguous() and bias.data_ptr() % 16 == 0
+        with _on_device(x.device):
             op = bw.SpconvBlockwiseOp().initialize(self.spfilter, n, h, w, self.stride, x_nhwc, out)
-            op(torch.cuda.current_stream(x.device))
-        if self.bias is not None:
-            out += self.bias.to(x.device)
+            op.run_with_bias(bias if fused else None, torch.cuda.current_stream(x.device))
+        if bias is not None and not fused:
+            out += bias
         return out.permute(0, 3, 1, 2)                       # NCHW view of the NHWC result (channels-last)
 
     def dense_weight(self) -> torch.Tensor:
