@@ -32,17 +32,19 @@ _VALUE_MODES = {"int9": VALUES_INT9_LIBC, "uniform": VALUES_UNIFORM}
 def _ptr(x) -> Optional[int]:
     if x is None:
         return None
-    if hasattr(x, "data_ptr"):
-        return int(x.data_ptr())
-    return int(x)
+    try:
+        return x.data_ptr()
+    except AttributeError:
+        return int(x)
 
 
 def _stream_ptr(stream) -> Optional[int]:
     if stream is None:
         return None
-    if hasattr(stream, "cuda_stream"):
-        return int(stream.cuda_stream)
-    return int(stream)
+    try:
+        return stream.cuda_stream
+    except AttributeError:
+        return int(stream)
 
 
 def uniform_half(stream_seed: int, n: int, offset: int = 0) -> np.ndarray:
@@ -242,7 +244,9 @@ class SpmmBlockwiseOp:
         return self
 
     def __call__(self, stream=None):
-        check(_cabi.lib().shflbw_spmm_exec(C.byref(self._state), _stream_ptr(stream)), "SpmmBlockwiseOp()")
+        status = _cabi.lib().shflbw_spmm_exec(self._state, _stream_ptr(stream))
+        if status:
+            check(status, "SpmmBlockwiseOp()")
 
     @property
     def launches_per_exec(self) -> int:
@@ -291,7 +295,9 @@ class SpconvBlockwiseOp:
         return self
 
     def __call__(self, stream=None):
-        check(_cabi.lib().shflbw_spconv_exec(C.byref(self._state), _stream_ptr(stream)), "SpconvBlockwiseOp()")
+        status = _cabi.lib().shflbw_spconv_exec(self._state, _stream_ptr(stream))
+        if status:
+            check(status, "SpconvBlockwiseOp()")
 
     def run_with_bias(self, bias, stream=None):
         """As a call, with bias[F] (fp16, 16-byte aligned; None: none) added to the fp16 result."""
@@ -356,7 +362,9 @@ class SpconvChainOp:
         return self
 
     def __call__(self, stream=None):
-        check(_cabi.lib().shflbw_spconv_exec(C.byref(self._state), _stream_ptr(stream)), "SpconvChainOp()")
+        status = _cabi.lib().shflbw_spconv_exec(self._state, _stream_ptr(stream))
+        if status:
+            check(status, "SpconvChainOp()")
 
     @property
     def launches_per_exec(self) -> int:

@@ -23,6 +23,9 @@ from . import blockwise as bw
 from .pruner import prune_conv_filter, prune_matrix
 
 
+_NOTHING = nullcontext()
+
+
 def _require_cuda_half(x: torch.Tensor, what: str):
     if not x.is_cuda or x.dtype != torch.float16:
         raise TypeError(f"{what}: expected a CUDA float16 tensor, got {x.device} {x.dtype}")
@@ -30,7 +33,21 @@ def _require_cuda_half(x: torch.Tensor, what: str):
 
 def _on_device(device: torch.device):
     """Makes `device` current where it is not."""
-    return nullcontext() if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+    return _NOTHING if device.index == torch.cuda.current_device() else torch.cuda.device(device)
+
+
+def _stream_of(device: torch.device) -> int:
+    """torch's current stream on `device` as a cudaStream_t (without building a Stream object, 3 us)."""
+    return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+def _fused_bias(bias, device: torch.device, n: int, align: int):
+    """(bias on `device`, whether the kernels can add it: fp16, one per output, contiguous, aligned)."""
+    if bias is None:
+        return None, False
+    if bias.device != device:
+        bias = bias.to(device)
+    return bias, bias.dtype == torch.float16 and bias.shape == (n,) and bias.is_contiguous() and bias.data_ptr() % align == 0
 
 
 class ShflBWLinear(nn.Module):
@@ -66,10 +83,9 @@ class ShflBWLinear(nn.Module):
         dev = xt.device
         self._upload(dev)
         out = torch.empty((self.out_features, n), dtype=torch.float16, device=dev)
-        bias = None if self.bias is None else self.bias.to(dev)
-        fused = bias is not None and bias.dtype == torch.float16 and bias.shape == (self.out_features,) and bias.is_contiguous()
+        bias, fused = _fused_bias(self.bias, dev, self.out_features, 2)
         with _on_device(dev):
-            bw.linear_exec(self.spmat, tokens, x, bias if fused else None, xt, n, out, torch.cuda.current_stream(dev))
+            bw.linear_exec(self.spmat, tokens, x, bias if fused else None, xt, n, out, _stream_of(dev))
         if bias is not None and not fused:
             out += bias[:, None]
         return out
@@ -88,7 +104,8 @@ class ShflBWLinear(nn.Module):
         padded = -(-tokens // 8) * 8
         xt = torch.empty((self.in_features, padded), dtype=torch.float16, device=x.device)
         yt = self._run(x2, tokens, xt, padded)
-        return yt[:, :tokens].t().reshape(*lead, self.out_features)
+        y = yt.as_strided((tokens, self.out_features), (1, padded))
+        return y if lead == (tokens,) else y.reshape(*lead, self.out_features)
 
     def dense_weight(self) -> torch.Tensor:
         """The pruned weights as a dense [out][in] fp16 tensor (rows in original order), for checks."""
@@ -132,12 +149,10 @@ class ShflBWConv2d(nn.Module):
         x_nhwc = x.permute(0, 2, 3, 1).contiguous()          # a view when x is channels-last
         ho, wo = -(-h // self.stride), -(-w // self.stride)
         out = torch.empty((n, ho, wo, self.out_channels), dtype=torch.float16, device=x.device)
-        bias = None if self.bias is None else self.bias.to(x.device)
-        fused = bias is not None and bias.dtype == torch.float16 and bias.shape == (self.out_channels,) and \
-            bias.is_contiguous() and bias.data_ptr() % 16 == 0
+        bias, fused = _fused_bias(self.bias, x.device, self.out_channels, 16)
         with _on_device(x.device):
             op = bw.SpconvBlockwiseOp().initialize(self.spfilter, n, h, w, self.stride, x_nhwc, out)
-            op.run_with_bias(bias if fused else None, torch.cuda.current_stream(x.device))
+            op.run_with_bias(bias if fused else None, _stream_of(x.device))
         if bias is not None and not fused:
             out += bias
         return out.permute(0, 3, 1, 2)                       # NCHW view of the NHWC result (channels-last)
