@@ -25,14 +25,15 @@ __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol
 // buffer with a zero halo: hp = hi + ph in [0, Hp), wp = wi + pw in [0, Wp); images n >= Bn and
 // halo pixels are written as zero, so every filter tap of every output pixel reads a valid
 // address and the gather needs no bounds logic.
-// step > 1 (1x1 filters, no halo): only the pixels that the stride visits are staged, hi = hp * step, and
+// STRIDED (1x1 filters, no halo): only the pixels that the stride visits are staged, hi = hp * step, and
 // Hp x Wp is the output's size -- a quarter of the bytes and of the blocks at stride 2.
 // One block: 64 channels x 128 (padded pixel, image) slots, images fastest.  Both global
 // accesses are 16 bytes per thread (8 channels in, 8 images out); the transpose happens in
 // shared memory, whose 8-slot groups are XOR-swizzled by the channel group so that neither
 // the 2-byte scatter nor the 16-byte read-back has bank conflicts.  C % 8 == 0, Bp % 8 == 0.
 constexpr int kRelayoutC = 64, kRelayoutSlots = 128;
-__global__ void __launch_bounds__(256, 8)
+template <bool STRIDED>
+__global__ void __launch_bounds__(256)
 relayout_nhwc_to_chwn(const __half* __restrict__ in, __half* __restrict__ Xs, int Bn, int Bp, int Hin, int Win,
                       int Hp, int Wp, int ph, int pw, int C, int step) {
     __shared__ __align__(16) __half tile[kRelayoutC * kRelayoutSlots];
@@ -52,7 +53,7 @@ relayout_nhwc_to_chwn(const __half* __restrict__ in, __half* __restrict__ Xs, in
         const int chunk = e & 7, slot = e >> 3;
         const int pl = slot / NT, nl = slot - pl * NT;
         const int pp = p0 + pl, n = nb + nl;
-        const int hp = pp / Wp, hi = hp * step - ph, wi = (pp - hp * Wp) * step - pw;
+        const int hp = pp / Wp, hi = STRIDED ? hp * step : hp - ph, wi = STRIDED ? (pp - hp * Wp) * step : pp - hp * Wp - pw;
         v[i] = make_uint4(0u, 0u, 0u, 0u);
         if (pl < PT && pp < PP && n < Bn && c0 + chunk * 8 < C && (unsigned)hi < (unsigned)Hin &&
             (unsigned)wi < (unsigned)Win)
@@ -147,6 +148,7 @@ __host__ __device__ inline int unperm_threads_per_pos(int F) {
     while (g < 64 && g * 8 < F) g *= 2;
     return g;
 }
+template <bool BIAS>
 __global__ void __launch_bounds__(kUnpermThreads)
 unpermute_filters(const __half* __restrict__ staged, __half* __restrict__ out, const int* __restrict__ perm,
                   const __half* __restrict__ bias, int num_pos, int F) {
@@ -179,7 +181,7 @@ unpermute_filters(const __half* __restrict__ staged, __half* __restrict__ out, c
 #pragma unroll 4
             for (int f8 = t * 8; f8 < F; f8 += G * 8) {
                 uint4 v = *(const uint4*)(mine + f8);
-                if (bias) v = add_bias8(v, __ldg((const uint4*)(bias + f8)));
+                if constexpr (BIAS) v = add_bias8(v, __ldg((const uint4*)(bias + f8)));
                 *(uint4*)(dst + f8) = v;
             }
         }
@@ -199,7 +201,7 @@ unpermute_filters(const __half* __restrict__ staged, __half* __restrict__ out, c
 // images n >= Bn are padding.  A launch covers pixels pix0 .. pix0 + npix of out_pix.
 // PLAIN (plane c of channel c, no halo): a token's place in its plane is its index, and a block moves one
 // 64 x 64 tile; the general form's start-up and registers cost 1.1 us of 4.8 at 3136 tokens x 2048 filters.
-template <bool PLAIN>
+template <bool PLAIN, bool BIAS>
 __global__ void __launch_bounds__(256)
 planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, const int* __restrict__ perm,
                const __half* __restrict__ bias, int Bn, int Bp, int pix0, int npix, int out_pix, int W, int Wp, int ph, int pw,
@@ -262,7 +264,7 @@ planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, cons
             const int pix = fast_div(tok, div_bp), n = tok - pix * Bp;
             if (tok < ntok && n < Bn && c * 8 < nf) {
                 uint4 o = *(const uint4*)(tile + t * 64 + ((c ^ ((t >> 3) & 7)) << 3));
-                if (bias) o = add_bias8(o, __ldg((const uint4*)(bias + f0 + c * 8)));
+                if constexpr (BIAS) o = add_bias8(o, __ldg((const uint4*)(bias + f0 + c * 8)));
                 *(uint4*)(out + ((size_t)n * out_pix + pix0 + pix) * F + f0 + c * 8) = o;
             }
         }

@@ -111,9 +111,8 @@ struct alignas(64) PanelParams {
     int ablate;              // tuning builds only (-DSHFLBW_ABLATE): 1 no MMA, 2 no gather, 4 no value copies, 8 no stores
     // SpMM
     const __half* B;         // [K][N]
-    const __half* C;         // [M][N] or nullptr; SpConv writing NHWC: bias[F] or nullptr
+    const __half* C;         // [M][N] or nullptr; kernels built with BIAS: one value per output row / filter
     __half* D;               // [M][N]
-    int c_row;               // C is one value per output row ([M], a bias) instead of a matrix
     int N;                   // dense columns (SpMM) / Ho*Wo*Bp (SpConv)
     // SpConv (input staged channel-major, batch innermost, with a zero halo:
     // Xs[c][Hp][Wp][Bp], Hp = Hin + R - 1, Wp = Win + S - 1, image origin at (R/2, S/2))
@@ -258,8 +257,11 @@ __device__ __forceinline__ uint4 broadcast8(const __half* p) {
 
 constexpr int kPanelMaxItemsPerCta = 512;  // capacity of the per-CTA item table
 
+// BIAS: C holds one value per output row (SpMM, added like C with beta = 1) or per filter (SpConv writing
+// NHWC in logical order).  Kernels of their own: as a branch of the others it made small products 1-2 %
+// slower (256-item launches of 5-9 us, where every instruction is fetched for the first time).
 template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int LAG_ = 1, int GATHER_ = kGatherCpAsync,
-          int EW_ = 8>
+          int EW_ = 8, bool BIAS = false>
 __global__ void __launch_bounds__(PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, LAG_, GATHER_, EW_>::THREADS, 1)
 panel_umma_kernel(const __grid_constant__ PanelParams p) {
     using Cfg = PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, LAG_, GATHER_, EW_>;
@@ -1066,7 +1068,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                                 if (tok0 + c * 8 < p.N) {                // N % 8 == 0: 8 tokens are valid as a whole
                                     if (use_c) {                         // (the rare beta != 0 case pays the load's latency here)
                                         uint4 cv;
-                                        if (p.c_row) cv = broadcast8(p.C + (p.perm ? __ldg(p.perm + blk * V + m) : blk * V + m));
+                                        if constexpr (BIAS) cv = broadcast8(p.C + (p.perm ? __ldg(p.perm + blk * V + m) : blk * V + m));
                                         else cv = *(const uint4*)(p.C + roff + tok0 + c * 8);
                                         __half* h = (__half*)&v[c];
                                         const __half* ch = (const __half*)&cv;
@@ -1172,14 +1174,14 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             // chunk's two chunks ahead.
             constexpr int NCH = COLS / CW;
             constexpr bool RES_AHEAD = Cfg::RES_BYTES > 0;
-            const bool ahead = RES_AHEAD && ((use_c && !p.c_row) || (MODE == kPanelConvChain && p.res != nullptr));
+            const bool ahead = RES_AHEAD && ((use_c && !BIAS) || (MODE == kPanelConvChain && p.res != nullptr));
             const bool add_res = MODE == kPanelConvChain && p.res != nullptr;
             const bool need_add = ok_g && (use_c || add_res);
             auto addend_at = [&](int blk_, uint32_t goff_, int cc, int i) -> const __half* {
                 const int m = mbase + cc + slot_row(i);
                 if (use_c) {
                     const int row = (p.perm && !(ablate & 1024)) ? __ldg(p.perm + blk_ * V + m) : blk_ * V + m;
-                    if (p.c_row) return p.C + row;
+                    if constexpr (BIAS) return p.C + row;
                     return p.C + (size_t)((uint32_t)row * (uint32_t)p.N) + (size_t)goff_;
                 }
                 const uint32_t rr = (uint32_t)(p.res_map ? __ldg(p.res_map + blk_ * V + m) : blk_ * V + m) * (uint32_t)p.out_plane;
@@ -1190,7 +1192,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 #pragma unroll
                 for (int i = 0; i < NSLOT; ++i) {
                     const __half* src = addend_at(blk_, goff_, cc, i);
-                    if (MODE == kPanelSpmm && p.c_row) dst[i] = broadcast8(src);
+                    if constexpr (MODE == kPanelSpmm && BIAS) dst[i] = broadcast8(src);
                     else dst[i] = *(const uint4*)src;
                 }
             };
@@ -1271,7 +1273,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                         sm100::cp_async_wait<NCH - 1>();     // this chunk's copies (each lane reads only its own)
 #pragma unroll
                         for (int i = 0; i < NSLOT; ++i) addend[0][i] = *(const uint4*)(my_res + (ch * 4 + i) * 512);
-                    } else if (need_add) {
+                    } else if (BIAS && need_add) {
                         fetch_addend(blk, goff, cc, addend[0]);
                     }
                 }
@@ -1356,7 +1358,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     for (int i = 0; i < 4; ++i) {
                         const int row = i * 8 + (lane >> 2), c = lane & 3;
                         uint4 v = *(const uint4*)(my_tile + row * 64 + ((c ^ ((row >> 1) & 3)) << 4));
-                        if (p.C != nullptr && c < CW / 8) {              // bias (stored order is logical order here)
+                        if (BIAS && c < CW / 8) {                        // (stored order is logical order here)
                             const uint4 bv = __ldg((const uint4*)(p.C + blk * V + mbase + cc + c * 8));
                             __half2* h = (__half2*)&v;
                             const __half2* bh = (const __half2*)&bv;

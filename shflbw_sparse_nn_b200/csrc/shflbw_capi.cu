@@ -109,10 +109,10 @@ using PanelKernel = void (*)(const shflbw::PanelParams);
 struct PanelChoice { PanelKernel fn; size_t smem; int tokens; int stages; int pw; int threads; int variant; int gather; };
 
 template <int V, int TM, int KS, int STAGES, int PW, int MODE, int GROUPS = 2, int LAG = 1, int GATHER = shflbw::kGatherCpAsync,
-          int EW = 8>
+          int EW = 8, bool BIAS = false>
 PanelChoice choice() {
     using Cfg = shflbw::PanelCfg<V, TM, KS, STAGES, PW, MODE, GROUPS, LAG, GATHER, EW>;
-    return {shflbw::panel_umma_kernel<V, TM, KS, STAGES, PW, MODE, GROUPS, LAG, GATHER, EW>, (size_t)Cfg::SMEM_BYTES, Cfg::T,
+    return {shflbw::panel_umma_kernel<V, TM, KS, STAGES, PW, MODE, GROUPS, LAG, GATHER, EW, BIAS>, (size_t)Cfg::SMEM_BYTES, Cfg::T,
             STAGES, PW, Cfg::THREADS, 0, GATHER};
 }
 
@@ -193,7 +193,7 @@ bool tuned_shape(PanelChoice* out) {
 
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
-template <int MODE>
+template <int MODE, bool BIAS = false>
 bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsync, bool wide_epilogue = false) {
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         // Shallow items (at most 64 non-zero columns): sixteen epilogue warps and three producer
@@ -202,7 +202,7 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
         // six items' inputs are in flight from HBM (five: 37.5 -> 40.5 us on 14x14x256 -> 1024 at batch
         // 256, the rest equal).  Built for 64-row blocks.
         if (wide_epilogue && tile == 256 && V == 64) {
-            *out = choice<64, 2, 32, 6, 3, MODE, 3, 1, shflbw::kGatherCpAsync, 16>();
+            *out = choice<64, 2, 32, 6, 3, MODE, 3, 1, shflbw::kGatherCpAsync, 16, BIAS>();
             return true;
         }
     }
@@ -215,30 +215,30 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
             // 16 light producer warps in four groups (measured 3-6 % faster than the cp.async gather
             // on the 4096^3 case; the copy engine also applies the swizzle and zero-fills the N residue)
             if (gather == shflbw::kGatherTma && V == 64 && tile == 256) {
-                *out = choice<64, 2, 64, 5, 16, MODE, 4, 1, shflbw::kGatherTma>();
+                *out = choice<64, 2, 64, 5, 16, MODE, 4, 1, shflbw::kGatherTma, 8, BIAS>();
                 return true;
             }
         }
         switch (V * 1000 + tile) {
-            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE>(); return true;
-            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE>(); return true;
-            case 128128: *out = choice<128, 1, 64, 6, 8, MODE>(); return true;
-            case 128256: *out = choice<128, 2, 64, 4, 8, MODE>(); return true;
+            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
+            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
+            case 128128: *out = choice<128, 1, 64, 6, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
+            case 128256: *out = choice<128, 2, 64, 4, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
             default: return false;
         }
     } else {
         if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConv) {
             // 16-row blocks: UMMA N = 16, one or two 128-token accumulators per item (18 / 34 KB stages)
-            if (V == 16 && tile == 128) { *out = choice<16, 1, 64, 8, 8, MODE>(); return true; }
-            if (V == 16 && tile == 256) { *out = choice<16, 2, 64, 5, 8, MODE>(); return true; }
+            if (V == 16 && tile == 128) { *out = choice<16, 1, 64, 8, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true; }
+            if (V == 16 && tile == 256) { *out = choice<16, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true; }
         }
         switch (V * 1000 + tile) {
-            case 32128:  *out = choice<32, 1, 64, 8, 8, MODE>(); return true;    // 20 KB stages
-            case 32256:  *out = choice<32, 2, 64, 5, 8, MODE>(); return true;    // 36 KB
-            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE>(); return true;    // 24 KB
-            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE>(); return true;    // 40 KB
-            case 128128: *out = choice<128, 1, 64, 6, 8, MODE>(); return true;   // 32 KB
-            case 128256: *out = choice<128, 2, 64, 4, 8, MODE>(); return true;   // 48 KB
+            case 32128:  *out = choice<32, 1, 64, 8, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 20 KB stages
+            case 32256:  *out = choice<32, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 36 KB
+            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 24 KB
+            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 40 KB
+            case 128128: *out = choice<128, 1, 64, 6, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;   // 32 KB
+            case 128256: *out = choice<128, 2, 64, 4, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;   // 48 KB
             default: return false;
         }
     }
@@ -516,15 +516,19 @@ static int spmm_exec_impl(const shflbw_spmm_state_t* st, const void* bias, void*
         // The state is a POD and may have been copied: re-derive the function pointer from the
         // recorded configuration (the shared-memory attribute was set at init).
         PanelChoice ch;
-        const bool found = st->variant == 1 ? lookup<shflbw::kPanelSpmmRows>(st->V, st->tokens_per_cta, &ch, st->gather)
-                                            : lookup<shflbw::kPanelSpmm>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync, st->variant == 2);
+        const bool wide = st->variant == 2;
+        const bool found =
+            bias ? st->variant == 1 ? lookup<shflbw::kPanelSpmmRows, true>(st->V, st->tokens_per_cta, &ch, st->gather)
+                                    : lookup<shflbw::kPanelSpmm, true>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync, wide)
+                 : st->variant == 1 ? lookup<shflbw::kPanelSpmmRows>(st->V, st->tokens_per_cta, &ch, st->gather)
+                                    : lookup<shflbw::kPanelSpmm>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync, wide);
         if (!found) return SHFLBW_ERR_INVALID_ARG;
         shflbw::PanelParams p{};
         p.blk_ptr = st->blk_ptr; p.blk_idx = st->blk_idx; p.blk_val = (const __half*)st->blk_val;
         p.perm = st->perm; p.status_word = st->status_word; p.alpha = st->alpha; p.beta = st->beta;
         p.wait_limit = g_wait_limit; p.inject_from = g_inject_from; p.idx_limit = (unsigned)(st->K - 1);
         p.B = (const __half*)st->B; p.C = (const __half*)st->C; p.D = (__half*)st->D; p.N = st->N;
-        if (bias) { p.C = (const __half*)bias; p.beta = 1.f; p.c_row = 1; }
+        if (bias) { p.C = (const __half*)bias; p.beta = 1.f; }
         p.wide_stores = (st->N % 16 == 0) && (((uintptr_t)st->D & 31) == 0);
         if (ch.gather != st->gather) return SHFLBW_ERR_INVALID_ARG;
         if (st->gather == shflbw::kGatherTma) std::memcpy(p.tmap_b, st->tmap_b, sizeof p.tmap_b);
@@ -539,6 +543,7 @@ static int spmm_exec_impl(const shflbw_spmm_state_t* st, const void* bias, void*
         if (const char* e = getenv("SHFLBW_ABLATE")) p.ablate = atoi(e);
         if (const char* e = getenv("SHFLBW_TRACE_PTR")) p.trace = (unsigned long long*)strtoull(e, nullptr, 0);
 #endif
+        if (bias) { const int rc = allow_smem(ch.fn, ch.smem); if (rc != SHFLBW_OK) return rc; }   // (init allowed the kernel without)
         CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
     }
     CK(cudaGetLastError());
@@ -664,7 +669,7 @@ static void launch_relayout(const __half* in, __half* staged, int B, int Bp, int
     const int NT = Bp < 32 ? Bp : 32, PT = shflbw::kRelayoutSlots / NT;
     const int n_tiles = (Bp + NT - 1) / NT;
     dim3 grid((unsigned)(((PP + PT - 1) / PT) * n_tiles), (unsigned)((C + shflbw::kRelayoutC - 1) / shflbw::kRelayoutC));
-    (void)launch(shflbw::relayout_nhwc_to_chwn, grid, dim3(256), 0, s, in, staged, B, Bp, Hin, Win, Hp, Wp, R / 2, S / 2, C, step);
+    (void)launch(step > 1 ? shflbw::relayout_nhwc_to_chwn<true> : shflbw::relayout_nhwc_to_chwn<false>, grid, dim3(256), 0, s, in, staged, B, Bp, Hin, Win, Hp, Wp, R / 2, S / 2, C, step);
 }
 
 // Dynamic shared memory of unpermute_filters: 16-bit permutation + one F-vector of fp16 per position.
@@ -686,7 +691,7 @@ static cudaError_t launch_planes_to_nhwc(const void* planes, void* out, const in
         if (gx < (tiles + 7) / 8) gx = (tiles + 7) / 8;
         const bool plain = !perm && Wp == W && Hp == H;
         if (gx > tiles || plain) gx = tiles;
-        const cudaError_t e = launch(plain ? shflbw::planes_to_nhwc<true> : shflbw::planes_to_nhwc<false>, dim3((unsigned)gx, (unsigned)fb), dim3(256), 0, s, (const __half*)planes,
+        const cudaError_t e = launch(!plain ? shflbw::planes_to_nhwc<false, false> : bias ? shflbw::planes_to_nhwc<true, true> : shflbw::planes_to_nhwc<true, false>, dim3((unsigned)gx, (unsigned)fb), dim3(256), 0, s, (const __half*)planes,
                                      (__half*)out, perm, (const __half*)bias, Bn, Bp, (int)pix0, n, (int)npix, W, Wp, ph, pw,
                                      (size_t)Hp * Wp * Bp, F, shflbw::make_fast_div(Bp), shflbw::make_fast_div(W));
         if (e != cudaSuccess) return e;
@@ -759,8 +764,8 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
             out->staged_out_bytes = (size_t)B * Ho * Wo * f->F * 2;
             if (unperm_smem_bytes(f->F) > 227 * 1024 || f->F > 65536) return SHFLBW_ERR_UNSUPPORTED;
             if (unperm_smem_bytes(f->F) > 48 * 1024)
-                CK(cudaFuncSetAttribute((const void*)shflbw::unpermute_filters,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)unperm_smem_bytes(f->F)));
+                for (const void* k : {(const void*)shflbw::unpermute_filters<false>, (const void*)shflbw::unpermute_filters<true>})
+                    CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)unperm_smem_bytes(f->F)));
         }
     }
     out->kernel = SHFLBW_KERNEL_TCGEN05;
@@ -808,7 +813,9 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     }
     const bool planes = !st->chain && st->variant == 1;     // NHWC call computed as planes, then transposed
     PanelChoice ch;
-    const bool ok_kernel = (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch)
+    const bool panel_bias = bias && !planes && !st->staged_out;   // no later pass: the panel kernel's epilogue adds the bias
+    const bool ok_kernel = panel_bias            ? lookup<shflbw::kPanelConv, true>(st->V, st->tokens_per_cta, &ch)
+                           : (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch)
                            : st->variant == 1      ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch)
                                                    : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync, st->variant == 2);
     if (!ok_kernel) return SHFLBW_ERR_INVALID_ARG;
@@ -853,7 +860,11 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     if (const char* e = getenv("SHFLBW_ABLATE")) p.ablate = atoi(e);
     if (const char* e = getenv("SHFLBW_TRACE_PTR")) p.trace = (unsigned long long*)strtoull(e, nullptr, 0);
 #endif
-    if (!planes && !st->staged_out) p.C = (const __half*)bias;   // last pass of this call: its epilogue adds the bias
+    if (panel_bias) {
+        p.C = (const __half*)bias;
+        const int rc = allow_smem(ch.fn, ch.smem);
+        if (rc != SHFLBW_OK) return rc;
+    }
     CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
     // 3. back to NHWC in logical channel order.
     if (planes) {
@@ -863,7 +874,7 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
         const int per_block = shflbw::kUnpermThreads / shflbw::unperm_threads_per_pos(st->F);
         int blocks = (num_pos + per_block - 1) / per_block;
         if (blocks > 148 * 16) blocks = 148 * 16;
-        CK(launch(shflbw::unpermute_filters, dim3(blocks), dim3(shflbw::kUnpermThreads), unperm_smem_bytes(st->F), s,
+        CK(launch(bias ? shflbw::unpermute_filters<true> : shflbw::unpermute_filters<false>, dim3(blocks), dim3(shflbw::kUnpermThreads), unperm_smem_bytes(st->F), s,
                   (const __half*)st->staged_out, (__half*)st->ofmap, st->perm, (const __half*)bias, num_pos, st->F));
     }
     CK(cudaGetLastError());
