@@ -17,7 +17,12 @@
 
 namespace shflbw {
 
-// Programmatic dependent launch (see sm100_ptx.cuh): both are no-ops for plain launches.
+// Programmatic dependent launch (see sm100_ptx.cuh): both are no-ops for plain launches.  A kernel lets the
+// next one in early where that one has a set-up to overlap (the panel kernel after a relayout).  The last
+// pass of a convolution call lets it in only after its own wait, when the panel kernel is done: the next call's relayout has nothing to set up,
+// and its blocks, resident and waiting through the panel kernel and the last pass of this call, took the
+// shared memory and the slots of theirs (calls back to back: 19.8 -> 14.8 us for 13x8x8x376 -> 2016 at stride 2,
+// 13.5 -> 10.8 for 12x15x13x144 -> 640, 12 % over 39 shapes drawn from 1..64 images).
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -158,8 +163,8 @@ unpermute_filters(const __half* __restrict__ staged, __half* __restrict__ out, c
     const int G = unperm_threads_per_pos(F), P = kUnpermThreads / G;
     const int slot = threadIdx.x / G, t = threadIdx.x - slot * G;   // position slot, thread within it
     for (int f = threadIdx.x; f < F; f += kUnpermThreads) sperm[f] = (unsigned short)__ldg(perm + f);
-    grid_dep_launch();
     grid_dep_wait();                         // the staged output is complete only when the panel kernel is
+    grid_dep_launch();                       // (after the wait: see above)
     __half* mine = vec + (size_t)slot * F;
     for (int q0 = blockIdx.x * P; q0 < num_pos; q0 += gridDim.x * P) {
         const int q = q0 + slot;
@@ -199,7 +204,7 @@ unpermute_filters(const __half* __restrict__ staged, __half* __restrict__ out, c
 // are found once, by a scan of perm.  (One pixel x 8 images x all channels per block, 16-byte reads of
 // scattered lines: 52 us for 256 x 7 x 7 x 2048, 103 MB; this kernel: 21 us.)  F % 8 == 0, Bp % 8 == 0;
 // images n >= Bn are padding.  A launch covers pixels pix0 .. pix0 + npix of out_pix.
-// PLAIN (plane c of channel c, no halo): a token's place in its plane is its index, and a block moves one
+// PLAIN (plane c of channel c, no halo, F % 64 == 0): a token's place in its plane is its index, and a block moves one
 // 64 x 64 tile; the general form's start-up and registers cost 1.1 us of 4.8 at 3136 tokens x 2048 filters.
 template <bool PLAIN, bool BIAS>
 __global__ void __launch_bounds__(256)
@@ -208,7 +213,6 @@ planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, cons
                size_t plane, int F, FastDiv div_bp, FastDiv div_w) {
     __shared__ __align__(16) __half tile[64 * 64];
     __shared__ int plane_of[64];                         // of the block's channels
-    grid_dep_launch();
     const int f0 = blockIdx.y * 64, nf = min(64, F - f0);
     if constexpr (!PLAIN) {
     if (perm) {
@@ -220,19 +224,21 @@ planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, cons
     __syncthreads();
     }
     grid_dep_wait();                                     // the planes are complete only when the panel kernel is
+    grid_dep_launch();                                   // (after the wait: see above)
     const int ntok = npix * Bp;
     const int c = threadIdx.x & 7, r0 = threadIdx.x >> 3;   // 16-byte chunk, row of the pass
     const __half* src[2];
 #pragma unroll
     for (int pass = 0; pass < 2; ++pass) {
         const int r = r0 + 32 * pass;
-        src[pass] = r < nf ? planes + (size_t)(PLAIN ? f0 + r : plane_of[r]) * plane : nullptr;
+        if constexpr (PLAIN) src[pass] = planes + (size_t)(f0 + r) * plane;
+        else src[pass] = r < nf ? planes + (size_t)plane_of[r] * plane : nullptr;
     }
     uint4 v[2];
     auto load = [&](int tok0) {
         const int tok = tok0 + c * 8;
         size_t off = 0;
-        if (PLAIN) off = (size_t)pix0 * Bp + tok;
+        if constexpr (PLAIN) off = (size_t)pix0 * Bp + tok;
         else if (tok < ntok) {
             const int lpix = fast_div(tok, div_bp), n = tok - lpix * Bp, pix = pix0 + lpix;
             const int h = fast_div(pix, div_w), w = pix - h * W;
@@ -241,7 +247,7 @@ planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, cons
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
             v[pass] = make_uint4(0u, 0u, 0u, 0u);
-            if (tok < ntok && src[pass]) v[pass] = *(const uint4*)(src[pass] + off);
+            if (tok < ntok && (PLAIN || src[pass])) v[pass] = *(const uint4*)(src[pass] + off);
         }
     };
     int tok0 = blockIdx.x * 64;
@@ -262,7 +268,7 @@ planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, cons
             const int t = r0 + 32 * pass;                    // token of the tile
             const int tok = tok0 + t;
             const int pix = fast_div(tok, div_bp), n = tok - pix * Bp;
-            if (tok < ntok && n < Bn && c * 8 < nf) {
+            if (tok < ntok && n < Bn && (PLAIN || c * 8 < nf)) {
                 uint4 o = *(const uint4*)(tile + t * 64 + ((c ^ ((t >> 3) & 7)) << 3));
                 if constexpr (BIAS) o = add_bias8(o, __ldg((const uint4*)(bias + f0 + c * 8)));
                 *(uint4*)(out + ((size_t)n * out_pix + pix0 + pix) * F + f0 + c * 8) = o;

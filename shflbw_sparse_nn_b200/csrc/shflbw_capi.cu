@@ -689,7 +689,7 @@ static cudaError_t launch_planes_to_nhwc(const void* planes, void* out, const in
         const long long tiles = ((long long)n * Bp + 63) / 64;
         long long gx = (148 * 16 + fb - 1) / fb;
         if (gx < (tiles + 7) / 8) gx = (tiles + 7) / 8;
-        const bool plain = !perm && Wp == W && Hp == H;
+        const bool plain = !perm && Wp == W && Hp == H && F % 64 == 0;
         if (gx > tiles || plain) gx = tiles;
         const cudaError_t e = launch(!plain ? shflbw::planes_to_nhwc<false, false> : bias ? shflbw::planes_to_nhwc<true, true> : shflbw::planes_to_nhwc<true, false>, dim3((unsigned)gx, (unsigned)fb), dim3(256), 0, s, (const __half*)planes,
                                      (__half*)out, perm, (const __half*)bias, Bn, Bp, (int)pix0, n, (int)npix, W, Wp, ph, pw,
