@@ -193,9 +193,8 @@ unpermute_filters(const __half* __restrict__ staged, __half* __restrict__ out, c
     }
 }
 
-// Channel-major planes -> NHWC: out[n][h][w][c] = planes[f][h + ph][w + pw][n] (+ bias[c]), where plane f
-// holds logical channel c = perm[f] (perm == nullptr: c = f).  Used for the output of an NHWC call computed
-// as planes (perm == nullptr, no halo) and to export a chain buffer.  Bound by HBM / L2 bandwidth: both
+// Chain buffer -> NHWC: out[n][h][w][c] = planes[f][h + ph][w + pw][n], where plane f holds logical channel
+// c = perm[f] (perm == nullptr: c = f).  Bound by HBM / L2 bandwidth: both
 // sides should move whole lines.  One block owns 64 channels and moves them 64 tokens (tok = pixel * Bp + n)
 // at a time through 8 KB of shared memory: 16-byte loads of 8 tokens of one plane, 2-byte scatters into
 // [token][channel] (8-channel groups XOR-swizzled by the token group, so neither side has bank conflicts),
@@ -204,17 +203,13 @@ unpermute_filters(const __half* __restrict__ staged, __half* __restrict__ out, c
 // are found once, by a scan of perm.  (One pixel x 8 images x all channels per block, 16-byte reads of
 // scattered lines: 52 us for 256 x 7 x 7 x 2048, 103 MB; this kernel: 21 us.)  F % 8 == 0, Bp % 8 == 0;
 // images n >= Bn are padding.  A launch covers pixels pix0 .. pix0 + npix of out_pix.
-// PLAIN (plane c of channel c, no halo, F % 64 == 0): a token's place in its plane is its index, and a block moves one
-// 64 x 64 tile; the general form's start-up and registers cost 1.1 us of 4.8 at 3136 tokens x 2048 filters.
-template <bool PLAIN, bool BIAS>
 __global__ void __launch_bounds__(256)
-planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, const int* __restrict__ perm,
-               const __half* __restrict__ bias, int Bn, int Bp, int pix0, int npix, int out_pix, int W, int Wp, int ph, int pw,
-               size_t plane, int F, FastDiv div_bp, FastDiv div_w) {
+export_planes_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, const int* __restrict__ perm,
+                   int Bn, int Bp, int pix0, int npix, int out_pix, int W, int Wp, int ph, int pw,
+                   size_t plane, int F, FastDiv div_bp, FastDiv div_w) {
     __shared__ __align__(16) __half tile[64 * 64];
     __shared__ int plane_of[64];                         // of the block's channels
     const int f0 = blockIdx.y * 64, nf = min(64, F - f0);
-    if constexpr (!PLAIN) {
     if (perm) {
         for (int f = threadIdx.x; f < F; f += 256) {     // a permutation: every channel is found exactly once
             const int c = __ldg(perm + f) - f0;
@@ -222,7 +217,6 @@ planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, cons
         }
     } else if (threadIdx.x < 64) plane_of[threadIdx.x] = f0 + threadIdx.x;
     __syncthreads();
-    }
     grid_dep_wait();                                     // the planes are complete only when the panel kernel is
     grid_dep_launch();                                   // (after the wait: see above)
     const int ntok = npix * Bp;
@@ -231,15 +225,13 @@ planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, cons
 #pragma unroll
     for (int pass = 0; pass < 2; ++pass) {
         const int r = r0 + 32 * pass;
-        if constexpr (PLAIN) src[pass] = planes + (size_t)(f0 + r) * plane;
-        else src[pass] = r < nf ? planes + (size_t)plane_of[r] * plane : nullptr;
+        src[pass] = r < nf ? planes + (size_t)plane_of[r] * plane : nullptr;
     }
     uint4 v[2];
     auto load = [&](int tok0) {
         const int tok = tok0 + c * 8;
         size_t off = 0;
-        if constexpr (PLAIN) off = (size_t)pix0 * Bp + tok;
-        else if (tok < ntok) {
+        if (tok < ntok) {
             const int lpix = fast_div(tok, div_bp), n = tok - lpix * Bp, pix = pix0 + lpix;
             const int h = fast_div(pix, div_w), w = pix - h * W;
             off = ((size_t)(h + ph) * Wp + w + pw) * Bp + n;
@@ -247,7 +239,7 @@ planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, cons
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
             v[pass] = make_uint4(0u, 0u, 0u, 0u);
-            if (tok < ntok && (PLAIN || src[pass])) v[pass] = *(const uint4*)(src[pass] + off);
+            if (tok < ntok && src[pass]) v[pass] = *(const uint4*)(src[pass] + off);
         }
     };
     int tok0 = blockIdx.x * 64;
@@ -262,20 +254,55 @@ planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, cons
             for (int j = 0; j < 8; ++j) tile[(c * 8 + j) * 64 + col] = h[j];
         }
         __syncthreads();
-        if constexpr (!PLAIN) load(tok0 + gridDim.x * 64);
+        load(tok0 + gridDim.x * 64);
 #pragma unroll
         for (int pass = 0; pass < 2; ++pass) {
             const int t = r0 + 32 * pass;                    // token of the tile
             const int tok = tok0 + t;
             const int pix = fast_div(tok, div_bp), n = tok - pix * Bp;
-            if (tok < ntok && n < Bn && (PLAIN || c * 8 < nf)) {
-                uint4 o = *(const uint4*)(tile + t * 64 + ((c ^ ((t >> 3) & 7)) << 3));
-                if constexpr (BIAS) o = add_bias8(o, __ldg((const uint4*)(bias + f0 + c * 8)));
-                *(uint4*)(out + ((size_t)n * out_pix + pix0 + pix) * F + f0 + c * 8) = o;
+            if (tok < ntok && n < Bn && c * 8 < nf) {
+                *(uint4*)(out + ((size_t)n * out_pix + pix0 + pix) * F + f0 + c * 8) =
+                    *(const uint4*)(tile + t * 64 + ((c ^ ((t >> 3) & 7)) << 3));
             }
         }
-        if constexpr (PLAIN) return;
         __syncthreads();
+    }
+}
+
+// planes[f][tok] -> out[n][pix][f] (+ bias[f]): the output of an NHWC call computed as planes (one row of
+// tok = pix * Bp + n tokens per LOGICAL filter f) transposed to NHWC.  The same tile as above, one per block,
+// without the plane search and the halo, whose start-up and registers cost 1.1 us of 4.8 at 3136 tokens x
+// 2048 filters.  F % 64 == 0, Bp % 8 == 0; images n >= Bn are padding.
+template <bool BIAS>
+__global__ void __launch_bounds__(256)
+planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, const __half* __restrict__ bias, int Bn, int Bp, int npix, int F) {
+    __shared__ __align__(16) __half tile[64 * 64];
+    grid_dep_wait();                                     // the planes are complete only when the panel kernel is
+    grid_dep_launch();                                   // (after the wait: see above)
+    const int ntok = npix * Bp;
+    const int tok0 = blockIdx.x * 64, f0 = blockIdx.y * 64;
+    const int c = threadIdx.x & 7, r0 = threadIdx.x >> 3;   // 16-byte chunk, row of the pass
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const int r = r0 + 32 * pass;                    // filter of the tile
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (tok0 + c * 8 < ntok) v = *(const uint4*)(planes + (size_t)(f0 + r) * ntok + tok0 + c * 8);
+        const __half* h = (const __half*)&v;
+        const int col = (((r >> 3) ^ c) << 3) | (r & 7);    // token group c: filter group XOR c
+#pragma unroll
+        for (int j = 0; j < 8; ++j) tile[(c * 8 + j) * 64 + col] = h[j];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int pass = 0; pass < 2; ++pass) {
+        const int t = r0 + 32 * pass;                    // token of the tile
+        const int tok = tok0 + t;
+        const int pix = tok / Bp, n = tok - pix * Bp;
+        if (tok < ntok && n < Bn) {
+            uint4 o = *(const uint4*)(tile + t * 64 + ((c ^ ((t >> 3) & 7)) << 3));
+            if constexpr (BIAS) o = add_bias8(o, __ldg((const uint4*)(bias + f0 + c * 8)));
+            *(uint4*)(out + ((size_t)n * npix + pix) * F + f0 + c * 8) = o;
+        }
     }
 }
 

@@ -677,9 +677,9 @@ static size_t unperm_smem_bytes(int F) {
     return (size_t)F * 2 * (1 + shflbw::kUnpermThreads / shflbw::unperm_threads_per_pos(F));
 }
 
-// Planes -> NHWC (see the kernel).  Two to eight 64-token steps per block where that leaves several blocks
+// Chain buffer -> NHWC (see the kernel).  Two to eight 64-token steps per block where that leaves several blocks
 // per SM, so that a block's scan of the permutation and its start-up are shared.
-static cudaError_t launch_planes_to_nhwc(const void* planes, void* out, const int* perm, const void* bias, int Bn, int Bp, int H, int W,
+static cudaError_t launch_export(const void* planes, void* out, const int* perm, int Bn, int Bp, int H, int W,
                                          int Hp, int Wp, int ph, int pw, int F, cudaStream_t s) {
     const int fb = (F + 63) / 64;
     const int per = (1 << 30) / Bp > 0 ? (1 << 30) / Bp : 1;            // pixels per launch: the kernel counts its tokens in 31 bits
@@ -689,11 +689,10 @@ static cudaError_t launch_planes_to_nhwc(const void* planes, void* out, const in
         const long long tiles = ((long long)n * Bp + 63) / 64;
         long long gx = (148 * 16 + fb - 1) / fb;
         if (gx < (tiles + 7) / 8) gx = (tiles + 7) / 8;
-        const bool plain = !perm && Wp == W && Hp == H && F % 64 == 0;
-        if (gx > tiles || plain) gx = tiles;
-        const cudaError_t e = launch(!plain ? shflbw::planes_to_nhwc<false, false> : bias ? shflbw::planes_to_nhwc<true, true> : shflbw::planes_to_nhwc<true, false>, dim3((unsigned)gx, (unsigned)fb), dim3(256), 0, s, (const __half*)planes,
-                                     (__half*)out, perm, (const __half*)bias, Bn, Bp, (int)pix0, n, (int)npix, W, Wp, ph, pw,
-                                     (size_t)Hp * Wp * Bp, F, shflbw::make_fast_div(Bp), shflbw::make_fast_div(W));
+        if (gx > tiles) gx = tiles;
+        const cudaError_t e = launch(shflbw::export_planes_nhwc, dim3((unsigned)gx, (unsigned)fb), dim3(256), 0, s, (const __half*)planes,
+                                     (__half*)out, perm, Bn, Bp, (int)pix0, n, (int)npix, W, Wp, ph, pw, (size_t)Hp * Wp * Bp, F,
+                                     shflbw::make_fast_div(Bp), shflbw::make_fast_div(W));
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -868,7 +867,10 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
     // 3. back to NHWC in logical channel order.
     if (planes) {
-        CK(launch_planes_to_nhwc(st->staged_out, st->ofmap, nullptr, bias, st->B, st->Bp, st->Ho, st->Wo, st->Ho, st->Wo, 0, 0, st->F, s));
+        const int npix = st->Ho * st->Wo;
+        CK(launch(bias ? shflbw::planes_to_nhwc<true> : shflbw::planes_to_nhwc<false>,
+                  dim3((unsigned)(((long long)npix * st->Bp + 63) / 64), (unsigned)(st->F / 64)), dim3(256), 0, s,
+                  (const __half*)st->staged_out, (__half*)st->ofmap, (const __half*)bias, st->B, st->Bp, npix, st->F));
     } else if (st->staged_out) {
         const int num_pos = st->B * st->Ho * st->Wo;
         const int per_block = shflbw::kUnpermThreads / shflbw::unperm_threads_per_pos(st->F);
@@ -963,7 +965,7 @@ int shflbw_chain_export_nhwc(const void* chain_buf, int B, int H, int W, int F, 
     if ((size_t)F * 16 > 227 * 1024) return SHFLBW_ERR_UNSUPPORTED;
     const int Bp = (B + 7) / 8 * 8;
     if ((long long)H * W * (Bp / 8) >= (1ll << 31)) return SHFLBW_ERR_UNSUPPORTED;
-    CK(launch_planes_to_nhwc(chain_buf, nhwc, perm, nullptr, B, Bp, H, W, H + R - 1, W + S - 1, R / 2, S / 2, F, (cudaStream_t)stream));
+    CK(launch_export(chain_buf, nhwc, perm, B, Bp, H, W, H + R - 1, W + S - 1, R / 2, S / 2, F, (cudaStream_t)stream));
     CK(cudaGetLastError());
     return SHFLBW_OK;
 }
