@@ -7,9 +7,10 @@ the library's C ABI on the caller's CUDA stream.
 The reference project has no such layer (it only ever builds random patterns,
 block_sparse/spmm/blockwise_format.h:70-123, and points to the paper for real models); this
 is the piece a user with a trained network needs in front of the hot path.  torch is the
-plumbing here (device buffers, the current stream, the bias add and layout views); pruning is
-`pruner.prune_matrix` / `prune_conv_filter` on the host, once, and every forward is the
-library's SpMM / SpConv kernel.  fp16 inference only; there is no backward pass.
+plumbing here (device buffers, the current stream, layout views, and the inputs and biases that a
+kernel cannot read where they are); pruning is `pruner.prune_matrix` / `prune_conv_filter` on the
+host, once, and every forward is the library's SpMM / SpConv kernels, which add the bias too.  fp16
+inference only; there is no backward pass through the product.
 """
 from __future__ import annotations
 
@@ -41,13 +42,22 @@ def _stream_of(device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(device.index)
 
 
+def _in_memory(x: torch.Tensor) -> bool:
+    """Whether x.data_ptr() addresses the values of `x`: not where a negation is still pending (the memory
+    holds -x) and not for a tensor without memory of its own (a wrapper subclass, whose pointer is 0)."""
+    return not x.is_neg() and x.data_ptr() != 0
+
+
 def _fused_bias(bias, device: torch.device, n: int, align: int):
-    """(bias on `device`, whether the kernels can add it: fp16, one per output, contiguous, aligned)."""
+    """(bias on `device`, whether the kernels can add it: fp16, one per output, contiguous, aligned and its
+    values in memory).  Every other bias is added by torch."""
     if bias is None:
         return None, False
     if bias.device != device:
         bias = bias.to(device)
-    return bias, bias.dtype == torch.float16 and bias.shape == (n,) and bias.is_contiguous() and bias.data_ptr() % align == 0
+    fused = bias.dtype == torch.float16 and bias.shape == (n,) and bias.is_contiguous() and _in_memory(bias) \
+        and bias.data_ptr() % align == 0
+    return bias, fused
 
 
 class ShflBWLinear(nn.Module):
@@ -94,6 +104,7 @@ class ShflBWLinear(nn.Module):
         _require_cuda_half(xt, "ShflBWLinear")
         if xt.dim() != 2 or xt.shape[0] != self.in_features or xt.shape[1] % 8 or not xt.is_contiguous():
             raise ValueError("expected a contiguous [in_features][tokens] tensor with tokens % 8 == 0")
+        xt = xt.resolve_neg()
         return self._run(None, xt.shape[1], xt, xt.shape[1])
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
@@ -102,7 +113,12 @@ class ShflBWLinear(nn.Module):
         x2 = x.reshape(-1, self.in_features).contiguous()
         tokens = x2.shape[0]
         padded = -(-tokens // 8) * 8
-        xt = torch.empty((self.in_features, padded), dtype=torch.float16, device=x.device)
+        if tokens == 0 or _in_memory(x2):
+            xt = torch.empty((self.in_features, padded), dtype=torch.float16, device=x.device)
+        else:                                                # torch reads it, and transposes it on the way
+            xt = torch.zeros((self.in_features, padded), dtype=torch.float16, device=x.device)
+            xt[:, :tokens] = x2.t()
+            x2 = None
         yt = self._run(x2, tokens, xt, padded)
         y = yt.as_strided((tokens, self.out_features), (1, padded))
         return y if lead == (tokens,) else y.reshape(*lead, self.out_features)
@@ -146,7 +162,7 @@ class ShflBWConv2d(nn.Module):
                 self.spfilter.transform_and_sync_device()
             self._uploaded_on = x.device
         n, _, h, w = x.shape
-        x_nhwc = x.permute(0, 2, 3, 1).contiguous()          # a view when x is channels-last
+        x_nhwc = x.permute(0, 2, 3, 1).contiguous().resolve_neg()   # a view when x is channels-last
         ho, wo = -(-h // self.stride), -(-w // self.stride)
         out = torch.empty((n, ho, wo, self.out_channels), dtype=torch.float16, device=x.device)
         bias, fused = _fused_bias(self.bias, x.device, self.out_channels, 16)
