@@ -19,6 +19,7 @@ from contextlib import nullcontext
 import numpy as np
 import torch
 from torch import nn
+from torch.autograd import forward_ad
 
 from . import blockwise as bw
 from .pruner import prune_conv_filter, prune_matrix
@@ -48,15 +49,22 @@ def _in_memory(x: torch.Tensor) -> bool:
     return not x.is_neg() and x.data_ptr() != 0
 
 
+def _carries_gradient(t: torch.Tensor) -> bool:
+    """Whether an operation of torch on `t` would record a gradient or carry a tangent along."""
+    if t.requires_grad and torch.is_grad_enabled():
+        return True
+    return forward_ad._current_level >= 0 and forward_ad.unpack_dual(t).tangent is not None
+
+
 def _fused_bias(bias, device: torch.device, n: int, align: int):
-    """(bias on `device`, whether the kernels can add it: fp16, one per output, contiguous, aligned and its
-    values in memory).  Every other bias is added by torch."""
+    """(bias on `device`, whether the kernels can add it: fp16, one per output, contiguous, aligned, its values
+    in memory and without a gradient to record).  Every other bias is added by torch."""
     if bias is None:
         return None, False
     if bias.device != device:
         bias = bias.to(device)
     fused = bias.dtype == torch.float16 and bias.shape == (n,) and bias.is_contiguous() and _in_memory(bias) \
-        and bias.data_ptr() % align == 0
+        and bias.data_ptr() % align == 0 and not _carries_gradient(bias)
     return bias, fused
 
 

@@ -1,8 +1,9 @@
 """Which tensors the module front end hands to the kernels by address.  A kernel reads memory, so a
-tensor whose memory does not hold its values (a pending negation, a wrapper subclass) must go
-through torch instead."""
+tensor whose memory does not hold its values (a pending negation, a wrapper subclass) or whose
+addition has to be recorded by autograd must go through torch instead."""
 import pytest
 import torch
+from torch.autograd import forward_ad
 from torch.utils._pytree import tree_map
 
 import shflbw_sparse_nn_b200.nn as sbnn
@@ -37,6 +38,16 @@ def test_bias_is_fused_only_where_the_kernel_can_read_it():
     assert sbnn._fused_bias(None, CPU, 16, 2) == (None, False)
 
 
+def test_bias_that_autograd_follows_is_not_fused():
+    b = torch.ones(16, dtype=torch.float16, requires_grad=True)
+    assert not sbnn._fused_bias(b, CPU, 16, 2)[1]
+    with torch.no_grad():
+        assert sbnn._fused_bias(b, CPU, 16, 2)[1]
+    with forward_ad.dual_level():
+        assert not sbnn._fused_bias(forward_ad.make_dual(torch.ones(16).half(), torch.ones(16).half()), CPU, 16, 2)[1]
+        assert sbnn._fused_bias(torch.ones(16).half(), CPU, 16, 2)[1]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("kind", ["plain", "neg", "wrapped"])
 def test_modules_compute_with_the_values_of_a_tensor_and_not_its_memory(kind):
@@ -53,3 +64,19 @@ def test_modules_compute_with_the_values_of_a_tensor_and_not_its_memory(kind):
         assert torch.equal(conv(as_kind(xc)), want_c)
     lin._buffers["bias"], conv._buffers["bias"] = as_kind(lin.bias), as_kind(conv.bias)
     assert torch.equal(lin(x), want) and torch.equal(conv(xc), want_c)
+
+
+@pytest.mark.gpu
+def test_gradient_of_a_bias():
+    lin = sbnn.ShflBWLinear.from_dense(torch.nn.Linear(128, 64), V=64, density=0.3).cuda()
+    conv = sbnn.ShflBWConv2d.from_dense(torch.nn.Conv2d(32, 64, 1), V=64, density=0.3).cuda()
+    x = (torch.rand(24, 128, device="cuda") * 2 - 1).half()
+    xc = (torch.rand(3, 32, 5, 7, device="cuda") * 2 - 1).half()
+    for module, inp, count in ((lin, x, 24), (conv, xc, 3 * 5 * 7)):
+        want = module(inp)
+        assert not want.requires_grad
+        module.bias.requires_grad_()
+        y = module(inp)
+        assert torch.equal(y.detach(), want)
+        y.float().sum().backward()
+        assert torch.equal(module.bias.grad, torch.full((64,), float(count), dtype=torch.float16, device="cuda"))
