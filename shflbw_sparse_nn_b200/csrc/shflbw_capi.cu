@@ -1026,35 +1026,39 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     if (!f || !st || !st->init_success || !st->chain || !res_chain) return SHFLBW_ERR_INVALID_ARG;
     if (!on_current_device(*f) || st->blk_ptr != f->d_kptr) return SHFLBW_ERR_INVALID_ARG;
     if ((uintptr_t)res_chain & 15) return SHFLBW_ERR_UNSUPPORTED;
+    if (map_host)
+        for (int i = 0; i < st->F; ++i)
+            if (map_host[i] < 0 || map_host[i] >= st->F) return SHFLBW_ERR_BAD_FORMAT;
     // The sixteen-epilogue-warp kernel copies the residual an item ahead, which pays up to two stages of
     // columns per block (7x7x512 -> 2048 with residual, batch 256: 38 -> 31 us); without a residual the
     // limit is one stage (pick_panel).
-    if (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
-        (f->kptr.empty() ? 0 : f->kptr.back()) <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count()) {
-        PanelChoice ch;
-        if (lookup<shflbw::kPanelConvChain>(64, 256, &ch, shflbw::kGatherCpAsync, true)) {
-            const int rc = allow_smem(ch.fn, ch.smem);
-            if (rc != SHFLBW_OK) return rc;
-            st->variant = 2; st->stages = ch.stages; st->producer_warps = ch.pw; st->block_x = ch.threads; st->shared_mem_size = ch.smem;
-        }
+    PanelChoice ch;
+    const bool wide = st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
+                      (f->kptr.empty() ? 0 : f->kptr.back()) <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count() &&
+                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, shflbw::kGatherCpAsync, true);
+    if (wide) {
+        const int rc = allow_smem(ch.fn, ch.smem);
+        if (rc != SHFLBW_OK) return rc;
     }
-    // A map buffer made by an earlier call for this state is one of the handle's retired buffers.
-    const int* prev_map = nullptr;
-    for (void* r : f->retired) if (r == (const void*)st->residual_map) prev_map = st->residual_map;
-    st->residual = res_chain;
-    st->residual_map = nullptr;
+    const int* map_dev = nullptr;
     if (map_host) {
-        for (int i = 0; i < st->F; ++i)
-            if (map_host[i] < 0 || map_host[i] >= st->F) return SHFLBW_ERR_BAD_FORMAT;
         // One device buffer per state: re-binding the residual of the same state (every step,
-        // say) overwrites it in place instead of allocating again.
-        void* d = const_cast<int*>(prev_map);
+        // say) overwrites the map of an earlier call, one of the handle's retired buffers, in place
+        // instead of allocating again.
+        void* d = nullptr;
+        for (void* r : f->retired) if (r == (const void*)st->residual_map) d = r;
         if (!d) {
             CK(cudaMalloc(&d, (size_t)st->F * sizeof(int)));
             f->retired.push_back(d);                   // lives as long as the filter's device copy
         }
         CK(cudaMemcpy(d, map_host, (size_t)st->F * sizeof(int), cudaMemcpyHostToDevice));
-        st->residual_map = (const int*)d;
+        map_dev = (const int*)d;
+    }
+    // Nothing can fail from here on: a refused call leaves the state as it was.
+    st->residual = res_chain;
+    st->residual_map = map_dev;
+    if (wide) {
+        st->variant = 2; st->stages = ch.stages; st->producer_warps = ch.pw; st->block_x = ch.threads; st->shared_mem_size = ch.smem;
     }
     return SHFLBW_OK;
 }

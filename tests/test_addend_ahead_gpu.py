@@ -3,11 +3,14 @@ to shared memory an item ahead.  It performs the arithmetic of the eight-warp ke
 order, so the two must agree bit for bit: with several items per block, with one item only for some
 of the blocks, with a ragged last token tile, with a halo around the output planes, with a plane map
 and with the residual added in place."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 import shflbw_sparse_nn_b200 as sb
+from shflbw_sparse_nn_b200 import _cabi
 from gpu_util import dev, epilogue_warps, host, operand_swap, run_spmm, tile
 
 pytestmark = pytest.mark.gpu
@@ -60,6 +63,24 @@ def test_residual_picks_the_sixteen_warp_kernel_for_two_stages_of_columns():
         f.device_status()
         got.append(host(out).view(np.uint16))
     assert np.array_equal(got[0], got[1])
+
+
+def test_refused_residual_leaves_the_state_as_it_was():
+    Cc, F, Bn, H = 512, 512, 64, 20           # a residual would switch to the sixteen-warp kernel
+    f = sb.BlockwiseSpFilter().init_random(F, 1, 1, Cc, 64, 1, 0.2, True, 8, values="uniform")
+    f.transform_and_sync_device()
+    x = dev(sb.uniform_half(9, sb.chain_buffer_elems(Cc, H, H, Bn, 1, 1)))
+    out = torch.zeros(sb.chain_buffer_elems(F, H, H, Bn, 1, 1), dtype=torch.float16, device="cuda")
+    op = sb.SpconvChainOp().initialize(f, Bn, H, H, 1, x, out, 1, 1)
+    before = bytes(op._state)
+    bad = np.arange(F, dtype=np.int32)
+    for value in (-1, F):
+        bad[-1] = value
+        rc = _cabi.lib().shflbw_spconv_chain_set_residual(f._h, C.byref(op._state), out.data_ptr(), bad.ctypes.data)
+        assert rc == _cabi.ERR_BAD_FORMAT and bytes(op._state) == before
+    bad[-1] = F - 1
+    assert _cabi.lib().shflbw_spconv_chain_set_residual(f._h, C.byref(op._state), out.data_ptr(), bad.ctypes.data) == 0
+    assert op._state.variant == 2 and op._state.residual == out.data_ptr() and op._state.residual_map
 
 
 @pytest.mark.parametrize("N", [256 * 37, 256 * 80 + 24])
