@@ -267,15 +267,13 @@ int sm_count() {
 // Opt a panel kernel in to its dynamic shared memory once per (device, kernel): the host-buffer
 // calls initialise an op per chunk, and the attribute call is not free.
 int allow_smem(PanelKernel fn, size_t bytes) {
-    struct Done { const void* fn; int dev; };
-    static Done done[256];
-    static int n_done = 0;
+    static shflbw::OncePerDevice done;
     int dev = 0;
     CK(cudaGetDevice(&dev));
-    for (int i = 0; i < n_done; ++i) if (done[i].fn == (const void*)fn && done[i].dev == dev) return SHFLBW_OK;
-    CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    if (n_done < 256) done[n_done++] = {(const void*)fn, dev};
-    return SHFLBW_OK;
+    return done.run((const void*)fn, dev, [&]() -> int {
+        CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+        return SHFLBW_OK;
+    });
 }
 
 // Tile selection.  A 256-token work item halves the value-panel traffic per token and is

@@ -4,7 +4,10 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <mutex>
+#include <set>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "shflbw.h"
@@ -74,6 +77,30 @@ struct shflbw_matrix {
 };
 
 namespace shflbw {
+
+// Remembers for which (kernel, device) pairs an idempotent set-up call has succeeded, so that it is made once
+// and not on every call.  Any number of threads and pairs; a pair counts as done only after its set-up returned.
+class OncePerDevice {
+public:
+    template <class SetUp>
+    int run(const void* kernel, int device, SetUp&& set_up) {   // SHFLBW_OK, or what set_up returned
+        const std::pair<const void*, int> key{kernel, device};
+        {
+            std::lock_guard<std::mutex> lock(mutex_);
+            if (done_.count(key)) return SHFLBW_OK;
+        }
+        const int rc = set_up();
+        if (rc == SHFLBW_OK) {
+            std::lock_guard<std::mutex> lock(mutex_);
+            done_.insert(key);
+        }
+        return rc;
+    }
+
+private:
+    std::mutex mutex_;
+    std::set<std::pair<const void*, int>> done_;
+};
 
 // fp16 helpers on raw bits (host).
 float half_bits_to_float(uint16_t h);
