@@ -28,6 +28,9 @@ thread_local char g_cuda_err[256] = "";
 // which one producer warp withholds its arrivals.  Process-wide; read when a launch is issued.
 long long g_wait_limit = shflbw::kWaitLimitCycles;
 int g_inject_from = -1;
+#ifdef SHFLBW_FAULT_INJECT
+int g_set_ups_left = -1;             // test builds: this many more shared-memory opt-ins succeed (< 0: all)
+#endif
 
 bool cuda_ok(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return true;
@@ -270,6 +273,10 @@ int allow_smem(PanelKernel fn, size_t bytes) {
     static shflbw::OncePerDevice done;
     int dev = 0;
     CK(cudaGetDevice(&dev));
+#ifdef SHFLBW_FAULT_INJECT
+    if (g_set_ups_left == 0) return SHFLBW_ERR_CUDA;
+    if (g_set_ups_left > 0) --g_set_ups_left;
+#endif
     return done.run((const void*)fn, dev, [&]() -> int {
         CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         return SHFLBW_OK;
@@ -398,6 +405,8 @@ int shflbw_set_wait_limit_cycles(long long cycles) {
 // Test builds only: launches issued after this call run with one producer warp withholding its
 // barrier arrivals from stage `stage` on (< 0: off), so that the consumer's bounded wait gives up.
 int shflbw_debug_withhold_arrivals_from(int stage) { g_inject_from = stage; return SHFLBW_OK; }
+// ... and after this call `n` kernels are allowed their shared memory, the next ones refused (n < 0: off).
+int shflbw_debug_fail_set_up_after(int n) { g_set_ups_left = n; return SHFLBW_OK; }
 #endif
 
 int shflbw_matrix_to_device(shflbw_matrix_t* m) {
@@ -502,68 +511,77 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
     return SHFLBW_OK;
 }
 
-// bias: nullptr, or one value per output row, added to the fp16 product (state without C; tensor-core kernels).
-static int spmm_exec_impl(const shflbw_spmm_state_t* st, const void* bias, void* stream) {
+// The panel kernel of an initialised SpMM state, allowed its shared memory.  The state is a POD and may have
+// been copied: the function pointer is re-derived from the recorded configuration.  bias: the instance that
+// adds a bias (init allowed the one without).
+static int spmm_panel(const shflbw_spmm_state_t* st, bool bias, PanelChoice* ch) {
+    const bool wide = st->variant == 2;
+    const bool found =
+        bias ? st->variant == 1 ? lookup<shflbw::kPanelSpmmRows, true>(st->V, st->tokens_per_cta, ch, st->gather)
+                                : lookup<shflbw::kPanelSpmm, true>(st->V, st->tokens_per_cta, ch, shflbw::kGatherCpAsync, wide)
+             : st->variant == 1 ? lookup<shflbw::kPanelSpmmRows>(st->V, st->tokens_per_cta, ch, st->gather)
+                                : lookup<shflbw::kPanelSpmm>(st->V, st->tokens_per_cta, ch, shflbw::kGatherCpAsync, wide);
+    if (!found || ch->gather != st->gather) return SHFLBW_ERR_INVALID_ARG;
+    return bias ? allow_smem(ch->fn, ch->smem) : SHFLBW_OK;
+}
+
+// bias: nullptr, or one value per output row, added to the fp16 product (state without C).
+static int launch_spmm_panel(const shflbw_spmm_state_t* st, const PanelChoice& ch, const void* bias, cudaStream_t s) {
+    shflbw::PanelParams p{};
+    p.blk_ptr = st->blk_ptr; p.blk_idx = st->blk_idx; p.blk_val = (const __half*)st->blk_val;
+    p.perm = st->perm; p.status_word = st->status_word; p.alpha = st->alpha; p.beta = st->beta;
+    p.wait_limit = g_wait_limit; p.inject_from = g_inject_from; p.idx_limit = (unsigned)(st->K - 1);
+    p.B = (const __half*)st->B; p.C = (const __half*)st->C; p.D = (__half*)st->D; p.N = st->N;
+    if (bias) { p.C = (const __half*)bias; p.beta = 1.f; }
+    p.wide_stores = (st->N % 16 == 0) && (((uintptr_t)st->D & 31) == 0);
+    if (st->gather == shflbw::kGatherTma) std::memcpy(p.tmap_b, st->tmap_b, sizeof p.tmap_b);
+    p.num_items = st->num_items; p.tiles_n = st->tiles_n;
+    p.div_tiles = shflbw::make_fast_div(st->tiles_n); p.div_bp = p.div_wo = shflbw::make_fast_div(1);
+    // Tile-major item order: concurrent CTAs gather from the same few token tiles of B (SHFLBW_ITEM_ORDER=0|1
+    // forces block-major / tile-major; tuning aid).
+    p.num_blocks = st->num_row_blocks; p.div_blocks = shflbw::make_fast_div(st->num_row_blocks);
+    p.tile_major = 1;
+    if (const char* e = getenv("SHFLBW_ITEM_ORDER")) p.tile_major = atoi(e) != 0;
+#if defined(SHFLBW_ABLATE) || defined(SHFLBW_COUNTERS)
+    if (const char* e = getenv("SHFLBW_ABLATE")) p.ablate = atoi(e);
+    if (const char* e = getenv("SHFLBW_TRACE_PTR")) p.trace = (unsigned long long*)strtoull(e, nullptr, 0);
+#endif
+    CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
+    CK(cudaGetLastError());
+    return SHFLBW_OK;
+}
+
+int shflbw_spmm_exec(const shflbw_spmm_state_t* st, void* stream) {
     if (!st || !st->init_success) return SHFLBW_ERR_INVALID_ARG;
     cudaStream_t s = (cudaStream_t)stream;
     if (st->kernel == SHFLBW_KERNEL_SIMT) {
         shflbw::simt_spmm<<<dim3(st->grid_x, st->grid_y), st->block_x, 0, s>>>(
             st->blk_ptr, st->blk_idx, (const __half*)st->blk_val, st->perm, (const __half*)st->B,
             (const __half*)st->C, (__half*)st->D, st->M, st->N, st->V, st->alpha, st->beta);
-    } else {
-        // The state is a POD and may have been copied: re-derive the function pointer from the
-        // recorded configuration (the shared-memory attribute was set at init).
-        PanelChoice ch;
-        const bool wide = st->variant == 2;
-        const bool found =
-            bias ? st->variant == 1 ? lookup<shflbw::kPanelSpmmRows, true>(st->V, st->tokens_per_cta, &ch, st->gather)
-                                    : lookup<shflbw::kPanelSpmm, true>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync, wide)
-                 : st->variant == 1 ? lookup<shflbw::kPanelSpmmRows>(st->V, st->tokens_per_cta, &ch, st->gather)
-                                    : lookup<shflbw::kPanelSpmm>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync, wide);
-        if (!found) return SHFLBW_ERR_INVALID_ARG;
-        shflbw::PanelParams p{};
-        p.blk_ptr = st->blk_ptr; p.blk_idx = st->blk_idx; p.blk_val = (const __half*)st->blk_val;
-        p.perm = st->perm; p.status_word = st->status_word; p.alpha = st->alpha; p.beta = st->beta;
-        p.wait_limit = g_wait_limit; p.inject_from = g_inject_from; p.idx_limit = (unsigned)(st->K - 1);
-        p.B = (const __half*)st->B; p.C = (const __half*)st->C; p.D = (__half*)st->D; p.N = st->N;
-        if (bias) { p.C = (const __half*)bias; p.beta = 1.f; }
-        p.wide_stores = (st->N % 16 == 0) && (((uintptr_t)st->D & 31) == 0);
-        if (ch.gather != st->gather) return SHFLBW_ERR_INVALID_ARG;
-        if (st->gather == shflbw::kGatherTma) std::memcpy(p.tmap_b, st->tmap_b, sizeof p.tmap_b);
-        p.num_items = st->num_items; p.tiles_n = st->tiles_n;
-        p.div_tiles = shflbw::make_fast_div(st->tiles_n); p.div_bp = p.div_wo = shflbw::make_fast_div(1);
-        // Tile-major item order: concurrent CTAs gather from the same few token tiles of B (SHFLBW_ITEM_ORDER=0|1
-        // forces block-major / tile-major; tuning aid).
-        p.num_blocks = st->num_row_blocks; p.div_blocks = shflbw::make_fast_div(st->num_row_blocks);
-        p.tile_major = 1;
-        if (const char* e = getenv("SHFLBW_ITEM_ORDER")) p.tile_major = atoi(e) != 0;
-#if defined(SHFLBW_ABLATE) || defined(SHFLBW_COUNTERS)
-        if (const char* e = getenv("SHFLBW_ABLATE")) p.ablate = atoi(e);
-        if (const char* e = getenv("SHFLBW_TRACE_PTR")) p.trace = (unsigned long long*)strtoull(e, nullptr, 0);
-#endif
-        if (bias) { const int rc = allow_smem(ch.fn, ch.smem); if (rc != SHFLBW_OK) return rc; }   // (init allowed the kernel without)
-        CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
+        CK(cudaGetLastError());
+        return SHFLBW_OK;
     }
-    CK(cudaGetLastError());
-    return SHFLBW_OK;
+    PanelChoice ch;
+    const int rc = spmm_panel(st, false, &ch);
+    return rc != SHFLBW_OK ? rc : launch_spmm_panel(st, ch, nullptr, s);
 }
-
-int shflbw_spmm_exec(const shflbw_spmm_state_t* st, void* stream) { return spmm_exec_impl(st, nullptr, stream); }
 
 int shflbw_linear_exec(const shflbw_matrix_t* m, int tokens, const void* x, const void* bias, void* xt, int N, void* out,
                        void* stream) {
     if (!m || !xt || !out || N <= 0 || tokens > N || (x && tokens <= 0)) return SHFLBW_ERR_INVALID_ARG;
     if (((uintptr_t)x | (uintptr_t)bias) & 1) return SHFLBW_ERR_UNSUPPORTED;
     shflbw_spmm_state_t st;
-    const int rc = shflbw_spmm_init(m, N, xt, 1.f, nullptr, 0.f, out, SHFLBW_KERNEL_AUTO, &st);   // (asks for 16-byte aligned xt, out and N % 8)
+    int rc = shflbw_spmm_init(m, N, xt, 1.f, nullptr, 0.f, out, SHFLBW_KERNEL_AUTO, &st);   // (asks for 16-byte aligned xt, out and N % 8)
     if (rc != SHFLBW_OK) return rc;
+    PanelChoice ch;                                          // all set-up comes before the first launch
+    if ((rc = spmm_panel(&st, bias != nullptr, &ch)) != SHFLBW_OK) return rc;
     if (x) {
         const long long tiles = (long long)((m->ncol + 63) / 64) * ((N + 63) / 64);   // < 2^31: ncol * N < 2^40 or refused above
         if (tiles >= (1ll << 31)) return SHFLBW_ERR_UNSUPPORTED;
         CK(launch(shflbw::transpose_tokens, dim3((unsigned)tiles), dim3(256), 0, (cudaStream_t)stream, (const __half*)x, (__half*)xt, tokens,
                   m->ncol, N, (int)(m->ncol % 8 == 0 && ((uintptr_t)x & 15) == 0)));
     }
-    return spmm_exec_impl(&st, bias, stream);
+    return launch_spmm_panel(&st, ch, bias, (cudaStream_t)stream);
 }
 
 int shflbw_spmm_launches_per_exec(const shflbw_spmm_state_t* st) { return st && st->init_success ? 1 : 0; }
@@ -816,6 +834,10 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
                            : st->variant == 1      ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch)
                                                    : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync, st->variant == 2);
     if (!ok_kernel) return SHFLBW_ERR_INVALID_ARG;
+    if (panel_bias) {                                       // (init allowed the kernel without; before anything is launched)
+        const int rc = allow_smem(ch.fn, ch.smem);
+        if (rc != SHFLBW_OK) return rc;
+    }
     // 1. NHWC -> channel-major, batch-innermost staging with a zero halo (chained layers get
     //    their input in that layout already).
     //    A strided 1x1 filter visits 1 / stride^2 of the pixels: only those are staged, as an image of the
@@ -857,11 +879,7 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     if (const char* e = getenv("SHFLBW_ABLATE")) p.ablate = atoi(e);
     if (const char* e = getenv("SHFLBW_TRACE_PTR")) p.trace = (unsigned long long*)strtoull(e, nullptr, 0);
 #endif
-    if (panel_bias) {
-        p.C = (const __half*)bias;
-        const int rc = allow_smem(ch.fn, ch.smem);
-        if (rc != SHFLBW_OK) return rc;
-    }
+    if (panel_bias) p.C = (const __half*)bias;
     CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
     // 3. back to NHWC in logical channel order.
     if (planes) {
