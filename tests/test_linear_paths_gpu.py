@@ -29,6 +29,8 @@ def _plain(m, x2, bias):
     (64, 203, 300, 1, None, 256), (16, 77, 130, None, None, None),
     (64, 200, 256 * 40 + 5, 0, 16, 256),             # sixteen epilogue warps
     (64, 640, 256 * 40 + 13, 1, None, 256),          # TMA gather
+    (64, 640, 256 * 40 + 3, 1, None, 256),           # and N % 16 == 8: 16-byte stores (32-byte ones above)
+    (128, 320, 300, 1, None, 256), (128, 320, 120, 1, None, 128),
 ])
 @pytest.mark.parametrize("bias", [True, False])
 def test_forward_equals_operator_plus_bias_bit_for_bit(V, K, tokens, swap, ew, t, bias):
