@@ -33,18 +33,20 @@ def _ptr(x) -> Optional[int]:
     if x is None:
         return None
     try:
-        return x.data_ptr()
+        x = x.data_ptr()
     except AttributeError:
-        return int(x)
+        pass
+    return int(x)
 
 
 def _stream_ptr(stream) -> Optional[int]:
     if stream is None:
         return None
     try:
-        return stream.cuda_stream
+        stream = stream.cuda_stream
     except AttributeError:
-        return int(stream)
+        pass
+    return int(stream)
 
 
 def uniform_half(stream_seed: int, n: int, offset: int = 0) -> np.ndarray:
