@@ -30,6 +30,7 @@ long long g_wait_limit = shflbw::kWaitLimitCycles;
 int g_inject_from = -1;
 #ifdef SHFLBW_FAULT_INJECT
 int g_set_ups_left = -1;             // test builds: this many more shared-memory opt-ins succeed (< 0: all)
+int g_export_pixels = 0;             // test builds: most pixels per chain-export launch (0: the product's limit)
 #endif
 
 bool cuda_ok(cudaError_t e, const char* what) {
@@ -693,26 +694,43 @@ static size_t unperm_smem_bytes(int F) {
     return (size_t)F * 2 * (1 + shflbw::kUnpermThreads / shflbw::unperm_threads_per_pos(F));
 }
 
-// Chain buffer -> NHWC (see the kernel).  Two to eight 64-token steps per block where that leaves several blocks
-// per SM, so that a block's scan of the permutation and its start-up are shared.
+// Blocks per 64 channels of a chain export: two to eight 64-token steps per block where that leaves several
+// blocks per SM, so that a block's scan of the permutation and its start-up are shared.
+static long long export_blocks(long long tiles, int F) {
+    const int fb = (F + 63) / 64;
+    long long gx = (148 * 16 + fb - 1) / fb;
+    if (gx < (tiles + 7) / 8) gx = (tiles + 7) / 8;
+    return gx < tiles ? gx : tiles;
+}
+
+// Chain buffer -> NHWC (see the kernel).
 static cudaError_t launch_export(const void* planes, void* out, const int* perm, int Bn, int Bp, int H, int W,
                                          int Hp, int Wp, int ph, int pw, int F, cudaStream_t s) {
-    const int fb = (F + 63) / 64;
-    const int per = (1 << 30) / Bp > 0 ? (1 << 30) / Bp : 1;            // pixels per launch: the kernel counts its tokens in 31 bits
+    int per = (1 << 30) / Bp > 0 ? (1 << 30) / Bp : 1;                  // pixels per launch: the kernel counts its tokens in 31 bits
+#ifdef SHFLBW_FAULT_INJECT
+    if (g_export_pixels > 0) per = g_export_pixels;
+#endif
     const long long npix = (long long)H * W;
     for (long long pix0 = 0; pix0 < npix; pix0 += per) {
         const int n = (int)(npix - pix0 < per ? npix - pix0 : per);
         const long long tiles = ((long long)n * Bp + 63) / 64;
-        long long gx = (148 * 16 + fb - 1) / fb;
-        if (gx < (tiles + 7) / 8) gx = (tiles + 7) / 8;
-        if (gx > tiles) gx = tiles;
-        const cudaError_t e = launch(shflbw::export_planes_nhwc, dim3((unsigned)gx, (unsigned)fb), dim3(256), 0, s, (const __half*)planes,
+        const cudaError_t e = launch(shflbw::export_planes_nhwc, dim3((unsigned)export_blocks(tiles, F), (unsigned)((F + 63) / 64)), dim3(256), 0, s, (const __half*)planes,
                                      (__half*)out, perm, Bn, Bp, (int)pix0, n, (int)npix, W, Wp, ph, pw, (size_t)Hp * Wp * Bp, F,
                                      shflbw::make_fast_div(Bp), shflbw::make_fast_div(W));
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
+
+#ifdef SHFLBW_FAULT_INJECT
+// Chain exports issued after this call cover at most `n` pixels per launch (n <= 0: the product's limit).
+int shflbw_debug_set_export_pixels(int n) { g_export_pixels = n; return SHFLBW_OK; }
+// The most 64-token steps that a block of a chain export of `tokens` (pixels * padded batch) and F channels takes.
+int shflbw_debug_export_steps(long long tokens, int F) {
+    const long long tiles = (tokens + 63) / 64, gx = export_blocks(tiles, F);
+    return (int)((tiles + gx - 1) / gx);
+}
+#endif
 
 // Launch plan of one NHWC SpConv call, without its scratch pointers: kernel choice, grid, and
 // the scratch each side needs.  Two plans exist.

@@ -2,6 +2,8 @@
 inverse filter permutation, the bias that the last pass adds, and the staging of a strided 1x1 filter's
 pixels.  The passes only move fp16 values and add one, so everything but the strided convolution is
 compared bit for bit."""
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
@@ -10,17 +12,31 @@ import oracle_api as oa
 import shflbw_sparse_nn_b200 as sb
 from conftest import assert_close_fp16
 from gpu_util import dev, host, run_spconv
+from shflbw_sparse_nn_b200 import _cabi
+from shflbw_sparse_nn_b200.build import build_fault_inject_library
 from shflbw_sparse_nn_b200.nn import ShflBWConv2d
 
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("Bn,H,W,F,R,permute", [
-    (1, 1, 1, 32, 1, True), (3, 5, 7, 96, 3, True), (8, 9, 4, 64, 1, False), (13, 6, 6, 160, 5, True),
-    (40, 7, 7, 2048, 1, True),          # several 64-token steps per block
-    (256, 14, 14, 128, 3, True),
+@pytest.fixture
+def flib():
+    """The test build, which tells how an export is split and can split it finer."""
+    lib = _cabi.load_library(build_fault_inject_library())
+    lib.shflbw_debug_export_steps.argtypes, lib.shflbw_debug_export_steps.restype = [C.c_longlong, C.c_int], C.c_int
+    lib.shflbw_debug_set_export_pixels.argtypes, lib.shflbw_debug_set_export_pixels.restype = [C.c_int], C.c_int
+    yield lib
+    lib.shflbw_debug_set_export_pixels(0)
+
+
+@pytest.mark.parametrize("Bn,H,W,F,R,permute,steps", [
+    (1, 1, 1, 32, 1, True, 1), (3, 5, 7, 96, 3, True, 1), (8, 9, 4, 64, 1, False, 1), (13, 6, 6, 160, 5, True, 1),
+    (40, 7, 7, 2048, 1, True, 1), (256, 14, 14, 128, 3, True, 1),
+    (250, 7, 7, 2048, 1, True, 3), (117, 7, 7, 1984, 3, True, 2),       # several 64-token steps per block, the last round ragged
+    (61, 9, 13, 4096, 1, False, 4),
 ])
-def test_chain_export_is_the_transpose_of_the_planes(Bn, H, W, F, R, permute):
+def test_chain_export_is_the_transpose_of_the_planes(flib, Bn, H, W, F, R, permute, steps):
+    assert flib.shflbw_debug_export_steps(H * W * (-(-Bn // 8) * 8), F) == steps
     f = sb.BlockwiseSpFilter().init_random(F, 1, 1, 8, 32, 1, 0.5, permute, 3, values="uniform")
     f.transform_and_sync_device()
     Bp = -(-Bn // 8) * 8
@@ -32,6 +48,20 @@ def test_chain_export_is_the_transpose_of_the_planes(Bn, H, W, F, R, permute):
     core = buf[:, R // 2:R // 2 + H, R // 2:R // 2 + W, :Bn].transpose(3, 1, 2, 0)
     want[..., f.row_permute_ids if permute else np.arange(F)] = core
     assert np.array_equal(host(y).view(np.uint16), want.view(np.uint16))
+
+
+@pytest.mark.parametrize("pixels", [1, 5, 34, 35])
+def test_chain_export_in_several_launches(flib, pixels):
+    Bn, H, W, F, R = 13, 5, 7, 200, 3
+    buf = sb.uniform_half(4, F * (H + R - 1) * (W + R - 1) * 16).reshape(F, H + R - 1, W + R - 1, 16)
+    y = torch.full((Bn, H, W, F), float("nan"), dtype=torch.float16, device="cuda")
+    planes = dev(buf)
+    flib.shflbw_debug_set_export_pixels(pixels)
+    assert flib.shflbw_chain_export_nhwc(planes.data_ptr(), Bn, H, W, F, R, R, None, y.data_ptr(),
+                                         torch.cuda.current_stream().cuda_stream) == _cabi.OK
+    torch.cuda.synchronize()
+    want = buf[:, 1:1 + H, 1:1 + W, :Bn].transpose(3, 1, 2, 0)
+    assert np.array_equal(host(y).view(np.uint16), np.ascontiguousarray(want).view(np.uint16))
 
 
 @pytest.mark.parametrize("V,F,C,R,permute", [
