@@ -68,3 +68,22 @@ def test_inputs_that_are_not_contiguous_or_aligned():
         lin(x[:0])
     torch.cuda.synchronize()
     m.device_status()
+
+
+@pytest.mark.parametrize("tokens", [512, 4099])
+def test_input_in_the_operands_order_is_copied_once(tokens):
+    """The result of one layer is feature-major memory: as the input of the next it needs no transposed copy."""
+    M, K = 256, 1024
+    m = sb.BlockwiseSpMatrix().init_random(M, K, 64, 1, 0.1, True, 19, values="uniform")
+    lin = ShflBWLinear(m, None).cuda()
+    padded = -(-tokens // 8) * 8
+    x = (torch.rand(K, padded, device="cuda") * 2 - 1).half()[:, :tokens].t()
+    lin(x)                                                # uploads the weights
+    want = _plain(m, x, None)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    y = lin(x)
+    peak = torch.cuda.max_memory_allocated() - before
+    assert torch.equal(y, want) and peak <= (K + M) * padded * 2 + 4096        # the operand, the result, rounding
+    m.device_status()
