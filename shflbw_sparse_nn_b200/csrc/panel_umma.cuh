@@ -155,7 +155,7 @@ constexpr int kGatherCpAsync = 0, kGatherTma = 1, kGatherCpAsyncArrive = 2;
 // latency-bound: sixteen warps, as two sets on alternate items, keep four such chains per
 // scheduler in flight instead of two.
 template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int LAG_ = 1, int GATHER_ = kGatherCpAsync,
-          int EW_ = 8>
+          int EW_ = 8, bool ADDEND_ = false>
 struct PanelCfg {
     static constexpr int EW = EW_;
     static_assert(EW == 8 || EW == 16, "epilogue warps");
@@ -201,9 +201,11 @@ struct PanelCfg {
     // rows / filters through 2 KB so that its global stores are 16 bytes per lane and 64-byte
     // runs.  With rows in lanes the stores go straight from registers.
     static constexpr int OUT_BYTES = (MODE == kPanelSpmmRows || MODE == kPanelConvChainRows) ? 0 : EW * 2048;
-    // With sixteen epilogue warps the addend of an item (C, or a chained layer's residual) is copied to
-    // shared memory an item ahead: each lane's own 16-byte pieces, 64 rows x 32 tokens per warp.
-    static constexpr int RES_BYTES = EW == 16 ? EW * 4096 : 0;
+    // Sixteen epilogue warps, instances built with ADDEND: the addend of an item (C, or a chained layer's
+    // residual) is copied to shared memory an item ahead: each lane's own 16-byte pieces, 64 rows x 32
+    // tokens per warp.  Without, the ring has that room.
+    static_assert(!ADDEND_ || EW == 16, "addend slots: sixteen epilogue warps");
+    static constexpr int RES_BYTES = ADDEND_ ? EW * 4096 : 0;
     static constexpr int BAR_BYTES = (STAGES * 2 + 12) * 8;  // mbarriers (ring, up to 4 + 4 accumulator, drain) + tmem slot + abort flag
     static constexpr int TAB_BYTES = 512 * 8;               // per-CTA item table (kPanelMaxItemsPerCta entries)
     static constexpr int IDX_AHEAD = LAG + 1;              // a group fetches row ids this many of its stages ahead
@@ -261,10 +263,10 @@ constexpr int kPanelMaxItemsPerCta = 512;  // capacity of the per-CTA item table
 // NHWC in logical order).  Kernels of their own: as a branch of the others it made small products 1-2 %
 // slower (256-item launches of 5-9 us, where every instruction is fetched for the first time).
 template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int LAG_ = 1, int GATHER_ = kGatherCpAsync,
-          int EW_ = 8, bool BIAS = false>
-__global__ void __launch_bounds__(PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, LAG_, GATHER_, EW_>::THREADS, 1)
+          int EW_ = 8, bool BIAS = false, bool ADDEND = false>
+__global__ void __launch_bounds__(PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, LAG_, GATHER_, EW_, ADDEND>::THREADS, 1)
 panel_umma_kernel(const __grid_constant__ PanelParams p) {
-    using Cfg = PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, LAG_, GATHER_, EW_>;
+    using Cfg = PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, LAG_, GATHER_, EW_, ADDEND>;
     constexpr int EW = Cfg::EW;                                             // epilogue warps 0..EW-1, MMA warp EW, producers after it
     constexpr bool SWAP = Cfg::SWAP;                                        // rows in TMEM lanes
     constexpr bool CONV = MODE == kPanelConv || MODE == kPanelConvChain || MODE == kPanelConvChainRows;  // implicit-GEMM gather
@@ -1133,7 +1135,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 #pragma unroll
                 for (int i = 0; i < 4; ++i) row_off[i] = __shfl_sync(0xffffffffu, mine, i * 8 + (lane >> 2));
             }
-            const bool use_c = MODE == kPanelSpmm && p.beta != 0.0f && p.C != nullptr;
+            const bool use_c = MODE == kPanelSpmm && (EW == 8 || BIAS || Cfg::RES_BYTES > 0) && p.beta != 0.0f && p.C != nullptr;
             if constexpr (ROWS_OUT) {
             // SpMM: thread = token, accumulator columns = the block's output rows.  For a fixed
             // row a warp's 32 tokens are only 64 contiguous bytes of D, and storing them straight
@@ -1185,8 +1187,9 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             // chunk's two chunks ahead.
             constexpr int NCH = COLS / CW;
             constexpr bool RES_AHEAD = Cfg::RES_BYTES > 0;
+            constexpr bool IN_REGS = EW == 8;     // (sixteen warps without ADDEND add nothing but a bias)
             const bool ahead = RES_AHEAD && ((use_c && !BIAS) || (MODE == kPanelConvChain && p.res != nullptr));
-            const bool add_res = MODE == kPanelConvChain && p.res != nullptr;
+            const bool add_res = (IN_REGS || RES_AHEAD) && MODE == kPanelConvChain && p.res != nullptr;
             const bool need_add = ok_g && (use_c || add_res);
             auto addend_at = [&](int blk_, uint32_t goff_, int cc, int i) -> const __half* {
                 const int m = mbase + cc + slot_row(i);
@@ -1198,7 +1201,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 const uint32_t rr = (uint32_t)(p.res_map ? __ldg(p.res_map + blk_ * V + m) : blk_ * V + m) * (uint32_t)p.out_plane;
                 return p.res + (size_t)rr + (size_t)goff_;
             };
-            uint4 addend[NCH > 1 && !RES_AHEAD ? 2 : 1][4];
+            uint4 addend[NCH > 1 && IN_REGS ? 2 : 1][4];
             auto fetch_addend = [&](int blk_, uint32_t goff_, int cc, uint4 (&dst)[4]) {
 #pragma unroll
                 for (int i = 0; i < NSLOT; ++i) {
@@ -1233,9 +1236,9 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                         goff_next = group_offset(item_tile(item_next) * T, ok_next);
                     }
                 }
-            } else if (need_add) {
+            } else if (IN_REGS && need_add) {
                 fetch_addend(blk, goff, 0, addend[0]);
-                if constexpr (NCH > 1) fetch_addend(blk, goff, CW, addend[1]);
+                if constexpr (NCH > 1 && IN_REGS) fetch_addend(blk, goff, CW, addend[1]);
             }
             if (!wait_accumulator()) break;
 #pragma unroll
@@ -1284,10 +1287,9 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                         sm100::cp_async_wait<NCH - 1>();     // this chunk's copies (each lane reads only its own)
 #pragma unroll
                         for (int i = 0; i < NSLOT; ++i) addend[0][i] = *(const uint4*)(my_res + (ch * 4 + i) * 512);
-                    } else if (BIAS && need_add) {
-                        fetch_addend(blk, goff, cc, addend[0]);
                     }
                 }
+                if constexpr (BIAS && !IN_REGS) { if (need_add) fetch_addend(blk, goff, cc, addend[0]); }
                 if (!(ablate & 512)) {
 #pragma unroll
                     for (int k = 0; k < NSLOT / 2; ++k) {
@@ -1305,14 +1307,14 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                             const size_t off = (size_t)roff[i] + (size_t)goff;
                             if (use_c) {
                                 __half* h = (__half*)&v;
-                                const __half* cadd = (const __half*)&addend[NCH > 1 && !RES_AHEAD ? (ch & 1) : 0][i];
+                                const __half* cadd = (const __half*)&addend[NCH > 1 && IN_REGS ? (ch & 1) : 0][i];
 #pragma unroll
                                 for (int e = 0; e < 8; ++e) h[e] = __hfma(h[e], alpha1, __hmul(cadd[e], beta1));
                             }
                             if constexpr (MODE == kPanelConvChain) {   // out = relu(alpha * conv + residual), fp16
                                 __half2* h = (__half2*)&v;
                                 if (add_res) {
-                                    const __half2* rh = (const __half2*)&addend[NCH > 1 && !RES_AHEAD ? (ch & 1) : 0][i];
+                                    const __half2* rh = (const __half2*)&addend[NCH > 1 && IN_REGS ? (ch & 1) : 0][i];
 #pragma unroll
                                     for (int e = 0; e < 4; ++e) h[e] = __hadd2(h[e], rh[e]);
                                 }
@@ -1327,7 +1329,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     }
                 }
                 if constexpr (RES_AHEAD) { if (ahead) copy_addend(blk_next, goff_next, ok_next, ch); }
-                else if constexpr (NCH > 2) { if (need_add && ch + 2 < NCH) fetch_addend(blk, goff, cc + 2 * CW, addend[ch & 1]); }
+                else if constexpr (NCH > 2 && IN_REGS) { if (need_add && ch + 2 < NCH) fetch_addend(blk, goff, cc + 2 * CW, addend[ch & 1]); }
                 __syncwarp();
             }
             } else {

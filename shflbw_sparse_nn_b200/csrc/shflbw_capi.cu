@@ -113,10 +113,10 @@ using PanelKernel = void (*)(const shflbw::PanelParams);
 struct PanelChoice { PanelKernel fn; size_t smem; int tokens; int stages; int pw; int threads; int variant; int gather; };
 
 template <int V, int TM, int KS, int STAGES, int PW, int MODE, int GROUPS = 2, int LAG = 1, int GATHER = shflbw::kGatherCpAsync,
-          int EW = 8, bool BIAS = false>
+          int EW = 8, bool BIAS = false, bool ADDEND = false>
 PanelChoice choice() {
-    using Cfg = shflbw::PanelCfg<V, TM, KS, STAGES, PW, MODE, GROUPS, LAG, GATHER, EW>;
-    return {shflbw::panel_umma_kernel<V, TM, KS, STAGES, PW, MODE, GROUPS, LAG, GATHER, EW, BIAS>, (size_t)Cfg::SMEM_BYTES, Cfg::T,
+    using Cfg = shflbw::PanelCfg<V, TM, KS, STAGES, PW, MODE, GROUPS, LAG, GATHER, EW, ADDEND>;
+    return {shflbw::panel_umma_kernel<V, TM, KS, STAGES, PW, MODE, GROUPS, LAG, GATHER, EW, BIAS, ADDEND>, (size_t)Cfg::SMEM_BYTES, Cfg::T,
             STAGES, PW, Cfg::THREADS, 0, GATHER};
 }
 
@@ -198,15 +198,17 @@ bool tuned_shape(PanelChoice* out) {
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
 template <int MODE, bool BIAS = false>
-bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsync, bool wide_epilogue = false) {
+bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsync, int wide_ring = 0) {
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         // Shallow items (at most 64 non-zero columns): sixteen epilogue warps and three producer
         // warps, each a group of its own (20 warps: 96 registers per thread); stages of 32 columns,
         // six of them beside the 32 KB of epilogue tiles and the 64 KB of addend slots, so that up to
         // six items' inputs are in flight from HBM (five: 37.5 -> 40.5 us on 14x14x256 -> 1024 at batch
-        // 256, the rest equal).  Built for 64-row blocks.
-        if (wide_epilogue && tile == 256 && V == 64) {
-            *out = choice<64, 2, 32, 6, 3, MODE, 3, 1, shflbw::kGatherCpAsync, 16, BIAS>();
+        // 256, the rest equal); eight in the instance without the slots.  Built for 64-row blocks.
+        // wide_ring: 6 or 8 stages, 0 for the regular kernels.
+        if (wide_ring && tile == 256 && V == 64) {
+            *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, 1, shflbw::kGatherCpAsync, 16, BIAS, false>()
+                                  : choice<64, 2, 32, 6, 3, MODE, 3, 1, shflbw::kGatherCpAsync, 16, BIAS, true>();
             return true;
         }
     }
@@ -288,7 +290,7 @@ int allow_smem(PanelKernel fn, size_t bytes) {
 // the default; 128 is used when the dense extent is too small to give every SM a few items.
 // SHFLBW_TILE=128|256 overrides (tuning aid).
 template <int MODE>
-int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols, PanelChoice* out) {
+int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols, PanelChoice* out, bool addend = false) {
     // Token tile: a persistent CTA works through ceil(items / SMs) items in turn; an item of
     // the 128-token tile was measured at ~2/3 of the time of a 256-token item (half the
     // gathered bytes, the same number of pipeline stages).
@@ -326,13 +328,23 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
     // then all epilogue; with two stages the four producers of that kernel were measured slower
     // than the eight of the regular one) and several items per SM: sixteen epilogue warps.  SHFLBW_EPILOGUE_WARPS=8|16 forces the choice
     // (tuning aid).
+    // Their ring: eight stages where nothing is added and a block takes two stages, which a ring of six holds for
+    // three items only (14x14x256 -> 1024, batch 256, no residual: 35.2 us with six, 34.3 with eight); blocks of one
+    // stage are as fast with six (28x28x128 -> 512: 48.3, with eight 49.2).
     bool wide = false;
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         wide = !swapped && tile == 256 && V == 64 && padded_cols <= 64ll * row_blocks && items256 >= 4ll * sms;
         if (const char* e = getenv("SHFLBW_EPILOGUE_WARPS")) wide = !swapped && tile == 256 && V == 64 && atoi(e) == 16;
     }
-    if (!swapped && !lookup<MODE>(V, tile, out, shflbw::kGatherCpAsync, wide)) return SHFLBW_ERR_UNSUPPORTED;
+    const int wide_ring = !wide ? 0 : !addend && padded_cols > 32ll * row_blocks ? 8 : 6;
+    if (!swapped && !lookup<MODE>(V, tile, out, shflbw::kGatherCpAsync, wide_ring)) return SHFLBW_ERR_UNSUPPORTED;
     out->variant = swapped ? 1 : wide ? 2 : 0;
+    if (wide_ring == 8) {                    // a residual may be bound to the state later on
+        PanelChoice with_addend;
+        if (!lookup<MODE>(V, tile, &with_addend, shflbw::kGatherCpAsync, 6)) return SHFLBW_ERR_UNSUPPORTED;
+        const int rc = allow_smem(with_addend.fn, with_addend.smem);
+        if (rc != SHFLBW_OK) return rc;
+    }
     return allow_smem(out->fn, out->smem);
 }
 
@@ -494,7 +506,7 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
         out->tokens_per_cta = 128; out->stages = 0; out->shared_mem_size = 0;
     } else {
         PanelChoice ch;
-        int rc = pick_panel<shflbw::kPanelSpmm>(m->brow, N, out->num_row_blocks, m->kptr.empty() ? 0 : m->kptr.back(), &ch);
+        int rc = pick_panel<shflbw::kPanelSpmm>(m->brow, N, out->num_row_blocks, m->kptr.empty() ? 0 : m->kptr.back(), &ch, beta != 0.f);
         if (rc != SHFLBW_OK) return rc;
         out->kernel = SHFLBW_KERNEL_TCGEN05;
         out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
@@ -516,12 +528,12 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
 // been copied: the function pointer is re-derived from the recorded configuration.  bias: the instance that
 // adds a bias (init allowed the one without).
 static int spmm_panel(const shflbw_spmm_state_t* st, bool bias, PanelChoice* ch) {
-    const bool wide = st->variant == 2;
+    const int wide_ring = st->variant != 2 ? 0 : st->beta != 0.f ? 6 : st->stages;   // (an addend needs its slots)
     const bool found =
         bias ? st->variant == 1 ? lookup<shflbw::kPanelSpmmRows, true>(st->V, st->tokens_per_cta, ch, st->gather)
-                                : lookup<shflbw::kPanelSpmm, true>(st->V, st->tokens_per_cta, ch, shflbw::kGatherCpAsync, wide)
+                                : lookup<shflbw::kPanelSpmm, true>(st->V, st->tokens_per_cta, ch, shflbw::kGatherCpAsync, wide_ring)
              : st->variant == 1 ? lookup<shflbw::kPanelSpmmRows>(st->V, st->tokens_per_cta, ch, st->gather)
-                                : lookup<shflbw::kPanelSpmm>(st->V, st->tokens_per_cta, ch, shflbw::kGatherCpAsync, wide);
+                                : lookup<shflbw::kPanelSpmm>(st->V, st->tokens_per_cta, ch, shflbw::kGatherCpAsync, wide_ring);
     if (!found || ch->gather != st->gather) return SHFLBW_ERR_INVALID_ARG;
     return bias ? allow_smem(ch->fn, ch->smem) : SHFLBW_OK;
 }
@@ -850,7 +862,8 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     const bool ok_kernel = panel_bias            ? lookup<shflbw::kPanelConv, true>(st->V, st->tokens_per_cta, &ch)
                            : (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch)
                            : st->variant == 1      ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch)
-                                                   : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync, st->variant == 2);
+                                                   : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync,
+                                                                                      st->variant != 2 ? 0 : st->residual ? 6 : st->stages);
     if (!ok_kernel) return SHFLBW_ERR_INVALID_ARG;
     if (panel_bias) {                                       // (init allowed the kernel without; before anything is launched)
         const int rc = allow_smem(ch.fn, ch.smem);
@@ -1067,9 +1080,10 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     // columns per block (7x7x512 -> 2048 with residual, batch 256: 38 -> 31 us); without a residual the
     // limit is one stage (pick_panel).
     PanelChoice ch;
-    const bool wide = st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
-                      (f->kptr.empty() ? 0 : f->kptr.back()) <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count() &&
-                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, shflbw::kGatherCpAsync, true);
+    const bool wide = (st->variant == 2 ||
+                       (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
+                        (f->kptr.empty() ? 0 : f->kptr.back()) <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count())) &&
+                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, shflbw::kGatherCpAsync, 6);
     if (wide) {
         const int rc = allow_smem(ch.fn, ch.smem);
         if (rc != SHFLBW_OK) return rc;

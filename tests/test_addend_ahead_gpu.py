@@ -83,6 +83,50 @@ def test_refused_residual_leaves_the_state_as_it_was():
     assert op._state.variant == 2 and op._state.residual == out.data_ptr() and op._state.residual_map
 
 
+@pytest.mark.parametrize("Cc,padded_cols,ring", [(64, 112, 6), (80, 128, 6), (88, 144, 8), (200, 272, 8)])
+def test_ring_of_the_sixteen_warp_kernel(Cc, padded_cols, ring):
+    """Eight stages where nothing is added and a block takes two of them, six with slots for an addend
+    otherwise; a residual bound later moves a layer to the six.  Same bits as the eight-warp kernel."""
+    F, Bn, H = 256, 40, 33
+    f = sb.BlockwiseSpFilter().init_random(F, 1, 1, Cc, 64, 1, 0.3, True, 5, values="uniform")
+    f.transform_and_sync_device()
+    assert sum(-(-np.diff(f.indptr) // 16) * 16) == padded_cols        # of four blocks
+    x = dev(sb.uniform_half(6, sb.chain_buffer_elems(Cc, H, H, Bn, 1, 1)))
+    n_out = sb.chain_buffer_elems(F, H, H, Bn, 1, 1)
+    res = dev(sb.uniform_half(7, n_out))
+    got = {}
+    for ew in (8, 16):
+        out = torch.zeros(n_out, dtype=torch.float16, device="cuda")
+        with operand_swap(0), epilogue_warps(ew), tile(256):
+            op = sb.SpconvChainOp().initialize(f, Bn, H, H, 1, x, out, 1, 1, relu=True)
+        if ew == 16:
+            assert (op._state.variant, op._state.stages) == (2, ring)
+        op(torch.cuda.current_stream())
+        plain = out.clone()
+        op.set_residual(res)
+        if ew == 16:
+            assert (op._state.variant, op._state.stages) == (2, 6)
+        op(torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        f.device_status()
+        got[ew] = host(plain).view(np.uint16), host(out).view(np.uint16)
+    assert np.array_equal(got[8][0], got[16][0]) and np.array_equal(got[8][1], got[16][1])
+    assert not np.array_equal(got[16][0], got[16][1])
+
+
+@pytest.mark.parametrize("N", [256 * 37, 256 * 80 + 24])
+def test_spmm_without_an_addend_matches_the_eight_warp_kernel(N):
+    m = sb.BlockwiseSpMatrix().init_random(512, 200, 64, 1, 0.2, True, 11, values="uniform")
+    B = sb.uniform_half(12, m.ncol * N).reshape(m.ncol, N)
+    got = []
+    for ew, stages in ((8, None), (16, 8)):
+        with operand_swap(0), epilogue_warps(ew):
+            y, op = run_spmm(m, N, B, alpha=0.5, tokens=256)
+        assert op._state.variant == (2 if ew == 16 else 0) and stages in (None, op._state.stages)
+        got.append(y.view(np.uint16))
+    assert np.array_equal(got[0], got[1])
+
+
 @pytest.mark.parametrize("N", [256 * 37, 256 * 80 + 24])
 def test_spmm_beta_matches_the_eight_warp_kernel(N):
     m = sb.BlockwiseSpMatrix().init_random(512, 200, 64, 1, 0.2, True, 11, values="uniform")

@@ -27,7 +27,8 @@ def _plain(m, x2, bias):
     (64, 320, 1, None, None, None), (64, 320, 37, 1, None, 128), (64, 328, 65, 0, None, 128), (128, 320, 63, 1, None, 128),
     (32, 203, 8, None, None, None),                  # K % 8 != 0: 2-byte loads
     (64, 203, 300, 1, None, 256), (16, 77, 130, None, None, None),
-    (64, 200, 256 * 40 + 5, 0, 16, 256),             # sixteen epilogue warps
+    (64, 200, 256 * 40 + 5, 0, 16, 256),             # sixteen epilogue warps, ring of eight stages
+    (64, 64, 256 * 40 + 5, 0, 16, 256),              # of six
     (64, 640, 256 * 40 + 13, 1, None, 256),          # TMA gather
     (64, 640, 256 * 40 + 3, 1, None, 256),           # and N % 16 == 8: 16-byte stores (32-byte ones above)
     (128, 320, 300, 1, None, 256), (128, 320, 120, 1, None, 128),
