@@ -36,7 +36,7 @@ def _ptr(x) -> Optional[int]:
         x = x.data_ptr()
     except AttributeError:
         pass
-    return int(x)
+    return x if type(x) is int else int(x)
 
 
 def _stream_ptr(stream) -> Optional[int]:
@@ -46,7 +46,7 @@ def _stream_ptr(stream) -> Optional[int]:
         stream = stream.cuda_stream
     except AttributeError:
         pass
-    return int(stream)
+    return stream if type(stream) is int else int(stream)
 
 
 def uniform_half(stream_seed: int, n: int, offset: int = 0) -> np.ndarray:

@@ -63,8 +63,11 @@ def _fused_bias(bias, device: torch.device, n: int, align: int):
         return None, False
     if bias.device != device:
         bias = bias.to(device)
-    fused = bias.dtype == torch.float16 and bias.shape == (n,) and bias.is_contiguous() and _in_memory(bias) \
-        and bias.data_ptr() % align == 0 and not _carries_gradient(bias)
+    fused = bias.dtype == torch.float16 and bias.shape == (n,) and bias.is_contiguous() and not bias.is_neg() \
+        and not _carries_gradient(bias)
+    if fused:
+        address = bias.data_ptr()
+        fused = address != 0 and address % align == 0        # (0: as in _in_memory)
     return bias, fused
 
 
@@ -117,8 +120,8 @@ class ShflBWLinear(nn.Module):
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         _require_cuda_half(x, "ShflBWLinear")
-        lead = x.shape[:-1]
-        x2 = x.reshape(-1, self.in_features)
+        shape = x.shape
+        x2 = x if len(shape) == 2 and shape[1] == self.in_features else x.reshape(-1, self.in_features)
         tokens = x2.shape[0]
         padded = -(-tokens // 8) * 8
         # Tokens in consecutive memory (the view that a layer like this one returns) are in the operand's order
@@ -126,10 +129,13 @@ class ShflBWLinear(nn.Module):
         # 45 us; made contiguous and then transposed by the kernel, as every other order is, 110.  A ragged count
         # needs a fill and a slice as well, 5 us of host time, and gains from a few million values on (4095 tokens:
         # 78 us against 110).
-        by_torch = x2.stride(0) == 1 and not x2.is_contiguous() and (tokens == padded or x2.numel() >= 1 << 22)
-        if not by_torch:
-            x2 = x2.contiguous()
-            by_torch = tokens > 0 and not _in_memory(x2)     # the kernel cannot read it
+        by_torch = False
+        if not x2.is_contiguous():
+            by_torch = x2.stride(0) == 1 and (tokens == padded or x2.numel() >= 1 << 22)
+            if not by_torch:
+                x2 = x2.contiguous()
+        if tokens and not _in_memory(x2):                    # the kernel cannot read it
+            by_torch = True
         if by_torch and tokens != padded:
             xt = torch.zeros((self.in_features, padded), dtype=torch.float16, device=x.device)
         else:
@@ -139,7 +145,7 @@ class ShflBWLinear(nn.Module):
             x2 = None
         yt = self._run(x2, tokens, xt, padded)
         y = yt.as_strided((tokens, self.out_features), (1, padded))
-        return y if lead == (tokens,) else y.reshape(*lead, self.out_features)
+        return y if len(shape) == 2 and shape[0] == tokens else y.reshape(*shape[:-1], self.out_features)
 
     def dense_weight(self) -> torch.Tensor:
         """The pruned weights as a dense [out][in] fp16 tensor (rows in original order), for checks."""
