@@ -122,6 +122,7 @@ struct alignas(64) PanelParams {
     // chained SpConv: out[f][OHp][OWp][Bp] with the next layer's halo (origin at (oph, opw))
     int OWp, oph, opw, out_plane, relu;
     int wide_stores;         // SpMM, rows in lanes: output rows are 32-byte aligned (N % 16 == 0, D % 32 == 0)
+    int trigger_late;        // SpConv ending with this kernel (no permutation): lets its dependents in when its producers are done
     int out_logical;         // chained kernels: output plane of stored filter f is perm[f] (logical channel order) instead of f
     const __half* res;       // optional residual in the OUTPUT's geometry ([planes][OHp][OWp][Bp]) or nullptr
     const int* res_map;      // stored filter -> plane of `res` (nullptr: same index)
@@ -346,9 +347,11 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     // the sparse operand, which no kernel writes) may overlap the tail of the previous kernel in
     // the stream; the dense operand, the residual and the output are touched only below.  The
     // next kernel may start its own prologue as soon as every block of this one got here.
-    // (A convolution call that ends with this kernel lets the next call in when it is done: that one starts
-    // with a relayout, whose waiting blocks would only be in the way.  17.5 -> 14.6 us for 24x16x16x160 ->
-    // 1856, back to back.)
+    // (A convolution call that ends with this kernel lets the next one in when its producers are done: early enough
+    // for the set-up of an SpMM or a chained layer behind it, 1.2 us, and late enough that few blocks of another
+    // convolution's relayout, which has no set-up, wait on this kernel's SMs; with those spread evenly (relayout_smem)
+    // calls back to back are 1-3 % slower than without any trigger.  24x16x16x160 -> 1856, 3x3, V = 32: 26.4 us and 30.0
+    // with a chained layer; without a trigger 26.1 and 31.4; at once, and the relayout not spread, 29.3 and 30.2.)
     if (MODE != kPanelConv || p.perm != nullptr) sm100::grid_dependency_launch();
     // The wait itself is executed per role, as late as each role allows: by the producers after
     // their first row ids (sparse operand) are on their way and before their first gather, by the
@@ -800,6 +803,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 #pragma unroll
         for (int i = 0; i < LAG; ++i)
             if (lane == 0 && pend[i] >= 0) sm100::mbar_arrive(&full_bar[pend[i]]);
+        if (MODE == kPanelConv && p.trigger_late) sm100::grid_dependency_launch();
         if (pw == 0 && lane == 0) CTRACE(2);
 #ifdef SHFLBW_COUNTERS
         if (lane == 0 && p.trace != nullptr && pidx < 8) {

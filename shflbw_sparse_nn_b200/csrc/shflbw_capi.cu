@@ -270,9 +270,9 @@ int sm_count() {
     return n;
 }
 
-// Opt a panel kernel in to its dynamic shared memory once per (device, kernel): the host-buffer
+// Opt a kernel in to its dynamic shared memory once per (device, kernel): the host-buffer
 // calls initialise an op per chunk, and the attribute call is not free.
-int allow_smem(PanelKernel fn, size_t bytes) {
+int allow_smem(const void* fn, size_t bytes) {
     static shflbw::OncePerDevice done;
     int dev = 0;
     CK(cudaGetDevice(&dev));
@@ -280,11 +280,12 @@ int allow_smem(PanelKernel fn, size_t bytes) {
     if (g_set_ups_left == 0) return SHFLBW_ERR_CUDA;
     if (g_set_ups_left > 0) --g_set_ups_left;
 #endif
-    return done.run((const void*)fn, dev, [&]() -> int {
-        CK(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    return done.run(fn, dev, [&]() -> int {
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
         return SHFLBW_OK;
     });
 }
+int allow_smem(PanelKernel fn, size_t bytes) { return allow_smem((const void*)fn, bytes); }
 
 // Tile selection.  A 256-token work item halves the value-panel traffic per token and is
 // the default; 128 is used when the dense extent is too small to give every SM a few items.
@@ -689,16 +690,44 @@ int shflbw_spmm_host_copies_only(shflbw_matrix_t* m, int N, const void* B_host, 
 
 // ---------------------------------------------------------------------------- SpConv --
 
+// Shared memory that a relayout of so many blocks asks for on top of its tile, so that an SM holds no more than its
+// even share of them (up to seven; eight fit by their threads).  The blocks of a call that follows another are
+// resident early, on the SMs that the kernel before leaves first, and wait there: without a limit they pile up on
+// those few, which then move everything (24x16x16x160 -> 1856, V = 64, 1x1, unpermuted, calls back to back: 17.3 us;
+// with the limit 14.3).  With less than one block per SM the share is one where the kernel before is likely to be
+// a panel kernel, as it is behind a call that ends with one (10x27x27x176 -> 624: 13.5 us without, 9.5 with), and
+// without a limit behind a last pass, whose blocks are short and everywhere and leave no room for blocks of half an
+// SM (4x20x26x96 -> 1312: 16.7 us with, 16.0 without).
+constexpr size_t kRelayoutTile = (size_t)shflbw::kRelayoutC * shflbw::kRelayoutSlots * 2;
+static size_t relayout_smem(long long blocks, bool has_last_pass) {
+    const int sms = sm_count() > 0 ? sm_count() : 148;
+    const long long per_sm = (blocks + sms - 1) / sms;
+    if (per_sm > 7 || (per_sm == 1 && has_last_pass)) return 0;
+    return (size_t)(per_sm == 1 ? 227 : 228 / per_sm - 1) * 1024 - kRelayoutTile;   // of 228 KB, 1 KB a block is the system's
+}
+
+#ifdef SHFLBW_FAULT_INJECT
+// The bytes of shared memory that a relayout of `blocks` blocks occupies per block.
+int shflbw_debug_relayout_smem(long long blocks, int has_last_pass) { return (int)(kRelayoutTile + relayout_smem(blocks, has_last_pass != 0)); }
+#endif
+
 // NHWC -> [C][Hin+R-1][Win+S-1][Bp] with a zero halo (origin at (R/2, S/2)); step > 1 (1x1 filters): only the
 // pixels that the stride visits, [C][ceil(Hin/step)][ceil(Win/step)][Bp].
-static void launch_relayout(const __half* in, __half* staged, int B, int Bp, int Hin, int Win, int C, int R, int S,
-                            cudaStream_t s, int step = 1) {
+// Returns the number of blocks per SM.
+static long long launch_relayout(const __half* in, __half* staged, int B, int Bp, int Hin, int Win, int C, int R, int S,
+                            cudaStream_t s, int step = 1, bool has_last_pass = true) {
     const int Hp = step > 1 ? (Hin + step - 1) / step : Hin + R - 1, Wp = step > 1 ? (Win + step - 1) / step : Win + S - 1;
     const int PP = Hp * Wp;
     const int NT = Bp < 32 ? Bp : 32, PT = shflbw::kRelayoutSlots / NT;
     const int n_tiles = (Bp + NT - 1) / NT;
     dim3 grid((unsigned)(((PP + PT - 1) / PT) * n_tiles), (unsigned)((C + shflbw::kRelayoutC - 1) / shflbw::kRelayoutC));
-    (void)launch(step > 1 ? shflbw::relayout_nhwc_to_chwn<true> : shflbw::relayout_nhwc_to_chwn<false>, grid, dim3(256), 0, s, in, staged, B, Bp, Hin, Win, Hp, Wp, R / 2, S / 2, C, step);
+    const auto kernel = step > 1 ? shflbw::relayout_nhwc_to_chwn<true> : shflbw::relayout_nhwc_to_chwn<false>;
+    const long long blocks = (long long)grid.x * grid.y;
+    size_t smem = relayout_smem(blocks, has_last_pass);
+    if (smem && allow_smem((const void*)kernel, relayout_smem(1, false)) != SHFLBW_OK) smem = 0;   // only a matter of speed
+    (void)launch(kernel, grid, dim3(256), smem, s, in, staged, B, Bp, Hin, Win, Hp, Wp, R / 2, S / 2, C, step);
+    const int sms = sm_count() > 0 ? sm_count() : 148;
+    return (blocks + sms - 1) / sms;
 }
 
 // Dynamic shared memory of unpermute_filters: 16-bit permutation + one F-vector of fp16 per position.
@@ -875,11 +904,16 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     //    output's size that is then read at stride 1 (27x27x256 -> 14x14x512, batch 5: 3.4 -> 2.5 us).
     const int step = !st->chain && st->R == 1 && st->S == 1 ? st->stride : 1;
     const int Hp = step > 1 ? st->Ho : st->Hin + st->R - 1, Wp = step > 1 ? st->Wo : st->Win + st->S - 1;
+    long long relayout_per_sm = 0;
     if (!st->chain)
-        launch_relayout((const __half*)st->ifmap, (__half*)st->staged_in, st->B, st->Bp, st->Hin, st->Win, st->C,
-                        st->R, st->S, s, step);
+        relayout_per_sm = launch_relayout((const __half*)st->ifmap, (__half*)st->staged_in, st->B, st->Bp, st->Hin, st->Win, st->C,
+                                          st->R, st->S, s, step, planes || st->staged_out);
     // 2. implicit-GEMM panel kernel.
     shflbw::PanelParams p{};
+    // Where it ends the call: see the kernel.  A call that stages many blocks per SM is likely to be followed by another
+    // one, whose first blocks cannot be spread over the SMs (26x48x48x1024 -> 96 at stride 2, back to back: 73 us, 76
+    // with the trigger); it is long enough not to miss the 1.2 us.
+    p.trigger_late = relayout_per_sm <= 7;
     p.blk_ptr = st->blk_ptr; p.blk_idx = st->blk_idx; p.blk_val = (const __half*)st->blk_val;
     p.perm = st->perm; p.status_word = st->status_word; p.alpha = st->alpha; p.beta = 0.f;
     p.wait_limit = g_wait_limit; p.inject_from = g_inject_from;
