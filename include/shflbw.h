@@ -204,7 +204,7 @@ int shflbw_spmm_exec(const shflbw_spmm_state_t* st, void* stream);
  * alignment) is transposed into xt[K][N] with zeros beyond `tokens`, and out[M][N] (feature-major) =
  * W . xt + bias[M] is formed with the bias added to the fp16 product in the kernel's epilogue.  x == NULL:
  * xt holds the operand already.  bias may be NULL.  xt and out are caller-owned device buffers,
- * 16-byte aligned, N % 8 == 0, N >= tokens.  Asynchronous on `stream`; two launches.  No counterpart in
+ * 16-byte aligned, N % 8 == 0, N >= tokens.  Asynchronous on `stream`; two launches, one with x == NULL.  No counterpart in
  * the reference (its operator takes the feature-major operand only). */
 int shflbw_linear_exec(const shflbw_matrix_t* m, int tokens, const void* x, const void* bias, void* xt, int N,
                        void* out, void* stream);
@@ -249,7 +249,8 @@ typedef struct shflbw_spconv_state {
     float alpha;
     const void* ifmap;       /* NHWC input (device)  */
     void* ofmap;             /* NHWC output (device) */
-    void* staged_in;         /* scratch: input as [C][Hin+R-1][Win+S-1][Bp], zero halo */
+    void* staged_in;         /* scratch: input as [C][Hin+R-1][Win+S-1][Bp], zero halo; a strided 1x1 filter
+                                keeps only the pixels it visits, [C][Ho][Wo][Bp], in the same buffer */
     void* staged_out;        /* scratch: output planes [F][Ho][Wo][Bp] (variant 1), [B*Ho*Wo][F] in stored
                                 filter order (variant 0, permuted filter), or NULL */
     size_t staged_in_bytes, staged_out_bytes;
@@ -312,7 +313,8 @@ size_t shflbw_chain_buffer_elems(int C, int H, int W, int B, int R_consumer, int
 int shflbw_chain_import_nhwc(const void* nhwc, int B, int H, int W, int C, int R_consumer, int S_consumer,
                              void* chain_buf, void* stream);
 /* Chain buffer written by `producer` (halo for R x S) -> NHWC in logical channel order
- * (producer's inverse filter permutation applied; producer == NULL: channels as stored). */
+ * (producer's inverse filter permutation applied; producer == NULL: channels as stored).  F % 8 == 0,
+ * F <= 14528 (SHFLBW_ERR_UNSUPPORTED beyond). */
 int shflbw_chain_export_nhwc(const void* chain_buf, int B, int H, int W, int F, int R_halo, int S_halo,
                              const shflbw_matrix_t* producer, void* nhwc, void* stream);
 /* New filter = `filter` with its input channels renumbered to the stored filter order of

@@ -19,10 +19,11 @@ namespace shflbw {
 
 // Programmatic dependent launch (see sm100_ptx.cuh): both are no-ops for plain launches.  A kernel lets the
 // next one in early where that one has a set-up to overlap (the panel kernel after a relayout).  The last
-// pass of a convolution call lets it in only after its own wait, when the panel kernel is done: the next call's relayout has nothing to set up,
-// and its blocks, resident and waiting through the panel kernel and the last pass of this call, took the
-// shared memory and the slots of theirs (calls back to back: 19.8 -> 14.8 us for 13x8x8x376 -> 2016 at stride 2,
-// 13.5 -> 10.8 for 12x15x13x144 -> 640, 12 % over 39 shapes drawn from 1..64 images).
+// pass of a convolution call lets it in only after its own wait, when the panel kernel is done: the next call's
+// relayout has nothing to set up, and its blocks, resident and waiting through the panel kernel and the last
+// pass of this call, took the shared memory and the slots of theirs (calls back to back: 21.1 -> 14.7 us for
+// 13x8x8x376 -> 2016 at stride 2, 14.9 -> 11.3 for 12x15x13x144 -> 640 at stride 2, V = 128; 2.7 % over 43 shapes
+// of 1..64 images, none slower by 1 %).
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -271,8 +272,8 @@ export_planes_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, 
 
 // planes[f][tok] -> out[n][pix][f] (+ bias[f]): the output of an NHWC call computed as planes (one row of
 // tok = pix * Bp + n tokens per LOGICAL filter f) transposed to NHWC.  The same tile as above, one per block,
-// without the plane search and the halo, whose start-up and registers cost 1.1 us of 4.8 at 3136 tokens x
-// 2048 filters.  F % 64 == 0, Bp % 8 == 0; images n >= Bn are padding.
+// without the plane search, the halo and the loop, which cost 0.3 to 1 us of a call (0.9 of 31.3 at 3136 tokens
+// x 2048 filters).  F % 64 == 0, Bp % 8 == 0; images n >= Bn are padding.
 template <bool BIAS>
 __global__ void __launch_bounds__(256)
 planes_to_nhwc(const __half* __restrict__ planes, __half* __restrict__ out, const __half* __restrict__ bias, int Bn, int Bp, int npix, int F) {

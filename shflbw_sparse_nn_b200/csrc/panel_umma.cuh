@@ -115,7 +115,8 @@ struct alignas(64) PanelParams {
     __half* D;               // [M][N]
     int N;                   // dense columns (SpMM) / Ho*Wo*Bp (SpConv)
     // SpConv (input staged channel-major, batch innermost, with a zero halo:
-    // Xs[c][Hp][Wp][Bp], Hp = Hin + R - 1, Wp = Win + S - 1, image origin at (R/2, S/2))
+    // Xs[c][Hp][Wp][Bp], Hp = Hin + R - 1, Wp = Win + S - 1, image origin at (R/2, S/2); a strided 1x1
+    // filter of an NHWC call is staged as the pixels it visits, Hp = Ho, Wp = Wo, and read at stride 1)
     const __half* Xs;
     __half* out;             // [B*Ho*Wo][F] (NHWC) -- final or staged in stored filter order
     int Bn, Bp, Hp, Wp, Cin, F, R, S, stride, Ho, Wo;
@@ -1186,7 +1187,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             // block's shared memory the L1 holds about 28 KB, less than one item's 32 KB: with them more
             // requests in flight made these layers slower (56x56x64 -> 256 with residual, batch 256:
             // 214 us with loads before the accumulator wait, 230 with two items' loads in flight, 187 with
-            // the copies; the same product without a residual takes 93).
+            // the copies; the same product without a residual takes 93.  All in the executed stack; back to back
+            // with the L2 warm 168 and 91).
             //   Eight: into registers, the first two chunks before the accumulator wait, each later
             // chunk's two chunks ahead.
             constexpr int NCH = COLS / CW;

@@ -851,7 +851,8 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     out->block_x = ch.threads;
     out->grid_x = persistent_grid(out->num_items, sms); out->grid_y = 1;
     out->shared_mem_size = ch.smem;
-    out->staged_in_bytes = (size_t)cs.staged_elems * 2;
+    out->staged_in_bytes = (size_t)cs.staged_elems * 2;     // the whole image, also where a strided 1x1 filter stages less:
+                                                            // callers size and check their scratch by the documented formula
     return SHFLBW_OK;
 }
 
@@ -1043,7 +1044,7 @@ int shflbw_chain_export_nhwc(const void* chain_buf, int B, int H, int W, int F, 
         if (!on_current_device(*producer)) return SHFLBW_ERR_NOT_ON_DEVICE;
         perm = producer->d_perm;
     }
-    if ((size_t)F * 16 > 227 * 1024) return SHFLBW_ERR_UNSUPPORTED;
+    if (F > 14528) return SHFLBW_ERR_UNSUPPORTED;           // the documented range; the kernel itself needs grid.y = F / 64 <= 65535
     const int Bp = (B + 7) / 8 * 8;
     if ((long long)H * W * (Bp / 8) >= (1ll << 31)) return SHFLBW_ERR_UNSUPPORTED;
     CK(launch_export(chain_buf, nhwc, perm, B, Bp, H, W, H + R - 1, W + S - 1, R / 2, S / 2, F, (cudaStream_t)stream));
