@@ -33,7 +33,7 @@
 //   warps EW+1.. with w % 4 != 0   producers (PW of them, in GROUPS groups that take the stages in
 //                    turn).  cp.async gather: 16-byte copies into 128-byte-swizzled stages; a
 //                    group publishes its previous stage half-way through issuing the next one,
-//                    with ONE mbarrier arrival per warp; row ids are prefetched LAG+1 of the
+//                    with ONE mbarrier arrival per warp; row ids are prefetched two of the
 //                    group's stages ahead by 4-byte cp.async into a shared-memory ring.  TMA
 //                    gather: one tile::gather4 per lane, completion by byte count.  One bulk copy
 //                    per stage for the value slice either way.
@@ -105,10 +105,8 @@ struct alignas(64) PanelParams {
     // stays in L2 (SpMM with a large dense operand).
     int tile_major, num_blocks;
     FastDiv div_blocks;
-    unsigned long long* trace;  // tuning builds only: per-role timestamps of CTA 0
     int inject_from;         // fault-injection builds only (-DSHFLBW_FAULT_INJECT): from this stage number on, one
                              // producer warp withholds its arrivals, so the consumer's bounded wait runs out (< 0: off)
-    int ablate;              // tuning builds only (-DSHFLBW_ABLATE): 1 no MMA, 2 no gather, 4 no value copies, 8 no stores
     // SpMM
     const __half* B;         // [K][N]
     const __half* C;         // [M][N] or nullptr; kernels built with BIAS: one value per output row / filter
@@ -145,28 +143,22 @@ constexpr int kPanelSpmm = 0, kPanelConv = 1, kPanelConvChain = 2, kPanelSpmmRow
 //                   tensor map covers this GPU's own B; no multicast), the copy engine applies
 //                   the 128-byte swizzle and completes the stage's barrier by byte count, so the
 //                   producers never wait for data.  SpMM with rows in lanes only.
-//   kGatherCpAsyncArrive  the same 16-byte cp.async copies, but every lane hands its stage to the
-//                   barrier with cp.async.mbarrier.arrive.noinc: the arrival fires when the lane's
-//                   copies have landed, so the producers never wait for data and need no publish
-//                   step; row ids travel in registers (loaded two stages ahead).
-constexpr int kGatherCpAsync = 0, kGatherTma = 1, kGatherCpAsyncArrive = 2;
+constexpr int kGatherCpAsync = 0, kGatherTma = 1;
 
 // EW: epilogue warps, 8 or 16.  A warp can read only the TMEM lane quadrant warp % 4, so the two
 // warps of a quadrant split the accumulator columns between them.  Items with few non-zero
 // columns are all epilogue, and one warp's chain (TMEM read, convert, transpose, store) is
 // latency-bound: sixteen warps, as two sets on alternate items, keep four such chains per
 // scheduler in flight instead of two.
-template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int LAG_ = 1, int GATHER_ = kGatherCpAsync,
+template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int GATHER_ = kGatherCpAsync,
           int EW_ = 8, bool ADDEND_ = false>
 struct PanelCfg {
     static constexpr int EW = EW_;
     static_assert(EW == 8 || EW == 16, "epilogue warps");
     static constexpr bool TMA = GATHER_ == kGatherTma;
-    static constexpr bool ARRIVE = GATHER_ == kGatherCpAsyncArrive;
     static constexpr int KS = KS_;                         // non-zero columns per pipeline stage
     static constexpr int T = 128 * TM;
     static constexpr int GROUPS = GROUPS_;                 // producer groups that take the stages in turn
-    static constexpr int LAG = LAG_;                       // a group publishes a stage while issuing its LAG-th next one
     // Warp w runs on scheduler partition w % 4.  The MMA warp (the first after the epilogue
     // warps: 8 or 16) sits on partition 0 and no producer shares it: the later warps with
     // w % 4 == 0 stay idle.  The MMA warp executes a
@@ -210,10 +202,10 @@ struct PanelCfg {
     static constexpr int RES_BYTES = ADDEND_ ? EW * 4096 : 0;
     static constexpr int BAR_BYTES = (STAGES * 2 + 12) * 8;  // mbarriers (ring, up to 4 + 4 accumulator, drain) + tmem slot + abort flag
     static constexpr int TAB_BYTES = 512 * 8;               // per-CTA item table (kPanelMaxItemsPerCta entries)
-    static constexpr int IDX_AHEAD = LAG + 1;              // a group fetches row ids this many of its stages ahead
+    static constexpr int IDX_AHEAD = 2;                    // a group fetches row ids this many of its stages ahead
     static constexpr int IDX_RING = (IDX_AHEAD + 1) * GROUPS <= 8 ? 8 : 16;   // stages of row ids kept in shared memory
     static_assert((IDX_AHEAD + 1) * GROUPS <= IDX_RING, "row-id ring too small");
-    static constexpr int IDX_BYTES = (TMA || ARRIVE) ? 0 : IDX_RING * KS * 4;   // (the TMA gather loads its row ids straight into registers)
+    static constexpr int IDX_BYTES = TMA ? 0 : IDX_RING * KS * 4;   // (the TMA gather loads its row ids straight into registers)
     static constexpr int SMEM_BYTES = PIPE_BYTES + OUT_BYTES + RES_BYTES + BAR_BYTES + TAB_BYTES + IDX_BYTES + 1024;  // + align slack
     static constexpr bool SWAP = MODE == kPanelSpmmRows || MODE == kPanelConvChainRows;
     static constexpr int KG_BYTES = SWAP ? T * 16 : 2048;   // 8 gathered rows (one K group) of the token tile
@@ -235,7 +227,7 @@ struct PanelCfg {
     static_assert((TMEM_COLS & (TMEM_COLS - 1)) == 0 && TMEM_COLS <= 512, "TMEM columns");
     static_assert(KS % 16 == 0 && PW % GROUPS == 0 && KS % (PW / GROUPS) == 0 && (KS / (PW / GROUPS)) % (32 / (T / 8)) == 0,
                   "rows per producer warp");
-    static_assert(LAG >= 1 && LAG <= 2 && (TMA || ARRIVE || STAGES > GROUPS * LAG), "publish lag");
+    static_assert(TMA || STAGES > GROUPS, "a group publishes a stage while issuing its next one");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
 };
 
@@ -264,11 +256,11 @@ constexpr int kPanelMaxItemsPerCta = 512;  // capacity of the per-CTA item table
 // BIAS: C holds one value per output row (SpMM, added like C with beta = 1) or per filter (SpConv writing
 // NHWC in logical order).  Kernels of their own: as a branch of the others it made small products 1-2 %
 // slower (256-item launches of 5-9 us, where every instruction is fetched for the first time).
-template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int LAG_ = 1, int GATHER_ = kGatherCpAsync,
+template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int GATHER_ = kGatherCpAsync,
           int EW_ = 8, bool BIAS = false, bool ADDEND = false>
-__global__ void __launch_bounds__(PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, LAG_, GATHER_, EW_, ADDEND>::THREADS, 1)
+__global__ void __launch_bounds__(PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, GATHER_, EW_, ADDEND>::THREADS, 1)
 panel_umma_kernel(const __grid_constant__ PanelParams p) {
-    using Cfg = PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, LAG_, GATHER_, EW_, ADDEND>;
+    using Cfg = PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, GATHER_, EW_, ADDEND>;
     constexpr int EW = Cfg::EW;                                             // epilogue warps 0..EW-1, MMA warp EW, producers after it
     constexpr bool SWAP = Cfg::SWAP;                                        // rows in TMEM lanes
     constexpr bool CONV = MODE == kPanelConv || MODE == kPanelConvChain || MODE == kPanelConvChainRows;  // implicit-GEMM gather
@@ -292,25 +284,11 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     int* idx_ring = (int*)(bar_area + Cfg::BAR_BYTES + Cfg::TAB_BYTES);  // [IDX_RING][KS] row ids of upcoming stages
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-#ifdef SHFLBW_ABLATE
-    const int ablate = p.ablate;
-    auto now = []() { unsigned long long t; asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t)); return t; };
-    const bool tracing = p.trace != nullptr && blockIdx.x == 0;
-#define TRACE(role, n, k) do { if (tracing && (n) < 256 && !(ablate & 256)) p.trace[(role) * 1024 + (n) * 4 + (k)] = now(); } while (0)
-#define CTRACE(k) do { if (p.trace != nullptr) p.trace[4096 + blockIdx.x * 8 + (k)] = now(); } while (0)
-#define PTRACE(w, n, k) do { if (tracing && (n) < 256 && !(ablate & 256)) p.trace[8192 + (w) * 1024 + (n) * 4 + (k)] = now(); } while (0)
-#else
-#define PTRACE(w, n, k) do { } while (0)
-#define CTRACE(k) do { } while (0)
-    constexpr int ablate = 0;
-#define TRACE(role, n, k) do { } while (0)
-#endif
     // This CTA's work items: blockIdx.x, blockIdx.x + gridDim.x, ...  (host guarantees nloc <= table size)
     const int nloc = (p.num_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
     auto item_block = [&](int item) { return p.tile_major ? item - fast_div(item, p.div_blocks) * p.num_blocks : fast_div(item, p.div_tiles); };
     auto item_tile = [&](int item) { return p.tile_major ? fast_div(item, p.div_blocks) : item - fast_div(item, p.div_tiles) * p.tiles_n; };
 
-    if (tid == 0) CTRACE(0);
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
             // One arrival per producer WARP.  Per-thread deferred arrivals
@@ -318,8 +296,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             // per thread, i.e. more than the copies themselves.
             // cp.async gather: one arrival per producer WARP of the group.  TMA gather: one arrival
             // (with the stage's byte count) by the group's first warp.
-            // Deferred arrivals: one per LANE of the group's warps.
-            sm100::mbar_init(&full_bar[s], Cfg::TMA ? 1 : Cfg::ARRIVE ? (PW / Cfg::GROUPS) * 32 : PW / Cfg::GROUPS);
+            sm100::mbar_init(&full_bar[s], Cfg::TMA ? 1 : PW / Cfg::GROUPS);
             sm100::mbar_init(&empty_bar[s], 1);   // one tcgen05.commit per drain
         }
         for (int b = 0; b < NBUF; ++b) {
@@ -358,8 +335,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     // their first row ids (sparse operand) are on their way and before their first gather, by the
     // epilogue warps at once (they read C / the residual and write the output); the MMA warp
     // touches no global memory and does not wait.
-    if (tid == 0) TRACE(3, 0, 0);
-    if (tid == 0) CTRACE(1);
 
     const int pidx = warp - (EW + 1) - (warp / 4 - EW / 4);   // producer number of a producer warp (warps after the MMA warp with warp % 4 != 0)
     if constexpr (Cfg::REG_SPLIT) {
@@ -414,9 +389,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         for (int g = 0; g < GROUPS; ++g) advance(pre);       // which covers the load's latency even with one group
         sm100::grid_dependency_wait();                       // the dense operand may be the previous kernel's output
         int it = 0;
-#ifdef SHFLBW_COUNTERS
-        long long pc_empty = 0, pc_n = 0, pc_t0 = clock64();
-#endif
         for (int li = 0; li < nloc; ++li) {
             const int2 ent = item_tab[li];
             const int num_k = (ent.y + KS - 1) / KS;
@@ -428,17 +400,11 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 if ((it % GROUPS) != grp) continue;
                 const int s = it % STAGES;
                 if (it >= STAGES) {
-#ifdef SHFLBW_COUNTERS
-                    const long long e0c = clock64();
-#endif
                     int ok = 1;
                     if (lane == 0)
                         ok = sm100::mbar_wait_bounded(&empty_bar[s], ((it / STAGES) - 1) & 1, cta_abort, p.status_word,
                                                       SHFLBW_DEVSTAT_TIMEOUT_EMPTY, p.wait_limit, 32);
                     if (!__shfl_sync(0xffffffffu, ok, 0)) goto tma_producer_done;
-#ifdef SHFLBW_COUNTERS
-                    pc_empty += clock64() - e0c; ++pc_n;
-#endif
                 }
                 const int rows_valid = min(KS, ent.y - kt * KS);    // multiple of 16
                 const uint32_t st_base = smem_base + s * Cfg::STAGE_BYTES;
@@ -448,12 +414,10 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     if (!(p.inject_from >= 0 && it >= p.inject_from && pidx == 0))   // the withheld arrival
 #endif
                     sm100::mbar_arrive_expect_tx(&full_bar[s], (uint32_t)(rows_valid * T * 2) + wbytes);
-                    if (!(ablate & 4)) sm100::bulk_copy_g2s(st_base + (uint32_t)Cfg::G_BYTES, wsrc + (size_t)kt * KS * V, wbytes, &full_bar[s]);
-                    else sm100::mbar_complete_tx(&full_bar[s], wbytes);
+                    sm100::bulk_copy_g2s(st_base + (uint32_t)Cfg::G_BYTES, wsrc + (size_t)kt * KS * V, wbytes, &full_bar[s]);
                 }
                 if (issuer && quad * 4 < rows_valid) {
-                    if (!(ablate & 2)) sm100::tma_gather4(st_base + dst_off, p.tmap_b, col, ids.x, ids.y, ids.z, ids.w, &full_bar[s]);
-                    else sm100::mbar_complete_tx(&full_bar[s], 512u);
+                    sm100::tma_gather4(st_base + dst_off, p.tmap_b, col, ids.x, ids.y, ids.z, ids.w, &full_bar[s]);
                 }
                 ids = ids_next;
                 ids_next = load_ids(pre);
@@ -461,144 +425,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             }
         }
     tma_producer_done:;
-#ifdef SHFLBW_COUNTERS
-        if (lane == 0 && p.trace != nullptr && pidx < 8) {
-            unsigned long long* o = p.trace + 148 * 16 + (blockIdx.x * 8 + pidx) * 4;
-            o[0] = pc_empty; o[1] = pc_n; o[2] = clock64() - pc_t0;
-        }
-#endif
-        }
-    } else if (warp > EW && Cfg::ARRIVE) {
-        // ------------------------------------- producers (cp.async, deferred arrivals) ----
-        // The GW warps of a group share a stage (RPW rows each); a warp instruction copies RPI
-        // rows of the token tile, 16 bytes per lane, straight into the swizzled layout.  After its
-        // copies of a stage every lane issues cp.async.mbarrier.arrive.noinc on the stage's
-        // barrier: the arrival is delivered when that lane's copies have landed.  Nothing here
-        // waits for data; the only wait is for a free stage.  (The consumer orders the generic-
-        // proxy writes before the tensor core's reads with a proxy fence after its own wait.)
-        if constexpr (Cfg::ARRIVE) {
-        constexpr int GROUPS = Cfg::GROUPS, GW = PW / GROUPS, RPW = KS / GW;
-        constexpr int CPR = T / 8, RPI = 32 / CPR, NQ = RPW / RPI;
-        constexpr int XT = NQ < 8 / RPI ? NQ : 8 / RPI;
-        static_assert((RPW % 8 == 0 || 8 % RPW == 0) && RPW <= 32, "rows per producer warp");
-        const int grp = pidx / GW, pw = pidx % GW;
-        const int chunk = lane % CPR;
-        const int sub = RPI == 2 ? (lane >> 4) : 0;
-        const int rbase = pw * RPW + sub;
-        const uint32_t gbase = SWAP ? (uint32_t)((pw * RPW / 8) * Cfg::KG_BYTES + (chunk >> 3) * 1024)
-                                    : (uint32_t)((chunk >> 4) * Cfg::G_ACC + (pw * RPW / 8) * 2048 + (((chunk & 15) >> 3)) * 1024);
-        uint32_t gx[XT];
-#pragma unroll
-        for (int j = 0; j < XT; ++j) {
-            const int r7 = (pw * RPW + j * RPI + sub) & 7;
-            gx[j] = (uint32_t)(r7 * 128 + (((chunk & 7) ^ r7) << 4));
-        }
-        struct Cursor { int li, kt, num_k, row_begin, rows_total; };
-        auto enter = [&](Cursor& c) {
-            c.kt = 0;
-            while (c.li < nloc) {
-                const int2 e = item_tab[c.li];
-                c.row_begin = e.x; c.rows_total = e.y; c.num_k = (e.y + KS - 1) / KS;
-                if (c.num_k > 0) return;
-                ++c.li;
-            }
-            c.num_k = 0; c.row_begin = 0; c.rows_total = 0;
-        };
-        auto advance = [&](Cursor& c) { if (++c.kt >= c.num_k) { ++c.li; enter(c); } };
-        // Lane j < RPW holds the id of row pw*RPW + j of a stage (for SpConv: its element offset);
-        // ids are loaded two of the group's stages ahead and handed out by shuffle.
-        auto load_id = [&](const Cursor& c) {
-            int v = 0;
-            const int r = c.kt * KS + pw * RPW + lane;
-            if (lane < RPW && c.li < nloc && r < c.rows_total) v = __ldg(p.blk_idx + c.row_begin + r);
-            if constexpr (CONV)
-                return (int)min((unsigned)(((v & 0xffff) * (p.Hp * p.Wp) + ((v >> 16) & 0xff) * p.Wp + ((v >> 24) & 0xff)) * p.Bp), p.idx_limit);
-            else
-                return (int)min((unsigned)v, p.idx_limit);
-        };
-        Cursor pre{0, 0, 0, 0, 0};
-        enter(pre);
-        for (int d = 0; d < grp; ++d) advance(pre);
-        int id_cur = load_id(pre);
-        for (int g = 0; g < GROUPS; ++g) advance(pre);
-        int id_next = load_id(pre);
-        for (int g = 0; g < GROUPS; ++g) advance(pre);
-        sm100::grid_dependency_wait();                       // the dense operand may be the previous kernel's output
-        int it = 0;
-#ifdef SHFLBW_COUNTERS
-        long long pc_empty = 0, pc_n = 0, pc_t0 = clock64();
-#endif
-        for (int li = 0; li < nloc; ++li) {
-            const int2 ent = item_tab[li];
-            const int num_k = (ent.y + KS - 1) / KS;
-            if (num_k == 0) continue;
-            const int item = (int)blockIdx.x + li * (int)gridDim.x;
-            const int tok0 = item_tile(item) * T + chunk * 8;
-            const bool chunk_ok = tok0 < p.N;
-            const uint32_t nbytes = chunk_ok ? 16u : 0u;
-            const __half* conv_src0 = p.Xs;
-            if constexpr (CONV) {
-                if (chunk_ok) {
-                    const int pix = fast_div(tok0, p.div_bp), nn = tok0 - pix * p.Bp;
-                    const int oh = fast_div(pix, p.div_wo), ow = pix - oh * p.Wo;
-                    conv_src0 = p.Xs + ((oh * p.stride * p.Wp + ow * p.stride) * p.Bp + nn);
-                }
-            }
-            const __half* lane_src0 = chunk_ok ? p.B + tok0 : p.B;
-            const uint32_t row_pitch = chunk_ok ? (uint32_t)p.N : 0u;
-            const __half* wsrc = p.blk_val + (size_t)ent.x * V;
-            for (int kt = 0; kt < num_k; ++kt, ++it) {
-                if ((it % GROUPS) != grp) continue;
-                const int s = it % STAGES;
-                if (it >= STAGES) {
-#ifdef SHFLBW_COUNTERS
-                    const long long e0c = clock64();
-#endif
-                    int ok = 1;
-                    if (lane == 0)
-                        ok = sm100::mbar_wait_bounded(&empty_bar[s], ((it / STAGES) - 1) & 1, cta_abort, p.status_word,
-                                                      SHFLBW_DEVSTAT_TIMEOUT_EMPTY, p.wait_limit, 32);
-                    if (!__shfl_sync(0xffffffffu, ok, 0)) goto arrive_producer_done;
-#ifdef SHFLBW_COUNTERS
-                    pc_empty += clock64() - e0c; ++pc_n;
-#endif
-                }
-                const int rows_valid = min(KS, ent.y - kt * KS);
-                const uint32_t st_base = smem_base + s * Cfg::STAGE_BYTES;
-                if (pw == 0 && lane == 0 && !(ablate & 4)) {
-                    const uint32_t wbytes = (uint32_t)(rows_valid * V * 2);
-                    sm100::mbar_expect_tx(&full_bar[s], wbytes);
-                    sm100::bulk_copy_g2s(st_base + (uint32_t)Cfg::G_BYTES, wsrc + (size_t)kt * KS * V, wbytes, &full_bar[s]);
-                }
-                int idq[NQ];
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) idq[q] = __shfl_sync(0xffffffffu, id_cur, q * RPI + sub);
-#pragma unroll
-                for (int q = 0; q < NQ; ++q) {
-                    if (rbase + q * RPI < rows_valid && !(ablate & 2)) {
-                        const uint32_t dst = st_base + gbase + (uint32_t)(((q * RPI) >> 3) * Cfg::KG_BYTES) + gx[q % XT];
-                        if constexpr (CONV) sm100::cp_async_16(dst, conv_src0 + idq[q], nbytes);
-                        else sm100::cp_async_16(dst, lane_src0 + (uint64_t)(uint32_t)idq[q] * row_pitch, nbytes);
-                    }
-                }
-#ifdef SHFLBW_FAULT_INJECT
-                if (!(p.inject_from >= 0 && it >= p.inject_from && pidx == 0))   // the withheld arrivals
-#endif
-                sm100::cp_async_arrive_noinc(&full_bar[s]);
-                id_cur = id_next;
-                id_next = load_id(pre);
-                for (int g = 0; g < GROUPS; ++g) advance(pre);
-            }
-        }
-    arrive_producer_done:
-        sm100::cp_async_commit();
-        sm100::cp_async_wait<0>();          // nothing of this warp is in flight when the block ends
-#ifdef SHFLBW_COUNTERS
-        if (lane == 0 && p.trace != nullptr && pidx < 8) {
-            unsigned long long* o = p.trace + 148 * 16 + (blockIdx.x * 8 + pidx) * 4;
-            o[0] = pc_empty; o[1] = pc_n; o[2] = clock64() - pc_t0;
-        }
-#endif
         }
     } else if (warp > EW) {
         // ------------------------------------------------------------- producers ----
@@ -607,7 +433,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         // (wait for the free stage, wait for its copies, publish) the other one issues copies,
         // so the load/store unit stays busy; with a single group the round trip (~400 clk)
         // simply added to every stage.
-        constexpr int GROUPS = Cfg::GROUPS, LAG = Cfg::LAG;
+        constexpr int GROUPS = Cfg::GROUPS;
         constexpr int GW = PW / GROUPS;        // warps that share one stage
         constexpr int RPW = KS / GW;           // rows of a stage owned by this warp
         constexpr int CPR = T / 8;             // 16-byte chunks per gathered row
@@ -646,13 +472,13 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         };
         auto advance = [&](Cursor& c) { if (++c.kt >= c.num_k) { ++c.li; enter(c); } };
         // Row ids are prefetched with 4-byte cp.async into a shared-memory ring (slot = stage %
-        // IDX_RING; this warp owns entries [pw*RPW, pw*RPW + RPW) of its group's slots), LAG + 1 of
+        // IDX_RING; this warp owns entries [pw*RPW, pw*RPW + RPW) of its group's slots), two of
         // the group's stages ahead: they travel in the first cp.async group of a stage, and the
-        // publish step of the group's (LAG + 1)-th stage before the one that reads them is the
+        // publish step of the group's second stage before the one that reads them is the
         // last wait that is certain to cover that group.
         // (A register prefetch would stall: rotating the registers waits for the load in flight.)
         auto prefetch_idx = [&](const Cursor& c, int stage_no) {
-            if (lane < RPW && !(ablate & 2048)) {
+            if (lane < RPW) {
                 const int r = c.kt * KS + pw * RPW + lane;
                 const bool ok = c.li < nloc && r < c.rows_total;
                 sm100::cp_async_4(sm100::smem_u32(idx_ring + (stage_no % Cfg::IDX_RING) * KS + pw * RPW + lane),
@@ -676,12 +502,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         sm100::grid_dependency_wait();                         // the dense operand may be the previous kernel's output
 
         int it = 0;        // stage counter across items (all groups count the same sequence)
-        int pend[LAG];     // this group's stages not yet published, oldest first
-#pragma unroll
-        for (int i = 0; i < LAG; ++i) pend[i] = -1;
-#ifdef SHFLBW_COUNTERS
-        long long pc_empty = 0, pc_n = 0, pc_t0 = clock64();
-#endif
+        int pend = -1;     // this group's stage not yet published
         for (int li = cur.li; li < nloc; ++li) {
             const int2 ent = item_tab[li];
             const int num_k = (ent.y + KS - 1) / KS;
@@ -709,44 +530,33 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 if ((it % GROUPS) != grp) continue;            // the other group's stage
                 const int s = it % STAGES, s_idx = it % Cfg::IDX_RING;
                 if (it >= STAGES) {  // one lane polls; the warp follows through the broadcast of its result
-#ifdef SHFLBW_COUNTERS
-                    const long long e0c = clock64();
-#endif
                     int ok = 1;
                     if (lane == 0)
                         ok = sm100::mbar_wait_bounded(&empty_bar[s], ((it / STAGES) - 1) & 1, cta_abort, p.status_word,
                                                       SHFLBW_DEVSTAT_TIMEOUT_EMPTY, p.wait_limit, 32);
                     if (!__shfl_sync(0xffffffffu, ok, 0)) goto producer_done;   // timed out or aborted: stop issuing
-#ifdef SHFLBW_COUNTERS
-                    pc_empty += clock64() - e0c; ++pc_n;
-#endif
                 }
-                if (pw == 0 && lane == 0) TRACE(0, it, 0);
-                if (lane == 0) PTRACE(pidx, it, 0);
                 const int rows_valid = min(KS, ent.y - kt * KS);  // multiple of 16
                 const uint32_t st_base = smem_base + s * Cfg::STAGE_BYTES;
-                // An earlier stage of the group (the LAG-th before this one) is published half-way
-                // through this stage's copies: every stage is committed as two cp.async groups, so
-                // "all but the newest 2*LAG - 1 groups" covers every copy of that stage -- issued
-                // at least LAG - 1/2 issue phases ago, so the wait does not stall, while the tensor
-                // core gets the stage half an issue phase earlier than if it were published at the
-                // end.
+                // The group's stage before this one is published half-way through this stage's
+                // copies: every stage is committed as two cp.async groups, so "all but the newest
+                // group" covers every copy of that stage, issued half an issue phase ago or more.
                 auto publish_prev = [&]() {
                     sm100::cp_async_commit();
-                    if (pend[0] >= 0) {
-                        sm100::cp_async_wait<2 * LAG - 1>();
+                    if (pend >= 0) {
+                        sm100::cp_async_wait<1>();
                         sm100::fence_proxy_async_smem();   // every lane: its generic-proxy writes -> tensor-core reads
                         __syncwarp();
 #ifdef SHFLBW_FAULT_INJECT
                         if (p.inject_from >= 0 && it >= p.inject_from && pidx == 0) return;   // the withheld arrival
 #endif
-                        if (lane == 0) sm100::mbar_arrive(&full_bar[pend[0]]);
+                        if (lane == 0) sm100::mbar_arrive(&full_bar[pend]);
                     }
                 };
                 // Value panel slice [rows_valid][V]: stored in global memory in the byte order of
                 // the shared-memory operand tile, so one bulk copy by the copy engine places it;
                 // its bytes are added to what the stage's barrier waits for.
-                if (pw == 0 && lane == 0 && !(ablate & 4)) {
+                if (pw == 0 && lane == 0) {
                     const uint32_t wbytes = (uint32_t)(rows_valid * V * 2);
                     sm100::mbar_expect_tx(&full_bar[s], wbytes);
                     sm100::bulk_copy_g2s(st_base + (uint32_t)Cfg::G_BYTES, wsrc + (size_t)kt * KS * V, wbytes, &full_bar[s]);
@@ -765,7 +575,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 #pragma unroll
                     for (int q = 0; q < NQ; ++q) {
                         if (q == NQ / 2) publish_prev();
-                        if (rbase + q * RPI < rows_valid && !(ablate & 2))
+                        if (rbase + q * RPI < rows_valid)
                             sm100::cp_async_16(st_base + gbase + (uint32_t)(((q * RPI) >> 3) * Cfg::KG_BYTES) + gx[q % XT],
                                                lane_src0 + (uint64_t)(uint32_t)idr[q] * row_pitch, nbytes);
                     }
@@ -781,19 +591,13 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 #pragma unroll
                     for (int q = 0; q < NQ; ++q) {
                         if (q == NQ / 2) publish_prev();
-                        if (rbase + q * RPI < rows_valid && !(ablate & 2))
+                        if (rbase + q * RPI < rows_valid)
                             sm100::cp_async_16(st_base + gbase + (uint32_t)(((q * RPI) >> 3) * Cfg::KG_BYTES) + gx[q % XT],
                                                conv_src0 + dq[q], nbytes);
                     }
                 }
                 sm100::cp_async_commit();
-                if (pw == 0 && lane == 0) TRACE(0, it, 1);
-                if (lane == 0) PTRACE(pidx, it, 1);
-#pragma unroll
-                for (int i = 0; i + 1 < LAG; ++i) pend[i] = pend[i + 1];
-                pend[LAG - 1] = s;
-                if (pw == 0 && lane == 0) TRACE(0, it, 2);
-                if (lane == 0) PTRACE(pidx, it, 2);
+                pend = s;
             }
         }
     producer_done:
@@ -801,17 +605,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         sm100::cp_async_wait<0>();
         sm100::fence_proxy_async_smem();
         __syncwarp();
-#pragma unroll
-        for (int i = 0; i < LAG; ++i)
-            if (lane == 0 && pend[i] >= 0) sm100::mbar_arrive(&full_bar[pend[i]]);
+        if (lane == 0 && pend >= 0) sm100::mbar_arrive(&full_bar[pend]);
         if (MODE == kPanelConv && p.trigger_late) sm100::grid_dependency_launch();
-        if (pw == 0 && lane == 0) CTRACE(2);
-#ifdef SHFLBW_COUNTERS
-        if (lane == 0 && p.trace != nullptr && pidx < 8) {
-            unsigned long long* o = p.trace + 148 * 16 + (blockIdx.x * 8 + pidx) * 4;
-            o[0] = pc_empty; o[1] = pc_n; o[2] = clock64() - pc_t0;
-        }
-#endif
     } else if (warp == EW) {
         // ------------------------------------------------------------ MMA warp ----
         constexpr uint32_t idesc = SWAP ? sm100::make_idesc_f16_mnmajor(V, T) : sm100::make_idesc_f16_mnmajor(128, V);
@@ -830,47 +625,25 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         // instead of being recomputed by division.
         if (lane == 0) {
             int it = 0;
-#ifdef SHFLBW_COUNTERS
-            long long cnt_wait = 0, cnt_n = 0, cnt_acc = 0, cnt_t0 = clock64();
-#endif
-#ifdef SHFLBW_ABLATE
-            int held = -1;              // stage whose release waits for the next one (tuning: paired releases)
-#endif
             uint32_t s = 0, ph = 0;     // ring slot of stage `it` and the parity of its full barrier
             bool ready = false;         // that barrier was already seen complete
             for (int li = 0; li < nloc; ++li) {
                 const int rows_total = item_tab[li].y;
                 const int num_k = (rows_total + KS - 1) / KS;
                 const int b = li % NBUF;
-#ifdef SHFLBW_COUNTERS
-                const long long a0c = clock64();
-#endif
                 if (li >= NBUF && !sm100::mbar_wait_bounded(&acc_empty[b], ((li / NBUF) - 1) & 1, cta_abort, p.status_word,
                                                          SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit, 20))
                     break;                                   // timed out or aborted: issue nothing more
-#ifdef SHFLBW_COUNTERS
-                cnt_acc += clock64() - a0c;
-#endif
                 const uint32_t acc_base = tmem_base + b * Cfg::ACC_COLS;
                 for (int kt = 0; kt < num_k; ++kt, ++it) {
-#ifdef SHFLBW_COUNTERS
-                    if (!ready) {
-                        const long long w0 = clock64();
-                        sm100::mbar_wait_bounded(&full_bar[s], ph, cta_abort, p.status_word,
-                                                 SHFLBW_DEVSTAT_TIMEOUT_FULL, p.wait_limit, 20);
-                        cnt_wait += clock64() - w0; ++cnt_n;
-                    }
-#else
                     if (!ready && !sm100::mbar_wait_bounded(&full_bar[s], ph, cta_abort, p.status_word,
                                                             SHFLBW_DEVSTAT_TIMEOUT_FULL, p.wait_limit, 20))
                         goto mma_done;                       // timed out or aborted: issue nothing more
-#endif
-                    TRACE(1, it, 0);
                     // cp.async (generic proxy) data -> tensor-core (async proxy) reads; the copy engine's
                     // writes of the TMA gather are in the async proxy already
-                    if (!Cfg::TMA && !(ablate & 16)) sm100::fence_proxy_async_smem();
+                    if (!Cfg::TMA) sm100::fence_proxy_async_smem();
                     sm100::tc_fence_after_sync();
-                    int nk = (ablate & 1) ? 0 : min(KS, rows_total - kt * KS) / 16;
+                    int nk = min(KS, rows_total - kt * KS) / 16;
                     uint64_t gdj = gdesc0 + (uint64_t)((s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
                     uint64_t wdj = wdesc0 + (uint64_t)((s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
                     uint32_t accum = (uint32_t)(kt != 0);
@@ -899,31 +672,14 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                         wdj += WSTEP >> 4;
                         accum = 1u;
                     }
-#ifdef SHFLBW_ABLATE
-                    if (ablate & 4096) {   // release stages in pairs: one pipeline drain per two stages
-                        if (held >= 0 || kt + 1 == num_k) {
-                            if (held >= 0) sm100::umma_commit(&empty_bar[held]);
-                            sm100::umma_commit(&empty_bar[s]);
-                            held = -1;
-                        } else held = (int)s;
-                    } else
-#endif
-                    if (ablate & 64) sm100::mbar_arrive(&empty_bar[s]);
-                    else sm100::umma_commit(&empty_bar[s]);  // stage may be refilled once these MMAs retire
-                    TRACE(1, it, 1);
+                    sm100::umma_commit(&empty_bar[s]);  // stage may be refilled once these MMAs retire
                     // Test the next stage's barrier now: the round trip hides behind the MMAs just issued.
                     if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
                     ready = sm100::mbar_test(&full_bar[s], ph);
                 }
-                if (num_k > 0 && !(ablate & 1)) sm100::umma_commit(&acc_full[b]);  // accumulator complete
+                if (num_k > 0) sm100::umma_commit(&acc_full[b]);  // accumulator complete
                 else sm100::mbar_arrive(&acc_full[b]);                             // nothing to wait for
             }
-#ifdef SHFLBW_COUNTERS
-            if (p.trace != nullptr) {
-                unsigned long long* o = p.trace + blockIdx.x * 16;
-                o[0] = cnt_wait; o[1] = cnt_n; o[2] = cnt_acc; o[3] = clock64() - cnt_t0; o[4] = it;
-            }
-#endif
         mma_done:
             if (*cta_abort) {
                 // Aborted: the MMAs issued so far must retire before TMEM is freed and the block's
@@ -933,7 +689,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             }
         }
         __syncwarp();
-        if (lane == 0) CTRACE(3);
     } else {
         // -------------------------------------------------------------- epilogue ----
         // Warp w reads TMEM lane quadrant w % 4 (tokens) and half w / 4 % 2 of the accumulator
@@ -949,18 +704,12 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         const bool reads = half_id < HALVES;
         const __half alpha1 = __float2half_rn(p.alpha), beta1 = __float2half_rn(p.beta);
         const __half2 alpha2 = __half2half2(alpha1);
-#ifdef SHFLBW_COUNTERS
-        long long ec_wait = 0, ec_t0 = clock64();
-#endif
         bool res_primed = false;               // addend copies (RES_BYTES) run an item ahead
         for (int li = Cfg::ESETS > 1 ? warp >> 3 : 0; li < nloc; li += Cfg::ESETS) {
-#ifdef SHFLBW_COUNTERS
-            const long long ew0 = clock64();
-#endif
             const int item = (int)blockIdx.x + li * (int)gridDim.x;
             const int blk = item_block(item);
             const int n0 = item_tile(item) * T;
-            const bool has_k = item_tab[li].y > 0 && !(ablate & 1);
+            const bool has_k = item_tab[li].y > 0;
             const int b = li % NBUF;
             // Wait for the item's accumulator (one lane polls, the warp follows).  false: the wait
             // timed out or the block is aborting -- store nothing more.
@@ -971,10 +720,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                                                       SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit, 32);
                 if (!__shfl_sync(0xffffffffu, acc_ok, 0)) return false;
                 sm100::tc_fence_after_sync();
-#ifdef SHFLBW_COUNTERS
-                ec_wait += clock64() - ew0;
-#endif
-                if (tid == 0) TRACE(2, li, 0);
                 return true;
             };
             // Rows in lanes: the bias of this lane's row is one value for the whole item, requested before the
@@ -1012,7 +757,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     roff = (size_t)plane * (size_t)p.out_plane;
                     if (use_res) rres = (size_t)(p.res_map ? __ldg(p.res_map + blk * V + m) : blk * V + m) * (size_t)p.out_plane;
                 } else {
-                    const int drow = (p.perm && !(ablate & 1024)) ? __ldg(p.perm + blk * V + m) : blk * V + m;
+                    const int drow = (p.perm) ? __ldg(p.perm + blk * V + m) : blk * V + m;
                     roff = (size_t)drow * (size_t)p.N;
                 }
                 __half* const obase = CHAIN ? p.out : p.D;
@@ -1062,9 +807,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                         sm100::tc_fence_before_sync();
                         __syncwarp();
                         if (lane == 0) sm100::mbar_arrive(&acc_empty[b]);
-                        if (tid == 0) TRACE(2, li, 1);
                     }
-                    if (lane < LR && !(ablate & 520)) {
+                    if (lane < LR) {
                     uint4 v[4];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
@@ -1118,7 +862,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     }
                     __syncwarp();                                        // the next TMEM load is warp-wide
                 }
-                if (tid == 0) TRACE(2, li, 3);
                 continue;
             }
             // columns [col0, col0 + COLS) of the accumulator set: accumulator a = col / V, row m = col % V
@@ -1128,7 +871,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             const int a0 = col0 / V;                       // this warp's columns lie in one accumulator
             const int tok = reads ? n0 + a0 * 128 + quad * 32 + lane : p.N;   // idle warps store nothing
             const int mbase = col0 % V;                    // first block row / filter of this warp
-            bool ok = tok < p.N && !(ablate & 8);
+            bool ok = tok < p.N;
             uint32_t row_off[4];                           // SpConv: output offsets of positions i*8 + lane/4
             if constexpr (MODE == kPanelConv) {
                 const int pix = fast_div(tok, p.div_bp), img = tok - pix * p.Bp;
@@ -1164,7 +907,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             // and are written as zeros).
             auto group_offset = [&](int n0_, bool& ok_) -> uint32_t {
                 const int tok_g = reads ? n0_ + a0 * 128 + quad * 32 + tg * 8 : p.N;
-                ok_ = tok_g < p.N && !(ablate & 8);
+                ok_ = tok_g < p.N;
                 uint32_t goff_ = (uint32_t)tok_g;
                 if constexpr (MODE == kPanelConvChain) {
                     if (ok_) {
@@ -1200,7 +943,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             auto addend_at = [&](int blk_, uint32_t goff_, int cc, int i) -> const __half* {
                 const int m = mbase + cc + slot_row(i);
                 if (use_c) {
-                    const int row = (p.perm && !(ablate & 1024)) ? __ldg(p.perm + blk_ * V + m) : blk_ * V + m;
+                    const int row = (p.perm) ? __ldg(p.perm + blk_ * V + m) : blk_ * V + m;
                     if constexpr (BIAS) return p.C + row;
                     return p.C + (size_t)((uint32_t)row * (uint32_t)p.N) + (size_t)goff_;
                 }
@@ -1255,7 +998,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 for (int i = 0; i < NSLOT; ++i) {
                     const int m = mbase + cc + slot_row(i);
                     if constexpr (MODE == kPanelSpmm) {
-                        const int row = (p.perm && !(ablate & 1024)) ? __ldg(p.perm + blk * V + m) : blk * V + m;
+                        const int row = (p.perm) ? __ldg(p.perm + blk * V + m) : blk * V + m;
                         roff[i] = (uint32_t)row * (uint32_t)p.N;
                     } else {
                         const int plane = (p.out_logical && p.perm) ? __ldg(p.perm + blk * V + m) : blk * V + m;
@@ -1276,7 +1019,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                         sm100::tc_fence_before_sync();
                         __syncwarp();
                         if (lane == 0) sm100::mbar_arrive(&acc_empty[b]);
-                        if (tid == 0) TRACE(2, li, 1);
                     }
                     // Same epilogue arithmetic as the reference: round to fp16, then alpha (and
                     // beta * C, applied after the transpose) in fp16.
@@ -1296,7 +1038,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     }
                 }
                 if constexpr (BIAS && !IN_REGS) { if (need_add) fetch_addend(blk, goff, cc, addend[0]); }
-                if (!(ablate & 512)) {
+                {
 #pragma unroll
                     for (int k = 0; k < NSLOT / 2; ++k) {
                         const int q = 8 * k + (lane >> 2);   // 8 tokens of this lane's k-th row pair
@@ -1362,7 +1104,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                         sm100::tc_fence_before_sync();
                         __syncwarp();
                         if (lane == 0) sm100::mbar_arrive(&acc_empty[b]);
-                        if (tid == 0) TRACE(2, li, 1);
                     }
                     uint4 v;
                     __half2* h = (__half2*)&v;
@@ -1372,7 +1113,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     *(uint4*)(my_tile + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = v;
                 }
                 __syncwarp();
-                if (!(ablate & 512)) {
+                {
 #pragma unroll
                     for (int i = 0; i < 4; ++i) {
                         const int row = i * 8 + (lane >> 2), c = lane & 3;
@@ -1390,16 +1131,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 __syncwarp();
             }
             }
-            if (tid == 0) TRACE(2, li, 3);
         }
         if constexpr (Cfg::RES_BYTES > 0) sm100::cp_async_wait<0>();   // nothing of this warp is in flight when the block ends
-#ifdef SHFLBW_COUNTERS
-        if (lane == 0 && p.trace != nullptr && warp < 8) {   // per epilogue warp: cycles waiting for an accumulator, cycles in the role
-            unsigned long long* o = p.trace + 148 * 48 + (blockIdx.x * 8 + warp) * 2;
-            o[0] = ec_wait; o[1] = clock64() - ec_t0;
-        }
-#endif
-        if (tid == 0) CTRACE(4);
     }
 
     if (*cta_abort) {
@@ -1412,16 +1145,11 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     }
     sm100::tc_fence_before_sync();
     __syncthreads();
-    if (tid == 0) TRACE(3, 0, 1);
-    if (tid == 0) CTRACE(5);
     if (warp == EW) {
         sm100::tc_fence_after_sync();
         sm100::tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
     }
 }
 
-#undef TRACE
-#undef CTRACE
-#undef PTRACE
 
 }  // namespace shflbw

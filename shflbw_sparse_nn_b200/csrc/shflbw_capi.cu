@@ -112,11 +112,11 @@ int host_pipeline(shflbw_matrix* m, cudaStream_t* s_in, cudaStream_t* s_k, cudaS
 using PanelKernel = void (*)(const shflbw::PanelParams);
 struct PanelChoice { PanelKernel fn; size_t smem; int tokens; int stages; int pw; int threads; int variant; int gather; };
 
-template <int V, int TM, int KS, int STAGES, int PW, int MODE, int GROUPS = 2, int LAG = 1, int GATHER = shflbw::kGatherCpAsync,
+template <int V, int TM, int KS, int STAGES, int PW, int MODE, int GROUPS = 2, int GATHER = shflbw::kGatherCpAsync,
           int EW = 8, bool BIAS = false, bool ADDEND = false>
 PanelChoice choice() {
-    using Cfg = shflbw::PanelCfg<V, TM, KS, STAGES, PW, MODE, GROUPS, LAG, GATHER, EW, ADDEND>;
-    return {shflbw::panel_umma_kernel<V, TM, KS, STAGES, PW, MODE, GROUPS, LAG, GATHER, EW, BIAS, ADDEND>, (size_t)Cfg::SMEM_BYTES, Cfg::T,
+    using Cfg = shflbw::PanelCfg<V, TM, KS, STAGES, PW, MODE, GROUPS, GATHER, EW, ADDEND>;
+    return {shflbw::panel_umma_kernel<V, TM, KS, STAGES, PW, MODE, GROUPS, GATHER, EW, BIAS, ADDEND>, (size_t)Cfg::SMEM_BYTES, Cfg::T,
             STAGES, PW, Cfg::THREADS, 0, GATHER};
 }
 
@@ -150,51 +150,6 @@ int encode_b_map(const void* B, int K, int N, unsigned long long out[16]) {
     return SHFLBW_OK;
 }
 
-#ifdef SHFLBW_TUNE
-// Tuning builds only: SHFLBW_SHAPE="pw,groups,lag" picks the pipeline shape of the V = 64,
-// 256-token kernels (read at init and at exec, so a state follows the variable).
-template <int MODE>
-bool tuned_shape(PanelChoice* out) {
-    const char* e = getenv("SHFLBW_SHAPE");
-    if (!e) return false;
-    int pw = 0, groups = 0, lag = 0;
-    if (sscanf(e, "%d,%d,%d", &pw, &groups, &lag) != 3) return false;
-    switch (pw * 100 + groups * 10 + lag) {
-        case 821:  *out = choice<64, 2, 64, 5, 8, MODE, 2, 1>(); return true;
-        case 822:  *out = choice<64, 2, 64, 5, 8, MODE, 2, 2>(); return true;
-        case 811:  *out = choice<64, 2, 64, 5, 8, MODE, 1, 1>(); return true;
-        case 812:  *out = choice<64, 2, 64, 5, 8, MODE, 1, 2>(); return true;
-        case 1621: *out = choice<64, 2, 64, 5, 16, MODE, 2, 1>(); return true;
-        case 1622: *out = choice<64, 2, 64, 5, 16, MODE, 2, 2>(); return true;
-        case 1611: *out = choice<64, 2, 64, 5, 16, MODE, 1, 1>(); return true;
-        case 1612: *out = choice<64, 2, 64, 5, 16, MODE, 1, 2>(); return true;
-        case 1641: *out = choice<64, 2, 64, 5, 16, MODE, 4, 1>(); return true;
-        default: break;
-    }
-    switch (pw * 100 + groups * 10 + lag) {               // lag 3: cp.async with deferred arrivals
-        case 813:  *out = choice<64, 2, 64, 5, 8, MODE, 1, 1, shflbw::kGatherCpAsyncArrive>(); return true;
-        case 823:  *out = choice<64, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherCpAsyncArrive>(); return true;
-        case 1613: *out = choice<64, 2, 64, 5, 16, MODE, 1, 1, shflbw::kGatherCpAsyncArrive>(); return true;
-        case 1623: *out = choice<64, 2, 64, 5, 16, MODE, 2, 1, shflbw::kGatherCpAsyncArrive>(); return true;
-        case 1643: *out = choice<64, 2, 64, 5, 16, MODE, 4, 1, shflbw::kGatherCpAsyncArrive>(); return true;
-        default: break;
-    }
-    if constexpr (MODE == shflbw::kPanelSpmmRows) {   // lag 0: TMA gather
-        switch (pw * 100 + groups * 10 + lag) {
-            case 410:  *out = choice<64, 2, 64, 5, 4, MODE, 1, 1, shflbw::kGatherTma>(); return true;
-            case 810:  *out = choice<64, 2, 64, 5, 8, MODE, 1, 1, shflbw::kGatherTma>(); return true;
-            case 820:  *out = choice<64, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherTma>(); return true;
-            case 1610: *out = choice<64, 2, 64, 5, 16, MODE, 1, 1, shflbw::kGatherTma>(); return true;
-            case 1620: *out = choice<64, 2, 64, 5, 16, MODE, 2, 1, shflbw::kGatherTma>(); return true;
-            case 1640: *out = choice<64, 2, 64, 5, 16, MODE, 4, 1, shflbw::kGatherTma>(); return true;
-            case 840:  *out = choice<64, 2, 64, 5, 8, MODE, 4, 1, shflbw::kGatherTma>(); return true;
-            default: break;
-        }
-    }
-    return false;
-}
-#endif
-
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
 template <int MODE, bool BIAS = false>
@@ -207,44 +162,41 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
         // 256, the rest equal); eight in the instance without the slots.  Built for 64-row blocks.
         // wide_ring: 6 or 8 stages, 0 for the regular kernels.
         if (wide_ring && tile == 256 && V == 64) {
-            *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, 1, shflbw::kGatherCpAsync, 16, BIAS, false>()
-                                  : choice<64, 2, 32, 6, 3, MODE, 3, 1, shflbw::kGatherCpAsync, 16, BIAS, true>();
+            *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, false>()
+                                  : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, true>();
             return true;
         }
     }
     if constexpr (MODE == shflbw::kPanelSpmmRows || MODE == shflbw::kPanelConvChainRows) {   // rows in TMEM lanes: V must be a legal UMMA M
-#ifdef SHFLBW_TUNE
-        if (V == 64 && tile == 256 && tuned_shape<MODE>(out)) return true;
-#endif
         if constexpr (MODE == shflbw::kPanelSpmmRows) {
             // SpMM, 64-row blocks, 256-token items: the rows of B come by TMA tile-gather, issued by
             // 16 light producer warps in four groups (measured 3-6 % faster than the cp.async gather
             // on the 4096^3 case; the copy engine also applies the swizzle and zero-fills the N residue)
             if (gather == shflbw::kGatherTma && V == 64 && tile == 256) {
-                *out = choice<64, 2, 64, 5, 16, MODE, 4, 1, shflbw::kGatherTma, 8, BIAS>();
+                *out = choice<64, 2, 64, 5, 16, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
                 return true;
             }
         }
         switch (V * 1000 + tile) {
-            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
-            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
-            case 128128: *out = choice<128, 1, 64, 6, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
-            case 128256: *out = choice<128, 2, 64, 4, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
+            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
+            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
+            case 128128: *out = choice<128, 1, 64, 6, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
+            case 128256: *out = choice<128, 2, 64, 4, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
             default: return false;
         }
     } else {
         if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConv) {
             // 16-row blocks: UMMA N = 16, one or two 128-token accumulators per item (18 / 34 KB stages)
-            if (V == 16 && tile == 128) { *out = choice<16, 1, 64, 8, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true; }
-            if (V == 16 && tile == 256) { *out = choice<16, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true; }
+            if (V == 16 && tile == 128) { *out = choice<16, 1, 64, 8, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true; }
+            if (V == 16 && tile == 256) { *out = choice<16, 2, 64, 5, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true; }
         }
         switch (V * 1000 + tile) {
-            case 32128:  *out = choice<32, 1, 64, 8, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 20 KB stages
-            case 32256:  *out = choice<32, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 36 KB
-            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 24 KB
-            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 40 KB
-            case 128128: *out = choice<128, 1, 64, 6, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;   // 32 KB
-            case 128256: *out = choice<128, 2, 64, 4, 8, MODE, 2, 1, shflbw::kGatherCpAsync, 8, BIAS>(); return true;   // 48 KB
+            case 32128:  *out = choice<32, 1, 64, 8, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 20 KB stages
+            case 32256:  *out = choice<32, 2, 64, 5, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 36 KB
+            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 24 KB
+            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 40 KB
+            case 128128: *out = choice<128, 1, 64, 6, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;   // 32 KB
+            case 128256: *out = choice<128, 2, 64, 4, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;   // 48 KB
             default: return false;
         }
     }
@@ -556,10 +508,6 @@ static int launch_spmm_panel(const shflbw_spmm_state_t* st, const PanelChoice& c
     p.num_blocks = st->num_row_blocks; p.div_blocks = shflbw::make_fast_div(st->num_row_blocks);
     p.tile_major = 1;
     if (const char* e = getenv("SHFLBW_ITEM_ORDER")) p.tile_major = atoi(e) != 0;
-#if defined(SHFLBW_ABLATE) || defined(SHFLBW_COUNTERS)
-    if (const char* e = getenv("SHFLBW_ABLATE")) p.ablate = atoi(e);
-    if (const char* e = getenv("SHFLBW_TRACE_PTR")) p.trace = (unsigned long long*)strtoull(e, nullptr, 0);
-#endif
     CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
     CK(cudaGetLastError());
     return SHFLBW_OK;
@@ -941,10 +889,6 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     // to their outputs (SHFLBW_ITEM_ORDER=1 forces tile-major; tuning aid).
     p.tile_major = 0;
     if (const char* e = getenv("SHFLBW_ITEM_ORDER")) p.tile_major = atoi(e) != 0;
-#if defined(SHFLBW_ABLATE) || defined(SHFLBW_COUNTERS)
-    if (const char* e = getenv("SHFLBW_ABLATE")) p.ablate = atoi(e);
-    if (const char* e = getenv("SHFLBW_TRACE_PTR")) p.trace = (unsigned long long*)strtoull(e, nullptr, 0);
-#endif
     if (panel_bias) p.C = (const __half*)bias;
     CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
     // 3. back to NHWC in logical channel order.

@@ -94,10 +94,6 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst_smem, const void* src
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
 }
-// Subtracts `bytes` from the pending transaction count by hand (tuning builds that skip a copy).
-__device__ __forceinline__ void mbar_complete_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
 // TMA tile::gather4: rows r0..r3 of a 2-D tensor (tensor map box = W columns x 1 row), columns
 // [col, col + W), land as 4 consecutive rows of W elements at dst (swizzled as the map says) and
 // complete 4*W*elemsize bytes on the barrier.  Columns or rows outside the tensor read as zero.
@@ -131,12 +127,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-// Deferred arrival: the mbarrier receives one arrival (already counted in its expected
-// count, hence .noinc) once all cp.async copies this thread has issued so far have landed.
-// The issuing thread does not wait.
-__device__ __forceinline__ void cp_async_arrive_noinc(uint64_t* bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 // Generic-proxy writes (cp.async, st.shared) -> visible to the async proxy (tcgen05.mma reads).
 __device__ __forceinline__ void fence_proxy_async_smem() {
