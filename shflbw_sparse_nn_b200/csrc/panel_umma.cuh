@@ -28,15 +28,15 @@
 //                    accumulator columns; sixteen warps are two sets that take the items in turn.  Tokens in lanes: TMEM -> registers -> fp16 -> transpose
 //                    of 32-row chunks through shared memory -> 16-byte global stores (inverse row
 //                    permutation fused for SpMM).  Rows in lanes: stores straight from registers.
-//   warp  EW         allocates TMEM; its lane 0 issues tcgen05.mma, releases stages and
+//   warp  EW         allocates TMEM; an elected lane issues tcgen05.mma, releases stages and
 //                    accumulators with tcgen05.commit
 //   warps EW+1.. with w % 4 != 0   producers (PW of them, in GROUPS groups that take the stages in
 //                    turn).  cp.async gather: 16-byte copies into 128-byte-swizzled stages; a
 //                    group publishes its previous stage half-way through issuing the next one,
 //                    with ONE mbarrier arrival per warp; row ids are prefetched two of the
 //                    group's stages ahead by 4-byte cp.async into a shared-memory ring.  TMA
-//                    gather: one tile::gather4 per lane, completion by byte count.  One bulk copy
-//                    per stage for the value slice either way.
+//                    gather: every warp fills stages of its own with tile::gather4 copies, completion by
+//                    byte count.  One bulk copy per stage for the value slice either way.
 //   later warps with w % 4 == 0   idle, so that no producer shares the MMA warp's scheduler partition.
 // The accumulator is double buffered in TMEM (four sets with EW = 16) so the epilogue of item i
 // overlaps the main loop of item i+1, and the stage ring runs across item boundaries without
@@ -139,10 +139,10 @@ constexpr int kPanelSpmm = 0, kPanelConv = 1, kPanelConvChain = 2, kPanelSpmmRow
 // GATHER: how the rows of the dense operand reach shared memory.
 //   kGatherCpAsync  16-byte cp.async per lane, written straight into the swizzled layout; the
 //                   producer warps wait for their copies and publish the stage themselves.
-//   kGatherTma      TMA tile::gather4: one instruction per lane fetches 4 rows x 64 tokens (the
-//                   tensor map covers this GPU's own B; no multicast), the copy engine applies
-//                   the 128-byte swizzle and completes the stage's barrier by byte count, so the
-//                   producers never wait for data.  SpMM with rows in lanes only.
+//   kGatherTma      TMA tile::gather4: one instruction fetches 4 rows x 64 tokens (the tensor map covers
+//                   this GPU's own dense operand; no multicast), the copy engine applies the 128-byte
+//                   swizzle and completes the stage's barrier by byte count, so the producers never
+//                   wait for data.
 constexpr int kGatherCpAsync = 0, kGatherTma = 1;
 
 // EW: epilogue warps, 8 or 16.  A warp can read only the TMEM lane quadrant warp % 4, so the two
@@ -164,26 +164,9 @@ struct PanelCfg {
     // w % 4 == 0 stay idle.  The MMA warp executes a
     // few dozen instructions per stage and was measured at ~20 clk per instruction when
     // producer code kept evicting its lines from the partition's instruction cache.
-    static constexpr int WARPS_USED = EW + 1 + PW + (PW - 1) / 3;   // epilogue + MMA + producers + idle
-    // Register budgets per role.  Up to 20 warps every thread can have the ~100 registers the
-    // epilogue wants.  Beyond that the block is padded to whole warpgroups (4 warps) and
-    // launched at 65536 / threads registers per thread; the producer / MMA warpgroups then give
-    // registers back (setmaxnreg.dec) and the two epilogue warpgroups take them (setmaxnreg.inc).
-    // (With 16 epilogue warps the block is 20 warps at 96 registers and is not split.)
-    static constexpr bool REG_SPLIT = EW == 8 && WARPS_USED > 20;
-    static_assert(EW == 8 || WARPS_USED <= 20, "16 epilogue warps: at most 3 producers (20 warps leave 96 registers per thread, 21-24 only 80)");
-    static constexpr int WARPS = REG_SPLIT ? (WARPS_USED + 3) / 4 * 4 : WARPS_USED;
+    static constexpr int WARPS = EW + 1 + PW + (PW - 1) / 3;   // epilogue + MMA + producers + idle
+    static_assert(EW == 8 || WARPS <= 20, "16 epilogue warps: at most 3 producers (20 warps leave 96 registers per thread, 21-24 only 80)");
     static constexpr int THREADS = WARPS * 32;
-    static constexpr int REGS_LEAN = 56;                                    // producers, MMA warp, idle warps
-    static constexpr int REGS_EPI_RAW = (65536 - (WARPS - 8) * 32 * REGS_LEAN) / 256 / 8 * 8;
-    static constexpr int REGS_EPI = REGS_EPI_RAW > 160 ? 160 : REGS_EPI_RAW;
-    static_assert(!REG_SPLIT || REGS_EPI >= 88, "epilogue register budget");
-    // Only the 32-warp block is used with the split: 1024 threads x 64 registers is exactly the
-    // register file, so what the lean warpgroups return is exactly what the epilogue's increase
-    // asks for.  (24-warp blocks launched at 80 registers were seen to block in setmaxnreg.inc:
-    // the allocation granularity leaves less in the pool than the arithmetic says, and that wait
-    // has no time limit.)
-    static_assert(!REG_SPLIT || WARPS == 32, "register split: 32-warp blocks only");
     static constexpr int G_ACC = KS * 256;                 // gathered tile of one accumulator: [KS][128] fp16
     static constexpr int G_BYTES = TM * G_ACC;
     static constexpr int W_BYTES = KS * V * 2;
@@ -205,7 +188,7 @@ struct PanelCfg {
     static constexpr int IDX_AHEAD = 2;                    // a group fetches row ids this many of its stages ahead
     static constexpr int IDX_RING = (IDX_AHEAD + 1) * GROUPS <= 8 ? 8 : 16;   // stages of row ids kept in shared memory
     static_assert((IDX_AHEAD + 1) * GROUPS <= IDX_RING, "row-id ring too small");
-    static constexpr int IDX_BYTES = TMA ? 0 : IDX_RING * KS * 4;   // (the TMA gather loads its row ids straight into registers)
+    static constexpr int IDX_BYTES = (TMA ? PW : IDX_RING) * KS * 4;     // (TMA gather: one stage of row ids per producer warp)
     static constexpr int SMEM_BYTES = PIPE_BYTES + OUT_BYTES + RES_BYTES + BAR_BYTES + TAB_BYTES + IDX_BYTES + 1024;  // + align slack
     static constexpr bool SWAP = MODE == kPanelSpmmRows || MODE == kPanelConvChainRows;
     static constexpr int KG_BYTES = SWAP ? T * 16 : 2048;   // 8 gathered rows (one K group) of the token tile
@@ -222,10 +205,10 @@ struct PanelCfg {
     static constexpr uint32_t TMEM_COLS = NBUF * ACC_COLS < 32 ? 32 : NBUF * ACC_COLS;
     static_assert(V == 16 || V == 32 || V == 64 || V == 128, "row-block height");
     static_assert(V != 16 || !SWAP, "16-row blocks: tokens in lanes");
-    static_assert(!TMA || (MODE == kPanelSpmmRows && V == 64), "TMA gather: SpMM with rows in lanes, 64-row blocks");
+    static_assert(!TMA || (GROUPS == PW && PW <= STAGES), "TMA gather: every producer warp fills stages of its own");
     static_assert(STAGE_BYTES % 1024 == 0, "stages must keep 1024-byte swizzle-atom alignment");
     static_assert((TMEM_COLS & (TMEM_COLS - 1)) == 0 && TMEM_COLS <= 512, "TMEM columns");
-    static_assert(KS % 16 == 0 && PW % GROUPS == 0 && KS % (PW / GROUPS) == 0 && (KS / (PW / GROUPS)) % (32 / (T / 8)) == 0,
+    static_assert(KS % 32 == 0 && PW % GROUPS == 0 && (TMA || (KS % (PW / GROUPS) == 0 && (KS / (PW / GROUPS)) % (32 / (T / 8)) == 0)),
                   "rows per producer warp");
     static_assert(TMA || STAGES > GROUPS, "a group publishes a stage while issuing its next one");
     static_assert(SMEM_BYTES <= 227 * 1024, "shared memory budget");
@@ -283,7 +266,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     int2* item_tab = (int2*)(bar_area + Cfg::BAR_BYTES);  // [nloc] (first padded row, padded row count)
     int* idx_ring = (int*)(bar_area + Cfg::BAR_BYTES + Cfg::TAB_BYTES);  // [IDX_RING][KS] row ids of upcoming stages
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     // This CTA's work items: blockIdx.x, blockIdx.x + gridDim.x, ...  (host guarantees nloc <= table size)
     const int nloc = (p.num_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;
     auto item_block = [&](int item) { return p.tile_major ? item - fast_div(item, p.div_blocks) * p.num_blocks : fast_div(item, p.div_tiles); };
@@ -291,11 +274,9 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 
     if (tid == 0) {
         for (int s = 0; s < STAGES; ++s) {
-            // One arrival per producer WARP.  Per-thread deferred arrivals
-            // (cp.async.mbarrier.arrive.noinc) were measured at ~3 clk of load/store-unit time
-            // per thread, i.e. more than the copies themselves.
-            // cp.async gather: one arrival per producer WARP of the group.  TMA gather: one arrival
-            // (with the stage's byte count) by the group's first warp.
+            // cp.async gather: one arrival per producer WARP of the group (per-thread deferred arrivals,
+            // cp.async.mbarrier.arrive.noinc, were measured at ~3 clk of load/store-unit time per thread,
+            // i.e. more than the copies themselves).  TMA gather: one arrival, with the stage's byte count.
             sm100::mbar_init(&full_bar[s], Cfg::TMA ? 1 : PW / Cfg::GROUPS);
             sm100::mbar_init(&empty_bar[s], 1);   // one tcgen05.commit per drain
         }
@@ -319,7 +300,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     sm100::tc_fence_before_sync();
     __syncthreads();
     sm100::tc_fence_after_sync();
-    const uint32_t tmem_base = *tmem_slot;
+    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t smem_base = sm100::smem_u32(smem);
     // Programmatic dependent launch: everything above (barriers, TMEM, the item table -- read from
     // the sparse operand, which no kernel writes) may overlap the tail of the previous kernel in
@@ -337,97 +318,110 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     // touches no global memory and does not wait.
 
     const int pidx = warp - (EW + 1) - (warp / 4 - EW / 4);   // producer number of a producer warp (warps after the MMA warp with warp % 4 != 0)
-    if constexpr (Cfg::REG_SPLIT) {
-        // Whole warpgroups change their register budget together: warps 0-7 (epilogue) grow,
-        // every other warpgroup (MMA warp, producers, idle and padding warps) shrinks first.
-        if (warp < EW) sm100::setmaxnreg_inc<Cfg::REGS_EPI>();
-        else sm100::setmaxnreg_dec<Cfg::REGS_LEAN>();
-    }
     if (warp > EW && ((warp & 3) == 0 || pidx >= PW)) {
-        // idle: keeps producers off the MMA warp's scheduler partition (or pads the last warpgroup)
+        // idle: keeps producers off the MMA warp's scheduler partition
     } else if (warp > EW && Cfg::TMA) {
         // ---------------------------------------------------- producers (TMA gather) ----
         // A stage is KS gathered rows x T tokens = (KS/4) row quads x (T/64) column boxes, one
-        // tile::gather4 each (4 rows x 128 bytes, landing as half a swizzle atom).  The GW warps
-        // of a group split the stage's operations, one per lane; the group's first warp also
-        // posts the stage's byte count and the bulk copy of the value slice.  Nobody waits for
-        // data: the barrier completes when the bytes have arrived.
+        // tile::gather4 each (4 rows x 128 bytes, landing as half a swizzle atom).  Every producer warp
+        // fills stages of its own (stage it by warp it % PW), all operations issued by an elected lane,
+        // and the stage's barrier completes by byte count: nobody waits for data.  Bound by the copy
+        // engine's 9.6 clk per operation, 53 bytes a clock and SM.  Four warps: one of them spends 970 clk
+        // on issuing a 64 x 256 stage, the ring passes one in 570-620 (two warps per stage 610, four 620;
+        // one operation per lane instead of an elected lane: 640 and 1540 clk of issue).  Stage time of
+        // the 4096^3 product: 1174 -> 620 clk.
+        // A warp shares its stages with no other warp: a warp of a shared stage that has no row to fetch (a
+        // short last stage) is not waited for by anyone, can fall a whole ring behind, miss the phase that it
+        // waits for and wait for good.
         if constexpr (Cfg::TMA) {
-        constexpr int GROUPS = Cfg::GROUPS, GW = PW / GROUPS;
-        constexpr int BOXES = T / 64;                       // column boxes per row quad
-        constexpr int OPS = (KS / 4) * BOXES / GW;          // operations per warp per stage
-        static_assert((KS / 4) * BOXES % GW == 0 && OPS >= 1 && OPS <= 32, "gather4 operations per producer warp");
-        const int grp = pidx / GW, pw = pidx % GW;
-        const int opj = pw * OPS + lane;                    // this lane's operation of a stage
-        const int quad = opj / BOXES, cbox = opj % BOXES;
-        const bool issuer = lane < OPS;
-        const uint32_t dst_off = (uint32_t)((quad >> 1) * Cfg::KG_BYTES + cbox * 1024 + (quad & 1) * 512);
-        struct Cursor { int li, kt, num_k, row_begin, rows_total; };
-        auto enter = [&](Cursor& c) {
-            c.kt = 0;
-            while (c.li < nloc) {
-                const int2 e = item_tab[c.li];
-                c.row_begin = e.x; c.rows_total = e.y; c.num_k = (e.y + KS - 1) / KS;
-                if (c.num_k > 0) return;
-                ++c.li;
+        constexpr int BOXES = T / 64, QUADS = KS / 4;       // column boxes per row quad, row quads
+        constexpr int IPL = KS / 32;                        // row ids per lane
+        int* const my_ids = idx_ring + pidx * KS;           // row ids of this warp's current stage
+        if (sm100::elect_one()) sm100::prefetch_tensormap(p.tmap_b);
+        // (item, stage of the item) of this warp's next stage
+        int li = 0, kt = pidx, row_begin = 0, rows_total = 0;
+        auto settle = [&]() {                               // stages beyond an item's end belong to the items after it
+            while (li < nloc) {
+                const int2 e = item_tab[li];
+                const int num_k = (e.y + KS - 1) / KS;
+                row_begin = e.x; rows_total = e.y;
+                if (kt < num_k) return;
+                kt -= num_k;
+                ++li;
             }
-            c.num_k = 0; c.row_begin = 0; c.rows_total = 0;
         };
-        auto advance = [&](Cursor& c) { if (++c.kt >= c.num_k) { ++c.li; enter(c); } };
-        // The 4 row ids of this lane's quad, loaded two of the group's stages ahead (registers).
-        auto load_ids = [&](const Cursor& c) {
-            const int r = c.kt * KS + quad * 4;
-            if (issuer && c.li < nloc && r < c.rows_total) return __ldg((const int4*)(p.blk_idx + c.row_begin + r));
-            return make_int4(0, 0, 0, 0);
+        int id[IPL];
+        auto load_ids = [&]() {
+#pragma unroll
+            for (int i = 0; i < IPL; ++i) {
+                const int r = kt * KS + i * 32 + lane;
+                id[i] = li < nloc && r < rows_total ? __ldg(p.blk_idx + row_begin + r) : 0;
+            }
         };
-        Cursor pre{0, 0, 0, 0, 0};
-        enter(pre);
-        for (int d = 0; d < grp; ++d) advance(pre);
-        int4 ids = load_ids(pre);                            // this group's first stage
-        for (int g = 0; g < GROUPS; ++g) advance(pre);
-        int4 ids_next = load_ids(pre);                       // and its second: two stages of ids are in flight,
-        for (int g = 0; g < GROUPS; ++g) advance(pre);       // which covers the load's latency even with one group
-        sm100::grid_dependency_wait();                       // the dense operand may be the previous kernel's output
-        int it = 0;
-        for (int li = 0; li < nloc; ++li) {
-            const int2 ent = item_tab[li];
-            const int num_k = (ent.y + KS - 1) / KS;
-            if (num_k == 0) continue;
-            const int item = (int)blockIdx.x + li * (int)gridDim.x;
-            const int col = item_tile(item) * T + cbox * 64;     // first token of this lane's box (beyond N: zero fill)
-            const __half* wsrc = p.blk_val + (size_t)ent.x * V;
-            for (int kt = 0; kt < num_k; ++kt, ++it) {
-                if ((it % GROUPS) != grp) continue;
-                const int s = it % STAGES;
-                if (it >= STAGES) {
-                    int ok = 1;
-                    if (lane == 0)
-                        ok = sm100::mbar_wait_bounded(&empty_bar[s], ((it / STAGES) - 1) & 1, cta_abort, p.status_word,
-                                                      SHFLBW_DEVSTAT_TIMEOUT_EMPTY, p.wait_limit, 32);
-                    if (!__shfl_sync(0xffffffffu, ok, 0)) goto tma_producer_done;
-                }
-                const int rows_valid = min(KS, ent.y - kt * KS);    // multiple of 16
+        settle();
+        load_ids();
+        sm100::grid_dependency_wait();                      // the dense operand may be the previous kernel's output
+        uint32_t s = pidx, ph = 1;                          // ring slot and the parity that says it is free (at first it is)
+        int xs[BOXES], nbox = 0, of_item = -1;              // first column of each box, boxes that hold any token
+        int it = pidx;
+        while (li < nloc) {
+            if (of_item != li) {
+                of_item = li;
+                const int tok0 = item_tile((int)blockIdx.x + li * (int)gridDim.x) * T;
+                nbox = min(BOXES, (p.N - tok0 + 63) / 64);   // columns beyond N are never stored: boxes past it are not fetched
+#pragma unroll
+                for (int b = 0; b < BOXES; ++b) xs[b] = tok0 + b * 64;
+            }
+#pragma unroll
+            for (int i = 0; i < IPL; ++i) my_ids[i * 32 + lane] = id[i];
+            const int rows_valid = min(KS, rows_total - kt * KS);   // multiple of 16
+            const __half* wsrc = p.blk_val + (size_t)(row_begin + kt * KS) * V;
+            if (!sm100::mbar_wait_warp(&empty_bar[s], ph, cta_abort, p.status_word, SHFLBW_DEVSTAT_TIMEOUT_EMPTY, p.wait_limit)) break;
+            __syncwarp();                                    // the row ids are in place
+            if (sm100::elect_one()) {
                 const uint32_t st_base = smem_base + s * Cfg::STAGE_BYTES;
-                if (pw == 0 && lane == 0) {
-                    const uint32_t wbytes = (uint32_t)(rows_valid * V * 2);
+                const uint32_t wbytes = (uint32_t)(rows_valid * V * 2), bytes = (uint32_t)(rows_valid * nbox * 128) + wbytes;
 #ifdef SHFLBW_FAULT_INJECT
-                    if (!(p.inject_from >= 0 && it >= p.inject_from && pidx == 0))   // the withheld arrival
+                if (p.inject_from >= 0 && it >= p.inject_from) sm100::mbar_expect_tx(&full_bar[s], bytes);   // the withheld arrival
+                else
 #endif
-                    sm100::mbar_arrive_expect_tx(&full_bar[s], (uint32_t)(rows_valid * T * 2) + wbytes);
-                    sm100::bulk_copy_g2s(st_base + (uint32_t)Cfg::G_BYTES, wsrc + (size_t)kt * KS * V, wbytes, &full_bar[s]);
+                sm100::mbar_arrive_expect_tx(&full_bar[s], bytes);
+                sm100::bulk_copy_g2s(st_base + (uint32_t)Cfg::G_BYTES, wsrc, wbytes, &full_bar[s]);
+                // All row ids come into registers before the first copy: the copies are ordered with
+                // respect to reads of shared memory, which would each add their latency.
+                int4 r[QUADS];
+#pragma unroll
+                for (int q = 0; q < QUADS; ++q) r[q] = *(const int4*)(my_ids + q * 4);
+                // rows in lanes: [K group][T/64 atoms]; tokens in lanes: [128-token half][K group][2 atoms]
+                auto copy = [&](int q, int b) {
+                    const uint32_t off = SWAP ? (uint32_t)((q >> 1) * Cfg::KG_BYTES + b * 1024 + (q & 1) * 512)
+                                              : (uint32_t)((b >> 1) * Cfg::G_ACC + (q >> 1) * 2048 + (b & 1) * 1024 + (q & 1) * 512);
+                    sm100::tma_gather4(st_base + off, p.tmap_b, xs[b], r[q].x, r[q].y, r[q].z, r[q].w, &full_bar[s]);
+                };
+                if (rows_valid == KS && nbox == BOXES) {     // a whole stage: straight-line code
+#pragma unroll
+                    for (int q = 0; q < QUADS; ++q)
+#pragma unroll
+                        for (int b = 0; b < BOXES; ++b) copy(q, b);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < QUADS; ++q)
+#pragma unroll
+                        for (int b = 0; b < BOXES; ++b)
+                            if (q * 4 < rows_valid && b < nbox) copy(q, b);
                 }
-                if (issuer && quad * 4 < rows_valid) {
-                    sm100::tma_gather4(st_base + dst_off, p.tmap_b, col, ids.x, ids.y, ids.z, ids.w, &full_bar[s]);
-                }
-                ids = ids_next;
-                ids_next = load_ids(pre);
-                for (int g = 0; g < GROUPS; ++g) advance(pre);
             }
+            __syncwarp();                                    // the row ids may be overwritten
+            it += PW; s += PW;
+            if (s >= (uint32_t)STAGES) { s -= STAGES; ph ^= 1u; }
+            kt += PW;
+            settle();
+            load_ids();
         }
-    tma_producer_done:;
         }
     } else if (warp > EW) {
-        // ------------------------------------------------------------- producers ----
+        // --------------------------------------------- producers (cp.async gather) ----
+        if constexpr (!Cfg::TMA) {
         // The PW producer warps form GROUPS groups that take the CTA's stages in turn (group g
         // fills stages g, g+GROUPS, ...).  While one group sits in its barrier round trip
         // (wait for the free stage, wait for its copies, publish) the other one issues copies,
@@ -529,13 +523,9 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             for (int kt = 0; kt < num_k; ++kt, ++it) {
                 if ((it % GROUPS) != grp) continue;            // the other group's stage
                 const int s = it % STAGES, s_idx = it % Cfg::IDX_RING;
-                if (it >= STAGES) {  // one lane polls; the warp follows through the broadcast of its result
-                    int ok = 1;
-                    if (lane == 0)
-                        ok = sm100::mbar_wait_bounded(&empty_bar[s], ((it / STAGES) - 1) & 1, cta_abort, p.status_word,
-                                                      SHFLBW_DEVSTAT_TIMEOUT_EMPTY, p.wait_limit, 32);
-                    if (!__shfl_sync(0xffffffffu, ok, 0)) goto producer_done;   // timed out or aborted: stop issuing
-                }
+                if (it >= STAGES && !sm100::mbar_wait_warp(&empty_bar[s], ((it / STAGES) - 1) & 1, cta_abort, p.status_word,
+                                                           SHFLBW_DEVSTAT_TIMEOUT_EMPTY, p.wait_limit))
+                    goto producer_done;                        // timed out or aborted: stop issuing
                 const int rows_valid = min(KS, ent.y - kt * KS);  // multiple of 16
                 const uint32_t st_base = smem_base + s * Cfg::STAGE_BYTES;
                 // The group's stage before this one is published half-way through this stage's
@@ -607,12 +597,12 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         __syncwarp();
         if (lane == 0 && pend >= 0) sm100::mbar_arrive(&full_bar[pend]);
         if (MODE == kPanelConv && p.trigger_late) sm100::grid_dependency_launch();
+        }
     } else if (warp == EW) {
         // ------------------------------------------------------------ MMA warp ----
         constexpr uint32_t idesc = SWAP ? sm100::make_idesc_f16_mnmajor(V, T) : sm100::make_idesc_f16_mnmajor(128, V);
         // Descriptors are built once; per MMA only the 16-byte-granular start address field
-        // (low bits) advances.  A single thread issues every MMA, so scalar work between two
-        // tcgen05.mma instructions directly limits the tensor-pipe issue rate.
+        // (low bits) advances.
         const uint64_t gdesc0 = sm100::make_smem_desc(smem_base, 1024, Cfg::KG_BYTES, sm100::kSwizzle128B);
         const uint64_t wdesc0 =
             V == 16 ? sm100::make_smem_desc(smem_base + Cfg::G_BYTES, 256, 256, sm100::kSwizzle32B)
@@ -620,73 +610,59 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
           : V == 64 ? sm100::make_smem_desc(smem_base + Cfg::G_BYTES, 1024, 1024, sm100::kSwizzle128B)
                     : sm100::make_smem_desc(smem_base + Cfg::G_BYTES, 1024, 2048, sm100::kSwizzle128B);
         constexpr uint32_t WSTEP = V * 32;  // bytes per K-step (16 rows) of the value tile
-        // One thread runs the whole role (tcgen05.mma / commit are single-thread instructions):
-        // no per-stage warp synchronisation, and the ring slot and its parity are carried
-        // instead of being recomputed by division.
-        if (lane == 0) {
-            int it = 0;
-            uint32_t s = 0, ph = 0;     // ring slot of stage `it` and the parity of its full barrier
-            bool ready = false;         // that barrier was already seen complete
-            for (int li = 0; li < nloc; ++li) {
-                const int rows_total = item_tab[li].y;
-                const int num_k = (rows_total + KS - 1) / KS;
-                const int b = li % NBUF;
-                if (li >= NBUF && !sm100::mbar_wait_bounded(&acc_empty[b], ((li / NBUF) - 1) & 1, cta_abort, p.status_word,
-                                                         SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit, 20))
-                    break;                                   // timed out or aborted: issue nothing more
-                const uint32_t acc_base = tmem_base + b * Cfg::ACC_COLS;
-                for (int kt = 0; kt < num_k; ++kt, ++it) {
-                    if (!ready && !sm100::mbar_wait_bounded(&full_bar[s], ph, cta_abort, p.status_word,
-                                                            SHFLBW_DEVSTAT_TIMEOUT_FULL, p.wait_limit, 20))
-                        goto mma_done;                       // timed out or aborted: issue nothing more
-                    // cp.async (generic proxy) data -> tensor-core (async proxy) reads; the copy engine's
-                    // writes of the TMA gather are in the async proxy already
-                    if (!Cfg::TMA) sm100::fence_proxy_async_smem();
-                    sm100::tc_fence_after_sync();
-                    int nk = min(KS, rows_total - kt * KS) / 16;
-                    uint64_t gdj = gdesc0 + (uint64_t)((s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
-                    uint64_t wdj = wdesc0 + (uint64_t)((s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
-                    uint32_t accum = (uint32_t)(kt != 0);
-                    if constexpr (SWAP) {
-                        // A full stage (the common case) is issued as straight-line code: one thread
-                        // issues every MMA, so the scalar work between two of them is what limits
-                        // the issue rate; the descriptor steps are immediates here.
-                        if (nk == KS / 16) {
+        // The warp runs the role in lock step and one elected lane issues (elect_one): the ring slot, its
+        // parity and the descriptors are then uniform to the compiler, and an MMA is a few instructions.
+        // (One thread running the role alone: 54 clk per MMA whatever its shape, 1174 clk per stage of the
+        // 4096^3 product at V = 64, 1420 at V = 128.)
+        bool ok = true;
+        uint32_t s = 0, ph = 0;         // ring slot of the next stage and the parity of its full barrier
+        for (int li = 0; li < nloc && ok; ++li) {
+            const int rows_total = __shfl_sync(0xffffffffu, item_tab[li].y, 0);
+            const int num_k = (rows_total + KS - 1) / KS;
+            const int b = li % NBUF;
+            if (li >= NBUF && !(ok = sm100::mbar_wait_warp(&acc_empty[b], ((li / NBUF) - 1) & 1, cta_abort, p.status_word,
+                                                           SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit)))
+                break;                                       // timed out or aborted: issue nothing more
+            const uint32_t acc_base = tmem_base + b * Cfg::ACC_COLS;
+            for (int kt = 0; kt < num_k; ++kt) {
+                if (!(ok = sm100::mbar_wait_warp(&full_bar[s], ph, cta_abort, p.status_word, SHFLBW_DEVSTAT_TIMEOUT_FULL, p.wait_limit)))
+                    break;
+                // cp.async (generic proxy) data -> tensor-core (async proxy) reads; the copy engine's
+                // writes of the TMA gather are in the async proxy already
+                if (!Cfg::TMA) sm100::fence_proxy_async_smem();
+                sm100::tc_fence_after_sync();
+                if (sm100::elect_one()) {
+                    const int nk = min(KS, rows_total - kt * KS) / 16;
+                    const uint64_t gd = gdesc0 + (uint64_t)((s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
+                    const uint64_t wd = wdesc0 + (uint64_t)((s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
 #pragma unroll
-                            for (int j = 0; j < KS / 16; ++j)
-                                sm100::umma_f16_ss(acc_base, wdj + (uint64_t)(j * (WSTEP >> 4)), gdj + (uint64_t)(j * ((2 * Cfg::KG_BYTES) >> 4)),
-                                                   idesc, j == 0 ? accum : 1u);
-                            nk = 0;
+                    for (int j = 0; j < KS / 16; ++j) {
+                        if (j < nk) {
+                            const uint64_t gdj = gd + (uint64_t)(j * ((2 * Cfg::KG_BYTES) >> 4)), wdj = wd + (uint64_t)(j * (WSTEP >> 4));
+                            const uint32_t accum = j > 0 || kt > 0;
+                            if constexpr (SWAP) {
+                                sm100::umma_f16_ss(acc_base, wdj, gdj, idesc, accum);   // D[row][token] += W^T . G
+                            } else {
+#pragma unroll
+                                for (int a = 0; a < TM; ++a)
+                                    sm100::umma_f16_ss(acc_base + a * V, gdj + (uint64_t)((a * Cfg::G_ACC) >> 4), wdj, idesc, accum);
+                            }
                         }
                     }
-#pragma unroll 1
-                    for (int j = 0; j < nk; ++j) {
-                        if constexpr (SWAP) {
-                            sm100::umma_f16_ss(acc_base, wdj, gdj, idesc, accum);   // D[row][token] += W^T . G
-                        } else {
-#pragma unroll
-                            for (int a = 0; a < TM; ++a)
-                                sm100::umma_f16_ss(acc_base + a * V, gdj + (uint64_t)((a * Cfg::G_ACC) >> 4), wdj, idesc, accum);
-                        }
-                        gdj += (2 * Cfg::KG_BYTES) >> 4;
-                        wdj += WSTEP >> 4;
-                        accum = 1u;
-                    }
-                    sm100::umma_commit(&empty_bar[s]);  // stage may be refilled once these MMAs retire
-                    // Test the next stage's barrier now: the round trip hides behind the MMAs just issued.
-                    if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
-                    ready = sm100::mbar_test(&full_bar[s], ph);
+                    sm100::umma_commit(&empty_bar[s]);       // stage may be refilled once these MMAs retire
+                    if (kt + 1 == num_k) sm100::umma_commit(&acc_full[b]);   // accumulator complete
                 }
-                if (num_k > 0) sm100::umma_commit(&acc_full[b]);  // accumulator complete
-                else sm100::mbar_arrive(&acc_full[b]);                             // nothing to wait for
+                __syncwarp();
+                if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
             }
-        mma_done:
-            if (*cta_abort) {
-                // Aborted: the MMAs issued so far must retire before TMEM is freed and the block's
-                // shared memory goes away.  One more commit, awaited with its own (short) limit.
-                sm100::umma_commit(drain_bar);
-                sm100::mbar_wait_bounded(drain_bar, 0, cta_abort, p.status_word, 0, 4000000LL, 100, /*heed_abort=*/false);
-            }
+            if (num_k == 0 && lane == 0) sm100::mbar_arrive(&acc_full[b]);   // nothing to wait for
+            __syncwarp();
+        }
+        if (__any_sync(0xffffffffu, *cta_abort) && sm100::elect_one()) {
+            // Aborted: the MMAs issued so far must retire before TMEM is freed and the block's
+            // shared memory goes away.  One more commit, awaited with its own (short) limit.
+            sm100::umma_commit(drain_bar);
+            sm100::mbar_wait_bounded(drain_bar, 0, cta_abort, p.status_word, 0, 4000000LL, /*heed_abort=*/false);
         }
         __syncwarp();
     } else {
@@ -711,14 +687,12 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             const int n0 = item_tile(item) * T;
             const bool has_k = item_tab[li].y > 0;
             const int b = li % NBUF;
-            // Wait for the item's accumulator (one lane polls, the warp follows).  false: the wait
+            // Wait for the item's accumulator (the whole warp).  false: the wait
             // timed out or the block is aborting -- store nothing more.
             auto wait_accumulator = [&]() -> bool {
-                int acc_ok = 1;
-                if (lane == 0)
-                    acc_ok = sm100::mbar_wait_bounded(&acc_full[b], (li / NBUF) & 1, cta_abort, p.status_word,
-                                                      SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit, 32);
-                if (!__shfl_sync(0xffffffffu, acc_ok, 0)) return false;
+                if (!sm100::mbar_wait_warp(&acc_full[b], (li / NBUF) & 1, cta_abort, p.status_word,
+                                           SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit))
+                    return false;
                 sm100::tc_fence_after_sync();
                 return true;
             };

@@ -152,6 +152,14 @@ int encode_b_map(const void* B, int K, int N, unsigned long long out[16]) {
 
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
+// Shapes of the TMA gather: four producer warps, each a group of its own.
+template <int V, int TM, int STAGES, int MODE, bool BIAS>
+PanelChoice regular(int gather) {
+    if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelSpmmRows) {
+        if (gather == shflbw::kGatherTma) return choice<V, TM, 64, STAGES, 4, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
+    }
+    return choice<V, TM, 64, STAGES, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>();
+}
 template <int MODE, bool BIAS = false>
 bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsync, int wide_ring = 0) {
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
@@ -162,41 +170,39 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
         // 256, the rest equal); eight in the instance without the slots.  Built for 64-row blocks.
         // wide_ring: 6 or 8 stages, 0 for the regular kernels.
         if (wide_ring && tile == 256 && V == 64) {
+            if constexpr (MODE == shflbw::kPanelSpmm) {
+                if (gather == shflbw::kGatherTma) {
+                    *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherTma, 16, BIAS, false>()
+                                          : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherTma, 16, BIAS, true>();
+                    return true;
+                }
+            }
             *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, false>()
                                   : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, true>();
             return true;
         }
     }
     if constexpr (MODE == shflbw::kPanelSpmmRows || MODE == shflbw::kPanelConvChainRows) {   // rows in TMEM lanes: V must be a legal UMMA M
-        if constexpr (MODE == shflbw::kPanelSpmmRows) {
-            // SpMM, 64-row blocks, 256-token items: the rows of B come by TMA tile-gather, issued by
-            // 16 light producer warps in four groups (measured 3-6 % faster than the cp.async gather
-            // on the 4096^3 case; the copy engine also applies the swizzle and zero-fills the N residue)
-            if (gather == shflbw::kGatherTma && V == 64 && tile == 256) {
-                *out = choice<64, 2, 64, 5, 16, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
-                return true;
-            }
-        }
         switch (V * 1000 + tile) {
-            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
-            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
-            case 128128: *out = choice<128, 1, 64, 6, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
-            case 128256: *out = choice<128, 2, 64, 4, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;
+            case 64128:  *out = regular<64, 1, 8, MODE, BIAS>(gather); return true;
+            case 64256:  *out = regular<64, 2, 5, MODE, BIAS>(gather); return true;
+            case 128128: *out = regular<128, 1, 6, MODE, BIAS>(gather); return true;
+            case 128256: *out = regular<128, 2, 4, MODE, BIAS>(gather); return true;
             default: return false;
         }
     } else {
         if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConv) {
             // 16-row blocks: UMMA N = 16, one or two 128-token accumulators per item (18 / 34 KB stages)
-            if (V == 16 && tile == 128) { *out = choice<16, 1, 64, 8, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true; }
-            if (V == 16 && tile == 256) { *out = choice<16, 2, 64, 5, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true; }
+            if (V == 16 && tile == 128) { *out = regular<16, 1, 8, MODE, BIAS>(gather); return true; }
+            if (V == 16 && tile == 256) { *out = regular<16, 2, 5, MODE, BIAS>(gather); return true; }
         }
         switch (V * 1000 + tile) {
-            case 32128:  *out = choice<32, 1, 64, 8, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 20 KB stages
-            case 32256:  *out = choice<32, 2, 64, 5, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 36 KB
-            case 64128:  *out = choice<64, 1, 64, 8, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 24 KB
-            case 64256:  *out = choice<64, 2, 64, 5, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;    // 40 KB
-            case 128128: *out = choice<128, 1, 64, 6, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;   // 32 KB
-            case 128256: *out = choice<128, 2, 64, 4, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>(); return true;   // 48 KB
+            case 32128:  *out = regular<32, 1, 8, MODE, BIAS>(gather); return true;    // 20 KB stages
+            case 32256:  *out = regular<32, 2, 5, MODE, BIAS>(gather); return true;    // 36 KB
+            case 64128:  *out = regular<64, 1, 8, MODE, BIAS>(gather); return true;    // 24 KB
+            case 64256:  *out = regular<64, 2, 5, MODE, BIAS>(gather); return true;    // 40 KB
+            case 128128: *out = regular<128, 1, 6, MODE, BIAS>(gather); return true;   // 32 KB
+            case 128256: *out = regular<128, 2, 4, MODE, BIAS>(gather); return true;   // 48 KB
             default: return false;
         }
     }
@@ -260,6 +266,9 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
     // SpMM and chained SpConv with V = 64 / 128 can run with the operands swapped (rows in TMEM
     // lanes, one MMA per 16 columns for the whole token tile); SHFLBW_SWAP=0|1 forces the choice
     // (tuning aid).
+    // SpMM gathers by TMA; SHFLBW_GATHER=0 takes cp.async (tuning aid).
+    int gather = MODE == shflbw::kPanelSpmm ? shflbw::kGatherTma : shflbw::kGatherCpAsync;
+    if (const char* g = getenv("SHFLBW_GATHER")) if (atoi(g) != 1) gather = shflbw::kGatherCpAsync;
     bool swapped = false;
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         const char* e = getenv("SHFLBW_SWAP");
@@ -268,13 +277,8 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
         // rows-in-lanes epilogue of a 64-row block keeps only half of each warp's lanes busy.
         const bool deep = padded_cols >= 192ll * row_blocks;
         if ((V == 64 || V == 128) && (e ? atoi(e) != 0 : deep)) {
-            // TMA gather (SHFLBW_GATHER=0 keeps cp.async; tuning aid) when every SM gets at least two items
-            int gather = shflbw::kGatherCpAsync;
-            if (MODE == shflbw::kPanelSpmm && V == 64 && tile == 256 && items256 >= 2ll * sms) gather = shflbw::kGatherTma;
-            if (const char* g = getenv("SHFLBW_GATHER")) gather = atoi(g) == 1 && V == 64 && tile == 256 && MODE == shflbw::kPanelSpmm && n_tokens >= 64
-                                                                      ? shflbw::kGatherTma : shflbw::kGatherCpAsync;
             swapped = MODE == shflbw::kPanelSpmm ? lookup<shflbw::kPanelSpmmRows>(V, tile, out, gather)
-                                                 : lookup<shflbw::kPanelConvChainRows>(V, tile, out);
+                                                 : lookup<shflbw::kPanelConvChainRows>(V, tile, out, gather);
         }
     }
     // Tokens in lanes with at most one stage of non-zero columns per block on average (an item is
@@ -290,11 +294,11 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
         if (const char* e = getenv("SHFLBW_EPILOGUE_WARPS")) wide = !swapped && tile == 256 && V == 64 && atoi(e) == 16;
     }
     const int wide_ring = !wide ? 0 : !addend && padded_cols > 32ll * row_blocks ? 8 : 6;
-    if (!swapped && !lookup<MODE>(V, tile, out, shflbw::kGatherCpAsync, wide_ring)) return SHFLBW_ERR_UNSUPPORTED;
+    if (!swapped && !lookup<MODE>(V, tile, out, gather, wide_ring)) return SHFLBW_ERR_UNSUPPORTED;
     out->variant = swapped ? 1 : wide ? 2 : 0;
     if (wide_ring == 8) {                    // a residual may be bound to the state later on
         PanelChoice with_addend;
-        if (!lookup<MODE>(V, tile, &with_addend, shflbw::kGatherCpAsync, 6)) return SHFLBW_ERR_UNSUPPORTED;
+        if (!lookup<MODE>(V, tile, &with_addend, gather, 6)) return SHFLBW_ERR_UNSUPPORTED;
         const int rc = allow_smem(with_addend.fn, with_addend.smem);
         if (rc != SHFLBW_OK) return rc;
     }
@@ -484,9 +488,9 @@ static int spmm_panel(const shflbw_spmm_state_t* st, bool bias, PanelChoice* ch)
     const int wide_ring = st->variant != 2 ? 0 : st->beta != 0.f ? 6 : st->stages;   // (an addend needs its slots)
     const bool found =
         bias ? st->variant == 1 ? lookup<shflbw::kPanelSpmmRows, true>(st->V, st->tokens_per_cta, ch, st->gather)
-                                : lookup<shflbw::kPanelSpmm, true>(st->V, st->tokens_per_cta, ch, shflbw::kGatherCpAsync, wide_ring)
+                                : lookup<shflbw::kPanelSpmm, true>(st->V, st->tokens_per_cta, ch, st->gather, wide_ring)
              : st->variant == 1 ? lookup<shflbw::kPanelSpmmRows>(st->V, st->tokens_per_cta, ch, st->gather)
-                                : lookup<shflbw::kPanelSpmm>(st->V, st->tokens_per_cta, ch, shflbw::kGatherCpAsync, wide_ring);
+                                : lookup<shflbw::kPanelSpmm>(st->V, st->tokens_per_cta, ch, st->gather, wide_ring);
     if (!found || ch->gather != st->gather) return SHFLBW_ERR_INVALID_ARG;
     return bias ? allow_smem(ch->fn, ch->smem) : SHFLBW_OK;
 }

@@ -25,57 +25,61 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
     asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" ::"r"(smem_u32(bar))
                  : "memory");
 }
-// Non-blocking phase test.
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+// Phase test that may suspend the thread in hardware until the phase completes or `hint_ns` pass.
+__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity, uint32_t hint_ns = 1000) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(hint_ns)
         : "memory");
     return ok != 0;
 }
 
-// Bounded wait.  Returns when the phase with the given parity completes, the CTA-wide abort
-// flag is raised, or `limit_cycles` SM clocks pass.  On timeout it raises the abort flag and
+// Bounded wait.  Returns true when the phase with the given parity completes, false when the CTA-wide
+// abort flag is raised or `limit_cycles` SM clocks pass.  On timeout it raises the abort flag and
 // records `code` in the global status word; the caller carries on (results are then garbage,
-// but every later wait returns at once and the kernel drains and exits).
-//
-// The already-complete case is one inlined test; the polling loop lives in a function that is
-// NOT inlined, so the hot loops of the kernel stay short and straight (the kernels proved
-// sensitive to instruction fetch: a taken branch to a cold line cost ~150 clk).  Between
-// polls the thread sleeps `backoff_ns` so waiting warps leave the issue slots to the others.
+// the host reads the status word), so a lost arrival can never hang the GPU.
 // `heed_abort = false` is for the clean-up wait of the abort path itself (the flag is already up
 // there); `code` 0 records nothing.
+//
+// The waiting thread is suspended by the hardware (try_wait): a wait costs a handful of instructions
+// instead of a stream of polls, each of which takes a slot of the load/store unit that the copy
+// issue, the arrivals and the epilogue's stores go through as well.  The loop lives in a function
+// that is NOT inlined, so the hot loops of the kernel stay short and straight.
 __device__ __noinline__ bool mbar_wait_slow(uint64_t* bar, uint32_t parity, volatile int* cta_abort,
-                                            int* status_word, int code, long long limit_cycles,
-                                            uint32_t backoff_ns, bool heed_abort) {
+                                            int* status_word, int code, long long limit_cycles, bool heed_abort) {
     const long long t0 = clock64();
-    uint32_t spins = 0;
     while (true) {
-        if (backoff_ns) __nanosleep(backoff_ns);
-        if (mbar_test(bar, parity)) return true;
-        if ((++spins & 0xf) == 0) {
-            if (heed_abort && *cta_abort) return false;
-            if (clock64() - t0 > limit_cycles) {
-                *cta_abort = 1;
-                if (code) atomicCAS(status_word, 0, code);
-                return false;
-            }
+        if (mbar_try_wait(bar, parity)) return true;
+        if (heed_abort && *cta_abort) return false;
+        if (clock64() - t0 > limit_cycles) {
+            *cta_abort = 1;
+            if (code) atomicCAS(status_word, 0, code);
+            return false;
         }
     }
 }
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, volatile int* cta_abort,
-                                                  int* status_word, int code, long long limit_cycles,
-                                                  uint32_t backoff_ns = 40, bool heed_abort = true) {
-    // Most waits in the kernels are short (a few hundred clocks): poll a handful of times in
-    // line before paying for the call and the first sleep of the slow path.
-#pragma unroll 1
-    for (int i = 0; i < 12; ++i)
-        if (mbar_test(bar, parity)) return true;
-    return mbar_wait_slow(bar, parity, cta_abort, status_word, code, limit_cycles, backoff_ns, heed_abort);
+                                                  int* status_word, int code, long long limit_cycles, bool heed_abort = true) {
+    return mbar_try_wait(bar, parity) || mbar_wait_slow(bar, parity, cta_abort, status_word, code, limit_cycles, heed_abort);
+}
+// The same by a whole warp, with one answer for all lanes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* cta_abort,
+                                               int* status_word, int code, long long limit_cycles) {
+    return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, cta_abort, status_word, code, limit_cycles));
+}
+
+// One lane of a converged warp, always the same one.  Instructions whose operands the hardware takes
+// from uniform registers (tcgen05.mma / commit, bulk and tensor copies) belong in a branch on this: behind
+// `lane == 0` the compiler cannot see that one lane is left and serialises each of them over the lanes
+// that might be there (54 clk per tcgen05.mma instead of 15, 59 clk per gather4 instead of 9).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r != 0;
 }
 
 // ----------------------------------------------------------------- bulk copy ----
@@ -93,6 +97,10 @@ __device__ __forceinline__ void bulk_copy_g2s(uint32_t dst_smem, const void* src
 // One arrival plus `bytes` added to the pending transaction count, in one operation.
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+// Fetches a tensor map (64-byte aligned, kernel parameter or global memory) ahead of its first use.
+__device__ __forceinline__ void prefetch_tensormap(const void* tmap) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
 }
 // TMA tile::gather4: rows r0..r3 of a 2-D tensor (tensor map box = W columns x 1 row), columns
 // [col, col + W), land as 4 consecutive rows of W elements at dst (swizzled as the map says) and
@@ -142,15 +150,6 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // data the previous kernel writes -- or buffers it still reads.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
-// ------------------------------------------------------- register budgets ----
-// Change the per-thread register budget of the executing warpgroup (4 consecutive warps, all
-// of which must execute the same instruction).  The count is a multiple of 8 in [24, 256].
-// .dec returns registers to the SM's pool at once; .inc waits until the pool holds enough.
-template <int N>
-__device__ __forceinline__ void setmaxnreg_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
-template <int N>
-__device__ __forceinline__ void setmaxnreg_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
 
 // ------------------------------------------------------------------- tcgen05 ----
 // TMEM allocation: one full warp; ncols a power of two in [32, 512].  The base address
