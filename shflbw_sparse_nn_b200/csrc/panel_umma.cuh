@@ -338,7 +338,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         constexpr int IPL = KS / 32;                        // row ids per lane
         int* const my_ids = idx_ring + pidx * KS;           // row ids of this warp's current stage
         if (sm100::elect_one()) sm100::prefetch_tensormap(p.tmap_b);
-        // (item, stage of the item) of this warp's next stage
+        // (item, stage of the item) of this warp's next stage; row ids are loaded while the stage before is filled
         int li = 0, kt = pidx, row_begin = 0, rows_total = 0;
         auto settle = [&]() {                               // stages beyond an item's end belong to the items after it
             while (li < nloc) {
@@ -376,6 +376,9 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             for (int i = 0; i < IPL; ++i) my_ids[i * 32 + lane] = id[i];
             const int rows_valid = min(KS, rows_total - kt * KS);   // multiple of 16
             const __half* wsrc = p.blk_val + (size_t)(row_begin + kt * KS) * V;
+            kt += PW;
+            settle();
+            load_ids();
             if (!sm100::mbar_wait_warp(&empty_bar[s], ph, cta_abort, p.status_word, SHFLBW_DEVSTAT_TIMEOUT_EMPTY, p.wait_limit)) break;
             __syncwarp();                                    // the row ids are in place
             if (sm100::elect_one()) {
@@ -414,9 +417,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             __syncwarp();                                    // the row ids may be overwritten
             it += PW; s += PW;
             if (s >= (uint32_t)STAGES) { s -= STAGES; ph ^= 1u; }
-            kt += PW;
-            settle();
-            load_ids();
         }
         }
     } else if (warp > EW) {
@@ -610,28 +610,30 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
           : V == 64 ? sm100::make_smem_desc(smem_base + Cfg::G_BYTES, 1024, 1024, sm100::kSwizzle128B)
                     : sm100::make_smem_desc(smem_base + Cfg::G_BYTES, 1024, 2048, sm100::kSwizzle128B);
         constexpr uint32_t WSTEP = V * 32;  // bytes per K-step (16 rows) of the value tile
-        // The warp runs the role in lock step and one elected lane issues (elect_one): the ring slot, its
-        // parity and the descriptors are then uniform to the compiler, and an MMA is a few instructions.
-        // (One thread running the role alone: 54 clk per MMA whatever its shape, 1174 clk per stage of the
-        // 4096^3 product at V = 64, 1420 at V = 128.)
-        bool ok = true;
-        uint32_t s = 0, ph = 0;         // ring slot of the next stage and the parity of its full barrier
-        for (int li = 0; li < nloc && ok; ++li) {
-            const int rows_total = __shfl_sync(0xffffffffu, item_tab[li].y, 0);
-            const int num_k = (rows_total + KS - 1) / KS;
-            const int b = li % NBUF;
-            if (li >= NBUF && !(ok = sm100::mbar_wait_warp(&acc_empty[b], ((li / NBUF) - 1) & 1, cta_abort, p.status_word,
-                                                           SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit)))
-                break;                                       // timed out or aborted: issue nothing more
-            const uint32_t acc_base = tmem_base + b * Cfg::ACC_COLS;
-            for (int kt = 0; kt < num_k; ++kt) {
-                if (!(ok = sm100::mbar_wait_warp(&full_bar[s], ph, cta_abort, p.status_word, SHFLBW_DEVSTAT_TIMEOUT_FULL, p.wait_limit)))
-                    break;
-                // cp.async (generic proxy) data -> tensor-core (async proxy) reads; the copy engine's
-                // writes of the TMA gather are in the async proxy already
-                if (!Cfg::TMA) sm100::fence_proxy_async_smem();
-                sm100::tc_fence_after_sync();
-                if (sm100::elect_one()) {
+        // One elected lane runs the whole role: the ring slot, its parity and the descriptors are then uniform to
+        // the compiler, an MMA is a few instructions, and a stage costs 118 clk of this loop plus its MMAs (the
+        // warp waiting in lock step and electing per stage: 228; a thread that is not elected, lane == 0: 54 clk per
+        // MMA whatever its shape, 1174 clk per stage of the 4096^3 product at V = 64, 1420 at V = 128).
+        if (sm100::elect_one()) {
+            uint32_t s = 0, ph = 0;     // ring slot of the next stage and the parity of its full barrier
+            bool ready = false;         // that barrier was already seen complete
+            for (int li = 0; li < nloc; ++li) {
+                const int rows_total = item_tab[li].y;
+                const int num_k = (rows_total + KS - 1) / KS;
+                const int b = li % NBUF;
+                if (li >= NBUF && !sm100::mbar_wait_bounded(&acc_empty[b], ((li / NBUF) - 1) & 1, cta_abort, p.status_word,
+                                                            SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit))
+                    break;                                   // timed out or aborted: issue nothing more
+                const uint32_t acc_base = tmem_base + b * Cfg::ACC_COLS;
+                for (int kt = 0; kt < num_k; ++kt) {
+                    if (!ready && !sm100::mbar_wait_bounded(&full_bar[s], ph, cta_abort, p.status_word, SHFLBW_DEVSTAT_TIMEOUT_FULL, p.wait_limit))
+                        goto mma_done;                       // timed out or aborted: issue nothing more
+                    // cp.async (generic proxy) data -> tensor-core (async proxy) reads; the copy engine's
+                    // writes of the TMA gather are in the async proxy already
+                    if (!Cfg::TMA) sm100::fence_proxy_async_smem();
+                    sm100::tc_fence_after_sync();
+                    const uint32_t sn = s + 1 == (uint32_t)STAGES ? 0 : s + 1;
+                    ready = sm100::mbar_test(&full_bar[sn], sn ? ph : ph ^ 1u);   // the round trip hides behind the MMAs
                     const int nk = min(KS, rows_total - kt * KS) / 16;
                     const uint64_t gd = gdesc0 + (uint64_t)((s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
                     const uint64_t wd = wdesc0 + (uint64_t)((s * (uint32_t)Cfg::STAGE_BYTES) >> 4);
@@ -651,18 +653,18 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     }
                     sm100::umma_commit(&empty_bar[s]);       // stage may be refilled once these MMAs retire
                     if (kt + 1 == num_k) sm100::umma_commit(&acc_full[b]);   // accumulator complete
+                    s = sn;
+                    if (sn == 0) ph ^= 1u;
                 }
-                __syncwarp();
-                if (++s == (uint32_t)STAGES) { s = 0; ph ^= 1u; }
+                if (num_k == 0) sm100::mbar_arrive(&acc_full[b]);   // nothing to wait for
             }
-            if (num_k == 0 && lane == 0) sm100::mbar_arrive(&acc_full[b]);   // nothing to wait for
-            __syncwarp();
-        }
-        if (__any_sync(0xffffffffu, *cta_abort) && sm100::elect_one()) {
-            // Aborted: the MMAs issued so far must retire before TMEM is freed and the block's
-            // shared memory goes away.  One more commit, awaited with its own (short) limit.
-            sm100::umma_commit(drain_bar);
-            sm100::mbar_wait_bounded(drain_bar, 0, cta_abort, p.status_word, 0, 4000000LL, /*heed_abort=*/false);
+        mma_done:
+            if (*cta_abort) {
+                // Aborted: the MMAs issued so far must retire before TMEM is freed and the block's
+                // shared memory goes away.  One more commit, awaited with its own (short) limit.
+                sm100::umma_commit(drain_bar);
+                sm100::mbar_wait_bounded(drain_bar, 0, cta_abort, p.status_word, 0, 4000000LL, /*heed_abort=*/false);
+            }
         }
         __syncwarp();
     } else {
