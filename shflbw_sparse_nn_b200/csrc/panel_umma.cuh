@@ -12,11 +12,9 @@
 //   tokens in lanes  tokens are the UMMA M dimension (128 TMEM lanes), the V rows of the block
 //                    the N dimension (32/64/128): TM instructions per 16 columns.  Used for
 //                    V = 32, for SpConv writing NHWC, and for blocks with few columns.
-//   rows in lanes    the V rows are M (64 or 128 lanes; M = 64 occupies the first 16 lanes of
-//                    every 32-lane quadrant) and the T tokens N (128 or 256): ONE instruction
-//                    per 16 columns.  An MMA costs >= 73 clk whatever its N up to 128 and 133
-//                    clk at N = 256, so this halves the instruction count at ~8 % less tensor
-//                    time, and the accumulator holds one output row per lane.  Default for
+//   rows in lanes    the V rows are M (64 or 128) and the T tokens N (128 or 256): ONE instruction
+//                    per 16 columns, 128 clk at 128 x 256, 80 clk at 64 x 256 (weight-stationary
+//                    form), and the accumulator holds one output row per lane.  Default for
 //                    SpMM and chained SpConv with V = 64 / 128 and >= 3 stages of columns.
 // The description below is written for the first orientation; the second differs in the
 // gathered tile's layout ([K group][T/64 swizzle atoms]), the MMA issue and the epilogue.
@@ -192,7 +190,10 @@ struct PanelCfg {
     static constexpr int SMEM_BYTES = PIPE_BYTES + OUT_BYTES + RES_BYTES + BAR_BYTES + TAB_BYTES + IDX_BYTES + 1024;  // + align slack
     static constexpr bool SWAP = MODE == kPanelSpmmRows || MODE == kPanelConvChainRows;
     static constexpr int KG_BYTES = SWAP ? T * 16 : 2048;   // 8 gathered rows (one K group) of the token tile
-    static constexpr uint32_t ACC_COLS = SWAP ? T : TM * V; // fp32 columns of one accumulator set
+    // 64 rows in lanes run as weight-stationary MMAs (tcgen05.mma.ws): 80 clk for 64 x 256 x 16 instead of 128, and
+    // the accumulator fills all lanes: token t of row m is lane m + 64 * (t / (T / 2)), column t % (T / 2).
+    static constexpr bool WS = SWAP && V == 64;
+    static constexpr uint32_t ACC_COLS = WS ? T / 2 : SWAP ? T : TM * V; // fp32 columns of one accumulator set
     static_assert(!SWAP || V == 64 || V == 128, "rows-in-lanes needs a legal UMMA M");
     // Accumulator sets in TMEM: two (the MMAs of item i+1 run while the epilogue reads item i);
     // four with sixteen epilogue warps, whose items are so short that the hand-over itself
@@ -201,7 +202,7 @@ struct PanelCfg {
     // Sixteen epilogue warps work as two sets of eight that take the items in turn, so that the chains
     // of two items (accumulator wait, TMEM read, transpose, stores) overlap.
     static constexpr int ESETS = EW / 8;
-    static constexpr int NBUF = (EW == 16 && ACC_COLS * 4 <= 512) ? 4 : 2;
+    static constexpr int NBUF = ((EW == 16 || WS) && ACC_COLS * 4 <= 512) ? 4 : 2;
     static constexpr uint32_t TMEM_COLS = NBUF * ACC_COLS < 32 ? 32 : NBUF * ACC_COLS;
     static_assert(V == 16 || V == 32 || V == 64 || V == 128, "row-block height");
     static_assert(V != 16 || !SWAP, "16-row blocks: tokens in lanes");
@@ -643,7 +644,9 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                             const uint64_t gdj = gd + (uint64_t)(j * ((2 * Cfg::KG_BYTES) >> 4)), wdj = wd + (uint64_t)(j * (WSTEP >> 4));
                             const uint32_t accum = j > 0 || kt > 0;
                             if constexpr (SWAP) {
-                                sm100::umma_f16_ss(acc_base, wdj, gdj, idesc, accum);   // D[row][token] += W^T . G
+                                // D[row][token] += W^T . G
+                                if constexpr (Cfg::WS) sm100::umma_ws_f16_ss(acc_base, wdj, gdj, idesc, accum);
+                                else sm100::umma_f16_ss(acc_base, wdj, gdj, idesc, accum);
                             } else {
 #pragma unroll
                                 for (int a = 0; a < TM; ++a)
@@ -704,25 +707,25 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             // took 68.0 us with a bias and 45.7 without; 45.7 now.)
             __half2 bias2 = __float2half2_rn(0.f);
             if constexpr (SWAP && BIAS) {
-                const int m = V == 64 ? quad * 16 + (lane & 15) : quad * 32 + lane;
+                const int m = (Cfg::WS ? quad & 1 : quad) * 32 + lane;
                 bias2 = __half2half2(__ldg(p.C + (p.perm ? __ldg(p.perm + blk * V + m) : blk * V + m)));
             }
             if constexpr (SWAP || !ROWS_OUT) {
                 if (!wait_accumulator()) break;
             }
             if constexpr (SWAP) {
-                // Rows in lanes: lane l of quadrant `quad` holds output row m of the block (V = 64:
-                // the quadrant's first 16 lanes, m = 16*quad + l; V = 128: all 32, m = 32*quad + l)
-                // and this warp reads token columns [half_id*T/2, +T/2), 32 at a time: a lane's 32
+                // Rows in lanes: lane l of quadrant `quad` holds output row m of the block (V = 128:
+                // m = 32*quad + l; V = 64: m = 32*(quad % 2) + l, the upper two quadrants the second half of the
+                // tokens), and the quadrant's two warps share its token columns, 32 at a time: a lane's 32
                 // tokens are 64 contiguous bytes of its output row.  They are packed to fp16 and
                 // stored straight from registers -- as two 32-byte stores (whole L2 sectors) when
                 // the output rows are 32-byte aligned, else as four 16-byte stores.  No shared
                 // memory is involved: the tensor core's operand reads and the gather's writes already
                 // use most of its bandwidth.
-                constexpr int LR = V == 64 ? 16 : 32;                    // rows (valid lanes) per quadrant
-                constexpr int HC = T / 2;                                // token columns of this warp
+                constexpr int HC = (int)Cfg::ACC_COLS / 2;               // token columns of this warp
                 const uint32_t acc0 = tmem_base + ((uint32_t)(quad * 32) << 16) + b * Cfg::ACC_COLS + half_id * HC;
-                const int m = quad * LR + (lane < LR ? lane : 0);
+                const int t0 = n0 + (Cfg::WS ? (quad >> 1) * (T / 2) : 0) + half_id * HC;   // its first token
+                const int m = (Cfg::WS ? quad & 1 : quad) * 32 + lane;
                 size_t roff;                                             // element offset of this lane's output row
                 size_t rres = 0;                                         // chained: offset of its residual row
                 const bool use_res = CHAIN && p.res != nullptr;
@@ -741,13 +744,13 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 const bool use_c = !CHAIN && !BIAS && p.beta != 0.0f && p.C != nullptr;
 #pragma unroll 1
                 for (int cc = 0; cc < HC; cc += 32) {
-                    const int tok0 = n0 + half_id * HC + cc;             // this lane's 32 tokens start here
+                    const int tok0 = t0 + cc;                            // this lane's 32 tokens start here
                     // Where the four 8-token groups go, and (chained layers) the residual that gets added
                     // to them: requested before the accumulator read, so that the global-memory latency
                     // hides behind it.
                     size_t goffs[4];
                     uint4 addend[4];
-                    if (lane < LR) {
+                    {
                         if constexpr (CHAIN) {
                             // 8 consecutive tokens are 8 images of one output pixel; the pixel's place in the
                             // consumer's halo-padded plane is found once and stepped from group to group
@@ -784,7 +787,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                         __syncwarp();
                         if (lane == 0) sm100::mbar_arrive(&acc_empty[b]);
                     }
-                    if (lane < LR) {
+                    {
                     uint4 v[4];
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
