@@ -33,8 +33,7 @@
 //                    group publishes its previous stage half-way through issuing the next one,
 //                    with ONE mbarrier arrival per warp; row ids are prefetched two of the
 //                    group's stages ahead by 4-byte cp.async into a shared-memory ring.  TMA
-//                    gather: every warp fills stages of its own with tile::gather4 copies, completion by
-//                    byte count.  One bulk copy per stage for the value slice either way.
+//                    gather: tile::gather4 copies, completion by byte count.  One bulk copy per stage for the value slice either way.
 //   later warps with w % 4 == 0   idle, so that no producer shares the MMA warp's scheduler partition.
 // The accumulator is double buffered in TMEM (four sets with EW = 16) so the epilogue of item i
 // overlaps the main loop of item i+1, and the stage ring runs across item boundaries without
@@ -162,7 +161,7 @@ struct PanelCfg {
     // w % 4 == 0 stay idle.  The MMA warp executes a
     // few dozen instructions per stage and was measured at ~20 clk per instruction when
     // producer code kept evicting its lines from the partition's instruction cache.
-    static constexpr int WARPS = EW + 1 + PW + (PW - 1) / 3;   // epilogue + MMA + producers + idle
+    static constexpr int WARPS = EW + 1 + PW + (TMA ? 0 : (PW - 1) / 3);   // epilogue + MMA + producers + idle
     static_assert(EW == 8 || WARPS <= 20, "16 epilogue warps: at most 3 producers (20 warps leave 96 registers per thread, 21-24 only 80)");
     static constexpr int THREADS = WARPS * 32;
     static constexpr int G_ACC = KS * 256;                 // gathered tile of one accumulator: [KS][128] fp16
@@ -206,7 +205,7 @@ struct PanelCfg {
     static constexpr uint32_t TMEM_COLS = NBUF * ACC_COLS < 32 ? 32 : NBUF * ACC_COLS;
     static_assert(V == 16 || V == 32 || V == 64 || V == 128, "row-block height");
     static_assert(V != 16 || !SWAP, "16-row blocks: tokens in lanes");
-    static_assert(!TMA || (GROUPS == PW && PW <= STAGES), "TMA gather: every producer warp fills stages of its own");
+    static_assert(!TMA || (GROUPS <= STAGES && (KS / 4) % (PW / GROUPS) == 0), "TMA gather: producer groups, row quads per warp");
     static_assert(STAGE_BYTES % 1024 == 0, "stages must keep 1024-byte swizzle-atom alignment");
     static_assert((TMEM_COLS & (TMEM_COLS - 1)) == 0 && TMEM_COLS <= 512, "TMEM columns");
     static_assert(KS % 32 == 0 && PW % GROUPS == 0 && (TMA || (KS % (PW / GROUPS) == 0 && (KS / (PW / GROUPS)) % (32 / (T / 8)) == 0)),
@@ -278,7 +277,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             // cp.async gather: one arrival per producer WARP of the group (per-thread deferred arrivals,
             // cp.async.mbarrier.arrive.noinc, were measured at ~3 clk of load/store-unit time per thread,
             // i.e. more than the copies themselves).  TMA gather: one arrival, with the stage's byte count.
-            sm100::mbar_init(&full_bar[s], Cfg::TMA ? 1 : PW / Cfg::GROUPS);
+            sm100::mbar_init(&full_bar[s], PW / Cfg::GROUPS);
             sm100::mbar_init(&empty_bar[s], 1);   // one tcgen05.commit per drain
         }
         for (int b = 0; b < NBUF; ++b) {
@@ -318,105 +317,136 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     // epilogue warps at once (they read C / the residual and write the output); the MMA warp
     // touches no global memory and does not wait.
 
-    const int pidx = warp - (EW + 1) - (warp / 4 - EW / 4);   // producer number of a producer warp (warps after the MMA warp with warp % 4 != 0)
-    if (warp > EW && ((warp & 3) == 0 || pidx >= PW)) {
+    const int pidx = Cfg::TMA ? warp - (EW + 1) : warp - (EW + 1) - (warp / 4 - EW / 4);   // producer number of a producer warp (warps after the MMA warp with warp % 4 != 0)
+    if (!Cfg::TMA && warp > EW && ((warp & 3) == 0 || pidx >= PW)) {
         // idle: keeps producers off the MMA warp's scheduler partition
     } else if (warp > EW && Cfg::TMA) {
         // ---------------------------------------------------- producers (TMA gather) ----
         // A stage is KS gathered rows x T tokens = (KS/4) row quads x (T/64) column boxes, one
-        // tile::gather4 each (4 rows x 128 bytes, landing as half a swizzle atom).  Every producer warp
-        // fills stages of its own (stage it by warp it % PW), all operations issued by an elected lane,
-        // and the stage's barrier completes by byte count: nobody waits for data.  Bound by the copy
-        // engine's 9.6 clk per operation, 53 bytes a clock and SM.  Four warps: one of them spends 970 clk
-        // on issuing a 64 x 256 stage, the ring passes one in 570-620 (two warps per stage 610, four 620;
-        // one operation per lane instead of an elected lane: 640 and 1540 clk of issue).  Stage time of
-        // the 4096^3 product: 1174 -> 620 clk.
-        // A warp shares its stages with no other warp: a warp of a shared stage that has no row to fetch (a
-        // short last stage) is not waited for by anyone, can fall a whole ring behind, miss the phase that it
-        // waits for and wait for good.
+        // tile::gather4 each (4 rows x 128 bytes, landing as half a swizzle atom).  GROUPS groups of GW warps
+        // take the stages in turn, a warp's row quads are issued by an elected lane, and the stage's barrier
+        // completes by byte count: nobody waits for data.
+        // Bound by the issue: an operation takes seven operands in uniform registers, 15 clk of a warp that has
+        // the issue slots for itself and 32 in here, where the copy engine would take one every 9.  Hence two
+        // warps a stage (11008x4096x512, V = 32, density 0.25: 34.9 us with one, 32.5 with two; 4096^3 at
+        // V = 16, 0.1: 77.4 and 72.3; sixteen warps, four to a stage: 33.3 and 74.0, but 25.3 instead of 26.4 us at
+        // V = 64), and a loop whose control the compiler can see to be uniform.
+        // Every warp of a stage arrives on its barrier, with the bytes it fetches.  If only one did, a warp
+        // without a row in a short last stage would be waited for by nobody, could fall a whole ring behind,
+        // miss the phase that it waits for and wait for good.
+        // The CTA's first stage is split between all warps: nothing else is in flight then, and the issue would be
+        // most of its time (256^3: 3.1 -> 2.6 us).
         if constexpr (Cfg::TMA) {
         constexpr int BOXES = T / 64, QUADS = KS / 4;       // column boxes per row quad, row quads
-        constexpr int IPL = KS / 32;                        // row ids per lane
+        constexpr int GROUPS = Cfg::GROUPS, GW = PW / GROUPS;   // GW warps share a stage
+        constexpr int WQ = QUADS / GW;                      // quads of a stage that a warp fetches
+        constexpr int IPL = (WQ * 4 + 31) / 32;             // row ids per lane
+        const int grp = pidx / GW, pw = pidx % GW;
         int* const my_ids = idx_ring + pidx * KS;           // row ids of this warp's current stage
         if (sm100::elect_one()) sm100::prefetch_tensormap(p.tmap_b);
         // (item, stage of the item) of this warp's next stage; row ids are loaded while the stage before is filled
-        int li = 0, kt = pidx, row_begin = 0, rows_total = 0;
+        int li = 0, kt = 0, row_begin = 0, rows_total = 0;
         auto settle = [&]() {                               // stages beyond an item's end belong to the items after it
             while (li < nloc) {
                 const int2 e = item_tab[li];
-                const int num_k = (e.y + KS - 1) / KS;
-                row_begin = e.x; rows_total = e.y;
+                row_begin = __shfl_sync(0xffffffffu, e.x, 0); rows_total = __shfl_sync(0xffffffffu, e.y, 0);   // (uniform to the compiler)
+                const int num_k = (rows_total + KS - 1) / KS;
                 if (kt < num_k) return;
                 kt -= num_k;
                 ++li;
             }
         };
+        auto row_id = [&](int r) { return li < nloc && r < rows_total ? __ldg(p.blk_idx + row_begin + r) : 0; };   // of the item's row r
         int id[IPL];
         auto load_ids = [&]() {
 #pragma unroll
-            for (int i = 0; i < IPL; ++i) {
-                const int r = kt * KS + i * 32 + lane;
-                id[i] = li < nloc && r < rows_total ? __ldg(p.blk_idx + row_begin + r) : 0;
-            }
+            for (int i = 0; i < IPL; ++i) id[i] = row_id(kt * KS + pw * WQ * 4 + i * 32 + lane);
         };
+        int xs[BOXES], nbox = 0, of_item = -1;              // first column of each box, boxes that hold any token
+        auto enter_item = [&]() {
+            of_item = li;
+            const int tok0 = item_tile((int)blockIdx.x + li * (int)gridDim.x) * T;
+            nbox = min(BOXES, (p.N - tok0 + 63) / 64);       // columns beyond N are never stored: boxes past it are not fetched
+#pragma unroll
+            for (int b = 0; b < BOXES; ++b) xs[b] = tok0 + b * 64;
+        };
+        // rows in lanes: [K group][T/64 atoms]; tokens in lanes: [128-token half][K group][2 atoms]
+        auto dst_off = [](int q, int b) {
+            return SWAP ? (uint32_t)((q >> 1) * Cfg::KG_BYTES + b * 1024 + (q & 1) * 512)
+                        : (uint32_t)((b >> 1) * Cfg::G_ACC + (q >> 1) * 2048 + (b & 1) * 1024 + (q & 1) * 512);
+        };
+        auto arm = [&](uint32_t slot, int it, int row0, int rows_valid, int rows_mine) {   // expect this warp's bytes of a stage; the first of its warps copies the value slice
+            const uint32_t wbytes = pw == 0 ? (uint32_t)(rows_valid * V * 2) : 0u, bytes = (uint32_t)(rows_mine * nbox * 128) + wbytes;
+#ifdef SHFLBW_FAULT_INJECT
+            if (p.inject_from >= 0 && it >= p.inject_from) sm100::mbar_expect_tx(&full_bar[slot], bytes);   // the withheld arrival
+            else
+#endif
+            sm100::mbar_arrive_expect_tx(&full_bar[slot], bytes);
+            if (pw == 0) sm100::bulk_copy_g2s(smem_base + slot * Cfg::STAGE_BYTES + (uint32_t)Cfg::G_BYTES, p.blk_val + (size_t)row0 * V, wbytes, &full_bar[slot]);
+        };
+        // The CTA's first stage: this warp's quads of it.
+        constexpr int QW = (QUADS + PW - 1) / PW;
+        settle();
+        const int first_li = li, first_row = row_begin, first_valid = li < nloc ? min(KS, rows_total) : 0;
+        if (lane < QW * 4) my_ids[lane] = row_id(pidx * QW * 4 + lane);
+        if (li < nloc) enter_item();
+        kt += 1 + grp;
         settle();
         load_ids();
+        __syncwarp();
         sm100::grid_dependency_wait();                      // the dense operand may be the previous kernel's output
-        uint32_t s = pidx, ph = 1;                          // ring slot and the parity that says it is free (at first it is)
-        int xs[BOXES], nbox = 0, of_item = -1;              // first column of each box, boxes that hold any token
-        int it = pidx;
-        while (li < nloc) {
-            if (of_item != li) {
-                of_item = li;
-                const int tok0 = item_tile((int)blockIdx.x + li * (int)gridDim.x) * T;
-                nbox = min(BOXES, (p.N - tok0 + 63) / 64);   // columns beyond N are never stored: boxes past it are not fetched
+        if (first_li < nloc && sm100::elect_one()) {
+            if (grp == 0) arm(0, 0, first_row, first_valid, pw == 0 ? first_valid : 0);
 #pragma unroll
-                for (int b = 0; b < BOXES; ++b) xs[b] = tok0 + b * 64;
+            for (int i = 0; i < QW; ++i) {
+                const int q = pidx * QW + i;
+                const int4 r = *(const int4*)(my_ids + i * 4);
+#pragma unroll
+                for (int b = 0; b < BOXES; ++b)
+                    if (q * 4 < first_valid && b < nbox) sm100::tma_gather4(smem_base + dst_off(q, b), p.tmap_b, xs[b], r.x, r.y, r.z, r.w, &full_bar[0]);
             }
+        }
+        __syncwarp();
+        uint32_t s = 1 + grp, ph = 1;                      // ring slot and the parity that says it is free (in the first lap it is)
+        if (s >= (uint32_t)STAGES) { s -= STAGES; ph ^= 1u; }
+        int it = 1 + grp;
+        while (li < nloc) {
+            if (of_item != li) enter_item();
 #pragma unroll
-            for (int i = 0; i < IPL; ++i) my_ids[i * 32 + lane] = id[i];
+            for (int i = 0; i < IPL; ++i) if (WQ * 4 % 32 == 0 || i * 32 + lane < WQ * 4) my_ids[i * 32 + lane] = id[i];
             const int rows_valid = min(KS, rows_total - kt * KS);   // multiple of 16
-            const __half* wsrc = p.blk_val + (size_t)(row_begin + kt * KS) * V;
-            kt += PW;
+            const int row0 = row_begin + kt * KS;
+            kt += GROUPS;
             settle();
             load_ids();
             if (!sm100::mbar_wait_warp(&empty_bar[s], ph, cta_abort, p.status_word, SHFLBW_DEVSTAT_TIMEOUT_EMPTY, p.wait_limit)) break;
             __syncwarp();                                    // the row ids are in place
             if (sm100::elect_one()) {
                 const uint32_t st_base = smem_base + s * Cfg::STAGE_BYTES;
-                const uint32_t wbytes = (uint32_t)(rows_valid * V * 2), bytes = (uint32_t)(rows_valid * nbox * 128) + wbytes;
-#ifdef SHFLBW_FAULT_INJECT
-                if (p.inject_from >= 0 && it >= p.inject_from) sm100::mbar_expect_tx(&full_bar[s], bytes);   // the withheld arrival
-                else
-#endif
-                sm100::mbar_arrive_expect_tx(&full_bar[s], bytes);
-                sm100::bulk_copy_g2s(st_base + (uint32_t)Cfg::G_BYTES, wsrc, wbytes, &full_bar[s]);
+                arm(s, it, row0, rows_valid, min(max(rows_valid - pw * WQ * 4, 0), WQ * 4));
                 // All row ids come into registers before the first copy: the copies are ordered with
                 // respect to reads of shared memory, which would each add their latency.
-                int4 r[QUADS];
+                int4 r[WQ];
 #pragma unroll
-                for (int q = 0; q < QUADS; ++q) r[q] = *(const int4*)(my_ids + q * 4);
-                // rows in lanes: [K group][T/64 atoms]; tokens in lanes: [128-token half][K group][2 atoms]
+                for (int q = 0; q < WQ; ++q) r[q] = *(const int4*)(my_ids + q * 4);
                 auto copy = [&](int q, int b) {
-                    const uint32_t off = SWAP ? (uint32_t)((q >> 1) * Cfg::KG_BYTES + b * 1024 + (q & 1) * 512)
-                                              : (uint32_t)((b >> 1) * Cfg::G_ACC + (q >> 1) * 2048 + (b & 1) * 1024 + (q & 1) * 512);
-                    sm100::tma_gather4(st_base + off, p.tmap_b, xs[b], r[q].x, r[q].y, r[q].z, r[q].w, &full_bar[s]);
+                    sm100::tma_gather4(st_base + pw * (uint32_t)((WQ >> 1) * (SWAP ? Cfg::KG_BYTES : 2048)) + dst_off(q, b), p.tmap_b, xs[b], r[q].x, r[q].y, r[q].z, r[q].w, &full_bar[s]);
                 };
                 if (rows_valid == KS && nbox == BOXES) {     // a whole stage: straight-line code
 #pragma unroll
-                    for (int q = 0; q < QUADS; ++q)
+                    for (int q = 0; q < WQ; ++q)
 #pragma unroll
                         for (int b = 0; b < BOXES; ++b) copy(q, b);
                 } else {
 #pragma unroll
-                    for (int q = 0; q < QUADS; ++q)
+                    for (int q = 0; q < WQ; ++q)
 #pragma unroll
                         for (int b = 0; b < BOXES; ++b)
-                            if (q * 4 < rows_valid && b < nbox) copy(q, b);
+                            if ((pw * WQ + q) * 4 < rows_valid && b < nbox) copy(q, b);
                 }
             }
             __syncwarp();                                    // the row ids may be overwritten
-            it += PW; s += PW;
+            it += GROUPS; s += GROUPS;
             if (s >= (uint32_t)STAGES) { s -= STAGES; ph ^= 1u; }
         }
         }

@@ -152,11 +152,11 @@ int encode_b_map(const void* B, int K, int N, unsigned long long out[16]) {
 
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
-// Shapes of the TMA gather: four producer warps, each a group of its own.
+// Shapes of the TMA gather: eight producer warps, two to a stage.
 template <int V, int TM, int STAGES, int MODE, bool BIAS>
 PanelChoice regular(int gather) {
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelSpmmRows) {
-        if (gather == shflbw::kGatherTma) return choice<V, TM, 64, STAGES, 4, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
+        if (gather == shflbw::kGatherTma) return choice<V, TM, 64, STAGES, 8, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
     }
     return choice<V, TM, 64, STAGES, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>();
 }
