@@ -80,8 +80,9 @@ __device__ __forceinline__ int fast_div(int n, const FastDiv& f) {
 }
 
 struct alignas(64) PanelParams {
-    // TMA gather only: tensor map of B ([K][N] fp16, box = 64 tokens x 1 row, 128-byte swizzle); first
-    // member so that it sits on the 64-byte boundary the copy engine wants
+    // TMA gather only: tensor map of the dense operand (SpMM: B[K][N]; SpConv: one row per pixel of the staged
+    // input, running from that pixel to the end of what a tap reads; box = 64 tokens x 1 row, 128-byte swizzle);
+    // first member so that it sits on the 64-byte boundary the copy engine wants
     unsigned long long tmap_b[16];
     // sparse operand (kernel image)
     const int* blk_ptr;      // [X+1] padded offsets (multiples of 16)
@@ -95,7 +96,7 @@ struct alignas(64) PanelParams {
     long long wait_limit;    // SM clocks after which a barrier wait gives up (kWaitLimitCycles unless the host overrides it)
     float alpha, beta;
     int num_items, tiles_n;  // work items = row blocks x token tiles; item -> (item / tiles_n, item % tiles_n)
-    FastDiv div_tiles, div_bp, div_wo;   // division by tiles_n, Bp, Wo (set by the host with make_fast_div)
+    FastDiv div_tiles, div_bp, div_row;  // division by tiles_n, Bp, row_pix (set by the host with make_fast_div)
     // Order of the work items.  0: item = block * tiles_n + tile (a CTA's neighbours work on the
     // same row block).  1: item = tile * num_blocks + block: the CTAs that run at the same time
     // share a few token tiles, so the rows of the dense operand they gather are a small set that
@@ -108,13 +109,17 @@ struct alignas(64) PanelParams {
     const __half* B;         // [K][N]
     const __half* C;         // [M][N] or nullptr; kernels built with BIAS: one value per output row / filter
     __half* D;               // [M][N]
-    int N;                   // dense columns (SpMM) / Ho*Wo*Bp (SpConv)
+    int N;                   // dense columns (SpMM) / Ho*row_pix*Bp (SpConv)
     // SpConv (input staged channel-major, batch innermost, with a zero halo:
     // Xs[c][Hp][Wp][Bp], Hp = Hin + R - 1, Wp = Win + S - 1, image origin at (R/2, S/2); a strided 1x1
     // filter of an NHWC call is staged as the pixels it visits, Hp = Ho, Wp = Wo, and read at stride 1)
     const __half* Xs;
     __half* out;             // [B*Ho*Wo][F] (NHWC) -- final or staged in stored filter order
     int Bn, Bp, Hp, Wp, Cin, F, R, S, stride, Ho, Wo;
+    // An output row counts as row_pix >= Wo pixels: with the TMA gather a row may be rounded up so that no box of 64
+    // tokens crosses from one into the next, where the input's halo makes addresses jump.  Tokens of pixels
+    // ow >= Wo are computed from whatever is there and stored nowhere.
+    int row_pix;
     // chained SpConv: out[f][OHp][OWp][Bp] with the next layer's halo (origin at (oph, opw))
     int OWp, oph, opw, out_plane, relu;
     int wide_stores;         // SpMM, rows in lanes: output rows are 32-byte aligned (N % 16 == 0, D % 32 == 0)
@@ -356,19 +361,35 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 ++li;
             }
         };
-        auto row_id = [&](int r) { return li < nloc && r < rows_total ? __ldg(p.blk_idx + row_begin + r) : 0; };   // of the item's row r
+        auto row_id = [&](int r) {                           // of the item's row r
+            int v = li < nloc && r < rows_total ? __ldg(p.blk_idx + row_begin + r) : 0;
+            // (SpConv: column ids come decoded as c | r << 16 | s << 24; the map's row is the pixel that the tap starts at)
+            if constexpr (CONV) v = ((v & 0xffff) * p.Hp + ((v >> 16) & 0xff)) * p.Wp + ((v >> 24) & 0xff);
+            return v;
+        };
         int id[IPL];
         auto load_ids = [&]() {
 #pragma unroll
             for (int i = 0; i < IPL; ++i) id[i] = row_id(kt * KS + pw * WQ * 4 + i * 32 + lane);
         };
-        int xs[BOXES], nbox = 0, of_item = -1;              // first column of each box, boxes that hold any token
+        int xs[BOXES], boxes = 0, nbox = 0, of_item = -1;   // first column of each box; boxes that hold any token
         auto enter_item = [&]() {
             of_item = li;
             const int tok0 = item_tile((int)blockIdx.x + li * (int)gridDim.x) * T;
-            nbox = min(BOXES, (p.N - tok0 + 63) / 64);       // columns beyond N are never stored: boxes past it are not fetched
+            boxes = 0;                                       // boxes without a token that is stored are not fetched
 #pragma unroll
-            for (int b = 0; b < BOXES; ++b) xs[b] = tok0 + b * 64;
+            for (int b = 0; b < BOXES; ++b) {
+                const int tok = tok0 + b * 64;
+                xs[b] = tok;
+                bool any = tok < p.N;
+                if constexpr (CONV) {
+                    const int pix = fast_div(tok, p.div_bp), oh = fast_div(pix, p.div_row), ow = pix - oh * p.row_pix;
+                    xs[b] = (oh * p.Wp + ow) * p.stride * p.Bp + tok - pix * p.Bp;
+                    any = any && ow < p.Wo;
+                }
+                boxes |= (int)any << b;
+            }
+            nbox = __popc(boxes);
         };
         // rows in lanes: [K group][T/64 atoms]; tokens in lanes: [128-token half][K group][2 atoms]
         auto dst_off = [](int q, int b) {
@@ -403,7 +424,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 const int4 r = *(const int4*)(my_ids + i * 4);
 #pragma unroll
                 for (int b = 0; b < BOXES; ++b)
-                    if (q * 4 < first_valid && b < nbox) sm100::tma_gather4(smem_base + dst_off(q, b), p.tmap_b, xs[b], r.x, r.y, r.z, r.w, &full_bar[0]);
+                    if (q * 4 < first_valid && (boxes >> b & 1)) sm100::tma_gather4(smem_base + dst_off(q, b), p.tmap_b, xs[b], r.x, r.y, r.z, r.w, &full_bar[0]);
             }
         }
         __syncwarp();
@@ -442,13 +463,14 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     for (int q = 0; q < WQ; ++q)
 #pragma unroll
                         for (int b = 0; b < BOXES; ++b)
-                            if ((pw * WQ + q) * 4 < rows_valid && b < nbox) copy(q, b);
+                            if ((pw * WQ + q) * 4 < rows_valid && (boxes >> b & 1)) copy(q, b);
                 }
             }
             __syncwarp();                                    // the row ids may be overwritten
             it += GROUPS; s += GROUPS;
             if (s >= (uint32_t)STAGES) { s -= STAGES; ph ^= 1u; }
         }
+        if (MODE == kPanelConv && p.trigger_late) sm100::grid_dependency_launch();
         }
     } else if (warp > EW) {
         // --------------------------------------------- producers (cp.async gather) ----
@@ -543,7 +565,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             if constexpr (CONV) {
                 if (chunk_ok) {
                     const int pix = fast_div(tok0, p.div_bp), nn = tok0 - pix * p.Bp;
-                    const int oh = fast_div(pix, p.div_wo), ow = pix - oh * p.Wo;
+                    const int oh = fast_div(pix, p.div_row), ow = pix - oh * p.row_pix;
                     conv_src0 = p.Xs + ((oh * p.stride * p.Wp + ow * p.stride) * p.Bp + nn);
                 }
             }
@@ -779,18 +801,20 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     // to them: requested before the accumulator read, so that the global-memory latency
                     // hides behind it.
                     size_t goffs[4];
+                    bool valid[4] = {};
                     uint4 addend[4];
                     {
                         if constexpr (CHAIN) {
                             // 8 consecutive tokens are 8 images of one output pixel; the pixel's place in the
                             // consumer's halo-padded plane is found once and stepped from group to group
                             int pix = fast_div(tok0, p.div_bp), nn = tok0 - pix * p.Bp;
-                            int oh = fast_div(pix, p.div_wo), ow = pix - oh * p.Wo;
+                            int oh = fast_div(pix, p.div_row), ow = pix - oh * p.row_pix;
 #pragma unroll
                             for (int c = 0; c < 4; ++c) {
                                 goffs[c] = (size_t)(((oh + p.oph) * p.OWp + ow + p.opw) * p.Bp + nn);
+                                valid[c] = tok0 + c * 8 < p.N && ow < p.Wo;
                                 nn += 8;
-                                if (nn >= p.Bp) { nn = 0; if (++ow >= p.Wo) { ow = 0; ++oh; } }
+                                if (nn >= p.Bp) { nn = 0; if (++ow >= p.row_pix) { ow = 0; ++oh; } }
                             }
                         } else {
 #pragma unroll
@@ -800,7 +824,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 #pragma unroll
                             for (int c = 0; c < 4; ++c) {
                                 addend[c] = make_uint4(0u, 0u, 0u, 0u);
-                                if (use_res && tok0 + c * 8 < p.N) addend[c] = *(const uint4*)(p.res + rres + goffs[c]);
+                                if (use_res && valid[c]) addend[c] = *(const uint4*)(p.res + rres + goffs[c]);
                             }
                         }
                     }
@@ -853,7 +877,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     } else {
 #pragma unroll
                         for (int c = 0; c < 4; ++c) {
-                            if (tok0 + c * 8 < p.N) {
+                            if (valid[c]) {
                                 __half2* h = (__half2*)&v[c];
                                 if (use_res) {                           // out = relu(alpha * conv + residual), fp16
                                     const __half2* rh = (const __half2*)&addend[c];
@@ -884,8 +908,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             uint32_t row_off[4];                           // SpConv: output offsets of positions i*8 + lane/4
             if constexpr (MODE == kPanelConv) {
                 const int pix = fast_div(tok, p.div_bp), img = tok - pix * p.Bp;
-                ok = ok && img < p.Bn;
-                const int oh = fast_div(pix, p.div_wo), ow = pix - oh * p.Wo;
+                const int oh = fast_div(pix, p.div_row), ow = pix - oh * p.row_pix;
+                ok = ok && img < p.Bn && ow < p.Wo;
                 // this position's F-vector at the block's filters (element offset; host checks it fits 32 bits)
                 const uint32_t mine = ok ? (uint32_t)((img * p.Ho + oh) * p.Wo + ow) * (uint32_t)p.F + (uint32_t)(blk * V + mbase)
                                          : 0xffffffffu;
@@ -921,7 +945,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 if constexpr (MODE == kPanelConvChain) {
                     if (ok_) {
                         const int pix = fast_div(tok_g, p.div_bp), nn = tok_g - pix * p.Bp;
-                        const int oh = fast_div(pix, p.div_wo), ow = pix - oh * p.Wo;
+                        const int oh = fast_div(pix, p.div_row), ow = pix - oh * p.row_pix;
+                        ok_ = ow < p.Wo;
                         goff_ = (uint32_t)(((oh + p.oph) * p.OWp + ow + p.opw) * p.Bp + nn);
                     }
                 }

@@ -120,10 +120,10 @@ PanelChoice choice() {
             STAGES, PW, Cfg::THREADS, 0, GATHER};
 }
 
-// TMA tensor map of the dense operand B ([K][N] fp16 row-major): box = 64 tokens x 1 row (what one
-// row of a tile::gather4 fetches), 128-byte swizzle (the layout tcgen05.mma reads), zero fill
-// outside the tensor.  The driver entry point is looked up once.
-int encode_b_map(const void* B, int K, int N, unsigned long long out[16]) {
+// TMA tensor map of a dense operand (`rows` rows of `cols` fp16, `pitch` bytes from one to the next; rows may
+// overlap): box = 64 tokens x 1 row (what one row of a tile::gather4 fetches), 128-byte swizzle (the layout
+// tcgen05.mma reads), zero fill outside the tensor.  The driver entry point is looked up once.
+int encode_map(const void* base, long long rows, long long cols, long long pitch, unsigned long long out[16]) {
     typedef CUresult (*Encode)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -137,9 +137,9 @@ int encode_b_map(const void* B, int K, int N, unsigned long long out[16]) {
     }
     static_assert(sizeof(CUtensorMap) == 128, "tensor map size");
     alignas(64) CUtensorMap tm;
-    const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)K}, strides[1] = {(cuuint64_t)N * 2};
+    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows}, strides[1] = {(cuuint64_t)pitch};
     const cuuint32_t box[2] = {64, 1}, estr[2] = {1, 1};
-    const CUresult r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(B), dims, strides, box, estr,
+    const CUresult r = enc(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, estr,
                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
@@ -152,12 +152,12 @@ int encode_b_map(const void* B, int K, int N, unsigned long long out[16]) {
 
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
+constexpr int kWideConvTmaWarps = 2;                          // (three would make a block as large as the cp.async one: conv_gather)
+
 // Shapes of the TMA gather: eight producer warps, two to a stage.
 template <int V, int TM, int STAGES, int MODE, bool BIAS>
 PanelChoice regular(int gather) {
-    if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelSpmmRows) {
-        if (gather == shflbw::kGatherTma) return choice<V, TM, 64, STAGES, 8, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
-    }
+    if (gather == shflbw::kGatherTma) return choice<V, TM, 64, STAGES, 8, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
     return choice<V, TM, 64, STAGES, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>();
 }
 template <int MODE, bool BIAS = false>
@@ -170,12 +170,11 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
         // 256, the rest equal); eight in the instance without the slots.  Built for 64-row blocks.
         // wide_ring: 6 or 8 stages, 0 for the regular kernels.
         if (wide_ring && tile == 256 && V == 64) {
-            if constexpr (MODE == shflbw::kPanelSpmm) {
-                if (gather == shflbw::kGatherTma) {
-                    *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherTma, 16, BIAS, false>()
-                                          : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherTma, 16, BIAS, true>();
-                    return true;
-                }
+            if (gather == shflbw::kGatherTma) {
+                constexpr int PW = MODE == shflbw::kPanelSpmm ? 3 : kWideConvTmaWarps;
+                *out = wide_ring == 8 ? choice<64, 2, 32, 8, PW, MODE, PW, shflbw::kGatherTma, 16, BIAS, false>()
+                                      : choice<64, 2, 32, 6, PW, MODE, PW, shflbw::kGatherTma, 16, BIAS, true>();
+                return true;
             }
             *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, false>()
                                   : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, true>();
@@ -228,6 +227,41 @@ int sm_count() {
     return n;
 }
 
+// A convolution's state says by its number of threads how it gathers.
+using ConvCpAsync = shflbw::PanelCfg<64, 2, 64, 5, 8, shflbw::kPanelConvChain, 2, shflbw::kGatherCpAsync, 8>;
+using ConvCpAsyncWide = shflbw::PanelCfg<64, 2, 32, 8, 3, shflbw::kPanelConvChain, 3, shflbw::kGatherCpAsync, 16>;
+int conv_gather(const shflbw_spconv_state_t& st) {
+    return st.block_x == (unsigned)(st.variant == 2 ? ConvCpAsyncWide::THREADS : ConvCpAsync::THREADS) ? shflbw::kGatherCpAsync : shflbw::kGatherTma;
+}
+
+// How a convolution counts its tokens when it gathers by TMA: a box is 64 consecutive tokens, and has to be 128
+// consecutive bytes of the staged input.  Without a halo (Wp == Wo) all tokens of an image plane are; with one
+// those of an output row, which then counts as so many pixels (a multiple of 64 tokens); with a stride those of one
+// pixel.  Returns the pixels that a row counts as, 0 where boxes do not fit.
+int tma_row_pix(int Wo, int Wp, int Bp, int stride) {
+    if (stride == 1 && Wp == Wo) return Wo;
+    int pixels = 1;                                           // that make up whole boxes
+    while (pixels * Bp % 64) pixels *= 2;
+    return stride > 1 && pixels > 1 ? 0 : (Wo + pixels - 1) / pixels * pixels;
+}
+
+// SHFLBW_GATHER=0 takes the cp.async gather everywhere (tuning aid).  Asked for when a state is made.
+bool tma_wanted() { const char* g = getenv("SHFLBW_GATHER"); return !g || atoi(g) == 1; }
+
+// The gather of a convolution, and the pixels that an output row counts as.  TMA, unless the padding of the rows
+// costs the SMs more than a quarter in rounds of items: a stage takes it about 650 clk and the cp.async gather 870
+// to 1000 (14x14x512 -> 2048, batch 16, V = 64, 3 -> 4 rounds: 28.0 us by cp.async, 28.6 by TMA; V = 32, 6 -> 7:
+// 35.9 and 33.5; 7x7x512 -> 512, batch 8: 12.6 and 10.9).
+struct ConvTokens { int row_pix; int gather; };
+ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int row_blocks) {
+    const ConvTokens plain{Wo, shflbw::kGatherCpAsync};
+    const int row_pix = tma_wanted() ? tma_row_pix(Wo, Wp, Bp, stride) : 0;
+    if (!row_pix || (long long)Ho * row_pix * Bp >= (1ll << 31)) return plain;
+    const int sms = sm_count() > 0 ? sm_count() : 148;
+    auto rounds = [&](int pix) { return (((long long)Ho * pix * Bp + 255) / 256 * row_blocks + sms - 1) / sms; };
+    return 4 * rounds(row_pix) > 5 * rounds(Wo) ? plain : ConvTokens{row_pix, shflbw::kGatherTma};
+}
+
 // Opt a kernel in to its dynamic shared memory once per (device, kernel): the host-buffer
 // calls initialise an op per chunk, and the attribute call is not free.
 int allow_smem(const void* fn, size_t bytes) {
@@ -249,7 +283,8 @@ int allow_smem(PanelKernel fn, size_t bytes) { return allow_smem((const void*)fn
 // the default; 128 is used when the dense extent is too small to give every SM a few items.
 // SHFLBW_TILE=128|256 overrides (tuning aid).
 template <int MODE>
-int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols, PanelChoice* out, bool addend = false) {
+int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols, PanelChoice* out, bool addend = false,
+               int gather = shflbw::kGatherTma) {
     // Token tile: a persistent CTA works through ceil(items / SMs) items in turn; an item of
     // the 128-token tile was measured at ~2/3 of the time of a 256-token item (half the
     // gathered bytes, the same number of pipeline stages).
@@ -266,9 +301,7 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
     // SpMM and chained SpConv with V = 64 / 128 can run with the operands swapped (rows in TMEM
     // lanes, one MMA per 16 columns for the whole token tile); SHFLBW_SWAP=0|1 forces the choice
     // (tuning aid).
-    // SpMM gathers by TMA; SHFLBW_GATHER=0 takes cp.async (tuning aid).
-    int gather = MODE == shflbw::kPanelSpmm ? shflbw::kGatherTma : shflbw::kGatherCpAsync;
-    if (const char* g = getenv("SHFLBW_GATHER")) if (atoi(g) != 1) gather = shflbw::kGatherCpAsync;
+    if (!tma_wanted()) gather = shflbw::kGatherCpAsync;
     bool swapped = false;
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         const char* e = getenv("SHFLBW_SWAP");
@@ -468,7 +501,7 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
         out->kernel = SHFLBW_KERNEL_TCGEN05;
         out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
         out->gather = ch.gather;
-        if (ch.gather == shflbw::kGatherTma && (rc = encode_b_map(B, m->ncol, N, out->tmap_b)) != SHFLBW_OK) return rc;
+        if (ch.gather == shflbw::kGatherTma && (rc = encode_map(B, m->ncol, N, 2ll * N, out->tmap_b)) != SHFLBW_OK) return rc;
         out->tiles_n = (N + ch.tokens - 1) / ch.tokens;
         out->num_items = out->tiles_n * out->num_row_blocks;
         const int sms = sm_count();
@@ -506,7 +539,7 @@ static int launch_spmm_panel(const shflbw_spmm_state_t* st, const PanelChoice& c
     p.wide_stores = (st->N % 16 == 0) && (((uintptr_t)st->D & 31) == 0);
     if (st->gather == shflbw::kGatherTma) std::memcpy(p.tmap_b, st->tmap_b, sizeof p.tmap_b);
     p.num_items = st->num_items; p.tiles_n = st->tiles_n;
-    p.div_tiles = shflbw::make_fast_div(st->tiles_n); p.div_bp = p.div_wo = shflbw::make_fast_div(1);
+    p.div_tiles = shflbw::make_fast_div(st->tiles_n); p.div_bp = p.div_row = shflbw::make_fast_div(1);
     // Tile-major item order: concurrent CTAs gather from the same few token tiles of B (SHFLBW_ITEM_ORDER=0|1
     // forces block-major / tile-major; tuning aid).
     p.num_blocks = st->num_row_blocks; p.div_blocks = shflbw::make_fast_div(st->num_row_blocks);
@@ -765,6 +798,11 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     const int row_blocks = f->F / f->brow;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
 
+    // the input as the panel kernel sees it: a strided 1x1 filter's pixels are staged side by side
+    const bool compact = f->R == 1 && f->S == 1;
+    const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, row_blocks);
+    const long long counted = (long long)Ho * ct.row_pix * Bp;
+
     // planes out?
     PanelChoice ch;
     bool planes = false;
@@ -774,7 +812,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
         bool want = padded_cols >= 192ll * row_blocks;      // same rule as the chained layers: >= 3 stages per block
         if (const char* e = getenv("SHFLBW_CONV_PLANES")) want = atoi(e) != 0;
         if (want) {
-            rc = pick_panel<shflbw::kPanelConvChain>(f->brow, tokens, row_blocks, want ? (1ll << 40) : 0, &ch);
+            rc = pick_panel<shflbw::kPanelConvChain>(f->brow, counted, row_blocks, want ? (1ll << 40) : 0, &ch, false, ct.gather);
             if (rc != SHFLBW_OK) return rc;
             planes = ch.variant == 1;
         }
@@ -783,7 +821,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
         out->variant = 1;
         out->staged_out_bytes = (size_t)f->F * (size_t)tokens * 2;
     } else {
-        rc = pick_panel<shflbw::kPanelConv>(f->brow, tokens, row_blocks, 0, &ch);
+        rc = pick_panel<shflbw::kPanelConv>(f->brow, counted, row_blocks, 0, &ch, false, ct.gather);
         if (rc != SHFLBW_OK) return rc;
         out->variant = 0;
         if (f->row_permute) {
@@ -796,7 +834,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     }
     out->kernel = SHFLBW_KERNEL_TCGEN05;
     out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw;
-    out->tiles_n = (int)((tokens + ch.tokens - 1) / ch.tokens);
+    out->tiles_n = (int)((counted + ch.tokens - 1) / ch.tokens);
     out->num_items = out->tiles_n * row_blocks;
     const int sms = sm_count();
     if (sms <= 0) return SHFLBW_ERR_CUDA;
@@ -841,10 +879,11 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     const bool planes = !st->chain && st->variant == 1;     // NHWC call computed as planes, then transposed
     PanelChoice ch;
     const bool panel_bias = bias && !planes && !st->staged_out;   // no later pass: the panel kernel's epilogue adds the bias
-    const bool ok_kernel = panel_bias            ? lookup<shflbw::kPanelConv, true>(st->V, st->tokens_per_cta, &ch)
-                           : (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch)
-                           : st->variant == 1      ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch)
-                                                   : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, shflbw::kGatherCpAsync,
+    const int gather = conv_gather(*st);
+    const bool ok_kernel = panel_bias            ? lookup<shflbw::kPanelConv, true>(st->V, st->tokens_per_cta, &ch, gather)
+                           : (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch, gather)
+                           : st->variant == 1      ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch, gather)
+                                                   : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, gather,
                                                                                       st->variant != 2 ? 0 : st->residual ? 6 : st->stages);
     if (!ok_kernel) return SHFLBW_ERR_INVALID_ARG;
     if (panel_bias) {                                       // (init allowed the kernel without; before anything is launched)
@@ -857,12 +896,23 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     //    output's size that is then read at stride 1 (27x27x256 -> 14x14x512, batch 5: 3.4 -> 2.5 us).
     const int step = !st->chain && st->R == 1 && st->S == 1 ? st->stride : 1;
     const int Hp = step > 1 ? st->Ho : st->Hin + st->R - 1, Wp = step > 1 ? st->Wo : st->Win + st->S - 1;
+    shflbw::PanelParams p{};
+    p.Xs = (const __half*)(st->chain ? st->ifmap : st->staged_in);
+    p.stride = st->stride / step;
+    p.row_pix = st->Wo;
+    if (gather == shflbw::kGatherTma) {
+        p.row_pix = tma_row_pix(st->Wo, Wp, st->Bp, p.stride);
+        // One row per pixel a tap of output pixel (0, 0) reads, `pitch` from one to the next, as long as from output
+        // pixel (0, 0) to the last: every address that the map allows is inside the staged input.
+        const int rc = encode_map(p.Xs, ((long long)st->C - 1) * Hp * Wp + (long long)(st->R - 1) * Wp + st->S,
+                                  (((long long)st->Ho - 1) * p.stride * Wp + ((long long)st->Wo - 1) * p.stride + 1) * st->Bp, 2ll * st->Bp, p.tmap_b);
+        if (rc != SHFLBW_OK) return rc;
+    }
     long long relayout_per_sm = 0;
     if (!st->chain)
         relayout_per_sm = launch_relayout((const __half*)st->ifmap, (__half*)st->staged_in, st->B, st->Bp, st->Hin, st->Win, st->C,
                                           st->R, st->S, s, step, planes || st->staged_out);
     // 2. implicit-GEMM panel kernel.
-    shflbw::PanelParams p{};
     // Where it ends the call: see the kernel.  A call that stages many blocks per SM is likely to be followed by another
     // one, whose first blocks cannot be spread over the SMs (26x48x48x1024 -> 96 at stride 2, back to back: 73 us, 76
     // with the trigger); it is long enough not to miss the 1.2 us.
@@ -870,8 +920,7 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     p.blk_ptr = st->blk_ptr; p.blk_idx = st->blk_idx; p.blk_val = (const __half*)st->blk_val;
     p.perm = st->perm; p.status_word = st->status_word; p.alpha = st->alpha; p.beta = 0.f;
     p.wait_limit = g_wait_limit; p.inject_from = g_inject_from;
-    p.N = st->Ho * st->Wo * st->Bp;
-    p.Xs = (const __half*)(st->chain ? st->ifmap : st->staged_in);
+    p.N = st->Ho * p.row_pix * st->Bp;
     p.out = (__half*)(st->staged_out ? st->staged_out : st->ofmap);
     if (st->chain) {
         p.res = (const __half*)st->residual; p.res_map = st->residual_map;
@@ -884,9 +933,9 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     }
     p.idx_limit = (unsigned)((((long long)st->C - 1) * Hp * Wp + (long long)(st->R - 1) * Wp + (st->S - 1)) * st->Bp);
     p.Bn = st->B; p.Bp = st->Bp; p.Hp = Hp; p.Wp = Wp; p.Cin = st->C; p.F = st->F;
-    p.R = st->R; p.S = st->S; p.stride = st->stride / step; p.Ho = st->Ho; p.Wo = st->Wo;
+    p.R = st->R; p.S = st->S; p.Ho = st->Ho; p.Wo = st->Wo;
     p.num_items = st->num_items; p.tiles_n = st->tiles_n;
-    p.div_tiles = shflbw::make_fast_div(st->tiles_n); p.div_bp = shflbw::make_fast_div(st->Bp); p.div_wo = shflbw::make_fast_div(st->Wo);
+    p.div_tiles = shflbw::make_fast_div(st->tiles_n); p.div_bp = shflbw::make_fast_div(st->Bp); p.div_row = shflbw::make_fast_div(p.row_pix);
     p.num_blocks = st->F / st->V; p.div_blocks = shflbw::make_fast_div(p.num_blocks);
     // Block-major item order for the convolutions: running a token tile's filter blocks at the same time
     // (tile-major) was measured equal on the ResNet-50 stack and on config 3, whose inputs are small next
@@ -1026,11 +1075,13 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     out->perm = f->d_perm; out->status_word = f->d_status;
     out->chain = 1; out->out_R = R_next; out->out_S = S_next; out->relu = relu != 0;
     PanelChoice ch;
-    int rc = pick_panel<shflbw::kPanelConvChain>(f->brow, tokens, f->F / f->brow, f->kptr.empty() ? 0 : f->kptr.back(), &ch);
+    const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, f->F / f->brow);
+    const long long counted = (long long)Ho * ct.row_pix * Bp;
+    int rc = pick_panel<shflbw::kPanelConvChain>(f->brow, counted, f->F / f->brow, f->kptr.empty() ? 0 : f->kptr.back(), &ch, false, ct.gather);
     if (rc != SHFLBW_OK) return rc;
     out->kernel = SHFLBW_KERNEL_TCGEN05;
     out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
-    out->tiles_n = (int)((tokens + ch.tokens - 1) / ch.tokens);
+    out->tiles_n = (int)((counted + ch.tokens - 1) / ch.tokens);
     out->num_items = out->tiles_n * (f->F / f->brow);
     const int sms = sm_count();
     if (sms <= 0) return SHFLBW_ERR_CUDA;
@@ -1066,7 +1117,7 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     const bool wide = (st->variant == 2 ||
                        (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
                         (f->kptr.empty() ? 0 : f->kptr.back()) <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count())) &&
-                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, shflbw::kGatherCpAsync, 6);
+                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, conv_gather(*st), 6);
     if (wide) {
         const int rc = allow_smem(ch.fn, ch.smem);
         if (rc != SHFLBW_OK) return rc;
