@@ -334,8 +334,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         // Bound by the issue: an operation takes seven operands in uniform registers, 15 clk of a warp that has
         // the issue slots for itself and 32 in here, where the copy engine would take one every 9.  Hence two
         // warps a stage (11008x4096x512, V = 32, density 0.25: 34.9 us with one, 32.5 with two; 4096^3 at
-        // V = 16, 0.1: 77.4 and 72.3; sixteen warps, four to a stage: 33.3 and 74.0, but 25.3 instead of 26.4 us at
-        // V = 64), and a loop whose control the compiler can see to be uniform.
+        // V = 16, 0.1: 77.4 and 72.3; sixteen warps, four to a stage: 33.3 and 74.0), four for SpMM with rows in
+        // lanes (4096^3, V = 64: 26.4 us with two, 25.3 with four), and a loop whose control the compiler can see to be uniform.
         // Every warp of a stage arrives on its barrier, with the bytes it fetches.  If only one did, a warp
         // without a row in a short last stage would be waited for by nobody, could fall a whole ring behind,
         // miss the phase that it waits for and wait for good.

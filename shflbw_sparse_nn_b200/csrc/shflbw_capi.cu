@@ -154,10 +154,13 @@ int encode_map(const void* base, long long rows, long long cols, long long pitch
 // as fit beside the 16 KB of epilogue tiles).
 constexpr int kWideConvTmaWarps = 2;                          // (three would make a block as large as the cp.async one: conv_gather)
 
-// Shapes of the TMA gather: eight producer warps, two to a stage.
+// Shapes of the TMA gather: four stages at a time, by two warps each, SpMM with rows in lanes by four: its items are
+// deep and its epilogue fits the 80 registers that 25 warps leave (4096^3 V = 64 26.7 -> 25.3 us, V = 128 21.2 -> 20.2,
+// 4096x4096x1024 density 0.5 24.8 -> 23.1; with tokens in lanes 11008x4096x512 V = 32 32.7 -> 33.3).
 template <int V, int TM, int STAGES, int MODE, bool BIAS>
 PanelChoice regular(int gather) {
-    if (gather == shflbw::kGatherTma) return choice<V, TM, 64, STAGES, 8, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
+    constexpr int PW = MODE == shflbw::kPanelSpmmRows ? 16 : 8;
+    if (gather == shflbw::kGatherTma) return choice<V, TM, 64, STAGES, PW, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
     return choice<V, TM, 64, STAGES, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>();
 }
 template <int MODE, bool BIAS = false>
