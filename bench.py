@@ -334,7 +334,7 @@ def run_ours(args):
                    "timing": f"{R} blocks of {args.steps} steps, median block (max over ranks) / steps",
                    "launch": (f"CUDA graph of {G} steps replayed {args.steps // G}x per block" if G else "one host launch per step"),
                    "power": ("a timed region of ~60 ms runs at the full SM clock; 100+ ms of back-to-back launches of this "
-                             "kernel reach the board's power cap (sw_power_cap, ~1.85-1.89 GHz measured: ~36.7 us per step)")},
+                             "kernel reach the board's power cap (sw_power_cap, lower SM clocks)")},
         "dense_equivalent_tflops": round(world * flops_dense / (ms_step * 1e-3) / 1e12, 2),
         "roofline": roofline, "gpu_launches": R * args.steps * ops[0].launches_per_exec, "clocks": clocks,
     }
