@@ -33,9 +33,10 @@
 //                    group publishes its previous stage half-way through issuing the next one,
 //                    with ONE mbarrier arrival per warp; row ids are prefetched two of the
 //                    group's stages ahead by 4-byte cp.async into a shared-memory ring.  TMA
-//                    gather: tile::gather4 copies, completion by byte count.  One bulk copy per stage for the value slice either way.
-//   later warps with w % 4 == 0   idle, so that no producer shares the MMA warp's scheduler partition.
-// The accumulator is double buffered in TMEM (four sets with EW = 16) so the epilogue of item i
+//                    gather (every warp after the MMA warp): tile::gather4 copies, completion by byte count.
+//                    One bulk copy per stage for the value slice either way.
+//   later warps with w % 4 == 0   beside cp.async producers idle, so that none shares the MMA warp's scheduler partition.
+// The accumulator is double buffered in TMEM (four sets with EW = 16 and with 64 rows in lanes) so the epilogue of item i
 // overlaps the main loop of item i+1, and the stage ring runs across item boundaries without
 // draining.
 //
@@ -162,10 +163,10 @@ struct PanelCfg {
     static constexpr int T = 128 * TM;
     static constexpr int GROUPS = GROUPS_;                 // producer groups that take the stages in turn
     // Warp w runs on scheduler partition w % 4.  The MMA warp (the first after the epilogue
-    // warps: 8 or 16) sits on partition 0 and no producer shares it: the later warps with
-    // w % 4 == 0 stay idle.  The MMA warp executes a
-    // few dozen instructions per stage and was measured at ~20 clk per instruction when
-    // producer code kept evicting its lines from the partition's instruction cache.
+    // warps: 8 or 16) sits on partition 0; beside cp.async producers the later warps with
+    // w % 4 == 0 stay idle: the MMA thread executes a few dozen instructions per stage and was
+    // measured at ~20 clk per instruction when their code kept evicting its lines from the
+    // partition's instruction cache.
     static constexpr int WARPS = EW + 1 + PW + (TMA ? 0 : (PW - 1) / 3);   // epilogue + MMA + producers + idle
     static_assert(EW == 8 || WARPS <= 20, "16 epilogue warps: at most 3 producers (20 warps leave 96 registers per thread, 21-24 only 80)");
     static constexpr int THREADS = WARPS * 32;
