@@ -185,7 +185,9 @@ typedef struct shflbw_spmm_state {
     const int* perm;         /* device row permutation or NULL */
     int* status_word;        /* device int: 0 ok, else a SHFLBW_DEVSTAT_* code */
     int gather;              /* 0: cp.async gather, 1: TMA tile-gather through tmap_b */
-    unsigned long long tmap_b[16]; /* TMA tensor map of B (opaque 128 bytes, built at init from B and N) */
+    unsigned long long tmap_b[16]; /* TMA tensor map of B (opaque 128 bytes, built at init) ... */
+    const void* tmap_of;     /* ... for this address and these extents; exec builds its own where B, N or K differ */
+    int tmap_cols, tmap_rows;
 } shflbw_spmm_state_t;
 
 /* Replaces SpmmBlockwiseOp::initialize / SpmmBlockwiseInitFn

@@ -38,6 +38,7 @@ class SpmmState(C.Structure):
         ("blk_ptr", C.c_void_p), ("blk_idx", C.c_void_p), ("blk_val", C.c_void_p),
         ("perm", C.c_void_p), ("status_word", C.c_void_p),
         ("gather", C.c_int), ("tmap_b", C.c_ulonglong * 16),
+        ("tmap_of", C.c_void_p), ("tmap_cols", C.c_int), ("tmap_rows", C.c_int),
     ]
 
 

@@ -504,7 +504,10 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
         out->kernel = SHFLBW_KERNEL_TCGEN05;
         out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
         out->gather = ch.gather;
-        if (ch.gather == shflbw::kGatherTma && (rc = encode_map(B, m->ncol, N, 2ll * N, out->tmap_b)) != SHFLBW_OK) return rc;
+        if (ch.gather == shflbw::kGatherTma) {
+            if ((rc = encode_map(B, m->ncol, N, 2ll * N, out->tmap_b)) != SHFLBW_OK) return rc;
+            out->tmap_of = B; out->tmap_cols = N; out->tmap_rows = m->ncol;
+        }
         out->tiles_n = (N + ch.tokens - 1) / ch.tokens;
         out->num_items = out->tiles_n * out->num_row_blocks;
         const int sms = sm_count();
@@ -540,7 +543,15 @@ static int launch_spmm_panel(const shflbw_spmm_state_t* st, const PanelChoice& c
     p.B = (const __half*)st->B; p.C = (const __half*)st->C; p.D = (__half*)st->D; p.N = st->N;
     if (bias) { p.C = (const __half*)bias; p.beta = 1.f; }
     p.wide_stores = (st->N % 16 == 0) && (((uintptr_t)st->D & 31) == 0);
-    if (st->gather == shflbw::kGatherTma) std::memcpy(p.tmap_b, st->tmap_b, sizeof p.tmap_b);
+    // The state is the caller's: an operand that they exchanged is gathered through a map of its own.
+    if (st->gather == shflbw::kGatherTma) {
+        if (st->tmap_of == st->B && st->tmap_cols == st->N && st->tmap_rows == st->K) {
+            std::memcpy(p.tmap_b, st->tmap_b, sizeof p.tmap_b);
+        } else {
+            const int rc = encode_map(st->B, st->K, st->N, 2ll * st->N, p.tmap_b);
+            if (rc != SHFLBW_OK) return rc;
+        }
+    }
     p.num_items = st->num_items; p.tiles_n = st->tiles_n;
     p.div_tiles = shflbw::make_fast_div(st->tiles_n); p.div_bp = p.div_row = shflbw::make_fast_div(1);
     // Tile-major item order: concurrent CTAs gather from the same few token tiles of B (SHFLBW_ITEM_ORDER=0|1
