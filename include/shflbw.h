@@ -267,6 +267,9 @@ typedef struct shflbw_spconv_state {
     int relu;                /* 1: max(x, 0) fused into the epilogue                    */
     const void* residual;    /* chained: optional residual chain buffer (output geometry) */
     const int* residual_map; /* chained: stored filter -> plane of `residual`, or NULL     */
+    int gather;              /* 0: cp.async gather, 1: TMA tile-gather                     */
+    int row_pix;             /* pixels that an output row counts as (>= Wo; the TMA gather may round rows up to whole
+                                boxes): tiles_n and num_items are of Ho * row_pix * Bp tokens */
 } shflbw_spconv_state_t;
 
 /* Replaces SpconvBlockwiseOp::initialize / SpconvBlockwiseInitFn

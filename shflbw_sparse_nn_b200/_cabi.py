@@ -58,6 +58,7 @@ class SpconvState(C.Structure):
         ("perm", C.c_void_p), ("status_word", C.c_void_p),
         ("chain", C.c_int), ("out_R", C.c_int), ("out_S", C.c_int), ("relu", C.c_int),
         ("residual", C.c_void_p), ("residual_map", C.c_void_p),
+        ("gather", C.c_int), ("row_pix", C.c_int),
     ]
 
 

@@ -152,7 +152,7 @@ int encode_map(const void* base, long long rows, long long cols, long long pitch
 
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
-constexpr int kWideConvTmaWarps = 2;                          // (three would make a block as large as the cp.async one: conv_gather)
+constexpr int kWideConvTmaWarps = 2;
 
 // Shapes of the TMA gather: four stages at a time, by two warps each, SpMM with rows in lanes by four: its items are
 // deep and its epilogue fits the 80 registers that 25 warps leave (4096^3 V = 64 26.7 -> 25.3 us, V = 128 21.2 -> 20.2,
@@ -228,13 +228,6 @@ int sm_count() {
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
     if (dev >= 0 && dev < kMaxDevices) cached[dev] = n;
     return n;
-}
-
-// A convolution's state says by its number of threads how it gathers.
-using ConvCpAsync = shflbw::PanelCfg<64, 2, 64, 5, 8, shflbw::kPanelConvChain, 2, shflbw::kGatherCpAsync, 8>;
-using ConvCpAsyncWide = shflbw::PanelCfg<64, 2, 32, 8, 3, shflbw::kPanelConvChain, 3, shflbw::kGatherCpAsync, 16>;
-int conv_gather(const shflbw_spconv_state_t& st) {
-    return st.block_x == (unsigned)(st.variant == 2 ? ConvCpAsyncWide::THREADS : ConvCpAsync::THREADS) ? shflbw::kGatherCpAsync : shflbw::kGatherTma;
 }
 
 // How a convolution counts its tokens when it gathers by TMA: a box is 64 consecutive tokens, and has to be 128
@@ -848,6 +841,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     }
     out->kernel = SHFLBW_KERNEL_TCGEN05;
     out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw;
+    out->gather = ch.gather; out->row_pix = ct.row_pix;
     out->tiles_n = (int)((counted + ch.tokens - 1) / ch.tokens);
     out->num_items = out->tiles_n * row_blocks;
     const int sms = sm_count();
@@ -893,7 +887,7 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     const bool planes = !st->chain && st->variant == 1;     // NHWC call computed as planes, then transposed
     PanelChoice ch;
     const bool panel_bias = bias && !planes && !st->staged_out;   // no later pass: the panel kernel's epilogue adds the bias
-    const int gather = conv_gather(*st);
+    const int gather = st->gather;
     const bool ok_kernel = panel_bias            ? lookup<shflbw::kPanelConv, true>(st->V, st->tokens_per_cta, &ch, gather)
                            : (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch, gather)
                            : st->variant == 1      ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch, gather)
@@ -913,9 +907,8 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     shflbw::PanelParams p{};
     p.Xs = (const __half*)(st->chain ? st->ifmap : st->staged_in);
     p.stride = st->stride / step;
-    p.row_pix = st->Wo;
+    p.row_pix = st->row_pix;
     if (gather == shflbw::kGatherTma) {
-        p.row_pix = tma_row_pix(st->Wo, Wp, st->Bp, p.stride);
         // One row per pixel a tap of output pixel (0, 0) reads, `pitch` from one to the next, as long as from output
         // pixel (0, 0) to the last: every address that the map allows is inside the staged input.
         const int rc = encode_map(p.Xs, ((long long)st->C - 1) * Hp * Wp + (long long)(st->R - 1) * Wp + st->S,
@@ -1095,6 +1088,7 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     if (rc != SHFLBW_OK) return rc;
     out->kernel = SHFLBW_KERNEL_TCGEN05;
     out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
+    out->gather = ch.gather; out->row_pix = ct.row_pix;
     out->tiles_n = (int)((counted + ch.tokens - 1) / ch.tokens);
     out->num_items = out->tiles_n * (f->F / f->brow);
     const int sms = sm_count();
@@ -1131,7 +1125,7 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     const bool wide = (st->variant == 2 ||
                        (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
                         (f->kptr.empty() ? 0 : f->kptr.back()) <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count())) &&
-                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, conv_gather(*st), 6);
+                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6);
     if (wide) {
         const int rc = allow_smem(ch.fn, ch.smem);
         if (rc != SHFLBW_OK) return rc;

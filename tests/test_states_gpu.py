@@ -54,3 +54,25 @@ def test_spconv_state_follows_exchanged_operands(V, R):
     op._state.ifmap, op._state.ofmap = xd.data_ptr(), yd.data_ptr()
     _call(op, f)
     assert np.array_equal(host(yd).view(np.uint16), y1.view(np.uint16))
+
+
+@pytest.mark.parametrize("Bn,H,W,R,stride,V,gather,row_pix", [
+    (8, 9, 16, 3, 1, 64, 1, 16),      # rows of whole 64-token boxes
+    (3, 9, 13, 3, 1, 32, 1, 16),      # rounded up to them
+    (64, 9, 13, 3, 2, 64, 1, 7),      # strided, a box per pixel
+    (16, 9, 9, 3, 2, 64, 0, 5),       # strided, no whole box: cp.async
+    (5, 9, 13, 1, 1, 128, 1, 13),     # no halo
+])
+def test_spconv_state_says_how_it_gathers(Bn, H, W, R, stride, V, gather, row_pix, monkeypatch):
+    """The gather and the pixels of a row are the plan's, and its item count is theirs; the other gather by request."""
+    f = sb.BlockwiseSpFilter().init_random(2 * V, R, R, 16, V, 1, 0.4, True, 19, values="uniform")
+    x = sb.uniform_half(20, Bn * H * W * 16).reshape(Bn, H, W, 16)
+    for env, want_gather, want_pix in ((None, gather, row_pix), ("0", 0, -(-W // stride))):
+        if env is None:
+            monkeypatch.delenv("SHFLBW_GATHER", raising=False)
+        else:
+            monkeypatch.setenv("SHFLBW_GATHER", env)
+        _, op = run_spconv(f, Bn, H, W, stride, x)
+        st = op._state
+        assert (st.gather, st.row_pix) == (want_gather, want_pix)
+        assert st.num_items == 2 * -(-(st.Ho * st.row_pix * st.Bp) // st.tokens_per_cta)
