@@ -152,8 +152,6 @@ int encode_map(const void* base, long long rows, long long cols, long long pitch
 
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
-constexpr int kWideConvTmaWarps = 2;
-
 // Shapes of the TMA gather: four stages at a time, by two warps each, SpMM with rows in lanes by four: its items are
 // deep and its epilogue fits the 80 registers that 25 warps leave (4096^3 V = 64 26.7 -> 25.3 us, V = 128 21.2 -> 20.2,
 // 4096x4096x1024 density 0.5 24.8 -> 23.1; with tokens in lanes 11008x4096x512 V = 32 32.7 -> 33.3).
@@ -172,11 +170,14 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
         // six items' inputs are in flight from HBM (five: 37.5 -> 40.5 us on 14x14x256 -> 1024 at batch
         // 256, the rest equal); eight in the instance without the slots.  Built for 64-row blocks.
         // wide_ring: 6 or 8 stages, 0 for the regular kernels.
+        // Three gather warps with a stage each at a time, whichever the gather: with two of them the TMA issue was the
+        // longest of an item's steps from 32 columns on (chained 14x14x256 -> 1024 with residual, batch 256, 102
+        // columns a block: 57.2 us, three 47.0, three by cp.async 49.9; 28x28x256 -> 512 without residual, batch
+        // 128, 48 columns: 36.8, 30.0, 33.1).
         if (wide_ring && tile == 256 && V == 64) {
             if (gather == shflbw::kGatherTma) {
-                constexpr int PW = MODE == shflbw::kPanelSpmm ? 3 : kWideConvTmaWarps;
-                *out = wide_ring == 8 ? choice<64, 2, 32, 8, PW, MODE, PW, shflbw::kGatherTma, 16, BIAS, false>()
-                                      : choice<64, 2, 32, 6, PW, MODE, PW, shflbw::kGatherTma, 16, BIAS, true>();
+                *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherTma, 16, BIAS, false>()
+                                      : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherTma, 16, BIAS, true>();
                 return true;
             }
             *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, false>()

@@ -8,7 +8,7 @@ import torch
 import oracle_api as oa
 import shflbw_sparse_nn_b200 as sb
 from conftest import assert_close_fp16
-from gpu_util import dev, epilogue_warps, host, operand_swap, run_spconv, run_spmm
+from gpu_util import dev, epilogue_warps, host, operand_swap, run_spconv, run_spmm, tile
 
 pytestmark = pytest.mark.gpu
 
@@ -66,7 +66,7 @@ def test_spconv(Bn, H, W, Cc, R, stride, V, tma, permute, monkeypatch):
     f = sb.BlockwiseSpFilter().init_random(F, R, R, Cc, V, 1, 0.5, permute, 41 + V, values="uniform")
     x = sb.uniform_half(42, Bn * H * W * Cc).reshape(Bn, H, W, Cc)
     (y, op), (y_cp, op_cp) = _both(monkeypatch, lambda: run_spconv(f, Bn, H, W, stride, x))
-    assert (op._state.block_x != op_cp._state.block_x) == tma
+    assert (op._state.gather, op_cp._state.gather) == (int(tma), 0)
     assert np.array_equal(y.view(np.uint16), y_cp.view(np.uint16))
     want = oa.spconv_ref_nhwc(Bn, H, W, Cc, F, R, R, stride, V, f.indptr, f.indices, f.values,
                               f.row_permute_ids if permute else None, x)
@@ -102,7 +102,7 @@ def test_chained_layer(Bn, H, stride, V, swap, ew, residual, monkeypatch):
         b1 = torch.zeros(sb.chain_buffer_elems(F, Ho, Wo, Bn, 3, 3), dtype=torch.float16, device="cuda")
         res = dev(sb.uniform_half(53, b1.numel()))
         sb.chain_import_nhwc(dev(x), Bn, H, W, Cc, 3, 3, b0, s)
-        with operand_swap(swap), epilogue_warps(ew):
+        with operand_swap(swap), epilogue_warps(ew), tile(256 if ew == 16 else None):
             op = sb.SpconvChainOp().initialize(f, Bn, H, W, stride, b0, b1, 3, 3, alpha=0.5, relu=True)
             if residual:
                 op.set_residual(res, None)
@@ -112,6 +112,8 @@ def test_chained_layer(Bn, H, stride, V, swap, ew, residual, monkeypatch):
         return host(b1), op
 
     (got, op), (want, op_cp) = _both(monkeypatch, run)
-    assert op._state.block_x != op_cp._state.block_x and op._state.variant == op_cp._state.variant
+    assert (op._state.gather, op_cp._state.gather) == (1, 0) and op._state.variant == op_cp._state.variant
+    if ew == 16:                                                 # three gather warps either way
+        assert op._state.variant == 2 and (op._state.producer_warps, op_cp._state.producer_warps) == (3, 3)
     assert np.array_equal(got.view(np.uint16), want.view(np.uint16))
     assert np.abs(got.astype(np.float32)).max() > 0
