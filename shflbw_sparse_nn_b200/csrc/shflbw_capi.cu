@@ -204,10 +204,17 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
             case 32256:  *out = regular<32, 2, 5, MODE, BIAS>(gather); return true;    // 36 KB
             case 64128:  *out = regular<64, 1, 8, MODE, BIAS>(gather); return true;    // 24 KB
             case 64256:  *out = regular<64, 2, 5, MODE, BIAS>(gather); return true;    // 40 KB
-            case 128128: *out = regular<128, 1, 6, MODE, BIAS>(gather); return true;   // 32 KB
-            case 128256: *out = regular<128, 2, 4, MODE, BIAS>(gather); return true;   // 48 KB
-            default: return false;
+            default: break;
         }
+        if constexpr (MODE == shflbw::kPanelConvChain) {
+            if (gather == shflbw::kGatherTma) return false;   // (conv_tokens)
+            if (V == 128 && tile == 128) { *out = choice<128, 1, 64, 6, 8, MODE>(); return true; }   // 32 KB
+            if (V == 128 && tile == 256) { *out = choice<128, 2, 64, 4, 8, MODE>(); return true; }   // 48 KB
+        } else {
+            if (V == 128 && tile == 128) { *out = regular<128, 1, 6, MODE, BIAS>(gather); return true; }
+            if (V == 128 && tile == 256) { *out = regular<128, 2, 4, MODE, BIAS>(gather); return true; }
+        }
+        return false;
     }
 }
 
@@ -249,15 +256,27 @@ bool tma_wanted() { const char* g = getenv("SHFLBW_GATHER"); return !g || atoi(g
 // costs the SMs more than a quarter in rounds of items: a stage takes it about 650 clk and the cp.async gather 870
 // to 1000 (14x14x512 -> 2048, batch 16, V = 64, 3 -> 4 rounds: 28.0 us by cp.async, 28.6 by TMA; V = 32, 6 -> 7:
 // 35.9 and 33.5; 7x7x512 -> 512, batch 8: 12.6 and 10.9).
+// Chained layers of 128 rows with tokens in lanes gather by cp.async: their items are an epilogue of 32 KB behind one to
+// three stages, and beside the TMA gather's operands that epilogue does not fit the 96 registers that 17 warps leave
+// (batch 128, 28x28x256 -> 256, 13 columns a block: 17.2 us, 18.3 by TMA; batch 64, 14x14x512 -> 1024 with residual,
+// 102 columns: 15.3 and 17.2).
 struct ConvTokens { int row_pix; int gather; };
-ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int row_blocks) {
+ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int row_blocks, bool chained_positions = false, int V = 0) {
     const ConvTokens plain{Wo, shflbw::kGatherCpAsync};
+    if (chained_positions && V == 128) return plain;
     const int row_pix = tma_wanted() ? tma_row_pix(Wo, Wp, Bp, stride) : 0;
     if (!row_pix || (long long)Ho * row_pix * Bp >= (1ll << 31)) return plain;
     const int sms = sm_count() > 0 ? sm_count() : 148;
     auto rounds = [&](int pix) { return (((long long)Ho * pix * Bp + 255) / 256 * row_blocks + sms - 1) / sms; };
     return 4 * rounds(row_pix) > 5 * rounds(Wo) ? plain : ConvTokens{row_pix, shflbw::kGatherTma};
 }
+
+// Whether the rows of the blocks lie in the TMEM lanes (SpMM, and SpConv that writes planes).
+bool rows_in_lanes(int V, bool deep) {
+    const char* e = getenv("SHFLBW_SWAP");                    // forces the choice (tuning aid)
+    return (V == 64 || V == 128) && (e ? atoi(e) != 0 : deep);
+}
+bool is_deep(long long padded_cols, int row_blocks) { return padded_cols >= 192ll * row_blocks; }
 
 // Opt a kernel in to its dynamic shared memory once per (device, kernel): the host-buffer
 // calls initialise an op per chunk, and the attribute call is not free.
@@ -296,20 +315,16 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
         if (V == 16) tile = 128;   // chained layers: the only shape built for 16-row blocks
     }
     // SpMM and chained SpConv with V = 64 / 128 can run with the operands swapped (rows in TMEM
-    // lanes, one MMA per 16 columns for the whole token tile); SHFLBW_SWAP=0|1 forces the choice
-    // (tuning aid).
+    // lanes, one MMA per 16 columns for the whole token tile).
     if (!tma_wanted()) gather = shflbw::kGatherCpAsync;
     bool swapped = false;
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
-        const char* e = getenv("SHFLBW_SWAP");
         // Worth it when the main loop dominates an item (>= 3 pipeline stages of non-zero columns
         // per block on average); with fewer columns the item is all epilogue, and the
         // rows-in-lanes epilogue of a 64-row block keeps only half of each warp's lanes busy.
-        const bool deep = padded_cols >= 192ll * row_blocks;
-        if ((V == 64 || V == 128) && (e ? atoi(e) != 0 : deep)) {
+        if (rows_in_lanes(V, is_deep(padded_cols, row_blocks)))
             swapped = MODE == shflbw::kPanelSpmm ? lookup<shflbw::kPanelSpmmRows>(V, tile, out, gather)
                                                  : lookup<shflbw::kPanelConvChainRows>(V, tile, out, gather);
-        }
     }
     // Tokens in lanes with at most one stage of non-zero columns per block on average (an item is
     // then all epilogue; with two stages the four producers of that kernel were measured slower
@@ -817,7 +832,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     const bool planes_possible = (f->brow == 64 || f->brow == 128) && f->F / 64 <= 65535 &&
                                  (long long)f->F * tokens < (1ll << 32) - 1;
     if (planes_possible) {
-        bool want = padded_cols >= 192ll * row_blocks;      // same rule as the chained layers: >= 3 stages per block
+        bool want = is_deep(padded_cols, row_blocks);       // same rule as the chained layers: >= 3 stages per block
         if (const char* e = getenv("SHFLBW_CONV_PLANES")) want = atoi(e) != 0;
         if (want) {
             rc = pick_panel<shflbw::kPanelConvChain>(f->brow, counted, row_blocks, want ? (1ll << 40) : 0, &ch, false, ct.gather);
@@ -1083,15 +1098,17 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     out->perm = f->d_perm; out->status_word = f->d_status;
     out->chain = 1; out->out_R = R_next; out->out_S = S_next; out->relu = relu != 0;
     PanelChoice ch;
-    const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, f->F / f->brow);
+    const int row_blocks = f->F / f->brow;
+    const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
+    const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, row_blocks, !rows_in_lanes(f->brow, is_deep(padded_cols, row_blocks)), f->brow);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
-    int rc = pick_panel<shflbw::kPanelConvChain>(f->brow, counted, f->F / f->brow, f->kptr.empty() ? 0 : f->kptr.back(), &ch, false, ct.gather);
+    int rc = pick_panel<shflbw::kPanelConvChain>(f->brow, counted, row_blocks, padded_cols, &ch, false, ct.gather);
     if (rc != SHFLBW_OK) return rc;
     out->kernel = SHFLBW_KERNEL_TCGEN05;
     out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
     out->gather = ch.gather; out->row_pix = ct.row_pix;
     out->tiles_n = (int)((counted + ch.tokens - 1) / ch.tokens);
-    out->num_items = out->tiles_n * (f->F / f->brow);
+    out->num_items = out->tiles_n * row_blocks;
     const int sms = sm_count();
     if (sms <= 0) return SHFLBW_ERR_CUDA;
     out->block_x = ch.threads;

@@ -3,7 +3,9 @@ import numpy as np
 import pytest
 import torch
 
+import oracle_api as oa
 import shflbw_sparse_nn_b200 as sb
+from conftest import assert_close_fp16
 from gpu_util import dev, host, operand_swap, run_spconv, run_spmm
 
 pytestmark = pytest.mark.gpu
@@ -76,3 +78,33 @@ def test_spconv_state_says_how_it_gathers(Bn, H, W, R, stride, V, gather, row_pi
         st = op._state
         assert (st.gather, st.row_pix) == (want_gather, want_pix)
         assert st.num_items == 2 * -(-(st.Ho * st.row_pix * st.Bp) // st.tokens_per_cta)
+
+
+@pytest.mark.parametrize("density,residual,gather", [(0.05, False, 0), (0.05, True, 0), (0.6, False, 0), (0.6, True, 0), (0.9, True, 1)])
+def test_chained_layers_of_128_rows_gather_by_what_is_faster_for_them(density, residual, gather):
+    """Up to two stages of columns a block: tokens in lanes, cp.async; from three on: rows in lanes, TMA.  Against the
+    oracle either way, max(1e-2 * |ref|, 1e-3) as for every fp16 result of fp32 sums, with a residual's fp16 sum on top."""
+    Bn, H, W, C, V, F = 8, 6, 9, 240, 128, 256
+    f = sb.BlockwiseSpFilter().init_random(F, 1, 1, C, V, 1, density, True, 23, values="uniform")
+    f.transform_and_sync_device()
+    x = sb.uniform_half(24, Bn * H * W * C).reshape(Bn, H, W, C)
+    s = torch.cuda.current_stream()
+    b0 = torch.zeros(sb.chain_buffer_elems(C, H, W, Bn), dtype=torch.float16, device="cuda")
+    b1 = torch.zeros(sb.chain_buffer_elems(F, H, W, Bn), dtype=torch.float16, device="cuda")
+    r = dev(sb.uniform_half(25, Bn * H * W * F).reshape(Bn, H, W, F))
+    br = torch.zeros_like(b1)
+    y = torch.empty((Bn, H, W, F), dtype=torch.float16, device="cuda")
+    sb.chain_import_nhwc(dev(x), Bn, H, W, C, 1, 1, b0, s)
+    sb.chain_import_nhwc(r, Bn, H, W, F, 1, 1, br, s)
+    op = sb.SpconvChainOp().initialize(f, Bn, H, W, 1, b0, b1)
+    if residual:
+        op.set_residual(br, None)
+    op(s)
+    sb.chain_export_nhwc(b1, Bn, H, W, F, 1, 1, f, y, s)
+    torch.cuda.synchronize()
+    f.device_status()
+    assert (op._state.variant, op._state.gather) == (gather, gather)
+    want = np.asarray(oa.spconv_ref_nhwc(Bn, H, W, C, F, 1, 1, 1, V, f.indptr, f.indices, f.values, f.row_permute_ids, x), np.float32)
+    if residual:
+        want = want.reshape(Bn, H, W, F) + host(r).astype(np.float32)
+    assert_close_fp16(host(y), want.reshape(Bn, H, W, F), what=f"density {density}")
