@@ -252,31 +252,54 @@ int tma_row_pix(int Wo, int Wp, int Bp, int stride) {
 // SHFLBW_GATHER=0 takes the cp.async gather everywhere (tuning aid).  Asked for when a state is made.
 bool tma_wanted() { const char* g = getenv("SHFLBW_GATHER"); return !g || atoi(g) == 1; }
 
-// The gather of a convolution, and the pixels that an output row counts as.  TMA, unless the padding of the rows
-// costs the SMs more than a quarter in rounds of items: a stage takes it about 650 clk and the cp.async gather 870
-// to 1000 (14x14x512 -> 2048, batch 16, V = 64, 3 -> 4 rounds: 28.0 us by cp.async, 28.6 by TMA; V = 32, 6 -> 7:
-// 35.9 and 33.5; 7x7x512 -> 512, batch 8: 12.6 and 10.9).
-// Chained layers of 128 rows with tokens in lanes gather by cp.async: their items are an epilogue of 32 KB behind one to
-// three stages, and beside the TMA gather's operands that epilogue does not fit the 96 registers that 17 warps leave
-// (batch 128, 28x28x256 -> 256, 13 columns a block: 17.2 us, 18.3 by TMA; batch 64, 14x14x512 -> 1024 with residual,
-// 102 columns: 15.3 and 17.2).
-struct ConvTokens { int row_pix; int gather; };
-ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int row_blocks, bool chained_positions = false, int V = 0) {
-    const ConvTokens plain{Wo, shflbw::kGatherCpAsync};
-    if (chained_positions && V == 128) return plain;
-    const int row_pix = tma_wanted() ? tma_row_pix(Wo, Wp, Bp, stride) : 0;
-    if (!row_pix || (long long)Ho * row_pix * Bp >= (1ll << 31)) return plain;
-    const int sms = sm_count() > 0 ? sm_count() : 148;
-    auto rounds = [&](int pix) { return (((long long)Ho * pix * Bp + 255) / 256 * row_blocks + sms - 1) / sms; };
-    return 4 * rounds(row_pix) > 5 * rounds(Wo) ? plain : ConvTokens{row_pix, shflbw::kGatherTma};
-}
-
 // Whether the rows of the blocks lie in the TMEM lanes (SpMM, and SpConv that writes planes).
 bool rows_in_lanes(int V, bool deep) {
     const char* e = getenv("SHFLBW_SWAP");                    // forces the choice (tuning aid)
     return (V == 64 || V == 128) && (e ? atoi(e) != 0 : deep);
 }
 bool is_deep(long long padded_cols, int row_blocks) { return padded_cols >= 192ll * row_blocks; }
+
+// Token tile: a persistent CTA works through ceil(items / SMs) items in turn; an item of 128 tokens takes about 2/3 of
+// the time of one of 256 (half the gathered bytes, the same number of pipeline stages).  256 halves the value-panel
+// traffic per token and is the default; 128 where the dense extent is too small to give every SM a few items.
+// SHFLBW_TILE=128|256 overrides (tuning aid).
+long long rounds_of_items(long long n_tokens, int tile, int row_blocks) {
+    const int sms = sm_count() > 0 ? sm_count() : 148;
+    return ((n_tokens + tile - 1) / tile * row_blocks + sms - 1) / sms;
+}
+int pick_tile(long long n_tokens, int row_blocks) {
+    if (const char* e = getenv("SHFLBW_TILE")) { const int t = atoi(e); if (t == 128 || t == 256) return t; }
+    return n_tokens <= 128 || rounds_of_items(n_tokens, 128, row_blocks) * 2 < rounds_of_items(n_tokens, 256, row_blocks) * 3 ? 128 : 256;
+}
+
+// The gather of a convolution, and the pixels that an output row counts as.  TMA, unless the padding of the rows
+// costs more time in rounds of items (those of the tile that each side takes) than the gather saves: a stage takes it
+// about 650 clk and the cp.async gather 870 to 1000.
+//   Rounds of one tile: up to a quarter more of them (14x14x512 -> 2048, batch 16, V = 64, 3 -> 4 rounds: 28.0 us by
+// cp.async, 28.6 by TMA; V = 32, 6 -> 7: 35.9 and 33.5; 13x13x256 -> 2048, batch 24, V = 64, 900 columns a block, 4 -> 5: 42.7 and 41.7); less than that for
+// taller blocks with tokens in lanes, whose items are more epilogue than gather (17x17x256, batch 24: chained -> 1024,
+// V = 64, 102 columns, 4 -> 5: 12.7 and 14.1; -> 2048 in NHWC, V = 128, 40 columns: 27.1 and 28.9).
+//   Padding that takes one or two rounds of 128-token items to as many of 256: only for blocks of less than a stage
+// (V = 32, 40 columns: 9.45 by cp.async, 8.95 by TMA; V = 64, 40: 4.07 and 3.99; 100: 4.2 and 5.2; 300: 5.5 and 6.3;
+// V = 128, 40: 10.2 and 10.9, 300: 12.9 and 15.7).
+//   Chained layers of 128 rows with tokens in lanes gather by cp.async: their items are an epilogue of 32 KB behind one to
+// three stages, and beside the TMA gather's operands that epilogue does not fit the 96 registers that 17 warps leave
+// (batch 128, 28x28x256 -> 256, 13 columns a block: 17.2 us, 18.3 by TMA; batch 64, 14x14x512 -> 1024 with residual,
+// 102 columns: 15.3 and 17.2).
+struct ConvTokens { int row_pix; int gather; };
+ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int V, int row_blocks, long long padded_cols, bool rows, bool chain) {
+    const ConvTokens plain{Wo, shflbw::kGatherCpAsync};
+    if (chain && !rows && V == 128) return plain;
+    const int row_pix = tma_wanted() ? tma_row_pix(Wo, Wp, Bp, stride) : 0;
+    const long long before = (long long)Ho * Wo * Bp, after = (long long)Ho * row_pix * Bp;
+    if (!row_pix || after >= (1ll << 31)) return plain;
+    const int tile0 = pick_tile(before, row_blocks), tile1 = pick_tile(after, row_blocks);
+    const long long cost0 = rounds_of_items(before, tile0, row_blocks) * (tile0 == 128 ? 2 : 3);
+    const long long cost1 = rounds_of_items(after, tile1, row_blocks) * (tile1 == 128 ? 2 : 3);
+    const bool short_items = tile1 > tile0 && V <= 64 && padded_cols <= 48ll * row_blocks;
+    const bool pays = short_items || (!rows && V >= 64 ? 5 * cost1 <= 6 * cost0 : 4 * cost1 <= 5 * cost0);
+    return pays ? ConvTokens{row_pix, shflbw::kGatherTma} : plain;
+}
 
 // Opt a kernel in to its dynamic shared memory once per (device, kernel): the host-buffer
 // calls initialise an op per chunk, and the attribute call is not free.
@@ -295,22 +318,10 @@ int allow_smem(const void* fn, size_t bytes) {
 }
 int allow_smem(PanelKernel fn, size_t bytes) { return allow_smem((const void*)fn, bytes); }
 
-// Tile selection.  A 256-token work item halves the value-panel traffic per token and is
-// the default; 128 is used when the dense extent is too small to give every SM a few items.
-// SHFLBW_TILE=128|256 overrides (tuning aid).
 template <int MODE>
 int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols, PanelChoice* out, bool addend = false,
                int gather = shflbw::kGatherTma) {
-    // Token tile: a persistent CTA works through ceil(items / SMs) items in turn; an item of
-    // the 128-token tile was measured at ~2/3 of the time of a 256-token item (half the
-    // gathered bytes, the same number of pipeline stages).
-    int tile = 256;
-    const int sms = sm_count() > 0 ? sm_count() : 148;
-    const long long items256 = ((n_tokens + 255) / 256) * row_blocks;
-    const long long items128 = ((n_tokens + 127) / 128) * row_blocks;
-    const long long waves256 = (items256 + sms - 1) / sms, waves128 = (items128 + sms - 1) / sms;
-    if (n_tokens <= 128 || waves128 * 2 < waves256 * 3) tile = 128;
-    if (const char* e = getenv("SHFLBW_TILE")) { int t = atoi(e); if (t == 128 || t == 256) tile = t; }
+    int tile = pick_tile(n_tokens, row_blocks);
     if constexpr (MODE != shflbw::kPanelSpmm && MODE != shflbw::kPanelConv) {
         if (V == 16) tile = 128;   // chained layers: the only shape built for 16-row blocks
     }
@@ -335,7 +346,8 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
     // stage are as fast with six (28x28x128 -> 512: 48.3, with eight 49.2).
     bool wide = false;
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
-        wide = !swapped && tile == 256 && V == 64 && padded_cols <= 64ll * row_blocks && items256 >= 4ll * sms;
+        wide = !swapped && tile == 256 && V == 64 && padded_cols <= 64ll * row_blocks &&
+               (n_tokens + 255) / 256 * row_blocks >= 4ll * (sm_count() > 0 ? sm_count() : 148);
         if (const char* e = getenv("SHFLBW_EPILOGUE_WARPS")) wide = !swapped && tile == 256 && V == 64 && atoi(e) == 16;
     }
     const int wide_ring = !wide ? 0 : !addend && padded_cols > 32ll * row_blocks ? 8 : 6;
@@ -821,31 +833,25 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     const int row_blocks = f->F / f->brow;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
 
-    // the input as the panel kernel sees it: a strided 1x1 filter's pixels are staged side by side
-    const bool compact = f->R == 1 && f->S == 1;
-    const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, row_blocks);
-    const long long counted = (long long)Ho * ct.row_pix * Bp;
-
     // planes out?
-    PanelChoice ch;
-    bool planes = false;
     const bool planes_possible = (f->brow == 64 || f->brow == 128) && f->F / 64 <= 65535 &&
                                  (long long)f->F * tokens < (1ll << 32) - 1;
-    if (planes_possible) {
-        bool want = is_deep(padded_cols, row_blocks);       // same rule as the chained layers: >= 3 stages per block
-        if (const char* e = getenv("SHFLBW_CONV_PLANES")) want = atoi(e) != 0;
-        if (want) {
-            rc = pick_panel<shflbw::kPanelConvChain>(f->brow, counted, row_blocks, want ? (1ll << 40) : 0, &ch, false, ct.gather);
-            if (rc != SHFLBW_OK) return rc;
-            planes = ch.variant == 1;
-        }
-    }
+    bool planes = is_deep(padded_cols, row_blocks);         // same rule as the chained layers: >= 3 stages per block
+    if (const char* e = getenv("SHFLBW_CONV_PLANES")) planes = atoi(e) != 0;
+    planes = planes && planes_possible && rows_in_lanes(f->brow, true);
+
+    // the input as the panel kernel sees it: a strided 1x1 filter's pixels are staged side by side
+    const bool compact = f->R == 1 && f->S == 1;
+    const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, f->brow, row_blocks, padded_cols, planes, false);
+    const long long counted = (long long)Ho * ct.row_pix * Bp;
+    PanelChoice ch;
+    rc = planes ? pick_panel<shflbw::kPanelConvChain>(f->brow, counted, row_blocks, 1ll << 40, &ch, false, ct.gather)
+                : pick_panel<shflbw::kPanelConv>(f->brow, counted, row_blocks, 0, &ch, false, ct.gather);
+    if (rc != SHFLBW_OK) return rc;
     if (planes) {
         out->variant = 1;
         out->staged_out_bytes = (size_t)f->F * (size_t)tokens * 2;
     } else {
-        rc = pick_panel<shflbw::kPanelConv>(f->brow, counted, row_blocks, 0, &ch, false, ct.gather);
-        if (rc != SHFLBW_OK) return rc;
         out->variant = 0;
         if (f->row_permute) {
             out->staged_out_bytes = (size_t)B * Ho * Wo * f->F * 2;
@@ -1100,7 +1106,8 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     PanelChoice ch;
     const int row_blocks = f->F / f->brow;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
-    const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, row_blocks, !rows_in_lanes(f->brow, is_deep(padded_cols, row_blocks)), f->brow);
+    const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, f->brow, row_blocks, padded_cols,
+                                      rows_in_lanes(f->brow, is_deep(padded_cols, row_blocks)), true);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
     int rc = pick_panel<shflbw::kPanelConvChain>(f->brow, counted, row_blocks, padded_cols, &ch, false, ct.gather);
     if (rc != SHFLBW_OK) return rc;

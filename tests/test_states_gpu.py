@@ -108,3 +108,25 @@ def test_chained_layers_of_128_rows_gather_by_what_is_faster_for_them(density, r
     if residual:
         want = want.reshape(Bn, H, W, F) + host(r).astype(np.float32)
     assert_close_fp16(host(y), want.reshape(Bn, H, W, F), what=f"density {density}")
+
+
+@pytest.mark.parametrize("H,Bn,V,F,density,gather,tile", [
+    (17, 24, 64, 128, 0.9, 0, 128),     # 55 tiles of 128 tokens, two blocks; rows of 24 pixels would make two rounds of 128
+    (17, 24, 64, 128, 0.2, 1, 256),     # less than a stage of columns a block: one round of 256 all the same
+    (17, 24, 128, 256, 0.2, 0, 128),    # ... not at 128 rows
+    (17, 24, 32, 64, 0.9, 0, 128),
+    (17, 24, 64, 1024, 0.6, 0, 256),    # four rounds of items; five with the rows padded
+    (17, 24, 32, 512, 0.6, 1, 256),
+])
+def test_padded_rows_are_weighed_in_the_tiles_that_each_side_takes(H, Bn, V, F, density, gather, tile):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the item counts are of 148 SMs")
+    C = 16
+    f = sb.BlockwiseSpFilter().init_random(F, 3, 3, C, V, 1, density, True, 27, values="uniform")
+    x = sb.uniform_half(28, Bn * H * H * C).reshape(Bn, H, H, C)
+    y, op = run_spconv(f, Bn, H, H, 1, x)
+    st = op._state
+    assert (st.gather, st.tokens_per_cta, st.row_pix) == (gather, tile, 24 if gather else 17)
+    n = 2 * H * H                                                # two images suffice for the oracle
+    want = oa.spconv_ref_nhwc(2, H, H, C, F, 3, 3, 1, V, f.indptr, f.indices, f.values, f.row_permute_ids, x[:2])
+    assert_close_fp16(y[:2].reshape(n, F), np.asarray(want).reshape(n, F), what=f"V={V} F={F}")
