@@ -249,8 +249,21 @@ int tma_row_pix(int Wo, int Wp, int Bp, int stride) {
     return stride > 1 && pixels > 1 ? 0 : (Wo + pixels - 1) / pixels * pixels;
 }
 
-// SHFLBW_GATHER=0 takes the cp.async gather everywhere (tuning aid).  Asked for when a state is made.
+// SHFLBW_GATHER=0 takes the cp.async gather everywhere, 1 has an SpMM gather by TMA where it would not by itself
+// (tuning aids).  Asked for when a state is made.
 bool tma_wanted() { const char* g = getenv("SHFLBW_GATHER"); return !g || atoi(g) == 1; }
+
+// The gather of an SpMM: TMA, unless the operand is a few KB of rows that share 32-byte sectors (an odd multiple of 8
+// tokens) and every row is wanted by many blocks.  The SMs then fetch the same few lines of L2 over and over, and the
+// copy engine's requests to one line queue up, the more so where a block takes neighbouring rows.  By TMA and by cp.async,
+// 8 tokens, density 0.5: K = 256, 700 blocks of 16 rows 15.3 and 8.6 us; K = 768, 148 of 16 9.9 and 5.8; K = 1024, 344 of
+// 64 19.1 and 12.5; K = 1536, 344 of 32 22.4 and 16.7 (at density 0.25, 16 rows, 9.2 and 10.4); K = 2048, 172 of 16 13.6
+// and 14.7; density 0.1, K = 512, 148 of 16 3.9 and 4.0.  24 tokens, K = 256, 700 blocks of 32: 18.4 and 9.8.  16 tokens,
+// whose rows are whole sectors, density 0.4, K = 256, 192 blocks of 16: 4.5 and 4.4; K = 1024: 5.5 and 7.4.
+int spmm_gather(long long K, int N, int row_blocks, long long padded_cols, int tile) {
+    const bool crowded = N % 16 == 8 && padded_cols >= 40 * K && (K * N <= 8192 || (K * N <= 12288 && 3 * padded_cols > K * row_blocks));
+    return crowded && tile == 128 && !getenv("SHFLBW_GATHER") ? shflbw::kGatherCpAsync : shflbw::kGatherTma;
+}
 
 // Whether the rows of the blocks lie in the TMEM lanes (SpMM, and SpConv that writes planes).
 bool rows_in_lanes(int V, bool deep) {
@@ -276,9 +289,10 @@ int pick_tile(long long n_tokens, int row_blocks) {
 // costs more time in rounds of items (those of the tile that each side takes) than the gather saves: a stage takes it
 // about 650 clk and the cp.async gather 870 to 1000.
 //   Rounds of one tile: up to a quarter more of them (14x14x512 -> 2048, batch 16, V = 64, 3 -> 4 rounds: 28.0 us by
-// cp.async, 28.6 by TMA; V = 32, 6 -> 7: 35.9 and 33.5; 13x13x256 -> 2048, batch 24, V = 64, 900 columns a block, 4 -> 5: 42.7 and 41.7); less than that for
-// taller blocks with tokens in lanes, whose items are more epilogue than gather (17x17x256, batch 24: chained -> 1024,
-// V = 64, 102 columns, 4 -> 5: 12.7 and 14.1; -> 2048 in NHWC, V = 128, 40 columns: 27.1 and 28.9).
+// cp.async, 28.6 by TMA; V = 32, 6 -> 7: 35.9 and 33.5; 13x13x256 -> 2048, batch 24, V = 64, 900 columns a block, 4 -> 5:
+// 42.7 and 41.7); less than that for taller blocks with tokens in lanes, whose items are more epilogue than gather
+// (17x17x256, batch 24: chained -> 1024, V = 64, 102 columns, 4 -> 5: 12.7 and 14.1; -> 2048 in NHWC, V = 128, 40 columns:
+// 27.1 and 28.9).
 //   Padding that takes one or two rounds of 128-token items to as many of 256: only for blocks of less than a stage
 // (V = 32, 40 columns: 9.45 by cp.async, 8.95 by TMA; V = 64, 40: 4.07 and 3.99; 100: 4.2 and 5.2; 300: 5.5 and 6.3;
 // V = 128, 40: 10.2 and 10.9, 300: 12.9 and 15.7).
@@ -520,7 +534,9 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
         out->tokens_per_cta = 128; out->stages = 0; out->shared_mem_size = 0;
     } else {
         PanelChoice ch;
-        int rc = pick_panel<shflbw::kPanelSpmm>(m->brow, N, out->num_row_blocks, m->kptr.empty() ? 0 : m->kptr.back(), &ch, beta != 0.f);
+        const long long padded_cols = m->kptr.empty() ? 0 : m->kptr.back();
+        int rc = pick_panel<shflbw::kPanelSpmm>(m->brow, N, out->num_row_blocks, padded_cols, &ch, beta != 0.f,
+                                                spmm_gather(m->ncol, N, out->num_row_blocks, padded_cols, pick_tile(N, out->num_row_blocks)));
         if (rc != SHFLBW_OK) return rc;
         out->kernel = SHFLBW_KERNEL_TCGEN05;
         out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;

@@ -5,6 +5,7 @@ import torch
 
 import oracle_api as oa
 import shflbw_sparse_nn_b200 as sb
+from shflbw_sparse_nn_b200 import blockwise as bw
 from conftest import assert_close_fp16
 from gpu_util import dev, host, operand_swap, run_spconv, run_spmm
 
@@ -130,3 +131,36 @@ def test_padded_rows_are_weighed_in_the_tiles_that_each_side_takes(H, Bn, V, F, 
     n = 2 * H * H                                                # two images suffice for the oracle
     want = oa.spconv_ref_nhwc(2, H, H, C, F, 3, 3, 1, V, f.indptr, f.indices, f.values, f.row_permute_ids, x[:2])
     assert_close_fp16(y[:2].reshape(n, F), np.asarray(want).reshape(n, F), what=f"V={V} F={F}")
+
+
+@pytest.mark.parametrize("V,K,N,dense,gather", [
+    (16, 256, 8, False, 0), (32, 1024, 8, False, 0), (64, 1024, 8, False, 0), (128, 256, 8, False, 0), (16, 256, 24, False, 0),
+    (32, 1032, 8, False, 1), (32, 1032, 8, True, 0), (16, 1544, 8, True, 1), (16, 512, 16, True, 1),
+])
+@pytest.mark.parametrize("beta", [0.0, -1.5])
+def test_spmm_on_few_shared_lines_gathers_by_cp_async(V, K, N, dense, gather, beta, monkeypatch):
+    """Rows that share sectors, wanted by many blocks: the same bits as by TMA, and the oracle's values; a linear layer's too."""
+    counts = ([K // 2, K, K // 2 + 1, K // 4, 17, 0] if dense else [0, 1, K // 4, K // 2, K - 1, 17]) * 28
+    M = V * len(counts)
+    rng = np.random.default_rng(K + V)
+    indptr = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    indices = np.concatenate([np.sort(rng.choice(K, c, replace=False)) for c in counts]).astype(np.int32)
+    m = sb.BlockwiseSpMatrix.from_arrays(M, K, V, indptr, indices, sb.uniform_half(3, indices.size * V),
+                                         rng.permutation(M).astype(np.int32))
+    B = sb.uniform_half(30, K * N).reshape(K, N)
+    Cm = sb.uniform_half(31, M * N).reshape(M, N) if beta else None
+    monkeypatch.delenv("SHFLBW_GATHER", raising=False)
+    D, op = run_spmm(m, N, B, alpha=0.5, Cm=Cm, beta=beta)
+    bias, bd = dev(sb.uniform_half(32, M)), dev(B)
+    out, forced = (torch.empty((M, N), dtype=torch.float16, device="cuda") for _ in range(2))
+    bw.linear_exec(m, N, None, bias, bd, N, out, torch.cuda.current_stream())
+    monkeypatch.setenv("SHFLBW_GATHER", "1")
+    E, op_tma = run_spmm(m, N, B, alpha=0.5, Cm=Cm, beta=beta)
+    bw.linear_exec(m, N, None, bias, bd, N, forced, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    assert (op._state.gather, op_tma._state.gather) == (gather, 1)
+    assert np.array_equal(D.view(np.uint16), E.view(np.uint16))
+    assert torch.equal(out.view(torch.int16), forced.view(torch.int16))
+    if K <= 256:                                                 # (a quick oracle)
+        want = oa.spmm_ref(M, N, V, indptr, indices, m.values, m.row_permute_ids, B, 0.5, Cm, beta)
+        assert_close_fp16(D, np.asarray(want).reshape(M, N), what=f"V={V} K={K} N={N}")
