@@ -158,8 +158,10 @@ int encode_map(const void* base, long long rows, long long cols, long long pitch
 template <int V, int TM, int STAGES, int MODE, bool BIAS>
 PanelChoice regular(int gather) {
     constexpr int PW = MODE == shflbw::kPanelSpmmRows ? 16 : 8;
-    if (gather == shflbw::kGatherTma) return choice<V, TM, 64, STAGES, PW, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
-    return choice<V, TM, 64, STAGES, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>();
+    constexpr bool SPMM = MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelSpmmRows;
+    if constexpr (!(SPMM && BIAS && TM == 2))                // (spmm_gather)
+        if (gather == shflbw::kGatherCpAsync) return choice<V, TM, 64, STAGES, 8, MODE, 2, shflbw::kGatherCpAsync, 8, BIAS>();
+    return choice<V, TM, 64, STAGES, PW, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
 }
 template <int MODE, bool BIAS = false>
 bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsync, int wide_ring = 0) {
@@ -180,9 +182,12 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
                                       : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherTma, 16, BIAS, true>();
                 return true;
             }
-            *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, false>()
-                                  : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, true>();
-            return true;
+            if constexpr (MODE == shflbw::kPanelConvChain) {
+                *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, false>()
+                                      : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherCpAsync, 16, BIAS, true>();
+                return true;
+            }
+            return false;
         }
     }
     if constexpr (MODE == shflbw::kPanelSpmmRows || MODE == shflbw::kPanelConvChainRows) {   // rows in TMEM lanes: V must be a legal UMMA M
@@ -260,9 +265,13 @@ bool tma_wanted() { const char* g = getenv("SHFLBW_GATHER"); return !g || atoi(g
 // 64 19.1 and 12.5; K = 1536, 344 of 32 22.4 and 16.7 (at density 0.25, 16 rows, 9.2 and 10.4); K = 2048, 172 of 16 13.6
 // and 14.7; density 0.1, K = 512, 148 of 16 3.9 and 4.0.  24 tokens, K = 256, 700 blocks of 32: 18.4 and 9.8.  16 tokens,
 // whose rows are whole sectors, density 0.4, K = 256, 192 blocks of 16: 4.5 and 4.4; K = 1024: 5.5 and 7.4.
-int spmm_gather(long long K, int N, int row_blocks, long long padded_cols, int tile) {
+// With a bias 256-token tiles are built for the TMA gather only, without one the other is there to compare with
+// (SHFLBW_GATHER=0).
+int spmm_gather(long long K, int N, int row_blocks, long long padded_cols, int tile, bool with_bias) {
+    if (tile == 256 && with_bias) return shflbw::kGatherTma;
+    if (getenv("SHFLBW_GATHER")) return tma_wanted() ? shflbw::kGatherTma : shflbw::kGatherCpAsync;
     const bool crowded = N % 16 == 8 && padded_cols >= 40 * K && (K * N <= 8192 || (K * N <= 12288 && 3 * padded_cols > K * row_blocks));
-    return crowded && tile == 128 && !getenv("SHFLBW_GATHER") ? shflbw::kGatherCpAsync : shflbw::kGatherTma;
+    return crowded && tile == 128 ? shflbw::kGatherCpAsync : shflbw::kGatherTma;
 }
 
 // Whether the rows of the blocks lie in the TMEM lanes (SpMM, and SpConv that writes planes).
@@ -341,7 +350,6 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
     }
     // SpMM and chained SpConv with V = 64 / 128 can run with the operands swapped (rows in TMEM
     // lanes, one MMA per 16 columns for the whole token tile).
-    if (!tma_wanted()) gather = shflbw::kGatherCpAsync;
     bool swapped = false;
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         // Worth it when the main loop dominates an item (>= 3 pipeline stages of non-zero columns
@@ -365,6 +373,7 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
         if (const char* e = getenv("SHFLBW_EPILOGUE_WARPS")) wide = !swapped && tile == 256 && V == 64 && atoi(e) == 16;
     }
     const int wide_ring = !wide ? 0 : !addend && padded_cols > 32ll * row_blocks ? 8 : 6;
+    if (wide && MODE == shflbw::kPanelSpmm) gather = shflbw::kGatherTma;   // (built for it only)
     if (!swapped && !lookup<MODE>(V, tile, out, gather, wide_ring)) return SHFLBW_ERR_UNSUPPORTED;
     out->variant = swapped ? 1 : wide ? 2 : 0;
     if (wide_ring == 8) {                    // a residual may be bound to the state later on
@@ -501,8 +510,8 @@ int shflbw_matrix_device_status(const shflbw_matrix_t* m) {
 
 // ------------------------------------------------------------------------------ SpMM --
 
-int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha, const void* C,
-                     float beta, void* D, int kernel, shflbw_spmm_state_t* out) {
+static int plan_spmm(const shflbw_matrix_t* m, int N, const void* B, float alpha, const void* C,
+                     float beta, void* D, int kernel, bool with_bias, shflbw_spmm_state_t* out) {
     if (!out) return SHFLBW_ERR_INVALID_ARG;
     std::memset(out, 0, sizeof *out);
     if (!m || !B || !D || N <= 0) return SHFLBW_ERR_INVALID_ARG;
@@ -536,7 +545,7 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
         PanelChoice ch;
         const long long padded_cols = m->kptr.empty() ? 0 : m->kptr.back();
         int rc = pick_panel<shflbw::kPanelSpmm>(m->brow, N, out->num_row_blocks, padded_cols, &ch, beta != 0.f,
-                                                spmm_gather(m->ncol, N, out->num_row_blocks, padded_cols, pick_tile(N, out->num_row_blocks)));
+                                                spmm_gather(m->ncol, N, out->num_row_blocks, padded_cols, pick_tile(N, out->num_row_blocks), with_bias));
         if (rc != SHFLBW_OK) return rc;
         out->kernel = SHFLBW_KERNEL_TCGEN05;
         out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
@@ -555,6 +564,11 @@ int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha
     }
     out->init_success = 1;
     return SHFLBW_OK;
+}
+
+int shflbw_spmm_init(const shflbw_matrix_t* m, int N, const void* B, float alpha, const void* C,
+                     float beta, void* D, int kernel, shflbw_spmm_state_t* out) {
+    return plan_spmm(m, N, B, alpha, C, beta, D, kernel, false, out);
 }
 
 // The panel kernel of an initialised SpMM state, allowed its shared memory.  The state is a POD and may have
@@ -621,7 +635,7 @@ int shflbw_linear_exec(const shflbw_matrix_t* m, int tokens, const void* x, cons
     if (!m || !xt || !out || N <= 0 || tokens > N || (x && tokens <= 0)) return SHFLBW_ERR_INVALID_ARG;
     if (((uintptr_t)x | (uintptr_t)bias) & 1) return SHFLBW_ERR_UNSUPPORTED;
     shflbw_spmm_state_t st;
-    int rc = shflbw_spmm_init(m, N, xt, 1.f, nullptr, 0.f, out, SHFLBW_KERNEL_AUTO, &st);   // (asks for 16-byte aligned xt, out and N % 8)
+    int rc = plan_spmm(m, N, xt, 1.f, nullptr, 0.f, out, SHFLBW_KERNEL_AUTO, bias != nullptr, &st);   // (asks for 16-byte aligned xt, out and N % 8)
     if (rc != SHFLBW_OK) return rc;
     PanelChoice ch;                                          // all set-up comes before the first launch
     if ((rc = spmm_panel(&st, bias != nullptr, &ch)) != SHFLBW_OK) return rc;

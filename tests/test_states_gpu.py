@@ -7,7 +7,7 @@ import oracle_api as oa
 import shflbw_sparse_nn_b200 as sb
 from shflbw_sparse_nn_b200 import blockwise as bw
 from conftest import assert_close_fp16
-from gpu_util import dev, host, operand_swap, run_spconv, run_spmm
+from gpu_util import dev, epilogue_warps, host, operand_swap, run_spconv, run_spmm, tile
 
 pytestmark = pytest.mark.gpu
 
@@ -164,3 +164,28 @@ def test_spmm_on_few_shared_lines_gathers_by_cp_async(V, K, N, dense, gather, be
     if K <= 256:                                                 # (a quick oracle)
         want = oa.spmm_ref(M, N, V, indptr, indices, m.values, m.row_permute_ids, B, 0.5, Cm, beta)
         assert_close_fp16(D, np.asarray(want).reshape(M, N), what=f"V={V} K={K} N={N}")
+
+
+@pytest.mark.parametrize("V,swap,ew,tokens", [(16, 0, 8, 256), (32, 0, 8, 128), (64, 0, 8, 256), (64, 1, 8, 256), (64, 0, 16, 256), (128, 1, 8, 256)])
+def test_linear_layers_where_cp_async_is_asked_for(V, swap, ew, tokens, monkeypatch):
+    """With a bias, and with sixteen epilogue warps, the SpMM kernels of 256-token tiles gather by TMA only: asking for
+    the other gather changes neither the bits nor what is accepted."""
+    K, N, M = 192, 200, 4 * V
+    m = sb.BlockwiseSpMatrix().init_random(M, K, V, 1, 0.3, True, 33 + V, values="uniform")
+    m.transform_and_sync_device()
+    B, bias = sb.uniform_half(34, K * N).reshape(K, N), sb.uniform_half(35, M)
+    bd, biasd, got = dev(B), dev(bias), []
+    for env in ("1", "0"):
+        monkeypatch.setenv("SHFLBW_GATHER", env)
+        out, plain = (torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda") for _ in range(2))
+        with operand_swap(swap), epilogue_warps(ew), tile(tokens):
+            bw.linear_exec(m, N, None, biasd, bd, N, out, torch.cuda.current_stream())
+            op = sb.SpmmBlockwiseOp().initialize(m, N, bd, plain)
+        _call(op, m)
+        assert op._state.gather == (1 if env == "1" or ew == 16 else 0)
+        got.append((host(out), host(plain)))
+    for a, b in zip(*got):
+        assert np.array_equal(a.view(np.uint16), b.view(np.uint16))
+    perm = m.row_permute_ids
+    want = np.asarray(oa.spmm_ref(M, N, V, m.indptr, m.indices, m.values, perm, B)).reshape(M, N) + bias.astype(np.float32)[:, None]
+    assert_close_fp16(got[1][0], want, what=f"V={V}")
