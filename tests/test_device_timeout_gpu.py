@@ -27,9 +27,11 @@ from shflbw_sparse_nn_b200.build import build_fault_inject_library
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("gather", [1, 0])
 @pytest.mark.parametrize("swap", ["1", "0"])
-def test_wait_limit_runs_out_and_the_library_recovers(swap, monkeypatch):
+def test_wait_limit_runs_out_and_the_library_recovers(swap, gather, monkeypatch):
     monkeypatch.setenv("SHFLBW_SWAP", swap)      # both kernel orientations share the failure path
+    monkeypatch.setenv("SHFLBW_GATHER", str(gather))         # each gather's producers have their own
     flib = _cabi.load_library(build_fault_inject_library())
     flib.shflbw_debug_withhold_arrivals_from.restype = C.c_int
     flib.shflbw_debug_withhold_arrivals_from.argtypes = [C.c_int]
@@ -43,7 +45,7 @@ def test_wait_limit_runs_out_and_the_library_recovers(swap, monkeypatch):
         st = _cabi.SpmmState()
         assert flib.shflbw_spmm_init(h, N, Bd.data_ptr(), 1.0, None, 0.0, Dd.data_ptr(), _cabi.KERNEL_AUTO,
                                      C.byref(st)) == _cabi.OK
-        assert st.variant == int(swap)
+        assert (st.variant, st.gather) == (int(swap), gather)
         stream = torch.cuda.current_stream().cuda_stream
 
         def launch():
