@@ -91,9 +91,10 @@ struct alignas(64) PanelParams {
     const __half* blk_val;   // value panels of the padded rows, element order kval_index() (shflbw_internal.hpp)
     const int* perm;         // [M] or nullptr
     int* status_word;
-    unsigned idx_limit;      // largest legal gather offset: K - 1 (SpMM, a row id) or the element offset of the last
-                             // (channel, tap) plane origin (SpConv); ids are clamped to it, so a corrupted id can
-                             // give wrong numbers but never an address outside the dense operand
+    unsigned idx_limit;      // cp.async gather: largest legal offset, K - 1 (SpMM, a row id) or the element offset of the
+                             // last (channel, tap) plane origin (SpConv).  Ids are clamped to it, so a corrupted id can
+                             // give wrong numbers but never an address outside the dense operand; the TMA gather reads
+                             // zeros for a row that its map does not have
     long long wait_limit;    // SM clocks after which a barrier wait gives up (kWaitLimitCycles unless the host overrides it)
     float alpha, beta;
     int num_items, tiles_n;  // work items = row blocks x token tiles; item -> (item / tiles_n, item % tiles_n)
@@ -134,8 +135,7 @@ struct alignas(64) PanelParams {
 // channel-major halo layout the next layer gathers from ("chained" layers).
 // 3 = SpMM with the operands swapped: the block's V rows are the UMMA M dimension (64 or 128
 // TMEM lanes) and the T tokens the N dimension, so ONE instruction per 16 columns covers the
-// whole token tile (the instruction rate, 73 clk minimum each, is what limits this kernel) and
-// the accumulator comes out with an output row per lane.
+// whole token tile and the accumulator comes out with an output row per lane.
 // 4 = chained SpConv with the operands swapped in the same way.
 constexpr int kPanelSpmm = 0, kPanelConv = 1, kPanelConvChain = 2, kPanelSpmmRows = 3, kPanelConvChainRows = 4;
 
@@ -282,7 +282,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         for (int s = 0; s < STAGES; ++s) {
             // cp.async gather: one arrival per producer WARP of the group (per-thread deferred arrivals,
             // cp.async.mbarrier.arrive.noinc, were measured at ~3 clk of load/store-unit time per thread,
-            // i.e. more than the copies themselves).  TMA gather: one arrival, with the stage's byte count.
+            // i.e. more than the copies themselves).  TMA gather: one arrival per warp of the group too, with the
+            // bytes that it fetches, whether it has a row in the stage or not (see the producers).
             sm100::mbar_init(&full_bar[s], PW / Cfg::GROUPS);
             sm100::mbar_init(&empty_bar[s], 1);   // one tcgen05.commit per drain
         }
@@ -312,11 +313,11 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     // the sparse operand, which no kernel writes) may overlap the tail of the previous kernel in
     // the stream; the dense operand, the residual and the output are touched only below.  The
     // next kernel may start its own prologue as soon as every block of this one got here.
-    // (A convolution call that ends with this kernel lets the next one in when its producers are done: early enough
-    // for the set-up of an SpMM or a chained layer behind it, 1.2 us, and late enough that few blocks of another
-    // convolution's relayout, which has no set-up, wait on this kernel's SMs; with those spread evenly (relayout_smem)
-    // calls back to back are 1-3 % slower than without any trigger.  24x16x16x160 -> 1856, 3x3, V = 32: 26.4 us and 30.0
-    // with a chained layer; without a trigger 26.1 and 31.4; at once, and the relayout not spread, 29.3 and 30.2.)
+    // (A convolution call that ends with this kernel lets the next one in when its producers have issued, or by
+    // cp.async completed, their last copies: early enough for the set-up of an SpMM or a chained layer behind it, about
+    // 1 us, and late enough that few blocks of another convolution's relayout, which has no set-up, wait on this kernel's
+    // SMs; with those spread evenly (relayout_smem) calls back to back are 1-3 % slower than without any trigger.
+    // 24x16x16x160 -> 1856, 3x3, V = 32: 23.9 us and 28.6 with a chained layer; without a trigger 23.7 and 29.8.)
     if (MODE != kPanelConv || p.perm != nullptr) sm100::grid_dependency_launch();
     // The wait itself is executed per role, as late as each role allows: by the producers after
     // their first row ids (sparse operand) are on their way and before their first gather, by the
@@ -1171,10 +1172,10 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     }
 
     if (*cta_abort) {
-        // A wait gave up somewhere in this block.  Every role has stopped issuing work; what is
-        // still in flight -- bulk copies of value slices (a few KB each) and gathers whose
-        // groups were awaited above -- gets a bounded ~100 us to land before the shared memory
-        // is released.
+        // A wait gave up somewhere in this block.  Every role has stopped issuing work, and cp.async copies were
+        // awaited above; what is still in flight -- bulk copies of value slices and tile gathers, at most a ring
+        // of stages, whose barriers nobody waits for any more -- gets a bounded ~100 us after each thread's last
+        // instruction to land before the shared memory is released.
         const long long t0 = clock64();
         while (clock64() - t0 < 200000LL) __nanosleep(1000);
     }

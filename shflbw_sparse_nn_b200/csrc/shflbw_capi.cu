@@ -282,8 +282,9 @@ bool rows_in_lanes(int V, bool deep) {
 bool is_deep(long long padded_cols, int row_blocks) { return padded_cols >= 192ll * row_blocks; }
 
 // Token tile: a persistent CTA works through ceil(items / SMs) items in turn; an item of 128 tokens takes about 2/3 of
-// the time of one of 256 (half the gathered bytes, the same number of pipeline stages).  256 halves the value-panel
-// traffic per token and is the default; 128 where the dense extent is too small to give every SM a few items.
+// the time of one of 256 (half the gathered bytes, the same number of pipeline stages; eight rounds of SpMM items, K =
+// 2048, density 0.2, by TMA: V = 16 0.66, 32 0.66, 64 0.63, 128 0.65; by cp.async 0.68 to 0.78).  256 halves the
+// value-panel traffic per token and is the default; 128 where the dense extent is too small to give every SM a few items.
 // SHFLBW_TILE=128|256 overrides (tuning aid).
 long long rounds_of_items(long long n_tokens, int tile, int row_blocks) {
     const int sms = sm_count() > 0 ? sm_count() : 148;
@@ -352,20 +353,24 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
     // lanes, one MMA per 16 columns for the whole token tile).
     bool swapped = false;
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
-        // Worth it when the main loop dominates an item (>= 3 pipeline stages of non-zero columns
-        // per block on average); with fewer columns the item is all epilogue, and the
-        // rows-in-lanes epilogue of a 64-row block keeps only half of each warp's lanes busy.
+        // From three stages of non-zero columns per block on (is_deep): with fewer an item is mostly epilogue, and
+        // lanes that hold a row each store, and read a residual, in pieces of 64 bytes.  The line was drawn when an MMA
+        // took 54 clk of issue whatever its shape, which rows in lanes halve.  With elected issue, tokens and rows in
+        // lanes, V = 64: SpMM 4096x1024x4096, 48 columns a block 12.5 and 11.9 us, 64 15.8 and 12.7, 176 17.9 and 15.7,
+        // 256 19.6 and 19.0 (1000 columns of B: within 5 %); chained 28x28x256 -> 256, batch 64, L2 warm, 48 columns 10.9
+        // and 15.4, 192 17.7 and 22.0, 400 22.7 and 26.2, 768 34.8 and 37.3, with a residual 38.0 and 43.9 (V = 128, 768
+        // columns: 29.5 and 27.6).  So SpMM would gain from 64 columns on, and chained layers lose up to about 800.
         if (rows_in_lanes(V, is_deep(padded_cols, row_blocks)))
             swapped = MODE == shflbw::kPanelSpmm ? lookup<shflbw::kPanelSpmmRows>(V, tile, out, gather)
                                                  : lookup<shflbw::kPanelConvChainRows>(V, tile, out, gather);
     }
-    // Tokens in lanes with at most one stage of non-zero columns per block on average (an item is
-    // then all epilogue; with two stages the four producers of that kernel were measured slower
-    // than the eight of the regular one) and several items per SM: sixteen epilogue warps.  SHFLBW_EPILOGUE_WARPS=8|16 forces the choice
-    // (tuning aid).
+    // Tokens in lanes with at most 64 non-zero columns per block on average, where an item is all epilogue, and several
+    // items per SM: sixteen epilogue warps (chained 28x28x256 -> 256, batch 128, eight and sixteen: 26 columns 18.7 and
+    // 15.1 us, 64 19.2 and 17.9, 96 21.3 and 21.1, 128 21.9 and 23.0; SpMM of the same size gains up to 128: 26.9 and
+    // 25.0).  SHFLBW_EPILOGUE_WARPS=8|16 forces the choice (tuning aid).
     // Their ring: eight stages where nothing is added and a block takes two stages, which a ring of six holds for
-    // three items only (14x14x256 -> 1024, batch 256, no residual: 35.2 us with six, 34.3 with eight); blocks of one
-    // stage are as fast with six (28x28x128 -> 512: 48.3, with eight 49.2).
+    // three items only (28x28x128 -> 512, batch 256, no residual, 40 columns: 56.6 us with six, 54.7 with eight); blocks
+    // of one stage are as fast with six (26 columns: 48.5, with eight 49.7).
     bool wide = false;
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         wide = !swapped && tile == 256 && V == 64 && padded_cols <= 64ll * row_blocks &&
@@ -866,7 +871,10 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     // planes out?
     const bool planes_possible = (f->brow == 64 || f->brow == 128) && f->F / 64 <= 65535 &&
                                  (long long)f->F * tokens < (1ll << 32) - 1;
-    bool planes = is_deep(padded_cols, row_blocks);         // same rule as the chained layers: >= 3 stages per block
+    bool planes = is_deep(padded_cols, row_blocks);         // the chained layers' rule (14x14x256 -> 1024, 3x3, batch 16, V = 64,
+                                                            // 112 columns a block, positions and planes: 16.8 and 14.8 us,
+                                                            // 192 17.3 and 15.0; 28x28x256 -> 256, 1x1, batch 64: 37.5 and
+                                                            // 38.7, 39.6 and 40.2)
     if (const char* e = getenv("SHFLBW_CONV_PLANES")) planes = atoi(e) != 0;
     planes = planes && planes_possible && rows_in_lanes(f->brow, true);
 
@@ -973,8 +981,8 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
                                           st->R, st->S, s, step, planes || st->staged_out);
     // 2. implicit-GEMM panel kernel.
     // Where it ends the call: see the kernel.  A call that stages many blocks per SM is likely to be followed by another
-    // one, whose first blocks cannot be spread over the SMs (26x48x48x1024 -> 96 at stride 2, back to back: 73 us, 76
-    // with the trigger); it is long enough not to miss the 1.2 us.
+    // one, whose first blocks cannot be spread over the SMs (26x48x48x1024 -> 96 at stride 2, back to back: 75.6 us, 78.9
+    // with the trigger); it is long enough not to miss the 1 us.
     p.trigger_late = relayout_per_sm <= 7;
     p.blk_ptr = st->blk_ptr; p.blk_idx = st->blk_idx; p.blk_val = (const __half*)st->blk_val;
     p.perm = st->perm; p.status_word = st->status_word; p.alpha = st->alpha; p.beta = 0.f;

@@ -87,7 +87,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
 // One lane of a converged warp, always the same one.  Instructions whose operands the hardware takes
 // from uniform registers (tcgen05.mma / commit, bulk and tensor copies) belong in a branch on this: behind
 // `lane == 0` the compiler cannot see that one lane is left and serialises each of them over the lanes
-// that might be there (54 clk per tcgen05.mma instead of 15, 59 clk per gather4 instead of 9).
+// that might be there (54 clk per tcgen05.mma instead of 15, 59 clk per gather4 instead of 15).
 __device__ __forceinline__ bool elect_one() {
     uint32_t r;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
