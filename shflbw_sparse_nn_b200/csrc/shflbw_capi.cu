@@ -1182,8 +1182,8 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
         for (int i = 0; i < st->F; ++i)
             if (map_host[i] < 0 || map_host[i] >= st->F) return SHFLBW_ERR_BAD_FORMAT;
     // The sixteen-epilogue-warp kernel copies the residual an item ahead, which pays up to two stages of
-    // columns per block (7x7x512 -> 2048 with residual, batch 256: 38 -> 31 us); without a residual the
-    // limit is one stage (pick_panel).
+    // columns per block (14x14x256 -> 1024 with residual, batch 128, 112 columns: 33.9 -> 26.5 us); without a
+    // residual the limit is one stage (pick_panel).
     PanelChoice ch;
     const bool wide = (st->variant == 2 ||
                        (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
