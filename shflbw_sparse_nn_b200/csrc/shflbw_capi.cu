@@ -211,13 +211,15 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
             case 64256:  *out = regular<64, 2, 5, MODE, BIAS>(gather); return true;    // 40 KB
             default: break;
         }
-        if constexpr (MODE == shflbw::kPanelConvChain) {
-            if (gather == shflbw::kGatherTma) return false;   // (conv_tokens)
-            if (V == 128 && tile == 128) { *out = choice<128, 1, 64, 6, 8, MODE>(); return true; }   // 32 KB
-            if (V == 128 && tile == 256) { *out = choice<128, 2, 64, 4, 8, MODE>(); return true; }   // 48 KB
-        } else {
-            if (V == 128 && tile == 128) { *out = regular<128, 1, 6, MODE, BIAS>(gather); return true; }
-            if (V == 128 && tile == 256) { *out = regular<128, 2, 4, MODE, BIAS>(gather); return true; }
+        if (V == 128 && tile == 128) { *out = regular<128, 1, 6, MODE, BIAS>(gather); return true; }   // 32 KB
+        if (V == 128 && tile == 256) {                                                                 // 48 KB
+            if constexpr (MODE == shflbw::kPanelConvChain) {
+                if (gather == shflbw::kGatherTma) return false;   // (conv_tokens)
+                *out = choice<128, 2, 64, 4, 8, MODE>();
+            } else {
+                *out = regular<128, 2, 4, MODE, BIAS>(gather);
+            }
+            return true;
         }
         return false;
     }
@@ -258,19 +260,22 @@ int tma_row_pix(int Wo, int Wp, int Bp, int stride) {
 // (tuning aids).  Asked for when a state is made.
 bool tma_wanted() { const char* g = getenv("SHFLBW_GATHER"); return !g || atoi(g) == 1; }
 
-// The gather of an SpMM: TMA, unless the operand is a few KB of rows that share 32-byte sectors (an odd multiple of 8
-// tokens) and every row is wanted by many blocks.  The SMs then fetch the same few lines of L2 over and over, and the
-// copy engine's requests to one line queue up, the more so where a block takes neighbouring rows.  By TMA and by cp.async,
-// 8 tokens, density 0.5: K = 256, 700 blocks of 16 rows 15.3 and 8.6 us; K = 768, 148 of 16 9.9 and 5.8; K = 1024, 344 of
-// 64 19.1 and 12.5; K = 1536, 344 of 32 22.4 and 16.7 (at density 0.25, 16 rows, 9.2 and 10.4); K = 2048, 172 of 16 13.6
-// and 14.7; density 0.1, K = 512, 148 of 16 3.9 and 4.0.  24 tokens, K = 256, 700 blocks of 32: 18.4 and 9.8.  16 tokens,
-// whose rows are whole sectors, density 0.4, K = 256, 192 blocks of 16: 4.5 and 4.4; K = 1024: 5.5 and 7.4.
+// The gather of an SpMM: TMA, unless rows share 32-byte sectors (8 or 24 tokens), there are few of them, and many blocks
+// want each.  The SMs then fetch the same few lines of L2 over and over, and the copy engine's requests to one line queue
+// up, the more so where a block takes neighbouring rows.  By TMA and by cp.async, 8 tokens, density 0.5: K = 256, 700
+// blocks of 16 rows 15.3 and 8.6 us; K = 768, 148 of 16 9.9 and 5.8; K = 1024, 344 of 64 19.1 and 12.5; K = 2360, 94 of
+// 32 14.9 and 9.6; K = 4000, 375 of 32 34.0 and 36.2.  Below 0.4: K = 1024, 688 of 16 at 0.25 19.5 and 11.8; K = 1272,
+// 175 of 16 at 0.39 8.4 and 8.8; K = 512, 148 of 16 at 0.1 3.9 and 4.0; a stage of 16 columns, K = 128, 362 of 16 4.7 and
+// 5.2.  24 tokens, K = 256, 700 of 32 at 0.5 18.4 and 9.8, 192 of 16 at 0.4 5.0 and 5.0; 40, K = 144, 313 of 32 5.4 and
+// 5.2; 16, whose rows are whole sectors, K = 1024, 688 of 16 at 0.25 8.2 and 11.8.
 // With a bias 256-token tiles are built for the TMA gather only, without one the other is there to compare with
 // (SHFLBW_GATHER=0).
 int spmm_gather(long long K, int N, int row_blocks, long long padded_cols, int tile, bool with_bias) {
     if (tile == 256 && with_bias) return shflbw::kGatherTma;
     if (getenv("SHFLBW_GATHER")) return tma_wanted() ? shflbw::kGatherTma : shflbw::kGatherCpAsync;
-    const bool crowded = N % 16 == 8 && padded_cols >= 40 * K && (K * N <= 8192 || (K * N <= 12288 && 3 * padded_cols > K * row_blocks));
+    const bool dense = 20 * padded_cols > 9 * K * row_blocks;
+    const bool crowded = padded_cols > 16ll * row_blocks && ((N == 8 && padded_cols >= 40 * K && K <= (dense ? 3072 : 1024)) ||
+                                                             (N == 24 && padded_cols >= 150 * K && K <= 341));
     return crowded && tile == 128 ? shflbw::kGatherCpAsync : shflbw::kGatherTma;
 }
 
@@ -297,31 +302,41 @@ int pick_tile(long long n_tokens, int row_blocks) {
 
 // The gather of a convolution, and the pixels that an output row counts as.  TMA, unless the padding of the rows
 // costs more time in rounds of items (those of the tile that each side takes) than the gather saves: a stage takes it
-// about 650 clk and the cp.async gather 870 to 1000.
-//   Rounds of one tile: up to a quarter more of them (14x14x512 -> 2048, batch 16, V = 64, 3 -> 4 rounds: 28.0 us by
-// cp.async, 28.6 by TMA; V = 32, 6 -> 7: 35.9 and 33.5; 13x13x256 -> 2048, batch 24, V = 64, 900 columns a block, 4 -> 5:
-// 42.7 and 41.7); less than that for taller blocks with tokens in lanes, whose items are more epilogue than gather
+// about 650 clk and the cp.async gather 870 to 1000.  cp.async and TMA in us:
+//   Rounds of one tile: up to a quarter more of them (14x14x512 -> 2048, batch 16, V = 64, 3 -> 4 rounds: 28.0 and 28.6; V
+// = 32, 6 -> 7: 35.9 and 33.5; 13x13x256 -> 2048, batch 24, V = 64, 900 columns a block, 4 -> 5: 42.7 and 41.7); a fifth for
+// taller blocks with tokens in lanes and one or two stages of columns, whose items are more epilogue than gather
 // (17x17x256, batch 24: chained -> 1024, V = 64, 102 columns, 4 -> 5: 12.7 and 14.1; -> 2048 in NHWC, V = 128, 40 columns:
-// 27.1 and 28.9).
-//   Padding that takes one or two rounds of 128-token items to as many of 256: only for blocks of less than a stage
-// (V = 32, 40 columns: 9.45 by cp.async, 8.95 by TMA; V = 64, 40: 4.07 and 3.99; 100: 4.2 and 5.2; 300: 5.5 and 6.3;
-// V = 128, 40: 10.2 and 10.9, 300: 12.9 and 15.7).
-//   Chained layers of 128 rows with tokens in lanes gather by cp.async: their items are an epilogue of 32 KB behind one to
-// three stages, and beside the TMA gather's operands that epilogue does not fit the 96 registers that 17 warps leave
-// (batch 128, 28x28x256 -> 256, 13 columns a block: 17.2 us, 18.3 by TMA; batch 64, 14x14x512 -> 1024 with residual,
-// 102 columns: 15.3 and 17.2).
+// 27.1 and 28.9; less than half a stage, chained 19x19x56 -> 320, batch 79, V = 64, 4 -> 5: 9.6 and 8.4).  Where there are
+// more of them the tokens count, too: at most 1.3 times as many (chained 17x17x952 -> 512, batch 51, V = 64, 4 -> 5 rounds of
+// 1.41 times the tokens: 67.6 and 71.5; 12x12x16 -> 1088, batch 50, V = 32, 8 -> 10, 1.33: 12.9 and 13.9; no more rounds,
+// 17x17x776 -> 608, batch 1, V = 32, 2 -> 2, 1.41: 44.6 and 34.9).
+//   Padding that takes one or two rounds of 128-token items to as many of 256: only for blocks of up to a stage of
+// columns (V = 32, 40 columns: 9.45 and 8.95, 54: 4.3 and 3.9, 100: 4.0 and 4.6; V = 64 chained, 40: 4.07 and 3.99, 64: 4.4
+// and 4.6, 300: 5.5 and 6.3; V = 128, 40: 10.2 and 10.9, 300: 12.9 and 15.7).
+//   128 rows with tokens in lanes write the longest items of all.  Into NHWC, padding that fills the chip leaves no SM to
+// the passes around (10x10x24 -> 1792, batch 6, 98 -> 140 items: 10.0 and 11.3).  Chained, they gather by cp.async: beside
+// the TMA gather's operands their epilogue does not fit the 96 registers that 17 warps leave (28x28x256 -> 256, batch 128,
+// 13 columns a block: 17.2 and 18.3; 14x14x512 -> 1024, batch 64, with residual, 102 columns: 15.3 and 17.2), except for
+// one stage on few SMs (7x7x48 -> 384, batch 8, 32 columns: 4.3 and 4.1).
 struct ConvTokens { int row_pix; int gather; };
 ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int V, int row_blocks, long long padded_cols, bool rows, bool chain) {
     const ConvTokens plain{Wo, shflbw::kGatherCpAsync};
-    if (chain && !rows && V == 128) return plain;
     const int row_pix = tma_wanted() ? tma_row_pix(Wo, Wp, Bp, stride) : 0;
     const long long before = (long long)Ho * Wo * Bp, after = (long long)Ho * row_pix * Bp;
     if (!row_pix || after >= (1ll << 31)) return plain;
     const int tile0 = pick_tile(before, row_blocks), tile1 = pick_tile(after, row_blocks);
-    const long long cost0 = rounds_of_items(before, tile0, row_blocks) * (tile0 == 128 ? 2 : 3);
-    const long long cost1 = rounds_of_items(after, tile1, row_blocks) * (tile1 == 128 ? 2 : 3);
-    const bool short_items = tile1 > tile0 && V <= 64 && padded_cols <= 48ll * row_blocks;
-    const bool pays = short_items || (!rows && V >= 64 ? 5 * cost1 <= 6 * cost0 : 4 * cost1 <= 5 * cost0);
+    const long long rounds0 = rounds_of_items(before, tile0, row_blocks), rounds1 = rounds_of_items(after, tile1, row_blocks);
+    const long long cost0 = rounds0 * (tile0 == 128 ? 2 : 3), cost1 = rounds1 * (tile1 == 128 ? 2 : 3);
+    if (V == 128 && !rows) {
+        if (chain && (tile1 == 256 || padded_cols > 64ll * row_blocks)) return plain;
+        if (!chain && 4 * after > 5 * before && rounds1 == 1 && 10 * ((after + tile1 - 1) / tile1 * row_blocks) > 9ll * (sm_count() > 0 ? sm_count() : 148))
+            return plain;
+    }
+    const bool short_items = tile1 > tile0 && V <= 64 && padded_cols <= (V == 64 && chain ? 48ll : 64ll) * row_blocks;
+    const bool tight = !rows && V >= 64 && padded_cols > 32ll * row_blocks && padded_cols <= 128ll * row_blocks;
+    const bool roomy = cost1 <= cost0 || padded_cols <= 32ll * row_blocks || 10 * after <= 13 * before;
+    const bool pays = short_items || (roomy && (tight ? 5 * cost1 <= 6 * cost0 : 4 * cost1 <= 5 * cost0));
     return pays ? ConvTokens{row_pix, shflbw::kGatherTma} : plain;
 }
 
