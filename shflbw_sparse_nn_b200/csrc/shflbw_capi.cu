@@ -164,7 +164,7 @@ PanelChoice regular(int gather) {
     return choice<V, TM, 64, STAGES, PW, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
 }
 template <int MODE, bool BIAS = false>
-bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsync, int wide_ring = 0) {
+bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsync, int wide_ring = 0, int wide_pw = 3) {
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         // Shallow items (at most 64 non-zero columns): sixteen epilogue warps and three producer
         // warps, each a group of its own (20 warps: 96 registers per thread); stages of 32 columns,
@@ -175,9 +175,14 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
         // Three gather warps with a stage each at a time, whichever the gather: with two of them the TMA issue was the
         // longest of an item's steps from 32 columns on (chained 14x14x256 -> 1024 with residual, batch 256, 102
         // columns a block: 57.2 us, three 47.0, three by cp.async 49.9; 28x28x256 -> 512 without residual, batch
-        // 128, 48 columns: 36.8, 30.0, 33.1).
+        // 128, 48 columns: 36.8, 30.0, 33.1).  With a residual and up to 48 columns two: the addends are what such a layer
+        // waits for, and fetching the stages ahead of them faster only gets in their way (in the network, batch 118, three
+        // and two: 56x56x64 -> 256, 10 columns, 87.6 and 78.4 us; 28x28x128 -> 512, 20, 48.6 and 45.2; 14x14x256 -> 1024,
+        // 40, 30.8 and 29.6; 7x7x512 -> 2048, 80, 22.5 both; without residual 56x56x64 -> 256 48.1 and 54.4).
         if (wide_ring && tile == 256 && V == 64) {
             if (gather == shflbw::kGatherTma) {
+                if constexpr (MODE == shflbw::kPanelConvChain)
+                    if (wide_ring == 6 && wide_pw == 2) { *out = choice<64, 2, 32, 6, 2, MODE, 2, shflbw::kGatherTma, 16, BIAS, true>(); return true; }
                 *out = wide_ring == 8 ? choice<64, 2, 32, 8, 3, MODE, 3, shflbw::kGatherTma, 16, BIAS, false>()
                                       : choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherTma, 16, BIAS, true>();
                 return true;
@@ -967,7 +972,7 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
                            : (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch, gather)
                            : st->variant == 1      ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch, gather)
                                                    : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, gather,
-                                                                                      st->variant != 2 ? 0 : st->residual ? 6 : st->stages);
+                                                                                      st->variant != 2 ? 0 : st->residual ? 6 : st->stages, st->producer_warps);
     if (!ok_kernel) return SHFLBW_ERR_INVALID_ARG;
     if (panel_bias) {                                       // (init allowed the kernel without; before anything is launched)
         const int rc = allow_smem(ch.fn, ch.smem);
@@ -1200,10 +1205,11 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     // columns per block (14x14x256 -> 1024 with residual, batch 128, 112 columns: 33.9 -> 26.5 us); without a
     // residual the limit is one stage (pick_panel).
     PanelChoice ch;
+    const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
     const bool wide = (st->variant == 2 ||
                        (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
-                        (f->kptr.empty() ? 0 : f->kptr.back()) <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count())) &&
-                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6);
+                        padded_cols <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count())) &&
+                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6, padded_cols <= 48ll * (st->F / st->V) ? 2 : 3);
     if (wide) {
         const int rc = allow_smem(ch.fn, ch.smem);
         if (rc != SHFLBW_OK) return rc;
