@@ -178,7 +178,9 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
         // 128, 48 columns: 36.8, 30.0, 33.1).  With a residual and up to 48 columns two: the addends are what such a layer
         // waits for, and fetching the stages ahead of them faster only gets in their way (in the network, batch 118, three
         // and two: 56x56x64 -> 256, 10 columns, 87.6 and 78.4 us; 28x28x128 -> 512, 20, 48.6 and 45.2; 14x14x256 -> 1024,
-        // 40, 30.8 and 29.6; 7x7x512 -> 2048, 80, 22.5 both; without residual 56x56x64 -> 256 48.1 and 54.4).
+        // 40, 30.8 and 29.6; 7x7x512 -> 2048, 80, 22.5 both; without residual 56x56x64 -> 256 48.1 and 54.4), unless the
+        // output is beyond 256 MB, where HBM decides (batch 256: 28x28x128 -> 512, 206 MB, 90.7 and 79.9; 56x56x64 -> 256,
+        // 411 MB, 183 and 202).  set_residual chooses.
         if (wide_ring && tile == 256 && V == 64) {
             if (gather == shflbw::kGatherTma) {
                 if constexpr (MODE == shflbw::kPanelConvChain)
@@ -1206,10 +1208,11 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     // residual the limit is one stage (pick_panel).
     PanelChoice ch;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
+    const bool two_warps = padded_cols <= 48ll * (st->F / st->V) && (long long)st->F * st->Ho * st->Wo * st->Bp * 2 <= (256ll << 20);   // (lookup)
     const bool wide = (st->variant == 2 ||
                        (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
                         padded_cols <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count())) &&
-                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6, padded_cols <= 48ll * (st->F / st->V) ? 2 : 3);
+                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6, two_warps ? 2 : 3);
     if (wide) {
         const int rc = allow_smem(ch.fn, ch.smem);
         if (rc != SHFLBW_OK) return rc;
