@@ -85,6 +85,7 @@ struct alignas(64) PanelParams {
     // input, running from that pixel to the end of what a tap reads; box = 64 tokens x 1 row, 128-byte swizzle);
     // first member so that it sits on the 64-byte boundary the copy engine wants
     unsigned long long tmap_b[16];
+    unsigned long long tmap_res[16];   // box epilogue only: tensor map of the residual's planes (box = 64 tokens x 1 plane)
     // sparse operand (kernel image)
     const int* blk_ptr;      // [X+1] padded offsets (multiples of 16)
     const int* blk_idx;      // padded column ids
@@ -154,7 +155,7 @@ constexpr int kGatherCpAsync = 0, kGatherTma = 1;
 // latency-bound: sixteen warps, as two sets on alternate items, keep four such chains per
 // scheduler in flight instead of two.
 template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int GATHER_ = kGatherCpAsync,
-          int EW_ = 8, bool ADDEND_ = false>
+          int EW_ = 8, bool ADDEND_ = false, int SLOTS_ = 0>
 struct PanelCfg {
     static constexpr int EW = EW_;
     static_assert(EW == 8 || EW == 16, "epilogue warps");
@@ -180,13 +181,16 @@ struct PanelCfg {
     // Epilogue tiles (tokens in lanes only): each epilogue warp transposes 32 tokens x 32 output
     // rows / filters through 2 KB so that its global stores are 16 bytes per lane and 64-byte
     // runs.  With rows in lanes the stores go straight from registers.
-    static constexpr int OUT_BYTES = (MODE == kPanelSpmmRows || MODE == kPanelConvChainRows) ? 0 : EW * 2048;
+    // Box epilogue: SLOTS slots of 32 rows x 64 tokens per pair of warps.
+    static constexpr int SLOTS = SLOTS_, SLOT_ROWS = 32, SLOT_BYTES = SLOT_ROWS * 128;
+    static constexpr int OUT_BYTES = (MODE == kPanelSpmmRows || MODE == kPanelConvChainRows) ? 0 : SLOTS ? EW / 2 * SLOTS * SLOT_BYTES : EW * 2048;
     // Sixteen epilogue warps, instances built with ADDEND: the addend of an item (C, or a chained layer's
     // residual) is copied to shared memory an item ahead: each lane's own 16-byte pieces, 64 rows x 32
     // tokens per warp.  Without, the ring has that room.
     static_assert(!ADDEND_ || EW == 16, "addend slots: sixteen epilogue warps");
-    static constexpr int RES_BYTES = ADDEND_ ? EW * 4096 : 0;
-    static constexpr int BAR_BYTES = (STAGES * 2 + 12) * 8;  // mbarriers (ring, up to 4 + 4 accumulator, drain) + tmem slot + abort flag
+    static constexpr int RES_BYTES = ADDEND_ ? EW * 4096 : SLOTS ? EW * SLOT_ROWS * 4 : 0;   // (box epilogue: row ids of a refill)
+    static constexpr int SLOT_BARS = SLOTS ? EW / 2 * (SLOTS + 1) : 0;       // per pair: one for each slot, one for its two warps
+    static constexpr int BAR_BYTES = (STAGES * 2 + 12 + SLOT_BARS) * 8;  // mbarriers (ring, up to 4 + 4 accumulator, drain) + tmem slot + abort flag
     static constexpr int TAB_BYTES = 512 * 8;               // per-CTA item table (kPanelMaxItemsPerCta entries)
     static constexpr int IDX_AHEAD = 2;                    // a group fetches row ids this many of its stages ahead
     static constexpr int IDX_RING = (IDX_AHEAD + 1) * GROUPS <= 8 ? 8 : 16;   // stages of row ids kept in shared memory
@@ -242,14 +246,155 @@ __device__ __forceinline__ uint4 broadcast8(const __half* p) {
 
 constexpr int kPanelMaxItemsPerCta = 512;  // capacity of the per-CTA item table
 
+// Epilogue of a chained layer with a residual that comes in boxes (64 consecutive tokens are 128 consecutive bytes of a
+// plane; tokens in lanes).  Such a layer is all epilogue, and what bounded it was the load/store unit: 2 250 wavefronts an
+// item of 64 x 256, 1 200 of them the residual's cp.async in 64-byte pieces.  Here the copy engine fetches the residual,
+// by tile::gather4 (its planes are permuted), into slots [row][64 tokens], 128-byte-swizzled.  The accumulator comes
+// out of TMEM as 8 x 8 tiles, is added to the residual in that form (ldmatrix transposes), goes back into the slot
+// (stmatrix) and leaves as 16-byte pieces of rows.  (Stores by TMA, a box at a time, were slower: 8 clk of the engine for
+// 128 bytes.)
+//
+// A pair of warps (TMEM quadrants 2 j and 2 j + 1, the same columns) shares a box and SLOTS slots, which its chunks of
+// 32 rows take in turn.  When warp q % 2 has finished chunk q + 1, and the other warp chunk q, it has chunk q's slot
+// refilled for chunk q + SLOTS.  All waits are on mbarriers and bounded.
+template <class Cfg, int V, class ItemBlock, class ItemTile>
+__device__ __forceinline__ void box_epilogue(const PanelParams& p, uint8_t* smem, uint32_t smem_base, uint32_t tmem_base, const int2* item_tab, int nloc,
+                                             uint64_t* acc_full, uint64_t* acc_empty, uint64_t* slot_bar, volatile int* cta_abort,
+                                             int warp, int lane, const ItemBlock& item_block, const ItemTile& item_tile) {
+    constexpr int NBUF = Cfg::NBUF, ESETS = Cfg::ESETS, T = Cfg::T, NS = Cfg::SLOTS, ROWS = Cfg::SLOT_ROWS, D = NS - 1;
+    constexpr int COLS = Cfg::ACC_COLS / 2, NCH = COLS / ROWS;
+    static_assert(NCH * ROWS == COLS && COLS <= V, "chunks of one accumulator");
+    static_assert(NS >= 2, "a chunk is added to while the one before is on its way out");
+    const int quad = warp & 3, half_id = (warp >> 2) & 1, first = ESETS > 1 ? warp >> 3 : 0;
+    const int a0 = half_id * COLS / V, mbase = half_id * COLS % V;     // accumulator and first block row of this warp
+    const int pair = first * 4 + half_id * 2 + (quad >> 1), me = quad & 1;
+    uint64_t* const ready = slot_bar + pair * NS;              // [NS] residual landed
+    uint64_t* const done = slot_bar + Cfg::EW / 2 * NS + pair;         // the warp that does not refill the slot is done with it
+    const uint32_t slots = smem_base + (uint32_t)(Cfg::PIPE_BYTES + pair * NS * Cfg::SLOT_BYTES);
+    int4* const ids = (int4*)(smem + Cfg::PIPE_BYTES + Cfg::OUT_BYTES + warp * (ROWS * 4));   // planes of the next refill
+    // stmatrix: lane 8 k + j names tokens 8 k.. of this warp's 32, row 8 i + j; the 16-byte chunk is XORed with j.  Pieces:
+    // lane 4 j + c takes tokens 8 c.., row 8 i + prow: rows r and r + 4 in turn, so that eight lanes read all banks.
+    const uint32_t lane_off = (uint32_t)((lane & 7) * 128 + (((me * 4 + (lane >> 3)) ^ (lane & 7)) << 4));
+    const int prow = ((lane >> 2) & 1) * 4 + (lane >> 3);
+    const uint32_t piece_off = (uint32_t)(prow * 128 + (((me * 4 + (lane & 3)) ^ prow) << 4));
+    const __half2 alpha2 = __half2half2(__float2half_rn(p.alpha)), zero2 = __float2half2_rn(0.f);
+    if (warp == 0 && sm100::elect_one()) sm100::prefetch_tensormap(p.tmap_res);
+    auto offset = [&](int tok) {                               // of a token's element in a plane
+        const int pix = fast_div(tok, p.div_bp), oh = fast_div(pix, p.div_row);
+        return ((oh + p.oph) * p.OWp + pix - oh * p.row_pix + p.opw) * p.Bp + tok - pix * p.Bp;
+    };
+    auto first_tok = [&](int item) { return item_tile(item) * T + a0 * 128 + (quad >> 1) * 64; };   // of the pair's box
+    auto load_ids = [&](int li, int ch) {                      // planes of four rows per lane, lanes 0..ROWS/4-1
+        const int f = item_block((int)blockIdx.x + li * (int)gridDim.x) * V + mbase + ch * ROWS + lane * 4;
+        return lane >= ROWS / 4 || li >= nloc ? make_int4(0, 0, 0, 0) : p.res_map ? __ldg((const int4*)(p.res_map + f)) : make_int4(f, f + 1, f + 2, f + 3);
+    };
+    auto refill = [&](int li, const int4& id, uint32_t slot) { // by one warp of the pair
+        const int tok = first_tok((int)blockIdx.x + li * (int)gridDim.x);
+        if (lane < ROWS / 4) ids[lane] = id;
+        __syncwarp();
+        if (sm100::elect_one()) {
+            if (tok < p.N) {
+                const int x = offset(tok);
+                int4 r[ROWS / 4];
+#pragma unroll
+                for (int i = 0; i < ROWS / 4; ++i) r[i] = ids[i];
+                sm100::mbar_arrive_expect_tx(&ready[slot], (uint32_t)Cfg::SLOT_BYTES);
+#pragma unroll
+                for (int i = 0; i < ROWS / 4; ++i)
+                    sm100::tma_gather4(slots + slot * (uint32_t)Cfg::SLOT_BYTES + (uint32_t)(i * 512), p.tmap_res, x, r[i].x, r[i].y, r[i].z, r[i].w, &ready[slot]);
+            } else {
+                sm100::mbar_arrive(&ready[slot]);
+            }
+        }
+        __syncwarp();
+    };
+#pragma unroll
+    for (int q = 0; q < NS; ++q)
+        if (first + q / NCH * ESETS < nloc && (q & 1) == me) refill(first + q / NCH * ESETS, load_ids(first + q / NCH * ESETS, q % NCH), (uint32_t)q);
+    uint32_t slot = 0, par = 0, q = 0, prev = 0;               // slot of chunk q, its parity; slot of chunk q - 1
+    for (int li = first; li < nloc; li += ESETS) {
+        const int item = (int)blockIdx.x + li * (int)gridDim.x, b = li % NBUF;
+        const bool has_k = item_tab[li].y > 0;
+        const int tok = first_tok(item) + me * 32 + (lane & 3) * 8;        // this lane's 8 tokens
+        const bool ok = tok < p.N;
+        __half* const dst = p.out + offset(tok);
+        const int f0 = item_block(item) * V + mbase;
+        const uint32_t acc = tmem_base + ((uint32_t)(quad * 32) << 16) + b * Cfg::ACC_COLS + half_id * COLS;
+        if (!sm100::mbar_wait_warp(&acc_full[b], (li / NBUF) & 1, cta_abort, p.status_word, SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit)) return;
+        sm100::tc_fence_after_sync();
+#pragma unroll
+        for (int ch = 0; ch < NCH; ++ch) {
+            const bool refills = (int)(q & 1) != me && q > 0;  // chunk q - 1's slot
+            const int li_n = li + (ch + D) / NCH * ESETS;
+            int4 id = make_int4(0, 0, 0, 0);
+            if (refills) id = load_ids(li_n, (ch + D) % NCH);
+            __half2 h[ROWS / 8][4];                            // tile of rows 8 i.., tokens 8 k..
+            {
+                uint32_t lo[ROWS / 2], hi[ROWS / 2];           // lanes 0-15 and 16-31 of the quadrant
+                if (has_k) {
+                    sm100::tmem_ld_16x256b(acc + ch * ROWS, lo);
+                    sm100::tmem_ld_16x256b(acc + (16u << 16) + ch * ROWS, hi);
+                    sm100::tmem_ld_wait();
+                } else {
+#pragma unroll
+                    for (int e = 0; e < ROWS / 2; ++e) lo[e] = hi[e] = 0u;
+                }
+                if (ch + 1 == NCH) {                           // last TMEM read of this item by this warp: release the buffer
+                    sm100::tc_fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) sm100::mbar_arrive(&acc_empty[b]);
+                }
+                // the arithmetic of the other epilogues: round to fp16, then alpha, the residual and ReLU in fp16
+#pragma unroll
+                for (int i = 0; i < ROWS / 8; ++i)
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const uint32_t* r = (k < 2 ? lo : hi) + 4 * i + 2 * (k & 1);
+                        h[i][k] = __hmul2(__floats2half2_rn(__uint_as_float(r[0]), __uint_as_float(r[1])), alpha2);
+                    }
+            }
+            if (!sm100::mbar_wait_warp(&ready[slot], par, cta_abort, p.status_word, SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit)) return;
+            const uint32_t tile = slots + slot * (uint32_t)Cfg::SLOT_BYTES;
+#pragma unroll
+            for (int i = 0; i < ROWS / 8; ++i) {
+                uint32_t r[4];
+                sm100::ldmatrix_x4_trans(tile + lane_off + i * 1024, r);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    h[i][k] = __hadd2(h[i][k], *(__half2*)&r[k]);
+                    if (p.relu) h[i][k] = __hmax2(h[i][k], zero2);
+                }
+                sm100::stmatrix_x4_trans(tile + lane_off + i * 1024, *(uint32_t*)&h[i][0], *(uint32_t*)&h[i][1], *(uint32_t*)&h[i][2], *(uint32_t*)&h[i][3]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < ROWS / 8; ++i) {
+                const uint4 v = *(const uint4*)(smem + (tile - smem_base) + piece_off + i * 1024);
+                if (ok) *(uint4*)(dst + (size_t)((uint32_t)(f0 + ch * ROWS + i * 8 + prow) * (uint32_t)p.out_plane)) = v;
+            }
+            sm100::fence_proxy_async_smem();                   // this warp's accesses before the copies of the refill
+            __syncwarp();
+            if ((int)(q & 1) != me) {                          // (phases of `done` in order: chunk q's arrival after chunk q - 1's)
+                if (q > 0 && !sm100::mbar_wait_warp(done, (q - 1) & 1, cta_abort, p.status_word, SHFLBW_DEVSTAT_TIMEOUT_ACCUM, p.wait_limit)) return;
+                if (lane == 0) sm100::mbar_arrive(done);
+                if (refills && li_n < nloc) refill(li_n, id, prev);
+            }
+            ++q;
+            prev = slot;
+            if (++slot == (uint32_t)NS) { slot = 0; par ^= 1u; }
+        }
+    }
+}
+
 // BIAS: C holds one value per output row (SpMM, added like C with beta = 1) or per filter (SpConv writing
 // NHWC in logical order).  Kernels of their own: as a branch of the others it made small products 1-2 %
 // slower (256-item launches of 5-9 us, where every instruction is fetched for the first time).
 template <int V, int TM, int KS_, int STAGES, int PW, int MODE, int GROUPS_ = 2, int GATHER_ = kGatherCpAsync,
-          int EW_ = 8, bool BIAS = false, bool ADDEND = false>
-__global__ void __launch_bounds__(PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, GATHER_, EW_, ADDEND>::THREADS, 1)
+          int EW_ = 8, bool BIAS = false, bool ADDEND = false, int SLOTS = 0>
+__global__ void __launch_bounds__(PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, GATHER_, EW_, ADDEND, SLOTS>::THREADS, 1)
 panel_umma_kernel(const __grid_constant__ PanelParams p) {
-    using Cfg = PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, GATHER_, EW_, ADDEND>;
+    using Cfg = PanelCfg<V, TM, KS_, STAGES, PW, MODE, GROUPS_, GATHER_, EW_, ADDEND, SLOTS>;
+    static_assert(SLOTS == 0 || (MODE == kPanelConvChain && !BIAS && !ADDEND), "box epilogue: chained layers with tokens in lanes");
     constexpr int EW = Cfg::EW;                                             // epilogue warps 0..EW-1, MMA warp EW, producers after it
     constexpr bool SWAP = Cfg::SWAP;                                        // rows in TMEM lanes
     constexpr bool CONV = MODE == kPanelConv || MODE == kPanelConvChain || MODE == kPanelConvChainRows;  // implicit-GEMM gather
@@ -269,6 +414,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     uint32_t* tmem_slot = (uint32_t*)(acc_empty + NBUF);
     volatile int* cta_abort = (volatile int*)(tmem_slot + 1);
     uint64_t* drain_bar = acc_empty + NBUF + 1;        // abort path only: MMA thread waits for its last MMAs
+    uint64_t* slot_bar = full_bar + STAGES * 2 + 12;   // [SLOT_BARS] box epilogue
     int2* item_tab = (int2*)(bar_area + Cfg::BAR_BYTES);  // [nloc] (first padded row, padded row count)
     int* idx_ring = (int*)(bar_area + Cfg::BAR_BYTES + Cfg::TAB_BYTES);  // [IDX_RING][KS] row ids of upcoming stages
 
@@ -291,6 +437,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             sm100::mbar_init(&acc_full[b], 1);
             sm100::mbar_init(&acc_empty[b], EW / Cfg::ESETS);  // one arrival per epilogue warp of the set that reads it
         }
+        for (int b = 0; b < Cfg::SLOT_BARS; ++b) sm100::mbar_init(&slot_bar[b], 1);
         sm100::mbar_init(drain_bar, 1);
         *cta_abort = 0;
         sm100::mbar_init_fence();
@@ -731,6 +878,9 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         // the items in turn: against all sixteen on one item (a quarter of the columns each), 108 ->
         // 93 us on 56x56x64 -> 256 at batch 256, since an item's chain of waits is most of its time.
         sm100::grid_dependency_wait();
+        if constexpr (SLOTS > 0) {
+            box_epilogue<Cfg, V>(p, smem, smem_base, tmem_base, item_tab, nloc, acc_full, acc_empty, slot_bar, cta_abort, warp, lane, item_block, item_tile);
+        } else {
         const int quad = warp & 3, half_id = (warp >> 2) & 1;
         // (a single 16- or 32-column accumulator is not split; two 16-column accumulators go to the two halves)
         constexpr int HALVES = (Cfg::ACC_COLS >= 64 || (V == 16 && TM == 2)) ? 2 : 1;
@@ -1169,6 +1319,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             }
         }
         if constexpr (Cfg::RES_BYTES > 0) sm100::cp_async_wait<0>();   // nothing of this warp is in flight when the block ends
+        }
     }
 
     if (*cta_abort) {

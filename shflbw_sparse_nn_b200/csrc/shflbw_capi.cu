@@ -113,10 +113,10 @@ using PanelKernel = void (*)(const shflbw::PanelParams);
 struct PanelChoice { PanelKernel fn; size_t smem; int tokens; int stages; int pw; int threads; int variant; int gather; };
 
 template <int V, int TM, int KS, int STAGES, int PW, int MODE, int GROUPS = 2, int GATHER = shflbw::kGatherCpAsync,
-          int EW = 8, bool BIAS = false, bool ADDEND = false>
+          int EW = 8, bool BIAS = false, bool ADDEND = false, int SLOTS = 0>
 PanelChoice choice() {
-    using Cfg = shflbw::PanelCfg<V, TM, KS, STAGES, PW, MODE, GROUPS, GATHER, EW, ADDEND>;
-    return {shflbw::panel_umma_kernel<V, TM, KS, STAGES, PW, MODE, GROUPS, GATHER, EW, BIAS, ADDEND>, (size_t)Cfg::SMEM_BYTES, Cfg::T,
+    using Cfg = shflbw::PanelCfg<V, TM, KS, STAGES, PW, MODE, GROUPS, GATHER, EW, ADDEND, SLOTS>;
+    return {shflbw::panel_umma_kernel<V, TM, KS, STAGES, PW, MODE, GROUPS, GATHER, EW, BIAS, ADDEND, SLOTS>, (size_t)Cfg::SMEM_BYTES, Cfg::T,
             STAGES, PW, Cfg::THREADS, 0, GATHER};
 }
 
@@ -150,6 +150,15 @@ int encode_map(const void* base, long long rows, long long cols, long long pitch
     return SHFLBW_OK;
 }
 
+// The same into `out` by way of a state's kept map: copied where that is of this very operand, made anew where not.
+int encode_map(const void* base, long long rows, long long cols, long long pitch, const shflbw_tensor_map_t& kept, unsigned long long out[16]) {
+    if (base && kept.of == base && kept.rows == rows && kept.cols == cols && kept.pitch == pitch) {
+        std::memcpy(out, kept.map, sizeof kept.map);
+        return SHFLBW_OK;
+    }
+    return encode_map(base, rows, cols, pitch, out);
+}
+
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
 // Shapes of the TMA gather: four stages at a time, by two warps each, SpMM with rows in lanes by four: its items are
@@ -164,7 +173,14 @@ PanelChoice regular(int gather) {
     return choice<V, TM, 64, STAGES, PW, MODE, 4, shflbw::kGatherTma, 8, BIAS>();
 }
 template <int MODE, bool BIAS = false>
-bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsync, int wide_ring = 0, int wide_pw = 3) {
+bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsync, int wide_ring = 0, int wide_pw = 3, bool box = false) {
+    if constexpr (MODE == shflbw::kPanelConvChain) {
+        if (box) {                                           // box epilogue (see the kernel)
+            if (gather != shflbw::kGatherTma || !wide_ring || tile != 256 || V != 64) return false;
+            *out = choice<64, 2, 32, 6, 3, MODE, 3, shflbw::kGatherTma, 16, false, false, 3>();
+            return true;
+        }
+    }
     if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
         // Shallow items (at most 64 non-zero columns): sixteen epilogue warps and three producer
         // warps, each a group of its own (20 warps: 96 registers per thread); stages of 32 columns,
@@ -850,6 +866,29 @@ int shflbw_debug_export_steps(long long tokens, int F) {
 }
 #endif
 
+// What a convolution's tensor maps are of.  Input: one row per pixel that a tap of output pixel (0, 0) reads, `pitch` from
+// one to the next, as long as from output pixel (0, 0) to the last: every address that the map allows is inside the
+// input.  Output and residual of a chained layer: its planes, up to the last pixel.
+struct PlaneMap { const void* base; long long rows, cols, pitch; };
+PlaneMap input_map(const shflbw_spconv_state_t& st, const void* base, int Hp, int Wp, int stride) {
+    return {base, ((long long)st.C - 1) * Hp * Wp + (long long)(st.R - 1) * Wp + st.S,
+            (((long long)st.Ho - 1) * stride * Wp + ((long long)st.Wo - 1) * stride + 1) * st.Bp, 2ll * st.Bp};
+}
+PlaneMap output_map(const shflbw_spconv_state_t& st, const void* base) {
+    const long long OWp = st.Wo + st.out_S - 1, OHp = st.Ho + st.out_R - 1;
+    return {base, st.F, ((st.out_R / 2 + st.Ho - 1) * OWp + st.out_S / 2 + st.Wo) * st.Bp, 2 * OHp * OWp * st.Bp};
+}
+// Whether 64 consecutive tokens of a chained layer are 128 consecutive bytes of an output plane throughout: the rows are
+// not padded, and either the output has no halo beside its rows or they are whole boxes.
+bool boxes_fit(const shflbw_spconv_state_t& st) {
+    return st.row_pix == st.Wo && (st.out_S == 1 || (long long)st.Wo * st.Bp % 64 == 0);
+}
+bool keep_map(shflbw_tensor_map_t* kept, const PlaneMap& m) {
+    if (encode_map(m.base, m.rows, m.cols, m.pitch, kept->map) != SHFLBW_OK) return false;
+    kept->of = m.base; kept->rows = m.rows; kept->cols = m.cols; kept->pitch = m.pitch;
+    return true;
+}
+
 // Launch plan of one NHWC SpConv call, without its scratch pointers: kernel choice, grid, and
 // the scratch each side needs.  Two plans exist.
 //   positions out   relayout -> panel kernel with tokens in TMEM lanes, writing [position][F] in
@@ -970,13 +1009,16 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     PanelChoice ch;
     const bool panel_bias = bias && !planes && !st->staged_out;   // no later pass: the panel kernel's epilogue adds the bias
     const int gather = st->gather;
+    // (the state is the caller's: a residual that they took away, or a map that the copies' row ids cannot be read from)
+    const bool box = st->chain && st->box_res && st->residual && !((uintptr_t)st->residual_map & 15);
     const bool ok_kernel = panel_bias            ? lookup<shflbw::kPanelConv, true>(st->V, st->tokens_per_cta, &ch, gather)
                            : (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch, gather)
                            : st->variant == 1      ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch, gather)
                                                    : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, gather,
-                                                                                      st->variant != 2 ? 0 : st->residual ? 6 : st->stages, st->producer_warps);
+                                                                                      st->variant != 2 ? 0 : st->residual ? 6 : st->stages,
+                                                                                      st->producer_warps, box);
     if (!ok_kernel) return SHFLBW_ERR_INVALID_ARG;
-    if (panel_bias) {                                       // (init allowed the kernel without; before anything is launched)
+    if (panel_bias || (st->box_res && !box)) {              // (init allowed the other kernel; before anything is launched)
         const int rc = allow_smem(ch.fn, ch.smem);
         if (rc != SHFLBW_OK) return rc;
     }
@@ -991,10 +1033,8 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     p.stride = st->stride / step;
     p.row_pix = st->row_pix;
     if (gather == shflbw::kGatherTma) {
-        // One row per pixel a tap of output pixel (0, 0) reads, `pitch` from one to the next, as long as from output
-        // pixel (0, 0) to the last: every address that the map allows is inside the staged input.
-        const int rc = encode_map(p.Xs, ((long long)st->C - 1) * Hp * Wp + (long long)(st->R - 1) * Wp + st->S,
-                                  (((long long)st->Ho - 1) * p.stride * Wp + ((long long)st->Wo - 1) * p.stride + 1) * st->Bp, 2ll * st->Bp, p.tmap_b);
+        const PlaneMap m = input_map(*st, p.Xs, Hp, Wp, p.stride);
+        const int rc = encode_map(m.base, m.rows, m.cols, m.pitch, st->map_in, p.tmap_b);
         if (rc != SHFLBW_OK) return rc;
     }
     long long relayout_per_sm = 0;
@@ -1016,6 +1056,12 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
         const int OHp = st->Ho + st->out_R - 1;
         p.OWp = st->Wo + st->out_S - 1; p.oph = st->out_R / 2; p.opw = st->out_S / 2;
         p.out_plane = OHp * p.OWp * st->Bp; p.relu = st->relu;
+        if (box) {
+            if (!boxes_fit(*st)) return SHFLBW_ERR_INVALID_ARG;
+            const PlaneMap m = output_map(*st, st->residual);
+            const int rc = encode_map(m.base, m.rows, m.cols, m.pitch, st->map_res, p.tmap_res);
+            if (rc != SHFLBW_OK) return rc;
+        }
     } else if (planes) {
         p.OWp = st->Wo; p.oph = 0; p.opw = 0; p.out_plane = st->Ho * st->Wo * st->Bp;
         p.out_logical = 1;                                   // plane index = logical channel
@@ -1169,11 +1215,13 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, f->brow, row_blocks, padded_cols,
                                       rows_in_lanes(f->brow, is_deep(padded_cols, row_blocks)), true);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
+    out->gather = ct.gather; out->row_pix = ct.row_pix;
     int rc = pick_panel<shflbw::kPanelConvChain>(f->brow, counted, row_blocks, padded_cols, &ch, false, ct.gather);
     if (rc != SHFLBW_OK) return rc;
+    if (ch.gather == shflbw::kGatherTma && !keep_map(&out->map_in, input_map(*out, in_chain, Hin + f->R - 1, Win + f->S - 1, stride))) return SHFLBW_ERR_CUDA;
     out->kernel = SHFLBW_KERNEL_TCGEN05;
     out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
-    out->gather = ch.gather; out->row_pix = ct.row_pix;
+    out->gather = ch.gather;
     out->tiles_n = (int)((counted + ch.tokens - 1) / ch.tokens);
     out->num_items = out->tiles_n * row_blocks;
     const int sms = sm_count();
@@ -1205,14 +1253,22 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
             if (map_host[i] < 0 || map_host[i] >= st->F) return SHFLBW_ERR_BAD_FORMAT;
     // The sixteen-epilogue-warp kernel copies the residual an item ahead, which pays up to two stages of
     // columns per block (14x14x256 -> 1024 with residual, batch 128, 112 columns: 33.9 -> 26.5 us); without a
-    // residual the limit is one stage (pick_panel).
+    // residual the limit is one stage (pick_panel).  Where the residual's rows come in whole boxes the copy engine
+    // fetches them (by cp.async and by TMA, 51 columns a block or fewer, back to back: 56x56x64 -> 256, batch 256 183 and
+    // 158 us, 118 73.1 and 70.0, 64 40.7 and 39.2; 14x14x256 -> 1024, batch 256 47.7 and 41.3, 118 23.8 and 21.4;
+    // 28x28x128 -> 512, batch 256 87.5 and 84.0 in the network, 84.0 and 87.1 alone, 118 39.3 and 36.9; 7x7x512 -> 2048, 256
+    // 27.3 and 26.4; a network of batch 256 2427 and 2298, 64 759 and 745, 32 501 and 499), with three gather warps.
     PanelChoice ch;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
     const bool two_warps = padded_cols <= 48ll * (st->F / st->V) && (long long)st->F * st->Ho * st->Wo * st->Bp * 2 <= (256ll << 20);   // (lookup)
+    const char* eb = getenv("SHFLBW_BOX");                   // 0: residual by cp.async (tuning aid)
+    const bool box = st->gather == shflbw::kGatherTma && boxes_fit(*st) && !(eb && atoi(eb) == 0);
     const bool wide = (st->variant == 2 ||
                        (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
                         padded_cols <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count())) &&
-                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6, two_warps ? 2 : 3);
+                      lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6, two_warps ? 2 : 3, box);
+    shflbw_tensor_map_t map_res{};
+    if (wide && box && !keep_map(&map_res, output_map(*st, res_chain))) return SHFLBW_ERR_CUDA;
     if (wide) {
         const int rc = allow_smem(ch.fn, ch.smem);
         if (rc != SHFLBW_OK) return rc;
@@ -1234,6 +1290,8 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     // Nothing can fail from here on: a refused call leaves the state as it was.
     st->residual = res_chain;
     st->residual_map = map_dev;
+    st->map_res = map_res;
+    st->box_res = wide && box;
     if (wide) {
         st->variant = 2; st->stages = ch.stages; st->producer_warps = ch.pw; st->block_x = ch.threads; st->shared_mem_size = ch.smem;
     }
