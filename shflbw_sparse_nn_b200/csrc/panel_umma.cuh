@@ -1070,20 +1070,30 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             }
             const bool use_c = MODE == kPanelSpmm && (EW == 8 || BIAS || Cfg::RES_BYTES > 0) && p.beta != 0.0f && p.C != nullptr;
             if constexpr (ROWS_OUT) {
-            // SpMM: thread = token, accumulator columns = the block's output rows.  For a fixed
-            // row a warp's 32 tokens are only 64 contiguous bytes of D, and storing them straight
-            // from registers is one 2-byte-per-lane store per row.  Instead each chunk of 32 rows
-            // goes through a tile in shared memory as 16 row PAIRS x 32 tokens of half2 (one
-            // packed conversion, one multiply and one 4-byte conflict-free write per pair) and
-            // comes back as 16-byte pieces: a lane reads 8 tokens of a pair (two 16-byte reads,
-            // the 16-byte units of odd pairs swapped so that a quarter warp covers all banks),
-            // splits them into the pair's two rows with byte permutes and stores 16 bytes of
-            // each; four lanes store one row's 64 bytes, eight rows per store instruction.  The
-            // inverse row permutation is the row index of those stores.
-            uint32_t* my_tile = (uint32_t*)(smem + Cfg::PIPE_BYTES + warp * 2048);
+            // TMEM lanes are tokens, accumulator columns the block's output rows.  For a fixed row a
+            // warp's 32 tokens are only 64 contiguous bytes of D, so each chunk of 32 rows is transposed
+            // through a tile in shared memory and comes back as 16-byte pieces: four lanes store one
+            // row's 64 bytes, eight rows per store instruction.  The inverse row permutation is the row
+            // index of those stores.
+            //   64 and 128 rows (TILES): the chunk leaves TMEM as 8 x 8 tiles, which stmatrix writes,
+            // transposed, as [row][32 tokens] (the 16-byte chunk c of row r at c ^ (r / 2 % 4): no bank
+            // conflicts either way).
+            //   16 and 32 rows: 16 row PAIRS x 32 tokens of half2, thread = token (one packed conversion,
+            // one multiply and one 4-byte conflict-free write per pair); a lane reads 8 tokens of a pair
+            // (two 16-byte reads, the 16-byte units of odd pairs swapped so that a quarter warp covers all
+            // banks) and splits them into the pair's two rows with byte permutes.
+            // Pairs and tiles, us: SpMM 4096x512x8192, V = 64, 51 columns a block 20.4 and 18.9, 4096x1024x4096 12.6 and
+            // 11.7; chained 56x56x64 -> 64, 3x3, batch 256 38.2 and 36.8; V = 128, 28x28x128 -> 256, batch 64, with
+            // residual 14.5 and 13.7, batch 8 5.1 and 4.35 (its TMA kernel does not spill any more); V = 32,
+            // 11008x4096x512 32.7 and 33.2, 256x256x256 2.78 and 2.93; V = 16, 3072x768x1000 14.5 and 14.9.
+            constexpr bool TILES = V >= 64;
+            uint8_t* const my_tile = smem + Cfg::PIPE_BYTES + warp * 2048;
             const int tg = lane & 3;                                    // 8-token group stored by this lane
-            // Slot j = 2i + h of a chunk is row 16i + 2*(lane/4) + h: pair 8i + lane/4, half h.
-            auto slot_row = [&](int j) { return 16 * (j >> 1) + 2 * (lane >> 2) + (j & 1); };
+            // stmatrix: lane 8 k + j names tokens 8 k.. of row 8 i + j
+            const uint32_t st_off = sm100::smem_u32(my_tile) + (uint32_t)((lane & 7) * 64 + (((lane >> 3) ^ ((lane >> 1) & 3)) << 4));
+            const uint8_t* const piece = my_tile + (lane >> 2) * 64 + ((tg ^ ((lane >> 3) & 3)) << 4);
+            // Row of a chunk that this lane's j-th piece is of (pairs: j = 2i + h is half h of pair 8i + lane/4).
+            auto slot_row = [&](int j) { return TILES ? 8 * j + (lane >> 2) : 16 * (j >> 1) + 2 * (lane >> 2) + (j & 1); };
             constexpr int NSLOT = CW / 8;                               // rows stored per lane and chunk
             // This lane's 8-token group of an item whose tile starts at token n0_: is it inside N
             // (N % 8 == 0: a group is valid as a whole), and its element offset inside an output
@@ -1191,15 +1201,15 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                         roff[i] = (uint32_t)plane * (uint32_t)p.out_plane;           // stored (chained) or logical order
                     }
                 }
-                {
-                    uint32_t r[CW];                       // the chunk's accumulator columns of this token
+                if constexpr (TILES) {
+                    uint32_t lo[CW / 2], hi[CW / 2];      // the chunk's columns of lanes 0-15 and 16-31 of the quadrant
                     if (has_k && reads) {
-                        if constexpr (CW == 32) sm100::tmem_ld_32x32b_x32(acc_base + cc, r);
-                        else sm100::tmem_ld_32x32b_x16(acc_base + cc, r);
+                        sm100::tmem_ld_16x256b(acc_base + cc, lo);
+                        sm100::tmem_ld_16x256b(acc_base + (16u << 16) + cc, hi);
                         sm100::tmem_ld_wait();
                     } else {
 #pragma unroll
-                        for (int e = 0; e < CW; ++e) r[e] = 0u;
+                        for (int e = 0; e < CW / 2; ++e) lo[e] = hi[e] = 0u;
                     }
                     if (cc + CW >= COLS) {  // last TMEM read of this item by this warp: release the buffer
                         sm100::tc_fence_before_sync();
@@ -1209,10 +1219,36 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     // Same epilogue arithmetic as the reference: round to fp16, then alpha (and
                     // beta * C, applied after the transpose) in fp16.
 #pragma unroll
+                    for (int i = 0; i < NSLOT; ++i) {     // rows 8 i..: four tiles of eight tokens
+                        __half2 h[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            const uint32_t* r = (k < 2 ? lo : hi) + 4 * i + 2 * (k & 1);
+                            h[k] = __floats2half2_rn(__uint_as_float(r[0]), __uint_as_float(r[1]));
+                            if (!use_c) h[k] = __hmul2(h[k], alpha2);
+                        }
+                        sm100::stmatrix_x4_trans(st_off + i * 512, *(uint32_t*)&h[0], *(uint32_t*)&h[1], *(uint32_t*)&h[2], *(uint32_t*)&h[3]);
+                    }
+                } else {
+                    uint32_t r[CW];                       // the chunk's accumulator columns of this token
+                    if (has_k && reads) {
+                        if constexpr (CW == 32) sm100::tmem_ld_32x32b_x32(acc_base + cc, r);
+                        else sm100::tmem_ld_32x32b_x16(acc_base + cc, r);
+                        sm100::tmem_ld_wait();
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < CW; ++e) r[e] = 0u;
+                    }
+                    if (cc + CW >= COLS) {
+                        sm100::tc_fence_before_sync();
+                        __syncwarp();
+                        if (lane == 0) sm100::mbar_arrive(&acc_empty[b]);
+                    }
+#pragma unroll
                     for (int q = 0; q < CW / 2; ++q) {
                         __half2 h = __floats2half2_rn(__uint_as_float(r[2 * q]), __uint_as_float(r[2 * q + 1]));
                         if (!use_c) h = __hmul2(h, alpha2);
-                        my_tile[q * 32 + (lane ^ ((q & 1) << 2))] = *(uint32_t*)&h;
+                        ((uint32_t*)my_tile)[q * 32 + (lane ^ ((q & 1) << 2))] = *(uint32_t*)&h;
                     }
                 }
                 __syncwarp();
@@ -1225,18 +1261,23 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                 }
                 if constexpr (BIAS && !IN_REGS) { if (need_add) fetch_addend(blk, goff, cc, addend[0]); }
                 {
+                    uint4 w0, w1;                            // pairs: 8 tokens of a row pair
 #pragma unroll
-                    for (int k = 0; k < NSLOT / 2; ++k) {
-                        const int q = 8 * k + (lane >> 2);   // 8 tokens of this lane's k-th row pair
-                        const uint32_t* src = my_tile + q * 32;
-                        const uint4 w0 = *(const uint4*)(src + (((2 * tg) ^ (q & 1)) << 2));
-                        const uint4 w1 = *(const uint4*)(src + (((2 * tg + 1) ^ (q & 1)) << 2));
-#pragma unroll
-                    for (int i = 2 * k; i < 2 * k + 2; ++i) {
-                        const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;   // the pair's second / first row
+                    for (int i = 0; i < NSLOT; ++i) {
                         uint4 v;
-                        v.x = __byte_perm(w0.x, w0.y, sel); v.y = __byte_perm(w0.z, w0.w, sel);
-                        v.z = __byte_perm(w1.x, w1.y, sel); v.w = __byte_perm(w1.z, w1.w, sel);
+                        if constexpr (TILES) {
+                            v = *(const uint4*)(piece + i * 512);
+                        } else {
+                            if (i % 2 == 0) {
+                                const int q = 4 * i + (lane >> 2);
+                                const uint32_t* src = (const uint32_t*)my_tile + q * 32;
+                                w0 = *(const uint4*)(src + (((2 * tg) ^ (q & 1)) << 2));
+                                w1 = *(const uint4*)(src + (((2 * tg + 1) ^ (q & 1)) << 2));
+                            }
+                            const uint32_t sel = (i & 1) ? 0x7632u : 0x5410u;   // the pair's second / first row
+                            v.x = __byte_perm(w0.x, w0.y, sel); v.y = __byte_perm(w0.z, w0.w, sel);
+                            v.z = __byte_perm(w1.x, w1.y, sel); v.w = __byte_perm(w1.z, w1.w, sel);
+                        }
                         if (ok_g) {
                             const size_t off = (size_t)roff[i] + (size_t)goff;
                             if (use_c) {
@@ -1259,7 +1300,6 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                             }
                             *(uint4*)(obase + off) = v;
                         }
-                    }
                     }
                 }
                 if constexpr (RES_AHEAD) { if (ahead) copy_addend(blk_next, goff_next, ok_next, ch); }
