@@ -235,15 +235,7 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
             default: break;
         }
         if (V == 128 && tile == 128) { *out = regular<128, 1, 6, MODE, BIAS>(gather); return true; }   // 32 KB
-        if (V == 128 && tile == 256) {                                                                 // 48 KB
-            if constexpr (MODE == shflbw::kPanelConvChain) {
-                if (gather == shflbw::kGatherTma) return false;   // (conv_tokens)
-                *out = choice<128, 2, 64, 4, 8, MODE>();
-            } else {
-                *out = regular<128, 2, 4, MODE, BIAS>(gather);
-            }
-            return true;
-        }
+        if (V == 128 && tile == 256) { *out = regular<128, 2, 4, MODE, BIAS>(gather); return true; }   // 48 KB
         return false;
     }
 }
@@ -338,10 +330,12 @@ int pick_tile(long long n_tokens, int row_blocks) {
 // columns (V = 32, 40 columns: 9.45 and 8.95, 54: 4.3 and 3.9, 100: 4.0 and 4.6; V = 64 chained, 40: 4.07 and 3.99, 64: 4.4
 // and 4.6, 300: 5.5 and 6.3; V = 128, 40: 10.2 and 10.9, 300: 12.9 and 15.7).
 //   128 rows with tokens in lanes write the longest items of all.  Into NHWC, padding that fills the chip leaves no SM to
-// the passes around (10x10x24 -> 1792, batch 6, 98 -> 140 items: 10.0 and 11.3).  Chained, they gather by cp.async: beside
-// the TMA gather's operands their epilogue does not fit the 96 registers that 17 warps leave (28x28x256 -> 256, batch 128,
-// 13 columns a block: 17.2 and 18.3; 14x14x512 -> 1024, batch 64, with residual, 102 columns: 15.3 and 17.2), except for
-// one stage on few SMs (7x7x48 -> 384, batch 8, 32 columns: 4.3 and 4.1).
+// the passes around (10x10x24 -> 1792, batch 6, 98 -> 140 items: 10.0 and 11.3).  Chained, with a stage of columns and part of
+// a second one, whose few copies the TMA gather's longer way to the first bytes does not repay, they gather by cp.async
+// (28x28x256 -> 256, 3x3, batch 64, 100 columns 12.2 and 12.1 without and 15.6 and 15.7 with a residual; 14x14x1024 -> 512,
+// batch 32, 6.4 and 7.0, 7.5 and 7.8; batch 8, 28x28x256 -> 256, 4.9 and 5.2), and up to three stages where there are fewer
+// items than SMs or the rows are padded (27x27x256 -> 256, 3x3, batch 100, 157 columns, with residual: 34.1 and 36.1).  Otherwise TMA: 16 columns 10.9 and 10.1, 48 14.4 and 13.1 with a residual, 200 13.8 and 12.9, 800 29.5 and
+// 26.2, 2000 59.8 and 49.3 (28x28x256 -> 256, batch 64).
 struct ConvTokens { int row_pix; int gather; };
 ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int V, int row_blocks, long long padded_cols, bool rows, bool chain) {
     const ConvTokens plain{Wo, shflbw::kGatherCpAsync};
@@ -352,7 +346,9 @@ ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int V, int ro
     const long long rounds0 = rounds_of_items(before, tile0, row_blocks), rounds1 = rounds_of_items(after, tile1, row_blocks);
     const long long cost0 = rounds0 * (tile0 == 128 ? 2 : 3), cost1 = rounds1 * (tile1 == 128 ? 2 : 3);
     if (V == 128 && !rows) {
-        if (chain && (tile1 == 256 || padded_cols > 64ll * row_blocks)) return plain;
+        const bool few = (after + tile1 - 1) / tile1 * row_blocks <= (sm_count() > 0 ? sm_count() : 148);
+        if (chain && (few || row_pix != Wo ? tile1 == 256 || padded_cols > 64ll * row_blocks
+                          : padded_cols > 64ll * row_blocks && padded_cols <= 128ll * row_blocks)) return plain;
         if (!chain && 4 * after > 5 * before && rounds1 == 1 && 10 * ((after + tile1 - 1) / tile1 * row_blocks) > 9ll * (sm_count() > 0 ? sm_count() : 148))
             return plain;
     }
@@ -380,45 +376,17 @@ int allow_smem(const void* fn, size_t bytes) {
 }
 int allow_smem(PanelKernel fn, size_t bytes) { return allow_smem((const void*)fn, bytes); }
 
+// The kernel of a plan, allowed its shared memory.  wide_ring: sixteen epilogue warps and that many stages (lookup), 0: eight.
 template <int MODE>
-int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols, PanelChoice* out, bool addend = false,
-               int gather = shflbw::kGatherTma) {
-    int tile = pick_tile(n_tokens, row_blocks);
-    if constexpr (MODE != shflbw::kPanelSpmm && MODE != shflbw::kPanelConv) {
-        if (V == 16) tile = 128;   // chained layers: the only shape built for 16-row blocks
-    }
-    // SpMM and chained SpConv with V = 64 / 128 can run with the operands swapped (rows in TMEM
-    // lanes, one MMA per 16 columns for the whole token tile).
-    bool swapped = false;
-    if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
-        // From three stages of non-zero columns per block on (is_deep): with fewer an item is mostly epilogue, and
-        // lanes that hold a row each store, and read a residual, in pieces of 64 bytes.  The line was drawn when an MMA
-        // took 54 clk of issue whatever its shape, which rows in lanes halve.  With elected issue, tokens and rows in
-        // lanes, V = 64: SpMM 4096x1024x4096, 48 columns a block 12.5 and 11.9 us, 64 15.8 and 12.7, 176 17.9 and 15.7,
-        // 256 19.6 and 19.0 (1000 columns of B: within 5 %); chained 28x28x256 -> 256, batch 64, L2 warm, 48 columns 10.9
-        // and 15.4, 192 17.7 and 22.0, 400 22.7 and 26.2, 768 34.8 and 37.3, with a residual 38.0 and 43.9 (V = 128, 768
-        // columns: 29.5 and 27.6).  So SpMM would gain from 64 columns on, and chained layers lose up to about 800.
-        if (rows_in_lanes(V, is_deep(padded_cols, row_blocks)))
-            swapped = MODE == shflbw::kPanelSpmm ? lookup<shflbw::kPanelSpmmRows>(V, tile, out, gather)
-                                                 : lookup<shflbw::kPanelConvChainRows>(V, tile, out, gather);
-    }
-    // Tokens in lanes with at most 64 non-zero columns per block on average, where an item is all epilogue, and several
-    // items per SM: sixteen epilogue warps (chained 28x28x256 -> 256, batch 128, eight and sixteen: 26 columns 18.7 and
-    // 15.1 us, 64 19.2 and 17.9, 96 21.3 and 21.1, 128 21.9 and 23.0; SpMM of the same size gains up to 128: 26.9 and
-    // 25.0).  SHFLBW_EPILOGUE_WARPS=8|16 forces the choice (tuning aid).
-    // Their ring: eight stages where nothing is added and a block takes two stages, which a ring of six holds for
-    // three items only (28x28x128 -> 512, batch 256, no residual, 40 columns: 56.6 us with six, 54.7 with eight); blocks
-    // of one stage are as fast with six (26 columns: 48.5, with eight 49.7).
-    bool wide = false;
-    if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConvChain) {
-        wide = !swapped && tile == 256 && V == 64 && padded_cols <= 64ll * row_blocks &&
-               (n_tokens + 255) / 256 * row_blocks >= 4ll * (sm_count() > 0 ? sm_count() : 148);
-        if (const char* e = getenv("SHFLBW_EPILOGUE_WARPS")) wide = !swapped && tile == 256 && V == 64 && atoi(e) == 16;
-    }
-    const int wide_ring = !wide ? 0 : !addend && padded_cols > 32ll * row_blocks ? 8 : 6;
-    if (wide && MODE == shflbw::kPanelSpmm) gather = shflbw::kGatherTma;   // (built for it only)
-    if (!swapped && !lookup<MODE>(V, tile, out, gather, wide_ring)) return SHFLBW_ERR_UNSUPPORTED;
-    out->variant = swapped ? 1 : wide ? 2 : 0;
+int pick_panel(int V, int tile, bool rows, int wide_ring, int gather, PanelChoice* out) {
+    if constexpr (MODE == shflbw::kPanelSpmm) { if (wide_ring) gather = shflbw::kGatherTma; }   // (built for it only)
+    bool found;
+    if (rows)
+        found = MODE == shflbw::kPanelSpmm ? lookup<shflbw::kPanelSpmmRows>(V, tile, out, gather) : lookup<shflbw::kPanelConvChainRows>(V, tile, out, gather);
+    else
+        found = lookup<MODE>(V, tile, out, gather, wide_ring);
+    if (!found) return SHFLBW_ERR_UNSUPPORTED;
+    out->variant = rows ? 1 : wide_ring ? 2 : 0;
     if (wide_ring == 8) {                    // a residual may be bound to the state later on
         PanelChoice with_addend;
         if (!lookup<MODE>(V, tile, &with_addend, gather, 6)) return SHFLBW_ERR_UNSUPPORTED;
@@ -426,6 +394,45 @@ int pick_panel(int V, long long n_tokens, int row_blocks, long long padded_cols,
         if (rc != SHFLBW_OK) return rc;
     }
     return allow_smem(out->fn, out->smem);
+}
+
+// Sixteen epilogue warps, tokens in lanes: SHFLBW_EPILOGUE_WARPS=8|16 forces the choice (tuning aid).
+bool wide_wanted(int V, int tile, bool pays) {
+    if (V != 64 || tile != 256) return false;
+    const char* e = getenv("SHFLBW_EPILOGUE_WARPS");
+    return e ? atoi(e) == 16 : pays;
+}
+// Their ring: eight stages where nothing is added and a block takes two stages, which a ring of six holds for
+// three items only (28x28x128 -> 512, batch 256, no residual, 40 columns: 56.6 us with six, 54.7 with eight); blocks
+// of one stage are as fast with six (26 columns: 48.5, with eight 49.7).
+int wide_ring_of(bool addend, long long padded_cols, int row_blocks) { return !addend && padded_cols > 32ll * row_blocks ? 8 : 6; }
+
+// Whether the rows of an SpMM's blocks lie in the TMEM lanes, and whether it runs with sixteen epilogue warps.  With rows in
+// lanes from three stages of non-zero columns per block on: with fewer an item is mostly epilogue.  The line was drawn when
+// an MMA took 54 clk of issue whatever its shape, which rows in lanes halve.
+bool spmm_rows(int V, long long padded_cols, int row_blocks) { return rows_in_lanes(V, is_deep(padded_cols, row_blocks)); }
+// At most 64 non-zero columns per block on average, where an item is all epilogue, and several items per SM.
+bool spmm_wide(int V, int tile, long long n_tokens, long long padded_cols, int row_blocks) {
+    return wide_wanted(V, tile, padded_cols <= 64ll * row_blocks && (n_tokens + 255) / 256 * row_blocks >= 4ll * (sm_count() > 0 ? sm_count() : 148));
+}
+
+// The same for chained layers, of `tokens` tokens counted with the padding of their rows.  Tokens in lanes, which write (and
+// read a residual) in runs of 64 bytes a row where rows in lanes scatter 16 bytes a lane, up to the depth where the MMA is
+// what an item waits for: at 64 rows two of 48 clk instead of one of 80 for the 256 tokens; at 128 rows it is 128 clk
+// either way.  Tokens and rows, us: V = 64, 28x28x256 -> 256, 3x3, batch 64: 256 columns 16.6 and 20.6 (with residual 20.7 and
+// 28.3), 800 35.4 and 36.9, 1200 49.0 and 48.2 (51.7 and 54.5), 2000 75.8 and 70.7 (78.4 and 76.6); 7x7x512 -> 512, batch 8,
+// 600 columns 6.2 and 6.3; V = 128: 400 17.1 and 20.9, 2000 49.3 and 48.9 (52.2 and 56.1).
+// Layers of fewer than 16 items, and those whose rows are no whole boxes of the TMA gather and go into an output with a halo
+// beside them, keep the line at three stages of columns.
+bool chain_rows(int V, bool padded_into_halo, long long items, long long padded_cols, int row_blocks) {
+    const bool deep = is_deep(padded_cols, row_blocks);
+    return rows_in_lanes(V, deep && (padded_into_halo || items < 16 || (V == 64 && padded_cols >= 1200ll * row_blocks)));
+}
+// At most 64 non-zero columns per block, and two or three items per SM (eight and sixteen, 13 / 40 / 60 columns: 2.7 items
+// 7.25 and 6.62 / 7.54 and 7.57 / 7.79 and 7.73, 3.6 8.6 and 7.6 / 9.1 and 8.8 / 9.2 and 9.0; 1.7 5.76 and 5.57 / 6.14 and 6.33 /
+// 6.32 and 6.33; 28x28x256 -> 256, batch 128, 64 columns 19.2 and 17.9, 96 21.3 and 21.1, 128 21.9 and 23.0).
+bool chain_wide(int V, int tile, long long items, long long padded_cols, int row_blocks) {
+    return wide_wanted(V, tile, padded_cols <= 64ll * row_blocks && 2 * items >= 5ll * (sm_count() > 0 ? sm_count() : 148));
 }
 
 // Argument and range checks shared by every NHWC SpConv entry point.  The kernels index the
@@ -587,8 +594,10 @@ static int plan_spmm(const shflbw_matrix_t* m, int N, const void* B, float alpha
     } else {
         PanelChoice ch;
         const long long padded_cols = m->kptr.empty() ? 0 : m->kptr.back();
-        int rc = pick_panel<shflbw::kPanelSpmm>(m->brow, N, out->num_row_blocks, padded_cols, &ch, beta != 0.f,
-                                                spmm_gather(m->ncol, N, out->num_row_blocks, padded_cols, pick_tile(N, out->num_row_blocks), with_bias));
+        const int blocks = out->num_row_blocks, tile = pick_tile(N, blocks);
+        const bool rows = spmm_rows(m->brow, padded_cols, blocks);
+        const int ring = !rows && spmm_wide(m->brow, tile, N, padded_cols, blocks) ? wide_ring_of(beta != 0.f, padded_cols, blocks) : 0;
+        int rc = pick_panel<shflbw::kPanelSpmm>(m->brow, tile, rows, ring, spmm_gather(m->ncol, N, blocks, padded_cols, tile, with_bias), &ch);
         if (rc != SHFLBW_OK) return rc;
         out->kernel = SHFLBW_KERNEL_TCGEN05;
         out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
@@ -944,8 +953,9 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, f->brow, row_blocks, padded_cols, planes, false);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
     PanelChoice ch;
-    rc = planes ? pick_panel<shflbw::kPanelConvChain>(f->brow, counted, row_blocks, 1ll << 40, &ch, false, ct.gather)
-                : pick_panel<shflbw::kPanelConv>(f->brow, counted, row_blocks, 0, &ch, false, ct.gather);
+    const int tile = pick_tile(counted, row_blocks);
+    rc = planes ? pick_panel<shflbw::kPanelConvChain>(f->brow, tile, true, 0, ct.gather, &ch)
+                : pick_panel<shflbw::kPanelConv>(f->brow, tile, false, 0, ct.gather, &ch);
     if (rc != SHFLBW_OK) return rc;
     if (planes) {
         out->variant = 1;
@@ -1216,7 +1226,11 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
                                       rows_in_lanes(f->brow, is_deep(padded_cols, row_blocks)), true);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
     out->gather = ct.gather; out->row_pix = ct.row_pix;
-    int rc = pick_panel<shflbw::kPanelConvChain>(f->brow, counted, row_blocks, padded_cols, &ch, false, ct.gather);
+    const int tile = pick_tile(counted, row_blocks);
+    const long long items = (counted + tile - 1) / tile * row_blocks;
+    const bool rows = chain_rows(f->brow, S_next > 1 && tma_row_pix(Wo, Win + f->S - 1, Bp, stride) > Wo, items, padded_cols, row_blocks);
+    const int ring = !rows && chain_wide(f->brow, tile, items, padded_cols, row_blocks) ? wide_ring_of(false, padded_cols, row_blocks) : 0;
+    int rc = pick_panel<shflbw::kPanelConvChain>(f->brow, tile, rows, ring, ct.gather, &ch);
     if (rc != SHFLBW_OK) return rc;
     if (ch.gather == shflbw::kGatherTma && !keep_map(&out->map_in, input_map(*out, in_chain, Hin + f->R - 1, Win + f->S - 1, stride))) return SHFLBW_ERR_CUDA;
     out->kernel = SHFLBW_KERNEL_TCGEN05;
@@ -1257,15 +1271,17 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     // fetches them (by cp.async and by TMA, 51 columns a block or fewer, back to back: 56x56x64 -> 256, batch 256 183 and
     // 158 us, 118 73.1 and 70.0, 64 40.7 and 39.2; 14x14x256 -> 1024, batch 256 47.7 and 41.3, 118 23.8 and 21.4;
     // 28x28x128 -> 512, batch 256 87.5 and 84.0 in the network, 84.0 and 87.1 alone, 118 39.3 and 36.9; 7x7x512 -> 2048, 256
-    // 27.3 and 26.4; a network of batch 256 2427 and 2298, 64 759 and 745, 32 501 and 499), with three gather warps.
+    // 27.3 and 26.4; a network of batch 256 2427 and 2298, 64 759 and 745, 32 501 and 499), with three gather warps, from six items
+    // per SM on; with fewer the slots' first laps are most of it (5.3 items per SM, 56x56x64 -> 256, batch 16: 12.1 and
+    // 12.5; 2.7, 28x28x128 -> 1024, batch 8, 60 columns: eight warps 9.38, sixteen by cp.async 9.02, by TMA 9.64).
     PanelChoice ch;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
     const bool two_warps = padded_cols <= 48ll * (st->F / st->V) && (long long)st->F * st->Ho * st->Wo * st->Bp * 2 <= (256ll << 20);   // (lookup)
     const char* eb = getenv("SHFLBW_BOX");                   // 0: residual by cp.async (tuning aid)
-    const bool box = st->gather == shflbw::kGatherTma && boxes_fit(*st) && !(eb && atoi(eb) == 0);
+    const bool box = st->gather == shflbw::kGatherTma && boxes_fit(*st) && (eb ? atoi(eb) != 0 : st->num_items >= 6ll * sm_count());
     const bool wide = (st->variant == 2 ||
                        (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
-                        padded_cols <= 128ll * (st->F / st->V) && st->num_items >= 4ll * sm_count())) &&
+                        padded_cols <= 128ll * (st->F / st->V) && 2ll * st->num_items >= 5ll * sm_count())) &&
                       lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6, two_warps ? 2 : 3, box);
     shflbw_tensor_map_t map_res{};
     if (wide && box && !keep_map(&map_res, output_map(*st, res_chain))) return SHFLBW_ERR_CUDA;

@@ -57,7 +57,8 @@ def test_box_residual_equals_cp_async_residual(Bn, H, R_next, F, density, mapped
     assert np.array_equal(got["0"], got["1"])
 
 
-def test_exchanged_and_removed_residuals_are_followed():
+def test_exchanged_and_removed_residuals_are_followed(monkeypatch):
+    monkeypatch.setenv("SHFLBW_BOX", "1")
     Bn, H, F = 64, 24, 256
     f = sb.BlockwiseSpFilter().init_random(F, 1, 1, 64, 64, 1, 0.3, True, 5, values="uniform")
     f.transform_and_sync_device()
@@ -89,6 +90,7 @@ def test_wait_limit_runs_out_beside_a_box_residual(monkeypatch):
     monkeypatch.setenv("SHFLBW_SWAP", "0")
     monkeypatch.setenv("SHFLBW_EPILOGUE_WARPS", "16")
     monkeypatch.setenv("SHFLBW_TILE", "256")
+    monkeypatch.setenv("SHFLBW_BOX", "1")
     flib = _cabi.load_library(build_fault_inject_library())
     flib.shflbw_debug_withhold_arrivals_from.restype = C.c_int
     flib.shflbw_debug_withhold_arrivals_from.argtypes = [C.c_int]
