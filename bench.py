@@ -450,7 +450,7 @@ def bench_spconv(sb, torch, dist, pk, steps=300, warmup=20, use_graph=True):
             "nonzero_tflops": round(dist.world * flops / t / 1e12, 3),
             "dense_equivalent_tflops": round(dist.world * 2.0 * npix * c["C"] * c["R"] * c["S"] * c["F"] / t / 1e12, 2),
             "launches_per_call": ops[0].launches_per_exec,
-            "plan": "planes out (filters in TMEM lanes) + transpose" if st.variant == 1 else "positions out (tokens in TMEM lanes)",
+            "plan": f"planes out ({'filters' if st.rows else 'tokens'} in TMEM lanes) + transpose" if st.variant == 1 else "positions out (tokens in TMEM lanes)",
             "launch": (f"CUDA graph of {G} calls" if G else "host launches"), "repeats": R,
             "t_roof_us": round(t_roof * 1e6, 3), "roofline_frac": round(t_roof / t, 4), "algorithmic_bytes": byt, "nnzb": f.nnzb,
             "launch_shares_ncu": ncu_spconv_shares() if st.variant == 1 else None}

@@ -250,8 +250,8 @@ typedef struct shflbw_spconv_state {
     int tokens_per_cta;
     int stages;
     int producer_warps;
-    int variant;             /* 0: tokens in TMEM lanes; 1: filters in TMEM lanes (NHWC calls: planes out + transpose);
-                                2: as 0 with 16 epilogue warps (chained layers) */
+    int variant;             /* chained layers 0: tokens in TMEM lanes; 1: filters in TMEM lanes; 2: as 0 with 16 epilogue
+                                warps.  NHWC calls 0: positions out; 1: planes out + transpose */
     int num_items, tiles_n;
     unsigned grid_x, grid_y, block_x;
     size_t shared_mem_size;
@@ -278,6 +278,8 @@ typedef struct shflbw_spconv_state {
     int gather;              /* 0: cp.async gather, 1: TMA tile-gather                     */
     int row_pix;             /* pixels that an output row counts as (>= Wo; the TMA gather may round rows up to whole
                                 boxes): tiles_n and num_items are of Ho * row_pix * Bp tokens */
+    int rows;                /* 1: filters in TMEM lanes, 0: tokens                        */
+    int wide;                /* 1: sixteen epilogue warps                                  */
     int box_res;             /* chained layers: 1 = the residual arrives in boxes of 64 tokens by TMA */
     shflbw_tensor_map_t map_in, map_res; /* chained layers: input and residual planes */
 } shflbw_spconv_state_t;

@@ -65,7 +65,7 @@ class SpconvState(C.Structure):
         ("chain", C.c_int), ("out_R", C.c_int), ("out_S", C.c_int), ("relu", C.c_int),
         ("residual", C.c_void_p), ("residual_map", C.c_void_p),
         ("gather", C.c_int), ("row_pix", C.c_int),
-        ("box_res", C.c_int), ("map_in", TensorMap), ("map_res", TensorMap),
+        ("rows", C.c_int), ("wide", C.c_int), ("box_res", C.c_int), ("map_in", TensorMap), ("map_res", TensorMap),
     ]
 
 

@@ -898,18 +898,33 @@ bool keep_map(shflbw_tensor_map_t* kept, const PlaneMap& m) {
     return true;
 }
 
+// Whether an NHWC call of a permuted filter is computed as planes (below): they leave the panel kernel in runs of 64 bytes,
+// the inverse permutation being an address, and the transposing pass reads and writes runs of 128.  Positions out and planes
+// out (tokens in lanes), 40 / 110 / 460 columns a block: 14x14x512 -> 2048, 3x3, batch 16, V = 64 17.6 and 15.7 / 18.6 and 16.7 /
+// 26.6 and 24.5; 14x14x256 -> 1024 15.4 and 12.1 / 16.8 and 13.5 / 21.3 and 18.0; 56x56x64 -> 64, batch 32 20.4 and 17.7 /
+// 21.7 and 19.4 / 27.8 and 24.6; V = 128 12 to 22 % less.  Not where the planes carry an eighth more images than there are
+// (28x28x256 -> 512, batch 1, 160 columns: 12.6 and 13.3), with less than an item of 256 tokens per SM (17x17x512 -> 256, 1x1,
+// batch 24, 74 columns: 12.1 and 13.4; 14x14x256 -> 512, batch 8, 460: 10.8 and 11.1), nor for less than a stage of columns
+// with padded rows (not looked at).  An unpermuted filter's positions need no further pass (28x28x256 -> 256, 1x1, batch 64,
+// 64 columns: 20.7, as planes 31.4; 14x14x512 -> 2048, 3x3, batch 16, 900: 29.0 and 33.2).
+// With filters in lanes (28.3 instead of 24.5 for 14x14x512 -> 2048, 460 columns) only at 64 rows from 1200 columns on, as
+// the chained layers (14x14x256 -> 1024, 1800 columns: 33.4, tokens 33.8).
+bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long items, bool padded_rows, long long padded_cols, int row_blocks) {
+    return f.row_permute && tile == 256 && items >= (sm_count() > 0 ? sm_count() : 148) && 8 * (Bp - B) <= Bp &&
+           (padded_cols >= 64ll * row_blocks || !padded_rows);
+}
+
 // Launch plan of one NHWC SpConv call, without its scratch pointers: kernel choice, grid, and
 // the scratch each side needs.  Two plans exist.
 //   positions out   relayout -> panel kernel with tokens in TMEM lanes, writing [position][F] in
 //                   stored filter order -> (with a filter permutation) unpermute_filters.
-//   planes out      relayout -> panel kernel with the filters in TMEM lanes, writing the output
-//                   as planes [F][Ho][Wo][Bp] with plane = LOGICAL channel (the permutation is
-//                   the row index of its stores, free) -> planes_to_nhwc transposes the planes
-//                   to NHWC.  Used for V = 64 / 128 filters with enough non-zero columns per
-//                   block: one MMA per 16 columns covers the whole token tile.
+//   planes out      relayout -> panel kernel writing the output as planes [F][Ho][Wo][Bp] with plane = LOGICAL
+//                   channel (the permutation is the row index of its stores, free) -> planes_to_nhwc
+//                   transposes the planes to NHWC.  Used for permuted V = 64 / 128 filters and outputs that
+//                   fill the chip (conv_planes), with tokens or, where deep, filters in TMEM lanes.
 // SHFLBW_CONV_PLANES=0|1 forces the choice (tuning aid).
 int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const void* ifmap, void* ofmap,
-              float alpha, int kernel, shflbw_spconv_state_t* out) {
+              float alpha, int kernel, shflbw_spconv_state_t* out, size_t scratch_limit = ~(size_t)0) {
     std::memset(out, 0, sizeof *out);
     if (check_kernel_arg(kernel) != SHFLBW_OK) return SHFLBW_ERR_INVALID_ARG;
     ConvShape cs;
@@ -940,22 +955,27 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
 
     // planes out?
     const bool planes_possible = (f->brow == 64 || f->brow == 128) && f->F / 64 <= 65535 &&
-                                 (long long)f->F * tokens < (1ll << 32) - 1;
-    bool planes = is_deep(padded_cols, row_blocks);         // the chained layers' rule (14x14x256 -> 1024, 3x3, batch 16, V = 64,
-                                                            // 112 columns a block, positions and planes: 16.8 and 14.8 us,
-                                                            // 192 17.3 and 15.0; 28x28x256 -> 256, 1x1, batch 64: 37.5 and
-                                                            // 38.7, 39.6 and 40.2)
-    if (const char* e = getenv("SHFLBW_CONV_PLANES")) planes = atoi(e) != 0;
-    planes = planes && planes_possible && rows_in_lanes(f->brow, true);
-
+                                 (long long)f->F * tokens < (1ll << 32) - 1 && rows_in_lanes(f->brow, true);
+    const char* ep = getenv("SHFLBW_CONV_PLANES");
     // the input as the panel kernel sees it: a strided 1x1 filter's pixels are staged side by side
     const bool compact = f->R == 1 && f->S == 1;
-    const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, f->brow, row_blocks, padded_cols, planes, false);
+    const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, f->brow, row_blocks, padded_cols,
+                                      planes_possible && (ep ? atoi(ep) != 0 : is_deep(padded_cols, row_blocks)), false);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
-    PanelChoice ch;
     const int tile = pick_tile(counted, row_blocks);
-    rc = planes ? pick_panel<shflbw::kPanelConvChain>(f->brow, tile, true, 0, ct.gather, &ch)
-                : pick_panel<shflbw::kPanelConv>(f->brow, tile, false, 0, ct.gather, &ch);
+    const long long items = (counted + tile - 1) / tile * row_blocks;
+    // (planes of up to an eighth more images than positions have: not where a fixed scratch holds only these)
+    const bool planes_fit = (size_t)cs.staged_elems * 2 + 256 + (size_t)f->F * (size_t)tokens * 2 + 256 <= scratch_limit;
+    const bool planes = planes_possible && planes_fit && (ep ? atoi(ep) != 0 : conv_planes(*f, B, Bp, tile, items, ct.row_pix != Wo, padded_cols, row_blocks));
+    PanelChoice ch;
+    if (planes) {
+        const int ring = chain_wide(f->brow, tile, items, padded_cols, row_blocks) ? wide_ring_of(false, padded_cols, row_blocks) : 0;
+        out->rows = f->brow == 64 && padded_cols >= 1200ll * row_blocks;
+        rc = pick_panel<shflbw::kPanelConvChain>(f->brow, tile, out->rows, out->rows ? 0 : ring, ct.gather, &ch);
+        out->wide = !out->rows && ring;
+    } else {
+        rc = pick_panel<shflbw::kPanelConv>(f->brow, tile, false, 0, ct.gather, &ch);
+    }
     if (rc != SHFLBW_OK) return rc;
     if (planes) {
         out->variant = 1;
@@ -1023,9 +1043,9 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     const bool box = st->chain && st->box_res && st->residual && !((uintptr_t)st->residual_map & 15);
     const bool ok_kernel = panel_bias            ? lookup<shflbw::kPanelConv, true>(st->V, st->tokens_per_cta, &ch, gather)
                            : (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch, gather)
-                           : st->variant == 1      ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch, gather)
+                           : st->rows              ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch, gather)
                                                    : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, gather,
-                                                                                      st->variant != 2 ? 0 : st->residual ? 6 : st->stages,
+                                                                                      !st->wide ? 0 : st->residual ? 6 : st->stages,
                                                                                       st->producer_warps, box);
     if (!ok_kernel) return SHFLBW_ERR_INVALID_ARG;
     if (panel_bias || (st->box_res && !box)) {              // (init allowed the other kernel; before anything is launched)
@@ -1235,7 +1255,7 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     if (ch.gather == shflbw::kGatherTma && !keep_map(&out->map_in, input_map(*out, in_chain, Hin + f->R - 1, Win + f->S - 1, stride))) return SHFLBW_ERR_CUDA;
     out->kernel = SHFLBW_KERNEL_TCGEN05;
     out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
-    out->gather = ch.gather;
+    out->gather = ch.gather; out->rows = rows; out->wide = ch.variant == 2;
     out->tiles_n = (int)((counted + ch.tokens - 1) / ch.tokens);
     out->num_items = out->tiles_n * row_blocks;
     const int sms = sm_count();
@@ -1309,7 +1329,7 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     st->map_res = map_res;
     st->box_res = wide && box;
     if (wide) {
-        st->variant = 2; st->stages = ch.stages; st->producer_warps = ch.pw; st->block_x = ch.threads; st->shared_mem_size = ch.smem;
+        st->variant = 2; st->wide = 1; st->stages = ch.stages; st->producer_warps = ch.pw; st->block_x = ch.threads; st->shared_mem_size = ch.smem;
     }
     return SHFLBW_OK;
 }
@@ -1320,7 +1340,7 @@ int shflbw_spconv_exec_static_scratch(const shflbw_matrix_t* f, int B, int Hin, 
     // unpermuted filter the output can bypass the array, so its capacity alone would not bound
     // the output offsets); only the scratch comes from somewhere else.
     shflbw_spconv_state_t st;
-    int rc = plan_conv(f, B, Hin, Win, stride, ifmap, ofmap, alpha, SHFLBW_KERNEL_TCGEN05, &st);
+    int rc = plan_conv(f, B, Hin, Win, stride, ifmap, ofmap, alpha, SHFLBW_KERNEL_TCGEN05, &st, SHFLBW_STATIC_SCRATCH_BYTES);
     if (rc != SHFLBW_OK) return rc;
 
     // Capacity check first: nothing is launched when the shape does not fit.

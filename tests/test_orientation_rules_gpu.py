@@ -6,6 +6,7 @@ import torch
 
 import shflbw_sparse_nn_b200 as sb
 from gpu_util import dev, host, operand_swap
+from shflbw_sparse_nn_b200 import _cabi
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +58,68 @@ def test_chained_layers(V, Bn, H, Cc, R, stride, R_next, cols, variant, gather, 
         assert (st.variant, st.gather) == (swap, 0)
         assert np.array_equal(got, other)
     assert np.abs(got.view(np.float16).astype(np.float32)).max() > 0
+
+
+@pytest.mark.parametrize("V,Bn,H,Cc,F,R,stride,cols,permute,variant,rows,wide", [
+    (64, 16, 14, 128, 1024, 3, 1, 230, True, 1, 0, 0),     # planes, tokens in lanes
+    (64, 16, 14, 256, 1024, 3, 1, 1300, True, 1, 1, 0),    # ... filters in lanes
+    (64, 31, 24, 64, 512, 1, 1, 20, True, 1, 0, 1),        # ... sixteen epilogue warps, a padding image
+    (64, 31, 24, 64, 512, 1, 1, 40, True, 1, 0, 1),
+    (128, 16, 14, 128, 2048, 3, 1, 100, True, 1, 0, 0),
+    (64, 8, 28, 64, 512, 3, 1, 40, True, 0, 0, 0),         # less than a stage of columns, padded rows: positions
+    (64, 9, 28, 64, 512, 1, 1, 40, True, 0, 0, 0),         # nine images in sixteen
+    (64, 8, 14, 128, 512, 3, 1, 230, True, 0, 0, 0),       # fewer items than SMs
+    (64, 16, 14, 128, 1024, 3, 1, 230, False, 0, 0, 0),    # nothing to permute
+    (128, 16, 28, 256, 2048, 3, 2, 230, True, 1, 0, 0),
+])
+def test_nhwc_calls(V, Bn, H, Cc, F, R, stride, cols, permute, variant, rows, wide, monkeypatch):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the item counts are of 148 SMs")
+    f = sb.BlockwiseSpFilter().init_random(F, R, R, Cc, V, 1, (cols + 0.5) / (R * R * Cc), permute, 5, values="uniform")
+    f.transform_and_sync_device()
+    x = dev(sb.uniform_half(3, Bn * H * H * Cc).reshape(Bn, H, H, Cc))
+    bias = dev(sb.uniform_half(4, F))
+    Ho = -(-H // stride)
+    got = {}
+    for planes in (None, "0", "1"):
+        if planes:
+            monkeypatch.setenv("SHFLBW_CONV_PLANES", planes)
+        y = torch.full((Bn, Ho, Ho, F), float("nan"), dtype=torch.float16, device="cuda")
+        op = sb.SpconvBlockwiseOp().initialize(f, Bn, H, H, stride, x, y, 0.25)
+        st = op._state
+        if planes:
+            assert st.variant == int(planes)
+        else:
+            assert (st.variant, st.rows, st.wide) == (variant, rows, wide)
+        out = []
+        for b in (None, bias):
+            op.run_with_bias(b, torch.cuda.current_stream())
+            torch.cuda.synchronize()
+            f.device_status()
+            out.append(host(y).view(np.uint16).copy())
+        got[planes] = out
+    for planes in ("0", "1"):
+        assert all(np.array_equal(a, b) for a, b in zip(got[None], got[planes]))
+    assert not np.array_equal(*got[None])
+
+
+def test_planes_that_do_not_fit_the_fixed_scratch_give_way_to_positions():
+    """Seven images, whose planes hold eight: at the smallest image whose planes are beyond the array the positions fit."""
+    H, Bn = 40, 7
+    f = sb.BlockwiseSpFilter().init_random(192, 1, 1, 8, 64, 1, 0.5, True, 9, values="uniform")
+    f.transform_and_sync_device()
+    need = lambda images: 2 * 8 * H * H * 8 + 2 * images * H * H * f.F
+    while need(8) <= _cabi.STATIC_SCRATCH_BYTES:
+        H += 1
+    assert need(7) + 512 <= _cabi.STATIC_SCRATCH_BYTES < need(8)
+    x = dev(sb.uniform_half(3, Bn * H * H * 8).reshape(Bn, H, H, 8))
+    y, want = (torch.full((Bn, H, H, f.F), float("nan"), dtype=torch.float16, device="cuda") for _ in range(2))
+    s = torch.cuda.current_stream()
+    rc = _cabi.lib().shflbw_spconv_exec_static_scratch(f._h, Bn, H, H, 1, x.data_ptr(), y.data_ptr(), 1.0, s.cuda_stream)
+    assert rc == 0
+    op = sb.SpconvBlockwiseOp().initialize(f, Bn, H, H, 1, x, want)
+    assert op._state.variant == 1
+    op(s)
+    torch.cuda.synchronize()
+    f.device_status()
+    assert torch.equal(y.view(torch.int16), want.view(torch.int16))
