@@ -294,11 +294,10 @@ int spmm_gather(long long K, int N, int row_blocks, long long padded_cols, int t
     return crowded && tile == 128 ? shflbw::kGatherCpAsync : shflbw::kGatherTma;
 }
 
-// Whether the rows of the blocks lie in the TMEM lanes (SpMM, and SpConv that writes planes).
-bool rows_in_lanes(int V, bool deep) {
-    const char* e = getenv("SHFLBW_SWAP");                    // forces the choice (tuning aid)
-    return (V == 64 || V == 128) && (e ? atoi(e) != 0 : deep);
-}
+// Whether the rows of the blocks lie in the TMEM lanes (SpMM, and SpConv that writes planes): `pays`, or what SHFLBW_SWAP=0|1
+// forces (tuning aid).
+bool swap_forced(int to) { const char* e = getenv("SHFLBW_SWAP"); return e && (atoi(e) != 0) == (to != 0); }
+bool rows_in_lanes(int V, bool pays) { return (V == 64 || V == 128) && !swap_forced(0) && (pays || swap_forced(1)); }
 bool is_deep(long long padded_cols, int row_blocks) { return padded_cols >= 192ll * row_blocks; }
 
 // Token tile: a persistent CTA works through ceil(items / SMs) items in turn; an item of 128 tokens takes about 2/3 of
@@ -407,13 +406,33 @@ bool wide_wanted(int V, int tile, bool pays) {
 // of one stage are as fast with six (26 columns: 48.5, with eight 49.7).
 int wide_ring_of(bool addend, long long padded_cols, int row_blocks) { return !addend && padded_cols > 32ll * row_blocks ? 8 : 6; }
 
-// Whether the rows of an SpMM's blocks lie in the TMEM lanes, and whether it runs with sixteen epilogue warps.  With rows in
-// lanes from three stages of non-zero columns per block on: with fewer an item is mostly epilogue.  The line was drawn when
-// an MMA took 54 clk of issue whatever its shape, which rows in lanes halve.
-bool spmm_rows(int V, long long padded_cols, int row_blocks) { return rows_in_lanes(V, is_deep(padded_cols, row_blocks)); }
-// At most 64 non-zero columns per block on average, where an item is all epilogue, and several items per SM.
-bool spmm_wide(int V, int tile, long long n_tokens, long long padded_cols, int row_blocks) {
-    return wide_wanted(V, tile, padded_cols <= 64ll * row_blocks && (n_tokens + 255) / 256 * row_blocks >= 4ll * (sm_count() > 0 ? sm_count() : 148));
+// Whether an SpMM runs with sixteen epilogue warps (tokens in lanes).  Few columns a block and several items per SM: an item is
+// all epilogue.  V = 64, N = 4096, 6.9 items per SM, eight warps / sixteen / rows in lanes: 16 columns 13.8 / 11.1 / 11.5 us, 64 15.1 /
+// 12.4 / 12.8, 80 15.4 / 13.1 / 13.3, 100 16.0 / 13.9 / 13.8, 128 16.8 / 15.5 / 14.7; with fewer items rows in lanes win (three: 48
+// columns 8.2 / 7.6 / 7.2).  Rows of B and D that are no whole 32-byte sectors (N % 16 = 8), where rows in lanes store 16 bytes
+// at a time: N = 4104, 16 columns 15.0 / 11.9 / 16.2, 80 17.4 / 15.4 / 19.3, 100 18.0 / 17.1 / 20.2, 128 19.0 / 19.3 / 21.3; N = 2056,
+// 3.8 items per SM, 16 / 48 / 90 columns 9.0 and 7.9 / 9.8 and 8.6 / 11.0 and 10.2.  `sectors`: whole ones.  With C: N = 4096, 16 columns 18.0 / 14.7 / 33.1,
+// 160 23.3 / 19.4 / 38.2; two items per SM, 16 / 48 / 90 columns 7.3 and 6.7 / 7.6 and 7.4 / 8.7 and 8.0; 1.35: 6.2 and 5.6 / 6.3 and
+// 6.6 / 8.0 and 7.2.
+bool spmm_wide(int V, int tile, int N, bool sectors, bool with_c, long long padded_cols, int row_blocks) {
+    const long long items = (N + 255) / 256 * (long long)row_blocks, sms = sm_count() > 0 ? sm_count() : 148;
+    const int most = with_c ? 160 : sectors ? 80 : 104;
+    return wide_wanted(V, tile, padded_cols <= (long long)most * row_blocks && (with_c ? items >= 2 * sms : sectors ? items >= 4 * sms : 2 * items >= 7 * sms));
+}
+// Whether its rows lie in the TMEM lanes where it does not.  They store 32 bytes a lane if D's rows are whole sectors: then
+// always (V = 64, 1024x1024x64, 16 / 96 / 256 columns, tokens and rows: 2.93 and 2.71 / 3.67 and 3.26 / 4.27 and 3.69;
+// 512x1024x16384 8.9 and 7.6 / 10.4 and 9.3 / 12.5 and 11.7; 4096x1024x4096, 256: 19.1 and 19.2; V = 128 13.9 and 11.2 / 16.1 and
+// 13.3 / 18.6 and 16.7).  If not, up to 64 tokens (4096x1024x40, 40 / 120 / 400 columns: 3.13 and 2.88 / 3.97 and 3.49 / 5.48 and
+// 4.73), and 64 rows in 128-token tiles from a stage and a half on (1024x4096x504: 3.31 and 3.41 / 4.11 and 4.09 / 5.62 and
+// 5.39), not beyond (4096x1024x3000, 120 / 400: 15.0 and 16.8 / 26.9 and 30.3; V = 128 14.1 and 15.5 / 21.4 and 22.6).  C is read
+// after the accumulator there, which pays for 64 rows from 1600 columns on (4096x4096x4096, 400 / 1600 / 3200: 31.4 and 45.6 /
+// 76.6 and 76.8 / 137 and 128; V = 128 33.1 and 49.5 / 59.0 and 65.2 / 102 and 103), and on 24 tokens or fewer, of which C has
+// little, from three stages on (8 tokens: 448x3704, V = 64, 977 columns 6.56 and 5.90, 8704x2312, V = 128, 187 columns 4.60 and
+// 4.24; 40 tokens, 4096x4096, 256 columns 4.70 and 5.03).
+bool spmm_rows(int V, int tile, int N, bool sectors, bool with_c, long long padded_cols, int row_blocks) {
+    const bool whole = sectors || N <= 64;
+    if (with_c) return rows_in_lanes(V, (V == 64 && whole && padded_cols >= 1600ll * row_blocks) || (N <= 24 && is_deep(padded_cols, row_blocks)));
+    return rows_in_lanes(V, whole || (V == 64 && tile == 128 && padded_cols >= 96ll * row_blocks));
 }
 
 // The same for chained layers, of `tokens` tokens counted with the padding of their rows.  Tokens in lanes, which write (and
@@ -595,8 +614,10 @@ static int plan_spmm(const shflbw_matrix_t* m, int N, const void* B, float alpha
         PanelChoice ch;
         const long long padded_cols = m->kptr.empty() ? 0 : m->kptr.back();
         const int blocks = out->num_row_blocks, tile = pick_tile(N, blocks);
-        const bool rows = spmm_rows(m->brow, padded_cols, blocks);
-        const int ring = !rows && spmm_wide(m->brow, tile, N, padded_cols, blocks) ? wide_ring_of(beta != 0.f, padded_cols, blocks) : 0;
+        const bool sectors = N % 16 == 0 && !((uintptr_t)D & 31);
+        const bool wide = !swap_forced(1) && spmm_wide(m->brow, tile, N, sectors, beta != 0.f, padded_cols, blocks);
+        const bool rows = !wide && spmm_rows(m->brow, tile, N, sectors, beta != 0.f, padded_cols, blocks);
+        const int ring = wide ? wide_ring_of(beta != 0.f, padded_cols, blocks) : 0;
         int rc = pick_panel<shflbw::kPanelSpmm>(m->brow, tile, rows, ring, spmm_gather(m->ncol, N, blocks, padded_cols, tile, with_bias), &ch);
         if (rc != SHFLBW_OK) return rc;
         out->kernel = SHFLBW_KERNEL_TCGEN05;

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import shflbw_sparse_nn_b200 as sb
-from gpu_util import dev, host, operand_swap
+from gpu_util import dev, host, operand_swap, run_spmm
 from shflbw_sparse_nn_b200 import _cabi
 
 pytestmark = pytest.mark.gpu
@@ -123,3 +123,45 @@ def test_planes_that_do_not_fit_the_fixed_scratch_give_way_to_positions():
     torch.cuda.synchronize()
     f.device_status()
     assert torch.equal(y.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("V,blocks,K,N,cols,beta,variant", [
+    (64, 40, 512, 4096, 40, 0.0, 2), (64, 40, 512, 4096, 100, 0.0, 1), (64, 40, 512, 1024, 40, 0.0, 1),    # whole sectors
+    (64, 40, 512, 4104, 90, 0.0, 2), (64, 40, 512, 4104, 130, 0.0, 0), (64, 40, 512, 1032, 40, 0.0, 0),    # not
+    (64, 10, 512, 504, 130, 0.0, 1), (64, 10, 512, 504, 40, 0.0, 0), (64, 10, 512, 40, 20, 0.0, 1),
+    (64, 40, 512, 4096, 120, -1.5, 2), (64, 40, 512, 4096, 300, -1.5, 0), (64, 4, 2048, 512, 1700, -1.5, 1), (64, 4, 2048, 24, 300, -1.5, 1),
+    (128, 20, 512, 4096, 20, 0.0, 1), (128, 20, 512, 4104, 300, 0.0, 0), (128, 20, 512, 64, 100, 0.0, 1), (128, 20, 512, 4096, 300, -1.5, 0),
+    (128, 2, 512, 8, 300, -1.5, 1),
+])
+def test_spmm(V, blocks, K, N, cols, beta, variant):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the item counts are of 148 SMs")
+    m = sb.BlockwiseSpMatrix().init_random(V * blocks, K, V, 1, (cols + 0.5) / K, True, 5, values="uniform")
+    B = sb.uniform_half(6, K * N).reshape(K, N)
+    Cm = sb.uniform_half(7, m.nrow * N).reshape(m.nrow, N) if beta else None
+    D, op = run_spmm(m, N, B, alpha=0.5, Cm=Cm, beta=beta)
+    assert op._state.variant == variant
+    for swap in (0, 1):
+        with operand_swap(swap):
+            E, op = run_spmm(m, N, B, alpha=0.5, Cm=Cm, beta=beta)
+        assert (op._state.variant == 1) == bool(swap)
+        assert np.array_equal(D.view(np.uint16), E.view(np.uint16))
+    assert np.abs(D.astype(np.float32)).max() > 0
+
+
+def test_rows_that_start_between_sectors_keep_tokens_in_lanes():
+    m = sb.BlockwiseSpMatrix().init_random(64 * 40, 512, 64, 1, 0.2, True, 5, values="uniform")
+    m.transform_and_sync_device()
+    B = dev(sb.uniform_half(6, 512 * 4096).reshape(512, 4096))
+    flat = torch.zeros(m.nrow * 4096 + 8, dtype=torch.float16, device="cuda")
+    s = torch.cuda.current_stream()
+    got = []
+    for off, variant in ((0, 1), (8, 0)):
+        D = flat[off:off + m.nrow * 4096]
+        op = sb.SpmmBlockwiseOp().initialize(m, 4096, B, D)
+        assert op._state.variant == variant
+        op(s)
+        torch.cuda.synchronize()
+        m.device_status()
+        got.append(host(D).view(np.uint16).copy())
+    assert np.array_equal(*got)
