@@ -424,22 +424,17 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     auto item_block = [&](int item) { return p.tile_major ? item - fast_div(item, p.div_blocks) * p.num_blocks : fast_div(item, p.div_tiles); };
     auto item_tile = [&](int item) { return p.tile_major ? fast_div(item, p.div_blocks) : item - fast_div(item, p.div_tiles) * p.tiles_n; };
 
-    if (tid == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            // cp.async gather: one arrival per producer WARP of the group (per-thread deferred arrivals,
-            // cp.async.mbarrier.arrive.noinc, were measured at ~3 clk of load/store-unit time per thread,
-            // i.e. more than the copies themselves).  TMA gather: one arrival per warp of the group too, with the
-            // bytes that it fetches, whether it has a row in the stage or not (see the producers).
-            sm100::mbar_init(&full_bar[s], PW / Cfg::GROUPS);
-            sm100::mbar_init(&empty_bar[s], 1);   // one tcgen05.commit per drain
-        }
-        for (int b = 0; b < NBUF; ++b) {
-            sm100::mbar_init(&acc_full[b], 1);
-            sm100::mbar_init(&acc_empty[b], EW / Cfg::ESETS);  // one arrival per epilogue warp of the set that reads it
-        }
-        for (int b = 0; b < Cfg::SLOT_BARS; ++b) sm100::mbar_init(&slot_bar[b], 1);
-        sm100::mbar_init(drain_bar, 1);
-        *cta_abort = 0;
+    if (warp == 0) {                                       // barriers, a lane each
+        static_assert(2 * STAGES + 2 * NBUF <= 32, "a barrier per lane");
+        // cp.async gather: one arrival per producer WARP of the group (per-thread deferred arrivals,
+        // cp.async.mbarrier.arrive.noinc, were measured at ~3 clk of load/store-unit time per thread,
+        // i.e. more than the copies themselves).  TMA gather: one arrival per warp of the group too, with the
+        // bytes that it fetches, whether it has a row in the stage or not (see the producers).  Stages are emptied by
+        // one tcgen05.commit, accumulators by an arrival of each epilogue warp of the set that reads them.
+        if (lane < 2 * STAGES + 2 * NBUF)
+            sm100::mbar_init(&full_bar[lane], lane < STAGES ? PW / Cfg::GROUPS : lane < 2 * STAGES + NBUF ? 1 : EW / Cfg::ESETS);
+        for (int b = lane; b < Cfg::SLOT_BARS; b += 32) sm100::mbar_init(&slot_bar[b], 1);
+        if (lane == 0) { sm100::mbar_init(drain_bar, 1); *cta_abort = 0; }
         sm100::mbar_init_fence();
     }
     for (int li = tid; li < nloc; li += blockDim.x) {
@@ -451,21 +446,24 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         sm100::tmem_alloc(tmem_slot, Cfg::TMEM_COLS);
         sm100::tmem_relinquish();
     }
-    sm100::tc_fence_before_sync();
-    __syncthreads();
-    sm100::tc_fence_after_sync();
-    const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
     const uint32_t smem_base = sm100::smem_u32(smem);
-    // Programmatic dependent launch: everything above (barriers, TMEM, the item table -- read from
+    // The end of the set-up, passed by every warp of the block, in its role: the producers of the TMA gather come with the
+    // row ids of their first stages under way.
+    // Programmatic dependent launch: everything before (barriers, TMEM, the item table, row ids -- read from
     // the sparse operand, which no kernel writes) may overlap the tail of the previous kernel in
-    // the stream; the dense operand, the residual and the output are touched only below.  The
+    // the stream; the dense operand, the residual and the output are touched only after the wait below.  The
     // next kernel may start its own prologue as soon as every block of this one got here.
     // (A convolution call that ends with this kernel lets the next one in when its producers have issued, or by
     // cp.async completed, their last copies: early enough for the set-up of an SpMM or a chained layer behind it, about
     // 1 us, and late enough that few blocks of another convolution's relayout, which has no set-up, wait on this kernel's
     // SMs; with those spread evenly (relayout_smem) calls back to back are 1-3 % slower than without any trigger.
     // 24x16x16x160 -> 1856, 3x3, V = 32: 23.9 us and 28.6 with a chained layer; without a trigger 23.7 and 29.8.)
-    if (MODE != kPanelConv || p.perm != nullptr) sm100::grid_dependency_launch();
+    auto set_up_done = [&]() {
+        sm100::tc_fence_before_sync();
+        asm volatile("bar.sync 0;" ::: "memory");
+        sm100::tc_fence_after_sync();
+        if (MODE != kPanelConv || p.perm != nullptr) sm100::grid_dependency_launch();
+    };
     // The wait itself is executed per role, as late as each role allows: by the producers after
     // their first row ids (sparse operand) are on their way and before their first gather, by the
     // epilogue warps at once (they read C / the residual and write the output); the MMA warp
@@ -473,7 +471,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
 
     const int pidx = Cfg::TMA ? warp - (EW + 1) : warp - (EW + 1) - (warp / 4 - EW / 4);   // producer number of a producer warp (warps after the MMA warp with warp % 4 != 0)
     if (!Cfg::TMA && warp > EW && ((warp & 3) == 0 || pidx >= PW)) {
-        // idle: keeps producers off the MMA warp's scheduler partition
+        set_up_done();                                      // idle: keeps producers off the MMA warp's scheduler partition
     } else if (warp > EW && Cfg::TMA) {
         // ---------------------------------------------------- producers (TMA gather) ----
         // A stage is KS gathered rows x T tokens = (KS/4) row quads x (T/64) column boxes, one
@@ -554,15 +552,39 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             sm100::mbar_arrive_expect_tx(&full_bar[slot], bytes);
             if (pw == 0) sm100::bulk_copy_g2s(smem_base + slot * Cfg::STAGE_BYTES + (uint32_t)Cfg::G_BYTES, p.blk_val + (size_t)row0 * V, wbytes, &full_bar[slot]);
         };
-        // The CTA's first stage: this warp's quads of it.
+        // The CTA's first stage: this warp's quads of it.  The first item's extent, the ids of these and those of the warp's
+        // first whole stage are read beside the block's set-up: a block that starts behind the last ones of the kernel before
+        // (grids of every SM) has them 0.5 us earlier (1024x1024x960, V = 32 4.91 -> 4.56 us, 4096^3 at V = 64 25.0 -> 23.4,
+        // 28x28x512 -> 128 chained, batch 8, 4.17 -> 3.96; read after the set-up, by its table, and one after the other before).
         constexpr int QW = (QUADS + PW - 1) / PW;
-        settle();
-        const int first_li = li, first_row = row_begin, first_valid = li < nloc ? min(KS, rows_total) : 0;
-        if (lane < QW * 4) my_ids[lane] = row_id(pidx * QW * 4 + lane);
-        if (li < nloc) enter_item();
-        kt += 1 + grp;
-        settle();
-        load_ids();
+        {
+            const int* const ext = p.blk_ptr + item_block((int)blockIdx.x);
+            const int e0 = __ldg(ext), e1 = __ldg(ext + 1);
+            enter_item();
+            row_begin = __shfl_sync(0xffffffffu, e0, 0); rows_total = __shfl_sync(0xffffffffu, e1, 0) - row_begin;
+        }
+        int first_li = 0, first_row = row_begin, first_valid = min(KS, rows_total), first_id = 0;
+        if (lane < QW * 4) first_id = row_id(pidx * QW * 4 + lane);
+        kt = 1 + grp;
+        const bool in_first = kt * KS < rows_total;
+        if (in_first) load_ids();
+        set_up_done();
+        if (first_valid == 0) {                             // an empty first item: on to one that is not
+            kt = 0;
+            settle();
+            first_li = li; first_row = row_begin;
+            if (li < nloc) {
+                first_valid = min(KS, rows_total);
+                if (lane < QW * 4) first_id = row_id(pidx * QW * 4 + lane);
+                enter_item();
+            }
+            kt += 1 + grp;
+        }
+        if (!in_first) {
+            settle();
+            load_ids();
+        }
+        if (lane < QW * 4) my_ids[lane] = first_id;
         __syncwarp();
         sm100::grid_dependency_wait();                      // the dense operand may be the previous kernel's output
         if (first_li < nloc && sm100::elect_one()) {
@@ -623,6 +645,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         }
     } else if (warp > EW) {
         // --------------------------------------------- producers (cp.async gather) ----
+        set_up_done();
         if constexpr (!Cfg::TMA) {
         // The PW producer warps form GROUPS groups that take the CTA's stages in turn (group g
         // fills stages g, g+GROUPS, ...).  While one group sits in its barrier round trip
@@ -802,6 +825,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         }
     } else if (warp == EW) {
         // ------------------------------------------------------------ MMA warp ----
+        set_up_done();
+        const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
         constexpr uint32_t idesc = SWAP ? sm100::make_idesc_f16_mnmajor(V, T) : sm100::make_idesc_f16_mnmajor(128, V);
         // Descriptors are built once; per MMA only the 16-byte-granular start address field
         // (low bits) advances.
@@ -877,6 +902,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         // columns (the block's output rows / filters).  Sixteen warps are two sets of eight that take
         // the items in turn: against all sixteen on one item (a quarter of the columns each), 108 ->
         // 93 us on 56x56x64 -> 256 at batch 256, since an item's chain of waits is most of its time.
+        set_up_done();
+        const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
         sm100::grid_dependency_wait();
         if constexpr (SLOTS > 0) {
             box_epilogue<Cfg, V>(p, smem, smem_base, tmem_base, item_tab, nloc, acc_full, acc_empty, slot_bar, cta_abort, warp, lane, item_block, item_tile);
@@ -1374,7 +1401,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     __syncthreads();
     if (warp == EW) {
         sm100::tc_fence_after_sync();
-        sm100::tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
+        sm100::tmem_dealloc(__shfl_sync(0xffffffffu, *tmem_slot, 0), Cfg::TMEM_COLS);
     }
 }
 
