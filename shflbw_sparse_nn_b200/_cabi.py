@@ -6,6 +6,7 @@ substitute for the CUDA path.
 from __future__ import annotations
 
 import ctypes as C
+import sys
 from pathlib import Path
 
 from .build import LIB_PATH
@@ -170,6 +171,33 @@ def lib() -> C.CDLL:
     if _lib is None:
         _lib = load_library(LIB_PATH)
     return _lib
+
+
+_native, _native_of = None, None
+
+
+def native():
+    """The native host path of a call (csrc/native_calls.cpp) bound to the loaded library; None where it has not been
+    built or torch, whose tensors it handles, is not in use: ctypes and the modules' Python code do the same."""
+    if _lib is not None and _native_of is _lib:
+        return _native
+    return _bind_native()
+
+
+def _bind_native():
+    global _native, _native_of
+    library = lib()
+    if "torch" not in sys.modules:
+        return None
+    try:
+        from . import _native as module
+    except ImportError:
+        module = None
+    if module is not None and not module.bind(*(C.cast(getattr(library, f"shflbw_{name}"), C.c_void_p).value for name in (
+            "spmm_exec", "spconv_exec", "spconv_exec_bias", "spconv_init", "linear_exec")), C.sizeof(SpconvState)):
+        module = None
+    _native, _native_of = module, library
+    return module
 
 
 def check(status: int, where: str) -> None:

@@ -246,7 +246,11 @@ class SpmmBlockwiseOp:
         return self
 
     def __call__(self, stream=None):
-        status = _cabi.lib().shflbw_spmm_exec(self._state, _stream_ptr(stream))
+        native = _cabi.native()
+        if native is not None:
+            status = native.spmm(C.addressof(self._state), stream)
+        else:
+            status = _cabi.lib().shflbw_spmm_exec(self._state, _stream_ptr(stream))
         if status:
             check(status, "SpmmBlockwiseOp()")
 
@@ -297,7 +301,11 @@ class SpconvBlockwiseOp:
         return self
 
     def __call__(self, stream=None):
-        status = _cabi.lib().shflbw_spconv_exec(self._state, _stream_ptr(stream))
+        native = _cabi.native()
+        if native is not None:
+            status = native.spconv(C.addressof(self._state), stream)
+        else:
+            status = _cabi.lib().shflbw_spconv_exec(self._state, _stream_ptr(stream))
         if status:
             check(status, "SpconvBlockwiseOp()")
 
@@ -364,7 +372,11 @@ class SpconvChainOp:
         return self
 
     def __call__(self, stream=None):
-        status = _cabi.lib().shflbw_spconv_exec(self._state, _stream_ptr(stream))
+        native = _cabi.native()
+        if native is not None:
+            status = native.spconv(C.addressof(self._state), stream)
+        else:
+            status = _cabi.lib().shflbw_spconv_exec(self._state, _stream_ptr(stream))
         if status:
             check(status, "SpconvChainOp()")
 

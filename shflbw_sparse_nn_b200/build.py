@@ -2,7 +2,8 @@
 
 `python -m shflbw_sparse_nn_b200.build` or `build_library()` compiles
 `csrc/shflbw_capi.cu` + `csrc/shflbw_format.cc` into `libshflbw_b200.so` next to this file.
-nvcc cross-compiles without a GPU.  The shared object is git-ignored; it is a build product.
+nvcc cross-compiles without a GPU.  `build_native()` compiles `csrc/native_calls.cpp`, the host path of the Python
+operators and modules, into `_native.so` (without it they go through ctypes).  Both are git-ignored build products.
 """
 from __future__ import annotations
 
@@ -86,6 +87,32 @@ def build_fault_inject_library(force: bool = False) -> Path:
     return FAULT_LIB_PATH
 
 
+NATIVE_PATH = PKG_DIR / "_native.so"
+NATIVE_SOURCE = PKG_DIR / "csrc" / "native_calls.cpp"
+
+
+def build_native(force: bool = False) -> Path:
+    """Compile the native host path (`_native.so`, a CPython module over torch's C++ tensors)."""
+    import sysconfig
+
+    import torch
+
+    deps = [NATIVE_SOURCE, REPO_ROOT / "include" / "shflbw.h"]
+    if not force and NATIVE_PATH.exists() and all(d.stat().st_mtime <= NATIVE_PATH.stat().st_mtime for d in deps):
+        return NATIVE_PATH
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(_nvcc()).resolve().parents[1]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           "-I", str(REPO_ROOT / "include"), "-I", sysconfig.get_paths()["include"], "-I", str(root / "include"),
+           "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"), "-I", str(cuda / "include"),
+           "-o", str(NATIVE_PATH), str(NATIVE_SOURCE),
+           "-L", str(root / "lib"), "-ltorch_python", "-ltorch_cpu", "-ltorch", "-lc10", "-lc10_cuda"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"g++ failed ({res.returncode}):\n{res.stdout}\n{res.stderr}")
+    return NATIVE_PATH
+
+
 TOOLS_DIR = PKG_DIR / "bin"
 TOOL_SOURCE = PKG_DIR / "csrc" / "benchmark_cli.cu"
 
@@ -114,6 +141,7 @@ def build_tools(force: bool = False) -> dict:
 
 if __name__ == "__main__":
     print(build_library(force="--force" in sys.argv, verbose="-v" in sys.argv))
+    print(build_native(force="--force" in sys.argv))
     if "--tools" in sys.argv:
         for exe in build_tools(force="--force" in sys.argv).values():
             print(exe)

@@ -68,8 +68,7 @@ struct FastDiv {
 inline FastDiv make_fast_div(int d) {
     FastDiv f{(unsigned)d, 0u, 0u};
     if (d > 1) {
-        unsigned c = 0;
-        while ((1ull << c) < (unsigned long long)d) ++c;         // ceil(log2 d)
+        const unsigned c = 32 - __builtin_clz((unsigned)d - 1);  // ceil(log2 d)
         const unsigned p = 31 + c;
         f.mul = (unsigned)(((1ull << p) + (unsigned long long)d - 1) / (unsigned long long)d);
         f.shr = p - 32;

@@ -16,6 +16,8 @@
 #include <cstring>
 #include <utility>
 
+#include <unistd.h>
+
 #include "aux_kernels.cuh"
 #include "panel_umma.cuh"
 #include "shflbw_internal.hpp"
@@ -40,6 +42,23 @@ bool cuda_ok(cudaError_t e, const char* what) {
     return false;
 }
 #define CK(call) do { if (!cuda_ok((call), #call)) return SHFLBW_ERR_CUDA; } while (0)
+
+// The tuning aids of a plan, read from the environment in one pass whenever one is made (50 ns a getenv, fourteen of them a plan).
+struct Tuning { const char *tile, *swap, *gather, *epilogue_warps, *conv_planes, *box; };
+thread_local Tuning g_tuning;
+void read_tuning() {
+    static const struct { const char* name; const char* Tuning::*at; } known[] = {
+        {"TILE", &Tuning::tile}, {"SWAP", &Tuning::swap}, {"GATHER", &Tuning::gather}, {"EPILOGUE_WARPS", &Tuning::epilogue_warps},
+        {"CONV_PLANES", &Tuning::conv_planes}, {"BOX", &Tuning::box}};
+    g_tuning = Tuning{};
+    for (char** e = environ; e && *e; ++e) {
+        if (strncmp(*e, "SHFLBW_", 7)) continue;
+        for (const auto& k : known) {
+            const size_t n = strlen(k.name);
+            if (!strncmp(*e + 7, k.name, n) && (*e)[7 + n] == '=' && !(g_tuning.*k.at)) g_tuning.*k.at = *e + 8 + n;
+        }
+    }
+}
 
 // Every kernel of this library is launched with the programmatic-stream-serialization attribute:
 // it may start while the previous kernel of the stream drains, sets itself up (barriers, TMEM,
@@ -273,7 +292,7 @@ int tma_row_pix(int Wo, int Wp, int Bp, int stride) {
 
 // SHFLBW_GATHER=0 takes the cp.async gather everywhere, 1 has an SpMM gather by TMA where it would not by itself
 // (tuning aids).  Asked for when a state is made.
-bool tma_wanted() { const char* g = getenv("SHFLBW_GATHER"); return !g || atoi(g) == 1; }
+bool tma_wanted() { return !g_tuning.gather || atoi(g_tuning.gather) == 1; }
 
 // The gather of an SpMM: TMA, unless rows share 32-byte sectors (8 or 24 tokens), there are few of them, and many blocks
 // want each.  The SMs then fetch the same few lines of L2 over and over, and the copy engine's requests to one line queue
@@ -287,7 +306,7 @@ bool tma_wanted() { const char* g = getenv("SHFLBW_GATHER"); return !g || atoi(g
 // (SHFLBW_GATHER=0).
 int spmm_gather(long long K, int N, int row_blocks, long long padded_cols, int tile, bool with_bias) {
     if (tile == 256 && with_bias) return shflbw::kGatherTma;
-    if (getenv("SHFLBW_GATHER")) return tma_wanted() ? shflbw::kGatherTma : shflbw::kGatherCpAsync;
+    if (g_tuning.gather) return tma_wanted() ? shflbw::kGatherTma : shflbw::kGatherCpAsync;
     const bool dense = 20 * padded_cols > 9 * K * row_blocks;
     const bool crowded = padded_cols > 16ll * row_blocks && ((N == 8 && padded_cols >= 40 * K && K <= (dense ? 3072 : 1024)) ||
                                                              (N == 24 && padded_cols >= 150 * K && K <= 341));
@@ -296,7 +315,7 @@ int spmm_gather(long long K, int N, int row_blocks, long long padded_cols, int t
 
 // Whether the rows of the blocks lie in the TMEM lanes (SpMM, and SpConv that writes planes): `pays`, or what SHFLBW_SWAP=0|1
 // forces (tuning aid).
-bool swap_forced(int to) { const char* e = getenv("SHFLBW_SWAP"); return e && (atoi(e) != 0) == (to != 0); }
+bool swap_forced(int to) { return g_tuning.swap && (atoi(g_tuning.swap) != 0) == (to != 0); }
 bool rows_in_lanes(int V, bool pays) { return (V == 64 || V == 128) && !swap_forced(0) && (pays || swap_forced(1)); }
 bool is_deep(long long padded_cols, int row_blocks) { return padded_cols >= 192ll * row_blocks; }
 
@@ -310,7 +329,7 @@ long long rounds_of_items(long long n_tokens, int tile, int row_blocks) {
     return ((n_tokens + tile - 1) / tile * row_blocks + sms - 1) / sms;
 }
 int pick_tile(long long n_tokens, int row_blocks) {
-    if (const char* e = getenv("SHFLBW_TILE")) { const int t = atoi(e); if (t == 128 || t == 256) return t; }
+    if (g_tuning.tile) { const int t = atoi(g_tuning.tile); if (t == 128 || t == 256) return t; }
     return n_tokens <= 128 || rounds_of_items(n_tokens, 128, row_blocks) * 2 < rounds_of_items(n_tokens, 256, row_blocks) * 3 ? 128 : 256;
 }
 
@@ -398,8 +417,7 @@ int pick_panel(int V, int tile, bool rows, int wide_ring, int gather, PanelChoic
 // Sixteen epilogue warps, tokens in lanes: SHFLBW_EPILOGUE_WARPS=8|16 forces the choice (tuning aid).
 bool wide_wanted(int V, int tile, bool pays) {
     if (V != 64 || tile != 256) return false;
-    const char* e = getenv("SHFLBW_EPILOGUE_WARPS");
-    return e ? atoi(e) == 16 : pays;
+    return g_tuning.epilogue_warps ? atoi(g_tuning.epilogue_warps) == 16 : pays;
 }
 // Their ring: eight stages where nothing is added and a block takes two stages, which a ring of six holds for
 // three items only (28x28x128 -> 512, batch 256, no residual, 40 columns: 56.6 us with six, 54.7 with eight); blocks
@@ -586,6 +604,7 @@ static int plan_spmm(const shflbw_matrix_t* m, int N, const void* B, float alpha
     if (!m || !B || !D || N <= 0) return SHFLBW_ERR_INVALID_ARG;
     if (check_kernel_arg(kernel) != SHFLBW_OK) return SHFLBW_ERR_INVALID_ARG;
     if (beta != 0.f && !C) return SHFLBW_ERR_INVALID_ARG;
+    read_tuning();
     if (!on_current_device(*m)) return SHFLBW_ERR_NOT_ON_DEVICE;  // reference: assert(device_synced)
     // The reference asserts bcol == 1 here (spmm/blockwise_op.h:86); the kernel image lists the
     // bcol columns of a block one by one, so wider blocks run on the same kernels.
@@ -948,6 +967,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
               float alpha, int kernel, shflbw_spconv_state_t* out, size_t scratch_limit = ~(size_t)0) {
     std::memset(out, 0, sizeof *out);
     if (check_kernel_arg(kernel) != SHFLBW_OK) return SHFLBW_ERR_INVALID_ARG;
+    read_tuning();
     ConvShape cs;
     int rc = check_conv_call(f, B, Hin, Win, stride, ifmap, ofmap, &cs);
     if (rc != SHFLBW_OK) return rc;
@@ -977,7 +997,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     // planes out?
     const bool planes_possible = (f->brow == 64 || f->brow == 128) && f->F / 64 <= 65535 &&
                                  (long long)f->F * tokens < (1ll << 32) - 1 && rows_in_lanes(f->brow, true);
-    const char* ep = getenv("SHFLBW_CONV_PLANES");
+    const char* ep = g_tuning.conv_planes;
     // the input as the panel kernel sees it: a strided 1x1 filter's pixels are staged side by side
     const bool compact = f->R == 1 && f->S == 1;
     const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, f->brow, row_blocks, padded_cols,
@@ -1261,6 +1281,7 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     out->perm = f->d_perm; out->status_word = f->d_status;
     out->chain = 1; out->out_R = R_next; out->out_S = S_next; out->relu = relu != 0;
     PanelChoice ch;
+    read_tuning();
     const int row_blocks = f->F / f->brow;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
     const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, f->brow, row_blocks, padded_cols,
@@ -1318,10 +1339,11 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     PanelChoice ch;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
     const bool two_warps = padded_cols <= 48ll * (st->F / st->V) && (long long)st->F * st->Ho * st->Wo * st->Bp * 2 <= (256ll << 20);   // (lookup)
-    const char* eb = getenv("SHFLBW_BOX");                   // 0: residual by cp.async (tuning aid)
+    read_tuning();
+    const char* eb = g_tuning.box;                           // SHFLBW_BOX=0: residual by cp.async (tuning aid)
     const bool box = st->gather == shflbw::kGatherTma && boxes_fit(*st) && (eb ? atoi(eb) != 0 : st->num_items >= 6ll * sm_count());
     const bool wide = (st->variant == 2 ||
-                       (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !getenv("SHFLBW_EPILOGUE_WARPS") &&
+                       (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !g_tuning.epilogue_warps &&
                         padded_cols <= 128ll * (st->F / st->V) && 2ll * st->num_items >= 5ll * sm_count())) &&
                       lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6, two_warps ? 2 : 3, box);
     shflbw_tensor_map_t map_res{};

@@ -21,7 +21,7 @@ import torch
 from torch import nn
 from torch.autograd import forward_ad
 
-from . import blockwise as bw
+from . import _cabi, blockwise as bw
 from .pruner import prune_conv_filter, prune_matrix
 
 
@@ -41,6 +41,11 @@ def _on_device(device: torch.device):
 def _stream_of(device: torch.device) -> int:
     """torch's current stream on `device` as a cudaStream_t (without building a Stream object, 3 us)."""
     return torch._C._cuda_getCurrentRawStream(device.index)
+
+
+def _bias_of(module: nn.Module):
+    """module.bias, without torch's look through its dictionaries where it is the buffer that it was made as."""
+    return module._buffers["bias"] if "bias" in module._buffers else module.bias
 
 
 def _in_memory(x: torch.Tensor) -> bool:
@@ -119,6 +124,11 @@ class ShflBWLinear(nn.Module):
         return self._run(None, xt.shape[1], xt, xt.shape[1])
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        native = _cabi.native()
+        if native is not None:                               # plain operands: everything below as one native call
+            y = native.linear(x, _bias_of(self), self.spmat._h.value or 0, self.in_features, self.out_features)
+            if y is not None:
+                return y
         _require_cuda_half(x, "ShflBWLinear")
         shape = x.shape
         x2 = x if len(shape) == 2 and shape[1] == self.in_features else x.reshape(-1, self.in_features)
@@ -178,6 +188,11 @@ class ShflBWConv2d(nn.Module):
         return cls(f, conv.stride[0], conv.bias, info)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        native = _cabi.native()
+        if native is not None:                               # plain operands: everything below as one native call
+            y = native.conv2d(x, _bias_of(self), self.spfilter._h.value or 0, self.stride, self.in_channels, self.out_channels)
+            if y is not None:
+                return y
         _require_cuda_half(x, "ShflBWConv2d")
         if x.dim() != 4 or x.shape[1] != self.in_channels:
             raise ValueError(f"expected [N][{self.in_channels}][H][W]")
