@@ -564,12 +564,14 @@ int shflbw_matrix_to_device(shflbw_matrix_t* m) {
     std::copy(m->row_permute_ids.begin(), m->row_permute_ids.end(), img.begin() + o_perm);
     std::copy(m->kcrs.begin(), m->kcrs.end(), img.begin() + o_crs);
     CK(cudaMalloc(&m->d_meta, total * sizeof(int)));
-    if (!cuda_ok(cudaMalloc(&m->d_val, m->kval.size() * 2), "cudaMalloc(values)")) {
+    if (!cuda_ok(cudaMalloc(&m->d_val, (m->kval.size() + m->kval_logical.size()) * 2), "cudaMalloc(values)")) {
         cudaFree(m->d_meta); m->d_meta = nullptr;
         return SHFLBW_ERR_CUDA;
     }
     CK(cudaMemcpy(m->d_meta, img.data(), total * sizeof(int), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(m->d_val, m->kval.data(), m->kval.size() * 2, cudaMemcpyHostToDevice));
+    if (!m->kval_logical.empty())
+        CK(cudaMemcpy((uint16_t*)m->d_val + m->kval.size(), m->kval_logical.data(), m->kval_logical.size() * 2, cudaMemcpyHostToDevice));
     const int* base = (const int*)m->d_meta;
     m->d_kptr = base + o_ptr;
     m->d_kidx = base + o_idx;
@@ -950,14 +952,14 @@ bool keep_map(shflbw_tensor_map_t* kept, const PlaneMap& m) {
 // With filters in lanes (28.3 instead of 24.5 for 14x14x512 -> 2048, 460 columns) only at 64 rows from 1200 columns on, as
 // the chained layers (14x14x256 -> 1024, 1800 columns: 33.4, tokens 33.8).
 bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long items, bool padded_rows, long long padded_cols, int row_blocks) {
-    return f.row_permute && tile == 256 && items >= (sm_count() > 0 ? sm_count() : 148) && 8 * (Bp - B) <= Bp &&
+    return f.row_permute && f.kval_logical.empty() && tile == 256 && items >= (sm_count() > 0 ? sm_count() : 148) && 8 * (Bp - B) <= Bp &&
            (padded_cols >= 64ll * row_blocks || !padded_rows);
 }
 
 // Launch plan of one NHWC SpConv call, without its scratch pointers: kernel choice, grid, and
 // the scratch each side needs.  Two plans exist.
 //   positions out   relayout -> panel kernel with tokens in TMEM lanes, writing [position][F] in
-//                   stored filter order -> (with a filter permutation) unpermute_filters.
+//                   stored filter order -> (with a filter permutation across blocks) unpermute_filters.
 //   planes out      relayout -> panel kernel writing the output as planes [F][Ho][Wo][Bp] with plane = LOGICAL
 //                   channel (the permutation is the row index of its stores, free) -> planes_to_nhwc
 //                   transposes the planes to NHWC.  Used for permuted V = 64 / 128 filters and outputs that
@@ -1023,9 +1025,14 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
         out->staged_out_bytes = (size_t)f->F * (size_t)tokens * 2;
     } else {
         out->variant = 0;
-        if (f->row_permute) {
+        if (f->row_permute && (unperm_smem_bytes(f->F) > 227 * 1024 || f->F > 65536)) return SHFLBW_ERR_UNSUPPORTED;
+        if (!f->kval_logical.empty()) {
+            // Rows in logical order: as an unpermuted filter, no pass behind the kernel (56x56x64 -> 64, 3x3, batch 32, V = 64,
+            // 115 columns: as planes 19.3 us, so 14.4; 25 filters of one block, 1x1 and 3x3, V = 16 to 128: 13 to 32 % less).
+            out->blk_val = (const uint16_t*)f->d_val + f->kval.size();
+            out->perm = nullptr;
+        } else if (f->row_permute) {
             out->staged_out_bytes = (size_t)B * Ho * Wo * f->F * 2;
-            if (unperm_smem_bytes(f->F) > 227 * 1024 || f->F > 65536) return SHFLBW_ERR_UNSUPPORTED;
             if (unperm_smem_bytes(f->F) > 48 * 1024)
                 for (const void* k : {(const void*)shflbw::unpermute_filters<false>, (const void*)shflbw::unpermute_filters<true>})
                     CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)unperm_smem_bytes(f->F)));

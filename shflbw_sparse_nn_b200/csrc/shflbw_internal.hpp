@@ -53,11 +53,14 @@ struct shflbw_matrix {
     std::vector<int> kptr, kidx;   // kernel image: padded offsets / column ids
     std::vector<int> kcrs;         // filters only: kidx decoded as c | r << 16 | s << 24 (k = (r*S + s)*C + c)
     std::vector<uint16_t> kval;    // kernel image: padded fp16 panels, element order kval_index()
+    // Filters whose permutation moves rows only within their blocks (a single block's always does): the panels once more
+    // with each block's rows in logical order, for NHWC calls, which then have nothing left to permute.  Else empty.
+    std::vector<uint16_t> kval_logical;
 
     // ---- device copy (owned) ----
     int device = -1;
     void* d_meta = nullptr;        // one int32 allocation: kptr | kidx | perm | kcrs | status word
-    void* d_val = nullptr;
+    void* d_val = nullptr;         // kval | kval_logical
     const int* d_kptr = nullptr;
     const int* d_kidx = nullptr;
     const int* d_kcrs = nullptr;   // filters with C < 65536 and R, S < 256 only
