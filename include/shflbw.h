@@ -219,6 +219,10 @@ int shflbw_spmm_exec(const shflbw_spmm_state_t* st, void* stream);
 int shflbw_linear_exec(const shflbw_matrix_t* m, int tokens, const void* x, const void* bias, void* xt, int N,
                        void* out, void* stream);
 
+/* The same of token-major activations on a handful of tokens in one launch, without xt: for layers where that is the
+ * faster way, SHFLBW_ERR_UNSUPPORTED (and nothing launched) for the others.  The same results, in out too. */
+int shflbw_linear_direct(const shflbw_matrix_t* m, int tokens, const void* x, const void* bias, int N, void* out, void* stream);
+
 /* Reads (and clears) the device status word of the matrix used by `st`; synchronises the
  * device.  SHFLBW_OK or SHFLBW_ERR_DEVICE_TIMEOUT. */
 int shflbw_matrix_device_status(const shflbw_matrix_t* m);

@@ -110,6 +110,7 @@ _PROTOS = {
                                    C.c_int, C.POINTER(SpmmState)]),
     "shflbw_spmm_exec": (C.c_int, [C.POINTER(SpmmState), C.c_void_p]),
     "shflbw_linear_exec": (C.c_int, [_H, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
+    "shflbw_linear_direct": (C.c_int, [_H, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "shflbw_spmm_host": (C.c_int, [_H, C.c_int, C.c_void_p, C.c_float, C.c_void_p, C.c_float, C.c_void_p]),
     "shflbw_spmm_host_copies_only": (C.c_int, [_H, C.c_int, C.c_void_p, C.c_void_p, C.c_int]),
     "shflbw_spmm_launches_per_exec": (C.c_int, [C.POINTER(SpmmState)]),
@@ -194,7 +195,7 @@ def _bind_native():
     except ImportError:
         module = None
     if module is not None and not module.bind(*(C.cast(getattr(library, f"shflbw_{name}"), C.c_void_p).value for name in (
-            "spmm_exec", "spconv_exec", "spconv_exec_bias", "spconv_init", "linear_exec")), C.sizeof(SpconvState)):
+            "spmm_exec", "spconv_exec", "spconv_exec_bias", "spconv_init", "linear_exec", "linear_direct")), C.sizeof(SpconvState)):
         module = None
     _native, _native_of = module, library
     return module

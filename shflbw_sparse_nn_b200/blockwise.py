@@ -273,6 +273,14 @@ def linear_exec(spmat: BlockwiseSpMatrix, tokens: int, x, bias, xt, N: int, out,
           "linear_exec")
 
 
+def linear_direct(spmat: BlockwiseSpMatrix, tokens: int, x, bias, N: int, out, stream=None) -> bool:
+    """The same of x[tokens][K] in one launch and without xt, or False (nothing launched) where two launches are faster."""
+    status = _cabi.lib().shflbw_linear_direct(spmat._h, tokens, _ptr(x), _ptr(bias), N, _ptr(out), _stream_ptr(stream))
+    if status != _cabi.ERR_UNSUPPORTED:
+        check(status, "linear_direct")
+    return status == 0
+
+
 def spmm_host(spmat: BlockwiseSpMatrix, N: int, B_host: np.ndarray, D_host: np.ndarray, alpha=1.0,
               C_host: Optional[np.ndarray] = None, beta=0.0) -> None:
     """End-to-end call with HOST buffers (numpy arrays or pinned torch CPU tensors)."""

@@ -20,6 +20,7 @@ SOURCES = [PKG_DIR / "csrc" / "shflbw_capi.cu", PKG_DIR / "csrc" / "shflbw_forma
 HEADERS = [
     PKG_DIR / "csrc" / "panel_umma.cuh",
     PKG_DIR / "csrc" / "aux_kernels.cuh",
+    PKG_DIR / "csrc" / "linear_direct.cuh",
     PKG_DIR / "csrc" / "sm100_ptx.cuh",
     PKG_DIR / "csrc" / "shflbw_internal.hpp",
     REPO_ROOT / "include" / "shflbw.h",

@@ -32,21 +32,23 @@ decltype(&shflbw_spconv_exec) spconv_exec = nullptr;
 decltype(&shflbw_spconv_exec_bias) spconv_exec_bias = nullptr;
 decltype(&shflbw_spconv_init) spconv_init = nullptr;
 decltype(&shflbw_linear_exec) linear_exec = nullptr;
+decltype(&shflbw_linear_direct) linear_direct = nullptr;
 PyObject* name_cuda_stream = nullptr;
 
 PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 6) { PyErr_SetString(PyExc_TypeError, "bind(spmm_exec, spconv_exec, spconv_exec_bias, spconv_init, linear_exec, size of a state)"); return nullptr; }
-    const long long size = PyLong_AsLongLong(args[5]);
+    if (n != 7) { PyErr_SetString(PyExc_TypeError, "bind(spmm_exec, spconv_exec, spconv_exec_bias, spconv_init, linear_exec, linear_direct, size of a state)"); return nullptr; }
+    const long long size = PyLong_AsLongLong(args[6]);
     if (PyErr_Occurred()) return nullptr;
     if (size != (long long)sizeof(shflbw_spconv_state_t)) Py_RETURN_FALSE;      // built beside another header
-    void* a[5];
-    for (int i = 0; i < 5; ++i)
+    void* a[6];
+    for (int i = 0; i < 6; ++i)
         if (!(a[i] = PyLong_AsVoidPtr(args[i]))) { if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address"); return nullptr; }
     spmm_exec = (decltype(spmm_exec))a[0];
     spconv_exec = (decltype(spconv_exec))a[1];
     spconv_exec_bias = (decltype(spconv_exec_bias))a[2];
     spconv_init = (decltype(spconv_init))a[3];
     linear_exec = (decltype(linear_exec))a[4];
+    linear_direct = (decltype(linear_direct))a[5];
     Py_RETURN_TRUE;
 }
 
@@ -132,9 +134,14 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t n) {
         Py_BEGIN_ALLOW_THREADS
         try {
             const int64_t tokens = x.size(0), padded = (tokens + 7) / 8 * 8;
-            const at::Tensor xt = at::empty({K, padded}, x.options()), out = at::empty({M, padded}, x.options());
-            rc = linear_exec(m, (int)tokens, x.const_data_ptr(), with_bias ? bias.const_data_ptr() : nullptr, xt.data_ptr(), (int)padded,
-                             out.data_ptr(), c10::cuda::getCurrentCUDAStream().stream());
+            const at::Tensor out = at::empty({M, padded}, x.options());
+            const void* const b = with_bias ? bias.const_data_ptr() : nullptr;
+            void* const stream = c10::cuda::getCurrentCUDAStream().stream();
+            rc = linear_direct(m, (int)tokens, x.const_data_ptr(), b, (int)padded, out.data_ptr(), stream);
+            if (rc == SHFLBW_ERR_UNSUPPORTED) {
+                const at::Tensor xt = at::empty({K, padded}, x.options());
+                rc = linear_exec(m, (int)tokens, x.const_data_ptr(), b, xt.data_ptr(), (int)padded, out.data_ptr(), stream);
+            }
             if (rc == SHFLBW_OK) y = out.as_strided({tokens, M}, {1, padded});
         } catch (...) {
             Py_BLOCK_THREADS

@@ -19,6 +19,7 @@
 #include <unistd.h>
 
 #include "aux_kernels.cuh"
+#include "linear_direct.cuh"
 #include "panel_umma.cuh"
 #include "shflbw_internal.hpp"
 
@@ -44,12 +45,13 @@ bool cuda_ok(cudaError_t e, const char* what) {
 #define CK(call) do { if (!cuda_ok((call), #call)) return SHFLBW_ERR_CUDA; } while (0)
 
 // The tuning aids of a plan, read from the environment in one pass whenever one is made (50 ns a getenv, fourteen of them a plan).
-struct Tuning { const char *tile, *swap, *gather, *epilogue_warps, *conv_planes, *box; };
+struct Tuning { const char *tile, *swap, *gather, *epilogue_warps, *conv_planes, *box, *linear_direct; };
 thread_local Tuning g_tuning;
 void read_tuning() {
     static const struct { const char* name; const char* Tuning::*at; } known[] = {
         {"TILE", &Tuning::tile}, {"SWAP", &Tuning::swap}, {"GATHER", &Tuning::gather}, {"EPILOGUE_WARPS", &Tuning::epilogue_warps},
-        {"CONV_PLANES", &Tuning::conv_planes}, {"BOX", &Tuning::box}};
+        {"CONV_PLANES", &Tuning::conv_planes}, {"BOX", &Tuning::box},
+        {"LINEAR_DIRECT", &Tuning::linear_direct}};
     g_tuning = Tuning{};
     for (char** e = environ; e && *e; ++e) {
         if (strncmp(*e, "SHFLBW_", 7)) continue;
@@ -528,6 +530,29 @@ void drop_device_copy(shflbw_matrix& m) {
 }
 }  // namespace shflbw
 
+namespace {
+// Whether a linear layer on a few tokens goes to the one-launch kernel: where its blocks, of 8 tokens each, are resident at
+// once and read little.  Device time, two launches and one: 4096 x 4096, V = 64, density 0.1 on 1 / 8 / 16 / 37 / 64 tokens
+// 5.4 / 5.7 / 5.1 / 5.5 / 5.4 and 2.8 / 3.3 / 4.1 / 5.0 / 9.2 us (64: 3.5 blocks an SM, of which 3 are resident); the host gains another
+// 2.2 us.  Over 160 shapes the two are equal near 270 KB an SM, of value panels and of the 32-byte sectors of x, less 20 KB for
+// every further pass over a block's columns (3712 x 7816, density 0.086, 18 tokens, 242 KB in two passes: 6.4 and 7.5;
+// 4096 x 4096 on 37 tokens: 245 KB in one), and from five blocks an SM on (1104 x 368, V = 16, 81 tokens: 4.6 and 5.5).  Up to 8 tokens
+// the panel kernel is no faster with so few (8608 x 440, V = 16, 3 tokens: 7.2 and 3.4): as far as 400 KB (9344 x 5224, V = 128, 5 tokens,
+// 319 KB in three passes: 8.9 and 7.4; 2304 x 4440, V = 128, 3 tokens, 382 KB in three: 8.4 and 8.3).
+bool linear_direct_pays(const shflbw_matrix& m, int tokens, int N, size_t smem) {
+    if (g_tuning.linear_direct) return atoi(g_tuning.linear_direct) != 0;
+    const long long sms = sm_count() > 0 ? sm_count() : 148, row_blocks = m.nrow / m.brow, blocks = row_blocks * (N / shflbw::kDirectTokens);
+    const long long resident = 228 * 1024 / ((long long)smem + 1024) < 8 ? 228 * 1024 / ((long long)smem + 1024) : 8;
+    const bool few = N == shflbw::kDirectTokens;
+    if (m.kptr.empty() || blocks > sms * (few || resident < 4 ? resident : 4)) return false;
+    const long long panels = m.kptr.back() * 2ll * m.brow, cols = m.kptr.back() / row_blocks;
+    const long long row = 2ll * m.ncol < 32 * cols ? 2ll * m.ncol : 32 * cols;           // bytes that a block reads of a token
+    const long long all = panels * (N / shflbw::kDirectTokens) + row_blocks * tokens * row;
+    const long long per_sm = all / (blocks < sms ? blocks : sms), passes = (m.max_cols + shflbw::kDirectCols - 1) / shflbw::kDirectCols;
+    return per_sm + 20 * 1024 * (passes - 1) <= (few ? 400 : 256) * 1024;
+}
+}  // namespace
+
 extern "C" {
 
 const char* shflbw_last_cuda_error(void) { return g_cuda_err; }
@@ -740,6 +765,32 @@ int shflbw_linear_exec(const shflbw_matrix_t* m, int tokens, const void* x, cons
                   m->ncol, N, (int)(m->ncol % 8 == 0 && ((uintptr_t)x & 15) == 0)));
     }
     return launch_spmm_panel(&st, ch, bias, (cudaStream_t)stream);
+}
+
+int shflbw_linear_direct(const shflbw_matrix_t* m, int tokens, const void* x, const void* bias, int N, void* out, void* stream) {
+    if (!m || !x || !out || N <= 0 || tokens <= 0 || tokens > N) return SHFLBW_ERR_INVALID_ARG;
+    if (((((uintptr_t)x | (uintptr_t)bias) & 1) | ((uintptr_t)out & 15)) || N % 8) return SHFLBW_ERR_UNSUPPORTED;
+    if (!on_current_device(*m)) return SHFLBW_ERR_NOT_ON_DEVICE;
+    if ((long long)m->nrow * N >= (1ll << 32) || (long long)m->ncol * N >= (1ll << 40)) return SHFLBW_ERR_UNSUPPORTED;   // as shflbw_spmm_init
+    read_tuning();
+    void (*fn)(const shflbw::DirectParams);
+    shflbw::DirectParams p{};
+    switch (m->brow) {
+        case 16: fn = shflbw::linear_direct<16>; break;
+        case 32: fn = shflbw::linear_direct<32>; break;
+        case 64: fn = shflbw::linear_direct<64>; break;
+        case 128: fn = shflbw::linear_direct<128>; break;
+        default: return SHFLBW_ERR_UNSUPPORTED;
+    }
+    const size_t smem = shflbw::direct_smem(m->brow, m->max_cols);
+    if (!linear_direct_pays(*m, tokens, N, smem)) return SHFLBW_ERR_UNSUPPORTED;
+    const int rc = allow_smem((const void*)fn, shflbw::direct_smem(m->brow, shflbw::kDirectCols));
+    if (rc != SHFLBW_OK) return rc;
+    p.blk_ptr = m->d_kptr; p.blk_idx = m->d_kidx; p.perm = m->d_perm; p.blk_val = (const __half*)m->d_val;
+    p.x = (const __half*)x; p.bias = (const __half*)bias; p.out = (__half*)out;
+    p.tokens = tokens; p.K = m->ncol; p.N = N; p.groups = N / shflbw::kDirectTokens;
+    CK(launch(fn, dim3((unsigned)(m->nrow / m->brow * p.groups)), dim3(256), smem, (cudaStream_t)stream, p));
+    return SHFLBW_OK;
 }
 
 int shflbw_spmm_launches_per_exec(const shflbw_spmm_state_t* st) { return st && st->init_success ? 1 : 0; }

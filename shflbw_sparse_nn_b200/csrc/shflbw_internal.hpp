@@ -51,6 +51,7 @@ struct shflbw_matrix {
     // ---- host images ----
     std::vector<int> meta_h;       // reference-compatible [indptr | indices*bcol | perm], pad 8
     std::vector<int> kptr, kidx;   // kernel image: padded offsets / column ids
+    int max_cols = 0;              // most padded columns of a row block
     std::vector<int> kcrs;         // filters only: kidx decoded as c | r << 16 | s << 24 (k = (r*S + s)*C + c)
     std::vector<uint16_t> kval;    // kernel image: padded fp16 panels, element order kval_index()
     // Filters whose permutation moves rows only within their blocks (a single block's always does): the panels once more

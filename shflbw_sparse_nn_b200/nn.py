@@ -104,14 +104,18 @@ class ShflBWLinear(nn.Module):
                 self.spmat.transform_and_sync_device()
             self._uploaded_on = device
 
-    def _run(self, x, tokens: int, xt: torch.Tensor, n: int) -> torch.Tensor:
-        """out[M][n] = W . xt + bias; x (token-major, or None when xt holds the operand) is transposed into xt first."""
-        dev = xt.device
+    def _run(self, x, tokens: int, xt, n: int) -> torch.Tensor:
+        """out[M][n] = W . xt + bias; x (token-major, or None when xt holds the operand) is read as it is, or transposed first."""
+        dev = xt.device if x is None else x.device
         self._upload(dev)
         out = torch.empty((self.out_features, n), dtype=torch.float16, device=dev)
         bias, fused = _fused_bias(self.bias, dev, self.out_features, 2)
         with _on_device(dev):
-            bw.linear_exec(self.spmat, tokens, x, bias if fused else None, xt, n, out, _stream_of(dev))
+            added, stream = bias if fused else None, _stream_of(dev)
+            if x is None or not bw.linear_direct(self.spmat, tokens, x, added, n, out, stream):
+                if xt is None:
+                    xt = torch.empty((self.in_features, n), dtype=torch.float16, device=dev)
+                bw.linear_exec(self.spmat, tokens, x, added, xt, n, out, stream)
         if bias is not None and not fused:
             out += bias[:, None]
         return out
@@ -146,11 +150,9 @@ class ShflBWLinear(nn.Module):
                 x2 = x2.contiguous()
         if tokens and not _in_memory(x2):                    # the kernel cannot read it
             by_torch = True
-        if by_torch and tokens != padded:
-            xt = torch.zeros((self.in_features, padded), dtype=torch.float16, device=x.device)
-        else:
-            xt = torch.empty((self.in_features, padded), dtype=torch.float16, device=x.device)
+        xt = None
         if by_torch:
+            xt = (torch.empty if tokens == padded else torch.zeros)((self.in_features, padded), dtype=torch.float16, device=x.device)
             (xt if tokens == padded else xt[:, :tokens]).copy_(x2.t())
             x2 = None
         yt = self._run(x2, tokens, xt, padded)
