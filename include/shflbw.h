@@ -376,8 +376,8 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* filter, shflbw_spconv_stat
  *  - ifmap / ofmap are NHWC device pointers exactly as for shflbw_spconv_init; the launch is
  *    asynchronous on `stream`.
  *  - Needs 2*C*(Hin+R-1)*(Win+S-1)*roundup8(B) bytes for the staged input, plus up to
- *    2*roundup8(B)*Ho*Wo*F for the staged output (not needed by unpermuted filters and by those
- *    whose permutation moves rows only within their blocks), each rounded up to 256.  More than the capacity ->
+ *    2*roundup8(B)*Ho*Wo*F for the staged output (not needed by unpermuted filters, by those
+ *    whose permutation moves rows only within their blocks, and by small outputs), each rounded up to 256.  More than the capacity ->
  *    SHFLBW_ERR_TOO_LARGE, nothing is launched.  The 32-bit range checks of shflbw_spconv_init
  *    apply as well (SHFLBW_ERR_UNSUPPORTED).
  *  - The first call on each device looks up the array's device address; make that first

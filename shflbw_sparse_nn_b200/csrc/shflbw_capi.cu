@@ -11,6 +11,7 @@
 
 #include <cuda.h>
 
+#include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -45,13 +46,13 @@ bool cuda_ok(cudaError_t e, const char* what) {
 #define CK(call) do { if (!cuda_ok((call), #call)) return SHFLBW_ERR_CUDA; } while (0)
 
 // The tuning aids of a plan, read from the environment in one pass whenever one is made (50 ns a getenv, fourteen of them a plan).
-struct Tuning { const char *tile, *swap, *gather, *epilogue_warps, *conv_planes, *box, *linear_direct; };
+struct Tuning { const char *tile, *swap, *gather, *epilogue_warps, *conv_planes, *box, *linear_direct, *conv_scatter; };
 thread_local Tuning g_tuning;
 void read_tuning() {
     static const struct { const char* name; const char* Tuning::*at; } known[] = {
         {"TILE", &Tuning::tile}, {"SWAP", &Tuning::swap}, {"GATHER", &Tuning::gather}, {"EPILOGUE_WARPS", &Tuning::epilogue_warps},
         {"CONV_PLANES", &Tuning::conv_planes}, {"BOX", &Tuning::box},
-        {"LINEAR_DIRECT", &Tuning::linear_direct}};
+        {"LINEAR_DIRECT", &Tuning::linear_direct}, {"CONV_SCATTER", &Tuning::conv_scatter}};
     g_tuning = Tuning{};
     for (char** e = environ; e && *e; ++e) {
         if (strncmp(*e, "SHFLBW_", 7)) continue;
@@ -533,7 +534,7 @@ void drop_device_copy(shflbw_matrix& m) {
 namespace {
 // Whether a linear layer on a few tokens goes to the one-launch kernel: where its blocks, of 8 tokens each, are resident at
 // once and read little.  Device time, two launches and one: 4096 x 4096, V = 64, density 0.1 on 1 / 8 / 16 / 37 / 64 tokens
-// 5.4 / 5.7 / 5.1 / 5.5 / 5.4 and 2.8 / 3.3 / 4.1 / 5.0 / 9.2 us (64: 3.5 blocks an SM, of which 3 are resident); the host gains another
+// 5.4 / 5.7 / 5.1 / 5.5 / 5.4 and 2.9 / 3.4 / 4.1 / 5.0 / 9.2 us (64: 3.5 blocks an SM, of which 3 are resident); the host gains another
 // 2.2 us.  Over 160 shapes the two are equal near 270 KB an SM, of value panels and of the 32-byte sectors of x, less 20 KB for
 // every further pass over a block's columns (3712 x 7816, density 0.086, 18 tokens, 242 KB in two passes: 6.4 and 7.5;
 // 4096 x 4096 on 37 tokens: 245 KB in one), and from five blocks an SM on (1104 x 368, V = 16, 81 tokens: 4.6 and 5.5).  Up to 8 tokens
@@ -1007,10 +1008,28 @@ bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long item
            (padded_cols >= 64ll * row_blocks || !padded_rows);
 }
 
+// Whether the panel kernel itself puts a permuted filter's positions in order, value by value: a pass less (2 us and a launch,
+// 2.2 us of the host's time), but every 32-byte sector of an F-vector is written once by each block that has a filter in it, and
+// the L2 takes some 80 of such partial sectors a clock.  So for small outputs, by the expected sectors that the busiest SM writes.
+// Device time with the pass and without, 75 shapes: up to 2500 sectors 0 to 27 % less (31x16x16x64 -> 48, V = 16, 960: 7.8 and 6.3;
+// 8x24x24x128 -> 448 at stride 2, V = 32, 2465: 7.5 and 6.8; 5x21x21x128 -> 192, V = 16, 2840: 9.9 and 8.8), then equal (5x27x27x256 -> 512
+// at stride 2, V = 32, 2860: 8.0 and 8.4, of a call that takes 12.5 us with the pass, the host's launches, and 9.6 without; 7x52x52x128 -> 208
+// at stride 2, V = 16, 4040: 21.8 and 22.0), from 5000 on up to twice as much.  Taller blocks are fewer, and more is seen of each one's
+// writes (V = 64, 5x19x19x64 -> 256, 2190: 8.0 and 7.3; 28x28x256 -> 512, 2560: 10.3 and 12.0; 3x34x34x512 -> 512 at stride 2, 3540: 10.0 and 11.1).
+bool conv_scatters(const shflbw_matrix& f, long long positions, long long items) {
+    if (g_tuning.conv_scatter) return atoi(g_tuning.conv_scatter) != 0;
+    const long long sms = sm_count() > 0 ? sm_count() : 148;
+    if (8 * items < sms) return false;                       // a few blocks keep the general form (2x12x12x128 -> 128: 6.35 us, 5.9 without the pass)
+    const double sectors = f.F / 16.0, chunk = f.brow < 32 ? f.brow : 32;
+    const double written = sectors * (1 - std::pow(1 - 1 / sectors, chunk)) * (f.F / chunk) * (double)positions;   // in all
+    return written / (double)items * (double)((items + sms - 1) / sms) <= (f.brow <= 32 ? 3200 : 2300);
+}
+
 // Launch plan of one NHWC SpConv call, without its scratch pointers: kernel choice, grid, and
 // the scratch each side needs.  Two plans exist.
 //   positions out   relayout -> panel kernel with tokens in TMEM lanes, writing [position][F] in
-//                   stored filter order -> (with a filter permutation across blocks) unpermute_filters.
+//                   stored filter order -> (with a filter permutation across blocks) unpermute_filters; small
+//                   outputs in logical order at once (conv_scatters).
 //   planes out      relayout -> panel kernel writing the output as planes [F][Ho][Wo][Bp] with plane = LOGICAL
 //                   channel (the permutation is the row index of its stores, free) -> planes_to_nhwc
 //                   transposes the planes to NHWC.  Used for permuted V = 64 / 128 filters and outputs that
@@ -1082,7 +1101,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
             // 115 columns: as planes 19.3 us, so 14.4; 25 filters of one block, 1x1 and 3x3, V = 16 to 128: 13 to 32 % less).
             out->blk_val = (const uint16_t*)f->d_val + f->kval.size();
             out->perm = nullptr;
-        } else if (f->row_permute) {
+        } else if (f->row_permute && !conv_scatters(*f, (long long)B * Ho * Wo, items)) {
             out->staged_out_bytes = (size_t)B * Ho * Wo * f->F * 2;
             if (unperm_smem_bytes(f->F) > 48 * 1024)
                 for (const void* k : {(const void*)shflbw::unpermute_filters<false>, (const void*)shflbw::unpermute_filters<true>})
@@ -1194,6 +1213,8 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     } else if (planes) {
         p.OWp = st->Wo; p.oph = 0; p.opw = 0; p.out_plane = st->Ho * st->Wo * st->Bp;
         p.out_logical = 1;                                   // plane index = logical channel
+    } else {
+        p.out_logical = st->perm && !st->staged_out;         // filters to their places, no further pass
     }
     p.idx_limit = (unsigned)((((long long)st->C - 1) * Hp * Wp + (long long)(st->R - 1) * Wp + (st->S - 1)) * st->Bp);
     p.Bn = st->B; p.Bp = st->Bp; p.Hp = Hp; p.Wp = Wp; p.Cin = st->C; p.F = st->F;

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("V,blocks,R,stride,shape", (
     (16, 1, 1, 1, (1, 5, 3, 24)), (32, 1, 3, 1, (5, 9, 7, 16)), (64, 1, 3, 1, (32, 56, 56, 64)), (128, 1, 3, 2, (9, 13, 13, 64)),
     (64, 3, 3, 1, (16, 14, 14, 64)), (16, 4, 1, 2, (3, 11, 11, 40))))
-def test_rows_within_blocks(V, blocks, R, stride, shape):
+def test_rows_within_blocks(monkeypatch, V, blocks, R, stride, shape):
     B, H, W, Cn = shape
     F, K = V * blocks, R * R * Cn
     rng = np.random.default_rng(V + blocks)
@@ -52,6 +52,7 @@ def test_rows_within_blocks(V, blocks, R, stride, shape):
         f = make(values, across.astype(np.int32))
         f.transform_and_sync_device()
         y = torch.empty((B, Ho, Wo, F), dtype=torch.float16, device="cuda")
+        monkeypatch.setenv("SHFLBW_CONV_SCATTER", "0")
         op = sb.SpconvBlockwiseOp().initialize(f, B, H, W, stride, x, y)
         assert op.launches_per_exec == 3
         op()
