@@ -126,8 +126,7 @@ struct alignas(64) PanelParams {
     int OWp, oph, opw, out_plane, relu;
     int wide_stores;         // SpMM, rows in lanes: output rows are 32-byte aligned (N % 16 == 0, D % 32 == 0)
     int trigger_late;        // SpConv ending with this kernel (nothing left to permute): lets its dependents in when its producers are done
-    int out_logical;         // chained kernels: output plane of stored filter f is perm[f] (logical channel order) instead of f;
-                             // SpConv: filter f of a position goes to perm[f]
+    int out_logical;         // chained kernels: output plane of stored filter f is perm[f] (logical channel order) instead of f
     const __half* res;       // optional residual in the OUTPUT's geometry ([planes][OHp][OWp][Bp]) or nullptr
     const int* res_map;      // stored filter -> plane of `res` (nullptr: same index)
 };
@@ -138,7 +137,9 @@ struct alignas(64) PanelParams {
 // TMEM lanes) and the T tokens the N dimension, so ONE instruction per 16 columns covers the
 // whole token tile and the accumulator comes out with an output row per lane.
 // 4 = chained SpConv with the operands swapped in the same way.
-constexpr int kPanelSpmm = 0, kPanelConv = 1, kPanelConvChain = 2, kPanelSpmmRows = 3, kPanelConvChainRows = 4;
+// 5 = SpConv writing NHWC in logical filter order, value by value (a kernel of its own: as a branch of 1 it cost that 1 to 3 %).
+constexpr int kPanelSpmm = 0, kPanelConv = 1, kPanelConvChain = 2, kPanelSpmmRows = 3, kPanelConvChainRows = 4,
+              kPanelConvScatter = 5;
 
 // GATHER: how the rows of the dense operand reach shared memory.
 //   kGatherCpAsync  16-byte cp.async per lane, written straight into the swizzled layout; the
@@ -397,7 +398,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
     static_assert(SLOTS == 0 || (MODE == kPanelConvChain && !BIAS && !ADDEND), "box epilogue: chained layers with tokens in lanes");
     constexpr int EW = Cfg::EW;                                             // epilogue warps 0..EW-1, MMA warp EW, producers after it
     constexpr bool SWAP = Cfg::SWAP;                                        // rows in TMEM lanes
-    constexpr bool CONV = MODE == kPanelConv || MODE == kPanelConvChain || MODE == kPanelConvChainRows;  // implicit-GEMM gather
+    constexpr bool NHWC = MODE == kPanelConv || MODE == kPanelConvScatter;
+    constexpr bool CONV = NHWC || MODE == kPanelConvChain || MODE == kPanelConvChainRows;  // implicit-GEMM gather
     constexpr bool CHAIN = MODE == kPanelConvChain || MODE == kPanelConvChainRows;
     constexpr bool ROWS_OUT = MODE == kPanelSpmm || MODE == kPanelConvChain; // transposing epilogue: rows out, tokens contiguous
     static_assert(EW == 8 || (ROWS_OUT && Cfg::ACC_COLS >= 128), "16 epilogue warps: transposing epilogue, >= 32 columns per warp");
@@ -462,7 +464,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         sm100::tc_fence_before_sync();
         asm volatile("bar.sync 0;" ::: "memory");
         sm100::tc_fence_after_sync();
-        if (MODE != kPanelConv || (p.perm != nullptr && !p.out_logical)) sm100::grid_dependency_launch();
+        if (!NHWC || (MODE == kPanelConv && p.perm != nullptr)) sm100::grid_dependency_launch();
     };
     // The wait itself is executed per role, as late as each role allows: by the producers after
     // their first row ids (sparse operand) are on their way and before their first gather, by the
@@ -641,7 +643,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             it += GROUPS; s += GROUPS;
             if (s >= (uint32_t)STAGES) { s -= STAGES; ph ^= 1u; }
         }
-        if (MODE == kPanelConv && p.trigger_late) sm100::grid_dependency_launch();
+        if (NHWC && p.trigger_late) sm100::grid_dependency_launch();
         }
     } else if (warp > EW) {
         // --------------------------------------------- producers (cp.async gather) ----
@@ -821,7 +823,7 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
         sm100::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && pend >= 0) sm100::mbar_arrive(&full_bar[pend]);
-        if (MODE == kPanelConv && p.trigger_late) sm100::grid_dependency_launch();
+        if (NHWC && p.trigger_late) sm100::grid_dependency_launch();
         }
     } else if (warp == EW) {
         // ------------------------------------------------------------ MMA warp ----
@@ -1085,7 +1087,8 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
             const int mbase = col0 % V;                    // first block row / filter of this warp
             bool ok = tok < p.N;
             uint32_t row_off[4], position = 0;             // SpConv: output offsets of positions i*8 + lane/4, of this lane's
-            if constexpr (MODE == kPanelConv) {
+            int positions = 0, nth = 0;
+            if constexpr (NHWC) {
                 const int pix = fast_div(tok, p.div_bp), img = tok - pix * p.Bp;
                 const int oh = fast_div(pix, p.div_row), ow = pix - oh * p.row_pix;
                 ok = ok && img < p.Bn && ow < p.Wo;
@@ -1094,7 +1097,12 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                                          : 0xffffffffu;
 #pragma unroll
                 for (int i = 0; i < 4; ++i) row_off[i] = __shfl_sync(0xffffffffu, mine, i * 8 + (lane >> 2));
-                position = ok ? mine - (uint32_t)(blk * V + mbase) : 0xffffffffu;
+                if constexpr (MODE == kPanelConvScatter) {
+                    position = mine - (uint32_t)(blk * V + mbase);
+                    const unsigned live = __ballot_sync(0xffffffffu, ok);    // not those of images beyond the batch, pixels beyond a row
+                    positions = __popc(live);
+                    nth = (int)__fns(live, 0, lane + 1);                     // the lane of the l-th of them (-1: fewer)
+                }
             }
             const bool use_c = MODE == kPanelSpmm && (EW == 8 || BIAS || Cfg::RES_BYTES > 0) && p.beta != 0.0f && p.C != nullptr;
             if constexpr (ROWS_OUT) {
@@ -1367,22 +1375,20 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     *(uint4*)(my_tile + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) = v;
                 }
                 __syncwarp();
-                if (p.perm != nullptr && p.out_logical) {
+                if constexpr (MODE == kPanelConvScatter) {
                     // Filters in logical order without a further pass: lane = filter of the chunk, one position's (CW = 16: two
                     // positions') values to wherever they belong in its F-vector.  Bound by partial sectors at the L2, about
                     // 80 a clock (5x14x14 positions of 512 filters: 2.3 us for 320,000).
                     constexpr int PER = 32 / CW;                         // positions of a store
                     const int f = __ldg(p.perm + blk * V + mbase + cc + lane % CW);
                     const uint32_t e = (uint32_t)(lane % CW);
-                    __half add = __float2half(0.f);
-                    if constexpr (BIAS) add = p.C[f];
+                    const __half add = p.C ? p.C[f] : __float2half(-0.f);   // (v + -0 is v, also for v = -0)
 #pragma unroll 8
-                    for (int i = 0; i < 32; i += PER) {
-                        const int row = i + lane / CW;
+                    for (int i = 0; i < positions; i += PER) {
+                        const int at = __shfl_sync(0xffffffffu, nth, i + lane / CW), row = at & 31;
                         const uint32_t to = __shfl_sync(0xffffffffu, position, row);
-                        __half v = *(const __half*)(my_tile + row * 64 + (((e >> 3) ^ ((row >> 1) & 3)) << 4) + (e & 7) * 2);
-                        if constexpr (BIAS) v = __hadd(v, add);
-                        if (to != 0xffffffffu) p.out[(size_t)to + f] = v;
+                        const __half v = *(const __half*)(my_tile + row * 64 + (((e >> 3) ^ ((row >> 1) & 3)) << 4) + (e & 7) * 2);
+                        if (at >= 0) p.out[(size_t)to + f] = __hadd(v, add);
                     }
                 } else {
 #pragma unroll

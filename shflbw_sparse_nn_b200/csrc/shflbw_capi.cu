@@ -244,7 +244,7 @@ bool lookup(int V, int tile, PanelChoice* out, int gather = shflbw::kGatherCpAsy
             default: return false;
         }
     } else {
-        if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConv) {
+        if constexpr (MODE == shflbw::kPanelSpmm || MODE == shflbw::kPanelConv || MODE == shflbw::kPanelConvScatter) {
             // 16-row blocks: UMMA N = 16, one or two 128-token accumulators per item (18 / 34 KB stages)
             if (V == 16 && tile == 128) { *out = regular<16, 1, 8, MODE, BIAS>(gather); return true; }
             if (V == 16 && tile == 256) { *out = regular<16, 2, 5, MODE, BIAS>(gather); return true; }
@@ -1011,18 +1011,18 @@ bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long item
 // Whether the panel kernel itself puts a permuted filter's positions in order, value by value: a pass less (2 us and a launch,
 // 2.2 us of the host's time), but every 32-byte sector of an F-vector is written once by each block that has a filter in it, and
 // the L2 takes some 80 of such partial sectors a clock.  So for small outputs, by the expected sectors that the busiest SM writes.
-// Device time with the pass and without, 75 shapes: up to 2500 sectors 0 to 27 % less (31x16x16x64 -> 48, V = 16, 960: 7.8 and 6.3;
-// 8x24x24x128 -> 448 at stride 2, V = 32, 2465: 7.5 and 6.8; 5x21x21x128 -> 192, V = 16, 2840: 9.9 and 8.8), then equal (5x27x27x256 -> 512
-// at stride 2, V = 32, 2860: 8.0 and 8.4, of a call that takes 12.5 us with the pass, the host's launches, and 9.6 without; 7x52x52x128 -> 208
-// at stride 2, V = 16, 4040: 21.8 and 22.0), from 5000 on up to twice as much.  Taller blocks are fewer, and more is seen of each one's
-// writes (V = 64, 5x19x19x64 -> 256, 2190: 8.0 and 7.3; 28x28x256 -> 512, 2560: 10.3 and 12.0; 3x34x34x512 -> 512 at stride 2, 3540: 10.0 and 11.1).
+// Device time with the pass and without, 75 shapes: up to 2500 sectors 0 to 18 % less (31x16x16x64 -> 48, V = 16, 960: 7.7 and 6.5;
+// 2x50x10x240 -> 320, 3x3, V = 64: 10.8 and 10.3; 8x24x24x128 -> 448 at stride 2, V = 32, 2465: 7.3 and 7.0; 28x28x256 -> 512, V = 64, 2560: 10.2
+// and 9.6; 5x21x21x128 -> 192, V = 16, 2840: 9.7 and 9.1), then equal (5x27x27x256 -> 512 at stride 2, V = 32, 2860: 8.1 and 8.3, of a call
+// that takes 12.5 us with the pass, the host's launches, and 9.5 without; 7x52x52x128 -> 208 at stride 2, V = 16, 4040: 21.8 and 22.0), from 5000 on
+// up to twice as much.  Taller blocks are fewer, and more is seen of each one's writes (V = 64, 3x34x34x512 -> 512 at stride 2, 3540: 9.9 and 10.8).
 bool conv_scatters(const shflbw_matrix& f, long long positions, long long items) {
     if (g_tuning.conv_scatter) return atoi(g_tuning.conv_scatter) != 0;
     const long long sms = sm_count() > 0 ? sm_count() : 148;
     if (8 * items < sms) return false;                       // a few blocks keep the general form (2x12x12x128 -> 128: 6.35 us, 5.9 without the pass)
     const double sectors = f.F / 16.0, chunk = f.brow < 32 ? f.brow : 32;
     const double written = sectors * (1 - std::pow(1 - 1 / sectors, chunk)) * (f.F / chunk) * (double)positions;   // in all
-    return written / (double)items * (double)((items + sms - 1) / sms) <= (f.brow <= 32 ? 3200 : 2300);
+    return written / (double)items * (double)((items + sms - 1) / sms) <= (f.brow <= 32 ? 3200 : 2600);
 }
 
 // Launch plan of one NHWC SpConv call, without its scratch pointers: kernel choice, grid, and
@@ -1080,12 +1080,15 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     // (planes of up to an eighth more images than positions have: not where a fixed scratch holds only these)
     const bool planes_fit = (size_t)cs.staged_elems * 2 + 256 + (size_t)f->F * (size_t)tokens * 2 + 256 <= scratch_limit;
     const bool planes = planes_possible && planes_fit && (ep ? atoi(ep) != 0 : conv_planes(*f, B, Bp, tile, items, ct.row_pix != Wo, padded_cols, row_blocks));
+    const bool scatter = !planes && f->row_permute && f->kval_logical.empty() && conv_scatters(*f, (long long)B * Ho * Wo, items);
     PanelChoice ch;
     if (planes) {
         const int ring = chain_wide(f->brow, tile, items, padded_cols, row_blocks) ? wide_ring_of(false, padded_cols, row_blocks) : 0;
         out->rows = f->brow == 64 && padded_cols >= 1200ll * row_blocks;
         rc = pick_panel<shflbw::kPanelConvChain>(f->brow, tile, out->rows, out->rows ? 0 : ring, ct.gather, &ch);
         out->wide = !out->rows && ring;
+    } else if (scatter) {
+        rc = pick_panel<shflbw::kPanelConvScatter>(f->brow, tile, false, 0, ct.gather, &ch);
     } else {
         rc = pick_panel<shflbw::kPanelConv>(f->brow, tile, false, 0, ct.gather, &ch);
     }
@@ -1101,7 +1104,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
             // 115 columns: as planes 19.3 us, so 14.4; 25 filters of one block, 1x1 and 3x3, V = 16 to 128: 13 to 32 % less).
             out->blk_val = (const uint16_t*)f->d_val + f->kval.size();
             out->perm = nullptr;
-        } else if (f->row_permute && !conv_scatters(*f, (long long)B * Ho * Wo, items)) {
+        } else if (f->row_permute && !scatter) {
             out->staged_out_bytes = (size_t)B * Ho * Wo * f->F * 2;
             if (unperm_smem_bytes(f->F) > 48 * 1024)
                 for (const void* k : {(const void*)shflbw::unpermute_filters<false>, (const void*)shflbw::unpermute_filters<true>})
@@ -1155,18 +1158,20 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     }
     const bool planes = !st->chain && st->variant == 1;     // NHWC call computed as planes, then transposed
     PanelChoice ch;
+    const bool scatter = !st->chain && !planes && st->perm && !st->staged_out;   // filters to their places, no later pass
     const bool panel_bias = bias && !planes && !st->staged_out;   // no later pass: the panel kernel's epilogue adds the bias
     const int gather = st->gather;
     // (the state is the caller's: a residual that they took away, or a map that the copies' row ids cannot be read from)
     const bool box = st->chain && st->box_res && st->residual && !((uintptr_t)st->residual_map & 15);
-    const bool ok_kernel = panel_bias            ? lookup<shflbw::kPanelConv, true>(st->V, st->tokens_per_cta, &ch, gather)
+    const bool ok_kernel = scatter               ? lookup<shflbw::kPanelConvScatter>(st->V, st->tokens_per_cta, &ch, gather)
+                           : panel_bias          ? lookup<shflbw::kPanelConv, true>(st->V, st->tokens_per_cta, &ch, gather)
                            : (!st->chain && !planes) ? lookup<shflbw::kPanelConv>(st->V, st->tokens_per_cta, &ch, gather)
                            : st->rows              ? lookup<shflbw::kPanelConvChainRows>(st->V, st->tokens_per_cta, &ch, gather)
                                                    : lookup<shflbw::kPanelConvChain>(st->V, st->tokens_per_cta, &ch, gather,
                                                                                       !st->wide ? 0 : st->residual ? 6 : st->stages,
                                                                                       st->producer_warps, box);
     if (!ok_kernel) return SHFLBW_ERR_INVALID_ARG;
-    if (panel_bias || (st->box_res && !box)) {              // (init allowed the other kernel; before anything is launched)
+    if ((panel_bias && !scatter) || (st->box_res && !box)) {              // (init allowed the other kernel; before anything is launched)
         const int rc = allow_smem(ch.fn, ch.smem);
         if (rc != SHFLBW_OK) return rc;
     }
@@ -1213,8 +1218,6 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     } else if (planes) {
         p.OWp = st->Wo; p.oph = 0; p.opw = 0; p.out_plane = st->Ho * st->Wo * st->Bp;
         p.out_logical = 1;                                   // plane index = logical channel
-    } else {
-        p.out_logical = st->perm && !st->staged_out;         // filters to their places, no further pass
     }
     p.idx_limit = (unsigned)((((long long)st->C - 1) * Hp * Wp + (long long)(st->R - 1) * Wp + (st->S - 1)) * st->Bp);
     p.Bn = st->B; p.Bp = st->Bp; p.Hp = Hp; p.Wp = Wp; p.Cin = st->C; p.F = st->F;
