@@ -1383,12 +1383,21 @@ panel_umma_kernel(const __grid_constant__ PanelParams p) {
                     const int f = __ldg(p.perm + blk * V + mbase + cc + lane % CW);
                     const uint32_t e = (uint32_t)(lane % CW);
                     const __half add = p.C ? p.C[f] : __float2half(-0.f);   // (v + -0 is v, also for v = -0)
-#pragma unroll 8
-                    for (int i = 0; i < positions; i += PER) {
-                        const int at = __shfl_sync(0xffffffffu, nth, i + lane / CW), row = at & 31;
-                        const uint32_t to = __shfl_sync(0xffffffffu, position, row);
-                        const __half v = *(const __half*)(my_tile + row * 64 + (((e >> 3) ^ ((row >> 1) & 3)) << 4) + (e & 7) * 2);
-                        if (at >= 0) p.out[(size_t)to + f] = __hadd(v, add);
+                    for (int i = 0; i < positions; i += 8 * PER) {       // eight stores' values first (one by one: 120 clocks each)
+                        int at[8];
+                        uint32_t to[8];
+                        __half v[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) at[j] = __shfl_sync(0xffffffffu, nth, i + j * PER + lane / CW);
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const int row = at[j] & 31;
+                            to[j] = __shfl_sync(0xffffffffu, position, row);
+                            v[j] = *(const __half*)(my_tile + row * 64 + (((e >> 3) ^ ((row >> 1) & 3)) << 4) + (e & 7) * 2);
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j)
+                            if (at[j] >= 0) p.out[(size_t)to[j] + f] = __hadd(v[j], add);
                     }
                 } else {
 #pragma unroll

@@ -1011,18 +1011,18 @@ bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long item
 // Whether the panel kernel itself puts a permuted filter's positions in order, value by value: a pass less (2 us and a launch,
 // 2.2 us of the host's time), but every 32-byte sector of an F-vector is written once by each block that has a filter in it, and
 // the L2 takes some 80 of such partial sectors a clock.  So for small outputs, by the expected sectors that the busiest SM writes.
-// Device time with the pass and without, 75 shapes: up to 2500 sectors 0 to 18 % less (31x16x16x64 -> 48, V = 16, 960: 7.7 and 6.5;
-// 2x50x10x240 -> 320, 3x3, V = 64: 10.8 and 10.3; 8x24x24x128 -> 448 at stride 2, V = 32, 2465: 7.3 and 7.0; 28x28x256 -> 512, V = 64, 2560: 10.2
-// and 9.6; 5x21x21x128 -> 192, V = 16, 2840: 9.7 and 9.1), then equal (5x27x27x256 -> 512 at stride 2, V = 32, 2860: 8.1 and 8.3, of a call
-// that takes 12.5 us with the pass, the host's launches, and 9.5 without; 7x52x52x128 -> 208 at stride 2, V = 16, 4040: 21.8 and 22.0), from 5000 on
-// up to twice as much.  Taller blocks are fewer, and more is seen of each one's writes (V = 64, 3x34x34x512 -> 512 at stride 2, 3540: 9.9 and 10.8).
+// Device time with the pass and without: up to 2600 sectors 1 to 15 % less (40x11x11x192 -> 96 at stride 2, V = 32, 720: 6.4 and 5.7;
+// 31x16x16x64 -> 48, V = 16, 960: 7.7 and 6.6; 2x34x34x408 -> 128, V = 32: 9.6 and 8.7; 8x24x24x128 -> 448 at stride 2, V = 32, 2465: 7.4 and 7.0;
+// 28x28x256 -> 512, V = 64, 2560: 10.2 and 10.0), then up to 5 % more, for 3 us less of the host's time (5x27x27x256 -> 512 at stride 2, V = 32,
+// 2860: 8.1 and 8.5 of a call that takes 12.5 us with the pass and 9.5 without), from 5000 on up to twice as much.  Taller blocks are
+// fewer, and more is seen of each one's writes (V = 64, 3x34x34x512 -> 512 at stride 2, 3540: 9.9 and 11.4).
 bool conv_scatters(const shflbw_matrix& f, long long positions, long long items) {
     if (g_tuning.conv_scatter) return atoi(g_tuning.conv_scatter) != 0;
     const long long sms = sm_count() > 0 ? sm_count() : 148;
     if (8 * items < sms) return false;                       // a few blocks keep the general form (2x12x12x128 -> 128: 6.35 us, 5.9 without the pass)
     const double sectors = f.F / 16.0, chunk = f.brow < 32 ? f.brow : 32;
     const double written = sectors * (1 - std::pow(1 - 1 / sectors, chunk)) * (f.F / chunk) * (double)positions;   // in all
-    return written / (double)items * (double)((items + sms - 1) / sms) <= (f.brow <= 32 ? 3200 : 2600);
+    return written / (double)items * (double)((items + sms - 1) / sms) <= (f.brow <= 32 ? 2900 : 2600);
 }
 
 // Launch plan of one NHWC SpConv call, without its scratch pointers: kernel choice, grid, and
