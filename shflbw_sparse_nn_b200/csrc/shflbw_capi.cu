@@ -998,13 +998,19 @@ bool keep_map(shflbw_tensor_map_t* kept, const PlaneMap& m) {
 // 26.6 and 24.5; 14x14x256 -> 1024 15.4 and 12.1 / 16.8 and 13.5 / 21.3 and 18.0; 56x56x64 -> 64, batch 32 20.4 and 17.7 /
 // 21.7 and 19.4 / 27.8 and 24.6; V = 128 12 to 22 % less.  Not where the planes carry an eighth more images than there are
 // (28x28x256 -> 512, batch 1, 160 columns: 12.6 and 13.3), with less than an item of 256 tokens per SM (17x17x512 -> 256, 1x1,
-// batch 24, 74 columns: 12.1 and 13.4; 14x14x256 -> 512, batch 8, 460: 10.8 and 11.1), nor for less than a stage of columns
+// batch 24, 74 columns: 12.1 and 13.4; 14x14x256 -> 512, batch 8, 460: 10.8 and 11.1) at 64 rows (at 128 from half an
+// item on: 14 shapes 4 to 12 % less, 31x31x336 -> 640, 1x1 at stride 2, batch 23, 152 columns 16.1 and 13.7), nor for less than a stage of columns
 // with padded rows (not looked at).  An unpermuted filter's positions need no further pass (28x28x256 -> 256, 1x1, batch 64,
 // 64 columns: 20.7, as planes 31.4; 14x14x512 -> 2048, 3x3, batch 16, 900: 29.0 and 33.2).
 // With filters in lanes (28.3 instead of 24.5 for 14x14x512 -> 2048, 460 columns) only at 64 rows from 1200 columns on, as
 // the chained layers (14x14x256 -> 1024, 1800 columns: 33.4, tokens 33.8).
-bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long items, bool padded_rows, long long padded_cols, int row_blocks) {
-    return f.row_permute && f.kval_logical.empty() && tile == 256 && items >= (sm_count() > 0 ? sm_count() : 148) && 8 * (Bp - B) <= Bp &&
+// Nor at 128 rows where the output is beyond 80 MB and of more than 640 filters: the last pass comes to planes that have left the
+// L2 (35x35x128 -> 1920, 1x1, batch 31, 146 MB: 112 and 142; 53x53x128 -> 768, 1x1, batch 24, 104 MB: 87 and 96; 28x28x128 -> 1280, 3x3, batch 64,
+// 128 MB: 106 and 111; but 42x42x256 -> 512, 3x3, batch 64, 116 MB: 170 and 161; 64 rows: 5 % less to 8 % more).
+bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long items, bool padded_rows, long long padded_cols, int row_blocks,
+                 long long out_bytes) {
+    if (f.brow == 128 && f.F > 640 && out_bytes > 80000000) return false;
+    return f.row_permute && f.kval_logical.empty() && tile == 256 && (f.brow == 128 || items >= (sm_count() > 0 ? sm_count() : 148)) && 8 * (Bp - B) <= Bp &&
            (padded_cols >= 64ll * row_blocks || !padded_rows);
 }
 
@@ -1079,7 +1085,8 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     const long long items = (counted + tile - 1) / tile * row_blocks;
     // (planes of up to an eighth more images than positions have: not where a fixed scratch holds only these)
     const bool planes_fit = (size_t)cs.staged_elems * 2 + 256 + (size_t)f->F * (size_t)tokens * 2 + 256 <= scratch_limit;
-    const bool planes = planes_possible && planes_fit && (ep ? atoi(ep) != 0 : conv_planes(*f, B, Bp, tile, items, ct.row_pix != Wo, padded_cols, row_blocks));
+    const bool planes = planes_possible && planes_fit && (ep ? atoi(ep) != 0 : conv_planes(*f, B, Bp, tile, items, ct.row_pix != Wo, padded_cols, row_blocks,
+                                                                                              2ll * B * Ho * Wo * f->F));
     const bool scatter = !planes && f->row_permute && f->kval_logical.empty() && conv_scatters(*f, (long long)B * Ho * Wo, items);
     PanelChoice ch;
     if (planes) {
