@@ -336,6 +336,21 @@ int pick_tile(long long n_tokens, int row_blocks) {
     return n_tokens <= 128 || rounds_of_items(n_tokens, 128, row_blocks) * 2 < rounds_of_items(n_tokens, 256, row_blocks) * 3 ? 128 : 256;
 }
 
+// The tile of an SpMM: also 128 tokens where that takes three quarters of the time's rounds (two of 256 or three of 128 for 1.0 to
+// 1.5 items per SM), from 100 columns a block on, at 128 rows from 48; and five sixths (three or five rounds) at 128 rows from 64
+// columns and at up to 32 rows from 200.  Below, an item is mostly epilogue, of which two tiles have more.  256 and 128 tokens, us:
+//   2944x1504x1752, V = 128, 246 columns 11.4 and 9.4; 9536x1256x232, V = 64, 116: 7.5 and 6.3; 5504x2744x152, V = 32, 496: 10.4 and 9.0;
+//   400x2312x1872, V = 16, 219: 6.3 and 5.9; 3712x280x1520, V = 128, 56: 6.9 and 5.9; 832x400x1520, V = 32, 39: 4.7 and 4.8;
+//   five sixths: 8576x728x1096, V = 128, 99: 15.5 and 14.0; 976x2488x1184, V = 16, 562: 13.2 and 12.3; 2912x352x416, V = 16, 123: 6.4 and 6.5;
+//   896x520x5536, V = 64, 182: 7.9 and 8.2.  Over 70 shapes on the 128 side 7 % less.
+int spmm_tile(int V, long long N, int row_blocks, long long padded_cols) {
+    const int tile = pick_tile(N, row_blocks);
+    if (tile == 128 || g_tuning.tile) return tile;
+    const long long r1 = rounds_of_items(N, 128, row_blocks), r2 = rounds_of_items(N, 256, row_blocks);
+    if (r1 * 4 <= r2 * 6 && padded_cols >= (V == 128 ? 48ll : 100ll) * row_blocks) return 128;
+    return r1 * 6 <= r2 * 10 && V != 64 && padded_cols >= (V == 128 ? 64ll : 200ll) * row_blocks ? 128 : 256;
+}
+
 // The gather of a convolution, and the pixels that an output row counts as.  TMA, unless the padding of the rows
 // costs more time in rounds of items (those of the tile that each side takes) than the gather saves: a stage takes it
 // about 650 clk and the cp.async gather 870 to 1000.  cp.async and TMA in us:
@@ -660,7 +675,7 @@ static int plan_spmm(const shflbw_matrix_t* m, int N, const void* B, float alpha
     } else {
         PanelChoice ch;
         const long long padded_cols = m->kptr.empty() ? 0 : m->kptr.back();
-        const int blocks = out->num_row_blocks, tile = pick_tile(N, blocks);
+        const int blocks = out->num_row_blocks, tile = spmm_tile(m->brow, N, blocks, padded_cols);
         const bool sectors = N % 16 == 0 && !((uintptr_t)D & 31);
         const bool wide = !swap_forced(1) && spmm_wide(m->brow, tile, N, sectors, beta != 0.f, padded_cols, blocks);
         const bool rows = !wide && spmm_rows(m->brow, tile, N, sectors, beta != 0.f, padded_cols, blocks);

@@ -165,3 +165,24 @@ def test_rows_that_start_between_sectors_keep_tokens_in_lanes():
         m.device_status()
         got.append(host(D).view(np.uint16).copy())
     assert np.array_equal(*got)
+
+
+@pytest.mark.parametrize("V,M,K,N,density,tile", (
+    (128, 2944, 1504, 1752, 0.164, 128), (64, 9536, 1256, 232, 0.093, 128), (32, 5504, 2744, 152, 0.181, 128), (16, 400, 2312, 1872, 0.095, 128),
+    (32, 832, 400, 1520, 0.099, 256), (16, 976, 2488, 1184, 0.226, 128), (64, 896, 520, 5536, 0.35, 256)))
+def test_spmm_tile_by_rounds(monkeypatch, V, M, K, N, density, tile):
+    """Two rounds of 256-token items or three of 128: the rule's sides, and the same bits either way."""
+    m = sb.BlockwiseSpMatrix().init_random(M, K, V, 1, density, True, 7, values="uniform")
+    m.transform_and_sync_device()
+    b = (torch.rand(K, N, device="cuda") * 2 - 1).half()
+    got = []
+    for forced in (None, "256", "128"):
+        if forced: monkeypatch.setenv("SHFLBW_TILE", forced)
+        d = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+        op = sb.SpmmBlockwiseOp().initialize(m, N, b, d)
+        if not forced and torch.cuda.get_device_properties(0).multi_processor_count == 148:
+            assert op._state.tokens_per_cta == tile
+        op()
+        torch.cuda.synchronize()
+        got.append(d)
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
