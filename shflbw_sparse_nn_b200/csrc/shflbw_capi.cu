@@ -343,11 +343,16 @@ int pick_tile(long long n_tokens, int row_blocks) {
 //   400x2312x1872, V = 16, 219: 6.3 and 5.9; 3712x280x1520, V = 128, 56: 6.9 and 5.9; 832x400x1520, V = 32, 39: 4.7 and 4.8;
 //   five sixths: 8576x728x1096, V = 128, 99: 15.5 and 14.0; 976x2488x1184, V = 16, 562: 13.2 and 12.3; 2912x352x416, V = 16, 123: 6.4 and 6.5;
 //   896x520x5536, V = 64, 182: 7.9 and 8.2.  Over 70 shapes on the 128 side 7 % less.
+// 16 rows and rows of B that are not whole sectors (N % 16 = 8; every second one is fetched in five sectors per box instead of four): from
+// 170 columns already at up to 19 rounds of 128 for 10 of 256 (3072x768x1000, 192 columns, 11 and 6 rounds: 14.7 and 13.5; 2880x3104x1208,
+// 415, 13 and 7: 24.0 and 23.2; 37 shapes 0.91 to 1.02, 4 % less; with whole sectors 3072x768x1024 10.9 and 12.0; 133 columns,
+// 9584x928x440: 14.4 and 15.3).
 int spmm_tile(int V, long long N, int row_blocks, long long padded_cols) {
     const int tile = pick_tile(N, row_blocks);
     if (tile == 128 || g_tuning.tile) return tile;
     const long long r1 = rounds_of_items(N, 128, row_blocks), r2 = rounds_of_items(N, 256, row_blocks);
     if (r1 * 4 <= r2 * 6 && padded_cols >= (V == 128 ? 48ll : 100ll) * row_blocks) return 128;
+    if (V == 16 && N % 16 && r2 >= 4 && r1 * 20 <= r2 * 38 && padded_cols >= 170ll * row_blocks) return 128;
     return r1 * 6 <= r2 * 10 && V != 64 && padded_cols >= (V == 128 ? 64ll : 200ll) * row_blocks ? 128 : 256;
 }
 

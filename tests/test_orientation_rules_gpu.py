@@ -169,7 +169,7 @@ def test_rows_that_start_between_sectors_keep_tokens_in_lanes():
 
 @pytest.mark.parametrize("V,M,K,N,density,tile", (
     (128, 2944, 1504, 1752, 0.164, 128), (64, 9536, 1256, 232, 0.093, 128), (32, 5504, 2744, 152, 0.181, 128), (16, 400, 2312, 1872, 0.095, 128),
-    (32, 832, 400, 1520, 0.099, 256), (16, 976, 2488, 1184, 0.226, 128), (64, 896, 520, 5536, 0.35, 256)))
+    (32, 832, 400, 1520, 0.099, 256), (16, 976, 2488, 1184, 0.226, 128), (64, 896, 520, 5536, 0.35, 256), (16, 3072, 768, 1000, 0.25, 128), (16, 3072, 768, 1024, 0.25, 256)))
 def test_spmm_tile_by_rounds(monkeypatch, V, M, K, N, density, tile):
     """Two rounds of 256-token items or three of 128: the rule's sides, and the same bits either way."""
     m = sb.BlockwiseSpMatrix().init_random(M, K, V, 1, density, True, 7, values="uniform")
