@@ -67,7 +67,8 @@ __global__ void __launch_bounds__(256) linear_direct(const DirectParams p) {
         sm100::cp_async_commit();
         int id[RUNS];
 #pragma unroll
-        for (int s = 0; s < RUNS; ++s) id[s] = mine && s * 32 + lane < n ? __ldg(p.blk_idx + row0 + c0 + s * 32 + lane) : -1;
+        for (int s = 0; s < RUNS; ++s)                        // (clamped: a corrupted id may give wrong numbers, never an address outside x)
+            id[s] = mine && s * 32 + lane < n ? (int)min((unsigned)__ldg(p.blk_idx + row0 + c0 + s * 32 + lane), (unsigned)p.K - 1u) : -1;
         if (c0 == 0) sm100::grid_dependency_wait();           // x may be the previous kernel's output
         unsigned short v[RUNS];                               // sixteen runs of 32 columns in flight
 #pragma unroll

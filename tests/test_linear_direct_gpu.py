@@ -87,3 +87,26 @@ def test_rule_and_module():
     assert not bw.linear_direct(odd, 8, x, None, 8, torch.empty(48, 8, dtype=torch.float16, device="cuda"))
     with pytest.raises(Exception):
         bw.linear_direct(m, 0, x, None, 8, x)
+
+
+class _Ints:
+    """Device memory as a tensor."""
+    def __init__(self, address, n):
+        self.__cuda_array_interface__ = {"shape": (n,), "typestr": "<i4", "data": (address, False), "version": 3}
+
+
+def test_ids_outside_the_layer_read_nothing_outside_x(monkeypatch):
+    """The ids lie in device memory: whatever stands there, the reads stay in x (the last column's, as the panel kernel's do)."""
+    monkeypatch.setenv("SHFLBW_LINEAR_DIRECT", "1")
+    K, tokens, N = 96, 11, 16
+    m = _matrix(32, K, (40, 96), True)
+    x = (torch.rand(tokens, K, device="cuda") * 2 - 1).half()
+    out = [torch.full((m.nrow, N), float("nan"), dtype=torch.float16, device="cuda") for _ in range(2)]
+    op = sb.SpmmBlockwiseOp().initialize(m, N, torch.zeros(K, N, device="cuda").half(), out[0])
+    ids = torch.as_tensor(_Ints(op._state.blk_idx, 48 + 96), device="cuda")
+    at = torch.tensor([0, 7, 39, 47, 48, 143], device="cuda")
+    for y, bad in zip(out, ([K, K + 5, 2 ** 31 - 1, -1, -2 ** 31, 1 << 20], [K - 1] * 6)):
+        ids[at] = torch.tensor(bad, dtype=torch.int32, device="cuda")
+        assert bw.linear_direct(m, tokens, x, None, N, y, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+    assert torch.equal(*out) and not out[0].isnan().any()
