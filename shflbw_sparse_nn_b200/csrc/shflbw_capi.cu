@@ -1105,9 +1105,16 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     const long long items = (counted + tile - 1) / tile * row_blocks;
     // (planes of up to an eighth more images than positions have: not where a fixed scratch holds only these)
     const bool planes_fit = (size_t)cs.staged_elems * 2 + 256 + (size_t)f->F * (size_t)tokens * 2 + 256 <= scratch_limit;
-    const bool planes = planes_possible && planes_fit && (ep ? atoi(ep) != 0 : conv_planes(*f, B, Bp, tile, items, ct.row_pix != Wo, padded_cols, row_blocks,
-                                                                                              2ll * B * Ho * Wo * f->F));
-    const bool scatter = !planes && f->row_permute && f->kval_logical.empty() && conv_scatters(*f, (long long)B * Ho * Wo, items);
+    // The last pass of permuted positions holds the permutation and an F-vector for each position of a block in shared memory
+    // (up to 23 244 filters).  Beyond, planes whatever they cost (the same for all sizes of a layer: no small output goes
+    // through the scattering kernel either).
+    const bool across = f->row_permute && f->kval_logical.empty();        // filters leave their blocks
+    const bool pass_fits = !across || (unperm_smem_bytes(f->F) <= 227 * 1024 && f->F <= 65536);
+    const bool planes = planes_possible && (ep ? planes_fit && atoi(ep) != 0
+                                               : !pass_fits || (planes_fit && conv_planes(*f, B, Bp, tile, items, ct.row_pix != Wo, padded_cols, row_blocks,
+                                                                                          2ll * B * Ho * Wo * f->F)));
+    if (!planes && !pass_fits) return SHFLBW_ERR_UNSUPPORTED;
+    const bool scatter = !planes && across && conv_scatters(*f, (long long)B * Ho * Wo, items);
     PanelChoice ch;
     if (planes) {
         const int ring = chain_wide(f->brow, tile, items, padded_cols, row_blocks) ? wide_ring_of(false, padded_cols, row_blocks) : 0;
@@ -1125,13 +1132,12 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
         out->staged_out_bytes = (size_t)f->F * (size_t)tokens * 2;
     } else {
         out->variant = 0;
-        if (f->row_permute && (unperm_smem_bytes(f->F) > 227 * 1024 || f->F > 65536)) return SHFLBW_ERR_UNSUPPORTED;
         if (!f->kval_logical.empty()) {
             // Rows in logical order: as an unpermuted filter, no pass behind the kernel (56x56x64 -> 64, 3x3, batch 32, V = 64,
             // 115 columns: as planes 19.3 us, so 14.4; 25 filters of one block, 1x1 and 3x3, V = 16 to 128: 13 to 32 % less).
             out->blk_val = (const uint16_t*)f->d_val + f->kval.size();
             out->perm = nullptr;
-        } else if (f->row_permute && !scatter) {
+        } else if (across && !scatter) {
             out->staged_out_bytes = (size_t)B * Ho * Wo * f->F * 2;
             if (unperm_smem_bytes(f->F) > 48 * 1024)
                 for (const void* k : {(const void*)shflbw::unpermute_filters<false>, (const void*)shflbw::unpermute_filters<true>})

@@ -14,7 +14,7 @@ from conftest import assert_close_fp16
 from gpu_util import dev, host, run_spconv
 from shflbw_sparse_nn_b200 import _cabi
 from shflbw_sparse_nn_b200.build import build_fault_inject_library
-from shflbw_sparse_nn_b200.nn import ShflBWConv2d
+from shflbw_sparse_nn_b200.nn import ShflBWConv2d, densify
 
 pytestmark = pytest.mark.gpu
 
@@ -100,3 +100,35 @@ def test_strided_1x1_filters_stage_only_the_pixels_they_visit(Bn, H, W, stride, 
     assert np.array_equal(y.view(np.uint16), sub.view(np.uint16))
     ref = oa.spconv_ref_nhwc(Bn, H, W, C, 2 * V, 1, 1, stride, V, f.indptr, f.indices, f.values, f.row_permute_ids, x)
     assert_close_fp16(y, ref, what="strided 1x1 vs oracle")
+
+
+@pytest.mark.parametrize("V,C,R,Bn,H", [
+    (64, 24, 3, 1, 4), (64, 24, 3, 9, 5), (128, 24, 3, 2, 5),      # 216 columns a block; images beyond the batch, 128-token tiles
+    (128, 24, 3, 16, 14),                                          # an output of 146 MB
+    (64, 24, 1, 3, 4),                                             # 24 columns
+])
+def test_more_filters_than_the_inverse_permutation_holds(V, C, R, Bn, H):
+    F = 23296                                                      # that pass: 10 F bytes of shared memory, 23 244 filters
+    f = sb.BlockwiseSpFilter().init_random(F, R, R, C, V, 1, 1.0, True, 33, values="uniform")
+    f.transform_and_sync_device()
+    x = dev(sb.uniform_half(34, Bn * H * H * C).reshape(Bn, H, H, C))
+    y = torch.full((Bn, H, H, F), float("nan"), dtype=torch.float16, device="cuda")
+    sb.SpconvBlockwiseOp().initialize(f, Bn, H, H, 1, x, y)(torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    f.device_status()
+    w = torch.from_numpy(densify(f)).cuda().double()
+    halo = torch.nn.functional.pad(x.double(), (0, 0, R // 2, R // 2, R // 2, R // 2))
+    cols = torch.cat([halo[:, r:r + H, s:s + H] for r in range(R) for s in range(R)], 3).reshape(-1, R * R * C)
+    want, size = cols @ w.t(), cols.abs() @ w.abs().t()
+    # 32-bit sums of n products in any order, n * 2^-23 * sum |a b| (sums chopped, not rounded), and a rounding to fp16
+    assert ((y.reshape(-1, F).double() - want).abs() <= R * R * C * 2.0 ** -23 * size + want.abs() * 2.0 ** -11 + 2.0 ** -25).all()
+
+
+def test_filters_of_few_rows_a_block_keep_that_limit():
+    for Bn in (1, 64):                                             # no planes for 32 rows: refused for every size
+        f = sb.BlockwiseSpFilter().init_random(23296, 1, 1, 8, 32, 1, 1.0, True, 35, values="uniform")
+        f.transform_and_sync_device()
+        x, y = (torch.zeros(Bn * 16 * n, dtype=torch.float16, device="cuda") for n in (8, 23296))
+        with pytest.raises(sb.ShflbwError) as e:
+            sb.SpconvBlockwiseOp().initialize(f, Bn, 4, 4, 1, x, y)
+        assert e.value.status == _cabi.ERR_UNSUPPORTED
