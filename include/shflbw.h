@@ -161,14 +161,6 @@ const int* shflbw_matrix_meta_image(const shflbw_matrix_t* m, size_t* n_int32);
 
 /* ------------------------------------------------------------------------- SpMM ---- */
 
-/* A TMA tensor map (opaque 128 bytes) kept in a state, and the address and extents that it is of: exec builds its own
- * where the state's owner has exchanged the operand. */
-typedef struct shflbw_tensor_map {
-    unsigned long long map[16];
-    const void* of;
-    long long rows, cols, pitch;
-} shflbw_tensor_map_t;
-
 /* Replaces SpmmBlockwiseOpState (block_sparse/spmm/blockwise_op.h:6-17): a POD the caller
  * may copy.  Holds non-owning device pointers: the matrix handle and B, C, D must outlive it. */
 typedef struct shflbw_spmm_state {
@@ -279,13 +271,13 @@ typedef struct shflbw_spconv_state {
     int relu;                /* 1: max(x, 0) fused into the epilogue                    */
     const void* residual;    /* chained: optional residual chain buffer (output geometry) */
     const int* residual_map; /* chained: stored filter -> plane of `residual`, or NULL     */
-    int gather;              /* 0: cp.async gather, 1: TMA tile-gather                     */
+    unsigned char gather;    /* 0: cp.async gather, 1: TMA tile-gather                     */
+    unsigned char rows;      /* 1: filters in TMEM lanes, 0: tokens                        */
+    unsigned char wide;      /* 1: sixteen epilogue warps                                  */
+    unsigned char box_res;   /* chained layers: 1 = the residual arrives in boxes of 64 tokens by TMA (these four bytes
+                                were `int gather`, which a caller built then finds in the low byte) */
     int row_pix;             /* pixels that an output row counts as (>= Wo; the TMA gather may round rows up to whole
                                 boxes): tiles_n and num_items are of Ho * row_pix * Bp tokens */
-    int rows;                /* 1: filters in TMEM lanes, 0: tokens                        */
-    int wide;                /* 1: sixteen epilogue warps                                  */
-    int box_res;             /* chained layers: 1 = the residual arrives in boxes of 64 tokens by TMA */
-    shflbw_tensor_map_t map_in, map_res; /* chained layers: input and residual planes */
 } shflbw_spconv_state_t;
 
 /* Replaces SpconvBlockwiseOp::initialize / SpconvBlockwiseInitFn

@@ -25,12 +25,6 @@ class ShflbwError(RuntimeError):
         super().__init__(f"{where}: status {status} ({detail})")
 
 
-class TensorMap(C.Structure):
-    """Mirror of shflbw_tensor_map_t."""
-    _fields_ = [("map", C.c_ulonglong * 16), ("of", C.c_void_p), ("rows", C.c_longlong), ("cols", C.c_longlong),
-                ("pitch", C.c_longlong)]
-
-
 class SpmmState(C.Structure):
     """Mirror of shflbw_spmm_state_t."""
     _fields_ = [
@@ -65,8 +59,7 @@ class SpconvState(C.Structure):
         ("perm", C.c_void_p), ("status_word", C.c_void_p),
         ("chain", C.c_int), ("out_R", C.c_int), ("out_S", C.c_int), ("relu", C.c_int),
         ("residual", C.c_void_p), ("residual_map", C.c_void_p),
-        ("gather", C.c_int), ("row_pix", C.c_int),
-        ("rows", C.c_int), ("wide", C.c_int), ("box_res", C.c_int), ("map_in", TensorMap), ("map_res", TensorMap),
+        ("gather", C.c_ubyte), ("rows", C.c_ubyte), ("wide", C.c_ubyte), ("box_res", C.c_ubyte), ("row_pix", C.c_int),
     ]
 
 

@@ -172,15 +172,6 @@ int encode_map(const void* base, long long rows, long long cols, long long pitch
     return SHFLBW_OK;
 }
 
-// The same into `out` by way of a state's kept map: copied where that is of this very operand, made anew where not.
-int encode_map(const void* base, long long rows, long long cols, long long pitch, const shflbw_tensor_map_t& kept, unsigned long long out[16]) {
-    if (base && kept.of == base && kept.rows == rows && kept.cols == cols && kept.pitch == pitch) {
-        std::memcpy(out, kept.map, sizeof kept.map);
-        return SHFLBW_OK;
-    }
-    return encode_map(base, rows, cols, pitch, out);
-}
-
 // Pipeline shape per (V, tile): non-zero columns per stage (KS) and ring depth (as many stages
 // as fit beside the 16 KB of epilogue tiles).
 // Shapes of the TMA gather: four stages at a time, by two warps each, SpMM with rows in lanes by four: its items are
@@ -643,6 +634,10 @@ int shflbw_matrix_device_status(const shflbw_matrix_t* m) {
     return SHFLBW_OK;
 }
 
+// Callers hold these states by value: their sizes belong to the version that shflbw_abi_version() gives, and a new field to a
+// new one (or into bytes that are there).
+static_assert(sizeof(shflbw_spmm_state_t) == 304 && sizeof(shflbw_spconv_state_t) == 232, "layout of ABI version 1");
+
 // ------------------------------------------------------------------------------ SpMM --
 
 static int plan_spmm(const shflbw_matrix_t* m, int N, const void* B, float alpha, const void* C,
@@ -1006,12 +1001,6 @@ PlaneMap output_map(const shflbw_spconv_state_t& st, const void* base) {
 bool boxes_fit(const shflbw_spconv_state_t& st) {
     return st.row_pix == st.Wo && (st.out_S == 1 || (long long)st.Wo * st.Bp % 64 == 0);
 }
-bool keep_map(shflbw_tensor_map_t* kept, const PlaneMap& m) {
-    if (encode_map(m.base, m.rows, m.cols, m.pitch, kept->map) != SHFLBW_OK) return false;
-    kept->of = m.base; kept->rows = m.rows; kept->cols = m.cols; kept->pitch = m.pitch;
-    return true;
-}
-
 // Whether an NHWC call of a permuted filter is computed as planes (below): they leave the panel kernel in runs of 64 bytes,
 // the inverse permutation being an address, and the transposing pass reads and writes runs of 128.  Positions out and planes
 // out (tokens in lanes), 40 / 110 / 460 columns a block: 14x14x512 -> 2048, 3x3, batch 16, V = 64 17.6 and 15.7 / 18.6 and 16.7 /
@@ -1220,7 +1209,7 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     p.row_pix = st->row_pix;
     if (gather == shflbw::kGatherTma) {
         const PlaneMap m = input_map(*st, p.Xs, Hp, Wp, p.stride);
-        const int rc = encode_map(m.base, m.rows, m.cols, m.pitch, st->map_in, p.tmap_b);
+        const int rc = encode_map(m.base, m.rows, m.cols, m.pitch, p.tmap_b);
         if (rc != SHFLBW_OK) return rc;
     }
     long long relayout_per_sm = 0;
@@ -1245,7 +1234,7 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
         if (box) {
             if (!boxes_fit(*st)) return SHFLBW_ERR_INVALID_ARG;
             const PlaneMap m = output_map(*st, st->residual);
-            const int rc = encode_map(m.base, m.rows, m.cols, m.pitch, st->map_res, p.tmap_res);
+            const int rc = encode_map(m.base, m.rows, m.cols, m.pitch, p.tmap_res);
             if (rc != SHFLBW_OK) return rc;
         }
     } else if (planes) {
@@ -1402,17 +1391,15 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, f->brow, row_blocks, padded_cols,
                                       rows_in_lanes(f->brow, is_deep(padded_cols, row_blocks)), true);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
-    out->gather = ct.gather; out->row_pix = ct.row_pix;
     const int tile = pick_tile(counted, row_blocks);
     const long long items = (counted + tile - 1) / tile * row_blocks;
     const bool rows = chain_rows(f->brow, S_next > 1 && tma_row_pix(Wo, Win + f->S - 1, Bp, stride) > Wo, items, padded_cols, row_blocks);
     const int ring = !rows && chain_wide(f->brow, tile, items, padded_cols, row_blocks) ? wide_ring_of(false, padded_cols, row_blocks) : 0;
     int rc = pick_panel<shflbw::kPanelConvChain>(f->brow, tile, rows, ring, ct.gather, &ch);
     if (rc != SHFLBW_OK) return rc;
-    if (ch.gather == shflbw::kGatherTma && !keep_map(&out->map_in, input_map(*out, in_chain, Hin + f->R - 1, Win + f->S - 1, stride))) return SHFLBW_ERR_CUDA;
     out->kernel = SHFLBW_KERNEL_TCGEN05;
     out->tokens_per_cta = ch.tokens; out->stages = ch.stages; out->producer_warps = ch.pw; out->variant = ch.variant;
-    out->gather = ch.gather; out->rows = rows; out->wide = ch.variant == 2;
+    out->gather = ch.gather; out->row_pix = ct.row_pix; out->rows = rows; out->wide = ch.variant == 2;
     out->tiles_n = (int)((counted + ch.tokens - 1) / ch.tokens);
     out->num_items = out->tiles_n * row_blocks;
     const int sms = sm_count();
@@ -1461,8 +1448,6 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
                        (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !g_tuning.epilogue_warps &&
                         padded_cols <= 128ll * (st->F / st->V) && 2ll * st->num_items >= 5ll * sm_count())) &&
                       lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6, two_warps ? 2 : 3, box);
-    shflbw_tensor_map_t map_res{};
-    if (wide && box && !keep_map(&map_res, output_map(*st, res_chain))) return SHFLBW_ERR_CUDA;
     if (wide) {
         const int rc = allow_smem(ch.fn, ch.smem);
         if (rc != SHFLBW_OK) return rc;
@@ -1484,7 +1469,6 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     // Nothing can fail from here on: a refused call leaves the state as it was.
     st->residual = res_chain;
     st->residual_map = map_dev;
-    st->map_res = map_res;
     st->box_res = wide && box;
     if (wide) {
         st->variant = 2; st->wide = 1; st->stages = ch.stages; st->producer_warps = ch.pw; st->block_x = ch.threads; st->shared_mem_size = ch.smem;

@@ -43,6 +43,19 @@ def test_state_structs_match_the_header_field_order():
         assert names == [f[0] for f in cls._fields_], struct
 
 
+def test_states_keep_the_size_that_belongs_to_the_abi_version():
+    """A caller holds a state by value, and an init clears it: not a byte beyond what a caller of this version has."""
+    l = _cabi.lib()
+    assert (l.shflbw_abi_version(), C.sizeof(_cabi.SpmmState), C.sizeof(_cabi.SpconvState)) == (1, 304, 232)
+    assert _cabi.SpconvState.gather.offset == 224 and _cabi.SpconvState.row_pix.offset == 228
+    for name, args, cls in (("spmm_init", (None, 64, 16, 1.0, None, 0.0, 32, 0), _cabi.SpmmState),
+                            ("spconv_init", (None, 8, 6, 6, 1, 16, 32, 1.0, 0), _cabi.SpconvState),
+                            ("spconv_chain_init", (None, 8, 6, 6, 1, 16, 32, 3, 3, 1.0, 0), _cabi.SpconvState)):
+        held = (C.c_ubyte * 1024)(*([0xAB] * 1024))
+        assert getattr(l, f"shflbw_{name}")(*args, C.cast(held, C.POINTER(cls))) == _cabi.ERR_INVALID_ARG
+        assert set(bytes(held)[C.sizeof(cls):]) == {0xAB}
+
+
 def test_strerror_covers_all_codes():
     l = _cabi.lib()
     texts = {l.shflbw_strerror(i).decode() for i in range(8)}
