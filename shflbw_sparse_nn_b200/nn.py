@@ -130,7 +130,8 @@ class ShflBWLinear(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         native = _cabi.native()
         if native is not None:                               # plain operands: everything below as one native call
-            y = native.linear(x, _bias_of(self), self.spmat._h.value or 0, self.in_features, self.out_features)
+            spmat = self.spmat                               # (held: the call has its address only, and lets other threads run)
+            y = native.linear(x, _bias_of(self), spmat._h.value or 0, self.in_features, self.out_features)
             if y is not None:
                 return y
         _require_cuda_half(x, "ShflBWLinear")
@@ -192,7 +193,8 @@ class ShflBWConv2d(nn.Module):
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         native = _cabi.native()
         if native is not None:                               # plain operands: everything below as one native call
-            y = native.conv2d(x, _bias_of(self), self.spfilter._h.value or 0, self.stride, self.in_channels, self.out_channels)
+            spfilter = self.spfilter                         # (held, as above)
+            y = native.conv2d(x, _bias_of(self), spfilter._h.value or 0, self.stride, self.in_channels, self.out_channels)
             if y is not None:
                 return y
         _require_cuda_half(x, "ShflBWConv2d")

@@ -1,12 +1,16 @@
 """Which tensors the module front end hands to the kernels by address.  A kernel reads memory, so a
 tensor whose memory does not hold its values (a pending negation, a wrapper subclass) or whose
 addition has to be recorded by autograd must go through torch instead."""
+import weakref
+
 import pytest
 import torch
 from torch.autograd import forward_ad
 from torch.utils._pytree import tree_map
 
+import shflbw_sparse_nn_b200 as sb
 import shflbw_sparse_nn_b200.nn as sbnn
+from shflbw_sparse_nn_b200 import _cabi
 
 CPU = torch.device("cpu")
 
@@ -46,6 +50,27 @@ def test_bias_that_autograd_follows_is_not_fused():
     with forward_ad.dual_level():
         assert not sbnn._fused_bias(forward_ad.make_dual(torch.ones(16).half(), torch.ones(16).half()), CPU, 16, 2)[1]
         assert sbnn._fused_bias(torch.ones(16).half(), CPU, 16, 2)[1]
+
+
+def test_a_native_call_holds_its_operand(monkeypatch):
+    """The call gets an address and releases the GIL: what another thread then binds to the module must not free it."""
+    lin = sbnn.ShflBWLinear(sb.BlockwiseSpMatrix().init_random(64, 64, 32, 1, 0.2, True, 1, values="uniform"), None)
+    conv = sbnn.ShflBWConv2d(sb.BlockwiseSpFilter().init_random(64, 1, 1, 8, 32, 1, 0.5, True, 1, values="uniform"), 1, None)
+    for module, name in ((lin, "spmat"), (conv, "spfilter")):
+        operand = weakref.ref(getattr(module, name))
+        alive = []
+
+        class Native:
+            @staticmethod
+            def linear(*args):
+                setattr(module, name, None)              # as another thread may meanwhile
+                alive.append(operand() is not None)
+                return args[0]
+            conv2d = linear
+
+        monkeypatch.setattr(_cabi, "native", lambda: Native)
+        x = torch.zeros(1)
+        assert module(x) is x and alive == [True] and operand() is None
 
 
 @pytest.mark.gpu
