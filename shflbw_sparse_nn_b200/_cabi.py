@@ -172,7 +172,8 @@ _native, _native_of = None, None
 
 def native():
     """The native host path of a call (csrc/native_calls.cpp) bound to the loaded library; None where it has not been
-    built or torch, whose tensors it handles, is not in use: ctypes and the modules' Python code do the same."""
+    built, or for another torch, or torch, whose tensors it handles, is not in use: ctypes and the modules' Python code
+    do the same."""
     if _lib is not None and _native_of is _lib:
         return _native
     return _bind_native()
@@ -187,9 +188,15 @@ def _bind_native():
         from . import _native as module
     except ImportError:
         module = None
-    if module is not None and not module.bind(*(C.cast(getattr(library, f"shflbw_{name}"), C.c_void_p).value for name in (
-            "spmm_exec", "spconv_exec", "spconv_exec_bias", "spconv_init", "linear_exec", "linear_direct")), C.sizeof(SpconvState)):
-        module = None
+    if module is not None:
+        addresses = [C.cast(getattr(library, f"shflbw_{name}"), C.c_void_p).value for name in (
+            "spmm_exec", "spconv_exec", "spconv_exec_bias", "spconv_init", "linear_exec", "linear_direct")]
+        try:
+            bound = module.bind(*addresses, C.sizeof(SpconvState), str(sys.modules["torch"].__version__))
+        except TypeError:                                    # built beside another version of this file
+            bound = False
+        if not bound:
+            module = None
     _native, _native_of = module, library
     return module
 

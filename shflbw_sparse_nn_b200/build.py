@@ -92,18 +92,25 @@ NATIVE_PATH = PKG_DIR / "_native.so"
 NATIVE_SOURCE = PKG_DIR / "csrc" / "native_calls.cpp"
 
 
+def native_is_current(torch_version: str) -> bool:
+    """Whether `_native.so` is as new as its sources and was compiled for this torch, whose tensors it takes apart."""
+    deps = [NATIVE_SOURCE, REPO_ROOT / "include" / "shflbw.h"]
+    return NATIVE_PATH.exists() and all(d.stat().st_mtime <= NATIVE_PATH.stat().st_mtime for d in deps) \
+        and f"compiled for torch {torch_version}\0".encode() in NATIVE_PATH.read_bytes()
+
+
 def build_native(force: bool = False) -> Path:
     """Compile the native host path (`_native.so`, a CPython module over torch's C++ tensors)."""
     import sysconfig
 
     import torch
 
-    deps = [NATIVE_SOURCE, REPO_ROOT / "include" / "shflbw.h"]
-    if not force and NATIVE_PATH.exists() and all(d.stat().st_mtime <= NATIVE_PATH.stat().st_mtime for d in deps):
+    if not force and native_is_current(str(torch.__version__)):
         return NATIVE_PATH
     root = Path(torch.__file__).resolve().parent
     cuda = Path(_nvcc()).resolve().parents[1]
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           f'-DSHFLBW_TORCH_VERSION="{torch.__version__}"',
            "-I", str(REPO_ROOT / "include"), "-I", sysconfig.get_paths()["include"], "-I", str(root / "include"),
            "-I", str(root / "include" / "torch" / "csrc" / "api" / "include"), "-I", str(cuda / "include"),
            "-o", str(NATIVE_PATH), str(NATIVE_SOURCE),

@@ -2,7 +2,8 @@
 // usually is.  A launch costs the driver 2.2 us; around it, through ctypes and torch's Python operators, a call of a bound operator
 // took 3.3 us, of a linear layer 19 (two launches, two allocations, a view), of a convolution module 23 (three launches).
 //
-//   bind               the addresses of the library's functions; False where the states of the two builds differ
+//   bind               the addresses of the library's functions; False where the states of the two builds differ, or torch is not
+//                      the one whose headers this module was compiled with (they lay out at::Tensor)
 //   spmm / spconv      one call of a bound operator, by the address of its state
 //   linear / conv2d    one forward of a module, for plain operands; None for everything else (subclasses, operands under a
 //                      transform, a mode or a trace, values not in memory, gradients to record, another device, layouts that
@@ -12,6 +13,8 @@
 // a call is enqueued, as ctypes does: a launch may wait for room in the queue.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
+
+#include <cstring>
 
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/core/Tensor.h>
@@ -36,10 +39,11 @@ decltype(&shflbw_linear_direct) linear_direct = nullptr;
 PyObject* name_cuda_stream = nullptr;
 
 PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
-    if (n != 7) { PyErr_SetString(PyExc_TypeError, "bind(spmm_exec, spconv_exec, spconv_exec_bias, spconv_init, linear_exec, linear_direct, size of a state)"); return nullptr; }
+    if (n != 8) { PyErr_SetString(PyExc_TypeError, "bind(spmm_exec, spconv_exec, spconv_exec_bias, spconv_init, linear_exec, linear_direct, size of a state, torch.__version__)"); return nullptr; }
     const long long size = PyLong_AsLongLong(args[6]);
+    const char* const torch_version = PyUnicode_AsUTF8(args[7]);
     if (PyErr_Occurred()) return nullptr;
-    if (size != (long long)sizeof(shflbw_spconv_state_t)) Py_RETURN_FALSE;      // built beside another header
+    if (size != (long long)sizeof(shflbw_spconv_state_t) || strcmp(torch_version, SHFLBW_TORCH_VERSION)) Py_RETURN_FALSE;
     void* a[6];
     for (int i = 0; i < 6; ++i)
         if (!(a[i] = PyLong_AsVoidPtr(args[i]))) { if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "null address"); return nullptr; }
@@ -194,7 +198,9 @@ PyMethodDef methods[] = {
     {"linear", (PyCFunction)(void (*)())linear, METH_FASTCALL, "forward of a linear layer, or None"},
     {"conv2d", (PyCFunction)(void (*)())conv2d, METH_FASTCALL, "forward of a convolution module, or None"},
     {nullptr, nullptr, 0, nullptr}};
-PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "host path of a call", -1, methods, nullptr, nullptr, nullptr, nullptr};
+// (build.py looks for the end of this text in the built file)
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_native", "host path of a call, compiled for torch " SHFLBW_TORCH_VERSION, -1, methods,
+                      nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 
