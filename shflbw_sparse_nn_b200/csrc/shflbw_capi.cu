@@ -11,13 +11,12 @@
 
 #include <cuda.h>
 
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
 #include <utility>
-
-#include <unistd.h>
 
 #include "aux_kernels.cuh"
 #include "linear_direct.cuh"
@@ -45,23 +44,10 @@ bool cuda_ok(cudaError_t e, const char* what) {
 }
 #define CK(call) do { if (!cuda_ok((call), #call)) return SHFLBW_ERR_CUDA; } while (0)
 
-// The tuning aids of a plan, read from the environment in one pass whenever one is made (50 ns a getenv, fourteen of them a plan).
-struct Tuning { const char *tile, *swap, *gather, *epilogue_warps, *conv_planes, *box, *linear_direct, *conv_scatter; };
-thread_local Tuning g_tuning;
-void read_tuning() {
-    static const struct { const char* name; const char* Tuning::*at; } known[] = {
-        {"TILE", &Tuning::tile}, {"SWAP", &Tuning::swap}, {"GATHER", &Tuning::gather}, {"EPILOGUE_WARPS", &Tuning::epilogue_warps},
-        {"CONV_PLANES", &Tuning::conv_planes}, {"BOX", &Tuning::box},
-        {"LINEAR_DIRECT", &Tuning::linear_direct}, {"CONV_SCATTER", &Tuning::conv_scatter}};
-    g_tuning = Tuning{};
-    for (char** e = environ; e && *e; ++e) {
-        if (strncmp(*e, "SHFLBW_", 7)) continue;
-        for (const auto& k : known) {
-            const size_t n = strlen(k.name);
-            if (!strncmp(*e + 7, k.name, n) && (*e)[7 + n] == '=' && !(g_tuning.*k.at)) g_tuning.*k.at = *e + 8 + n;
-        }
-    }
-}
+// A tuning aid: the number that the environment gives at this moment, kUnset without one.  Read where it is asked for (50 ns), so that
+// no pointer into the environment, which another thread may change, is kept.
+constexpr int kUnset = INT_MIN;
+int tuned(const char* name) { const char* e = getenv(name); return e ? atoi(e) : kUnset; }
 
 // Every kernel of this library is launched with the programmatic-stream-serialization attribute:
 // it may start while the previous kernel of the stream drains, sets itself up (barriers, TMEM,
@@ -286,7 +272,7 @@ int tma_row_pix(int Wo, int Wp, int Bp, int stride) {
 
 // SHFLBW_GATHER=0 takes the cp.async gather everywhere, 1 has an SpMM gather by TMA where it would not by itself
 // (tuning aids).  Asked for when a state is made.
-bool tma_wanted() { return !g_tuning.gather || atoi(g_tuning.gather) == 1; }
+bool tma_wanted() { const int e = tuned("SHFLBW_GATHER"); return e == kUnset || e == 1; }
 
 // The gather of an SpMM: TMA, unless rows share 32-byte sectors (8 or 24 tokens), there are few of them, and many blocks
 // want each.  The SMs then fetch the same few lines of L2 over and over, and the copy engine's requests to one line queue
@@ -300,7 +286,7 @@ bool tma_wanted() { return !g_tuning.gather || atoi(g_tuning.gather) == 1; }
 // (SHFLBW_GATHER=0).
 int spmm_gather(long long K, int N, int row_blocks, long long padded_cols, int tile, bool with_bias) {
     if (tile == 256 && with_bias) return shflbw::kGatherTma;
-    if (g_tuning.gather) return tma_wanted() ? shflbw::kGatherTma : shflbw::kGatherCpAsync;
+    if (const int e = tuned("SHFLBW_GATHER"); e != kUnset) return e == 1 ? shflbw::kGatherTma : shflbw::kGatherCpAsync;
     const bool dense = 20 * padded_cols > 9 * K * row_blocks;
     const bool crowded = padded_cols > 16ll * row_blocks && ((N == 8 && padded_cols >= 40 * K && K <= (dense ? 3072 : 1024)) ||
                                                              (N == 24 && padded_cols >= 150 * K && K <= 341));
@@ -309,8 +295,11 @@ int spmm_gather(long long K, int N, int row_blocks, long long padded_cols, int t
 
 // Whether the rows of the blocks lie in the TMEM lanes (SpMM, and SpConv that writes planes): `pays`, or what SHFLBW_SWAP=0|1
 // forces (tuning aid).
-bool swap_forced(int to) { return g_tuning.swap && (atoi(g_tuning.swap) != 0) == (to != 0); }
-bool rows_in_lanes(int V, bool pays) { return (V == 64 || V == 128) && !swap_forced(0) && (pays || swap_forced(1)); }
+bool rows_in_lanes(int V, bool pays) {
+    if (V != 64 && V != 128) return false;
+    const int e = tuned("SHFLBW_SWAP");
+    return e == kUnset ? pays : e != 0;
+}
 bool is_deep(long long padded_cols, int row_blocks) { return padded_cols >= 192ll * row_blocks; }
 
 // Token tile: a persistent CTA works through ceil(items / SMs) items in turn; an item of 128 tokens takes about 2/3 of
@@ -323,7 +312,7 @@ long long rounds_of_items(long long n_tokens, int tile, int row_blocks) {
     return ((n_tokens + tile - 1) / tile * row_blocks + sms - 1) / sms;
 }
 int pick_tile(long long n_tokens, int row_blocks) {
-    if (g_tuning.tile) { const int t = atoi(g_tuning.tile); if (t == 128 || t == 256) return t; }
+    if (const int e = tuned("SHFLBW_TILE"); e == 128 || e == 256) return e;
     return n_tokens <= 128 || rounds_of_items(n_tokens, 128, row_blocks) * 2 < rounds_of_items(n_tokens, 256, row_blocks) * 3 ? 128 : 256;
 }
 
@@ -340,7 +329,7 @@ int pick_tile(long long n_tokens, int row_blocks) {
 // 9584x928x440: 14.4 and 15.3).
 int spmm_tile(int V, long long N, int row_blocks, long long padded_cols) {
     const int tile = pick_tile(N, row_blocks);
-    if (tile == 128 || g_tuning.tile) return tile;
+    if (tile == 128 || tuned("SHFLBW_TILE") != kUnset) return tile;
     const long long r1 = rounds_of_items(N, 128, row_blocks), r2 = rounds_of_items(N, 256, row_blocks);
     if (r1 * 4 <= r2 * 6 && padded_cols >= (V == 128 ? 48ll : 100ll) * row_blocks) return 128;
     if (V == 16 && N % 16 && r2 >= 4 && r1 * 20 <= r2 * 38 && padded_cols >= 170ll * row_blocks) return 128;
@@ -431,7 +420,8 @@ int pick_panel(int V, int tile, bool rows, int wide_ring, int gather, PanelChoic
 // Sixteen epilogue warps, tokens in lanes: SHFLBW_EPILOGUE_WARPS=8|16 forces the choice (tuning aid).
 bool wide_wanted(int V, int tile, bool pays) {
     if (V != 64 || tile != 256) return false;
-    return g_tuning.epilogue_warps ? atoi(g_tuning.epilogue_warps) == 16 : pays;
+    const int e = tuned("SHFLBW_EPILOGUE_WARPS");
+    return e == kUnset ? pays : e == 16;
 }
 // Their ring: eight stages where nothing is added and a block takes two stages, which a ring of six holds for
 // three items only (28x28x128 -> 512, batch 256, no residual, 40 columns: 56.6 us with six, 54.7 with eight); blocks
@@ -552,7 +542,7 @@ namespace {
 // the panel kernel is no faster with so few (8608 x 440, V = 16, 3 tokens: 7.2 and 3.4): as far as 400 KB (9344 x 5224, V = 128, 5 tokens,
 // 319 KB in three passes: 8.9 and 7.4; 2304 x 4440, V = 128, 3 tokens, 382 KB in three: 8.4 and 8.3).
 bool linear_direct_pays(const shflbw_matrix& m, int tokens, int N, size_t smem) {
-    if (g_tuning.linear_direct) return atoi(g_tuning.linear_direct) != 0;
+    if (const int e = tuned("SHFLBW_LINEAR_DIRECT"); e != kUnset) return e != 0;
     const long long sms = sm_count() > 0 ? sm_count() : 148, row_blocks = m.nrow / m.brow, blocks = row_blocks * (N / shflbw::kDirectTokens);
     const long long resident = 228 * 1024 / ((long long)smem + 1024) < 8 ? 228 * 1024 / ((long long)smem + 1024) : 8;
     const bool few = N == shflbw::kDirectTokens;
@@ -647,7 +637,6 @@ static int plan_spmm(const shflbw_matrix_t* m, int N, const void* B, float alpha
     if (!m || !B || !D || N <= 0) return SHFLBW_ERR_INVALID_ARG;
     if (check_kernel_arg(kernel) != SHFLBW_OK) return SHFLBW_ERR_INVALID_ARG;
     if (beta != 0.f && !C) return SHFLBW_ERR_INVALID_ARG;
-    read_tuning();
     if (!on_current_device(*m)) return SHFLBW_ERR_NOT_ON_DEVICE;  // reference: assert(device_synced)
     // The reference asserts bcol == 1 here (spmm/blockwise_op.h:86); the kernel image lists the
     // bcol columns of a block one by one, so wider blocks run on the same kernels.
@@ -677,7 +666,8 @@ static int plan_spmm(const shflbw_matrix_t* m, int N, const void* B, float alpha
         const long long padded_cols = m->kptr.empty() ? 0 : m->kptr.back();
         const int blocks = out->num_row_blocks, tile = spmm_tile(m->brow, N, blocks, padded_cols);
         const bool sectors = N % 16 == 0 && !((uintptr_t)D & 31);
-        const bool wide = !swap_forced(1) && spmm_wide(m->brow, tile, N, sectors, beta != 0.f, padded_cols, blocks);
+        const int swap = tuned("SHFLBW_SWAP");
+        const bool wide = (swap == kUnset || swap == 0) && spmm_wide(m->brow, tile, N, sectors, beta != 0.f, padded_cols, blocks);
         const bool rows = !wide && spmm_rows(m->brow, tile, N, sectors, beta != 0.f, padded_cols, blocks);
         const int ring = wide ? wide_ring_of(beta != 0.f, padded_cols, blocks) : 0;
         int rc = pick_panel<shflbw::kPanelSpmm>(m->brow, tile, rows, ring, spmm_gather(m->ncol, N, blocks, padded_cols, tile, with_bias), &ch);
@@ -744,7 +734,7 @@ static int launch_spmm_panel(const shflbw_spmm_state_t* st, const PanelChoice& c
     // forces block-major / tile-major; tuning aid).
     p.num_blocks = st->num_row_blocks; p.div_blocks = shflbw::make_fast_div(st->num_row_blocks);
     p.tile_major = 1;
-    if (const char* e = getenv("SHFLBW_ITEM_ORDER")) p.tile_major = atoi(e) != 0;
+    if (const int e = tuned("SHFLBW_ITEM_ORDER"); e != kUnset) p.tile_major = e != 0;
     CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
     CK(cudaGetLastError());
     return SHFLBW_OK;
@@ -788,7 +778,6 @@ int shflbw_linear_direct(const shflbw_matrix_t* m, int tokens, const void* x, co
     if (((((uintptr_t)x | (uintptr_t)bias) & 1) | ((uintptr_t)out & 15)) || N % 8) return SHFLBW_ERR_UNSUPPORTED;
     if (!on_current_device(*m)) return SHFLBW_ERR_NOT_ON_DEVICE;
     if ((long long)m->nrow * N >= (1ll << 32) || (long long)m->ncol * N >= (1ll << 40)) return SHFLBW_ERR_UNSUPPORTED;   // as shflbw_spmm_init
-    read_tuning();
     void (*fn)(const shflbw::DirectParams);
     shflbw::DirectParams p{};
     switch (m->brow) {
@@ -837,7 +826,7 @@ static int spmm_host_impl(shflbw_matrix_t* m, int N, const void* B_host, float a
     // chunk width: a quarter of N rounded up to whole 256-token tiles; narrow operands go in one piece
     int w = N;
     int want = 4;
-    if (const char* e = getenv("SHFLBW_HOST_CHUNKS")) want = atoi(e) > 0 && atoi(e) <= 8 ? atoi(e) : 4;
+    if (const int e = tuned("SHFLBW_HOST_CHUNKS"); e > 0 && e <= 8) want = e;
     if (N >= 2048 && want > 1) w = ((N + want - 1) / want + 255) / 256 * 256;
     const int chunks = (N + w - 1) / w;
     constexpr int kMaxChunks = 8;
@@ -1032,7 +1021,7 @@ bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long item
 // 2860: 8.1 and 8.5 of a call that takes 12.5 us with the pass and 9.5 without), from 5000 on up to twice as much.  Taller blocks are
 // fewer, and more is seen of each one's writes (V = 64, 3x34x34x512 -> 512 at stride 2, 3540: 9.9 and 11.4).
 bool conv_scatters(const shflbw_matrix& f, long long positions, long long items) {
-    if (g_tuning.conv_scatter) return atoi(g_tuning.conv_scatter) != 0;
+    if (const int e = tuned("SHFLBW_CONV_SCATTER"); e != kUnset) return e != 0;
     const long long sms = sm_count() > 0 ? sm_count() : 148;
     if (8 * items < sms) return false;                       // a few blocks keep the general form (2x12x12x128 -> 128: 6.35 us, 5.9 without the pass)
     const double sectors = f.F / 16.0, chunk = f.brow < 32 ? f.brow : 32;
@@ -1054,7 +1043,6 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
               float alpha, int kernel, shflbw_spconv_state_t* out, size_t scratch_limit = ~(size_t)0) {
     std::memset(out, 0, sizeof *out);
     if (check_kernel_arg(kernel) != SHFLBW_OK) return SHFLBW_ERR_INVALID_ARG;
-    read_tuning();
     ConvShape cs;
     int rc = check_conv_call(f, B, Hin, Win, stride, ifmap, ofmap, &cs);
     if (rc != SHFLBW_OK) return rc;
@@ -1084,11 +1072,11 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     // planes out?
     const bool planes_possible = (f->brow == 64 || f->brow == 128) && f->F / 64 <= 65535 &&
                                  (long long)f->F * tokens < (1ll << 32) - 1 && rows_in_lanes(f->brow, true);
-    const char* ep = g_tuning.conv_planes;
+    const int ep = tuned("SHFLBW_CONV_PLANES");
     // the input as the panel kernel sees it: a strided 1x1 filter's pixels are staged side by side
     const bool compact = f->R == 1 && f->S == 1;
     const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, f->brow, row_blocks, padded_cols,
-                                      planes_possible && (ep ? atoi(ep) != 0 : is_deep(padded_cols, row_blocks)), false);
+                                      planes_possible && (ep != kUnset ? ep != 0 : is_deep(padded_cols, row_blocks)), false);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
     const int tile = pick_tile(counted, row_blocks);
     const long long items = (counted + tile - 1) / tile * row_blocks;
@@ -1099,7 +1087,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     // through the scattering kernel either).
     const bool across = f->row_permute && f->kval_logical.empty();        // filters leave their blocks
     const bool pass_fits = !across || (unperm_smem_bytes(f->F) <= 227 * 1024 && f->F <= 65536);
-    const bool planes = planes_possible && (ep ? planes_fit && atoi(ep) != 0
+    const bool planes = planes_possible && (ep != kUnset ? planes_fit && ep != 0
                                                : !pass_fits || (planes_fit && conv_planes(*f, B, Bp, tile, items, ct.row_pix != Wo, padded_cols, row_blocks,
                                                                                           2ll * B * Ho * Wo * f->F)));
     if (!planes && !pass_fits) return SHFLBW_ERR_UNSUPPORTED;
@@ -1251,7 +1239,7 @@ int shflbw_spconv_exec_bias(const shflbw_spconv_state_t* st, const void* bias, v
     // (tile-major) was measured equal on the ResNet-50 stack and on config 3, whose inputs are small next
     // to their outputs (SHFLBW_ITEM_ORDER=1 forces tile-major; tuning aid).
     p.tile_major = 0;
-    if (const char* e = getenv("SHFLBW_ITEM_ORDER")) p.tile_major = atoi(e) != 0;
+    if (const int e = tuned("SHFLBW_ITEM_ORDER"); e != kUnset) p.tile_major = e != 0;
     if (panel_bias) p.C = (const __half*)bias;
     CK(launch(ch.fn, dim3(st->grid_x, st->grid_y), dim3(ch.threads), ch.smem, s, p));
     // 3. back to NHWC in logical channel order.
@@ -1385,7 +1373,6 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     out->perm = f->d_perm; out->status_word = f->d_status;
     out->chain = 1; out->out_R = R_next; out->out_S = S_next; out->relu = relu != 0;
     PanelChoice ch;
-    read_tuning();
     const int row_blocks = f->F / f->brow;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
     const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, f->brow, row_blocks, padded_cols,
@@ -1441,11 +1428,10 @@ int shflbw_spconv_chain_set_residual(shflbw_matrix_t* f, shflbw_spconv_state_t* 
     PanelChoice ch;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
     const bool two_warps = padded_cols <= 48ll * (st->F / st->V) && (long long)st->F * st->Ho * st->Wo * st->Bp * 2 <= (256ll << 20);   // (lookup)
-    read_tuning();
-    const char* eb = g_tuning.box;                           // SHFLBW_BOX=0: residual by cp.async (tuning aid)
-    const bool box = st->gather == shflbw::kGatherTma && boxes_fit(*st) && (eb ? atoi(eb) != 0 : st->num_items >= 6ll * sm_count());
+    const int eb = tuned("SHFLBW_BOX");                      // 0: residual by cp.async (tuning aid)
+    const bool box = st->gather == shflbw::kGatherTma && boxes_fit(*st) && (eb != kUnset ? eb != 0 : st->num_items >= 6ll * sm_count());
     const bool wide = (st->variant == 2 ||
-                       (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && !g_tuning.epilogue_warps &&
+                       (st->variant == 0 && st->V == 64 && st->tokens_per_cta == 256 && tuned("SHFLBW_EPILOGUE_WARPS") == kUnset &&
                         padded_cols <= 128ll * (st->F / st->V) && 2ll * st->num_items >= 5ll * sm_count())) &&
                       lookup<shflbw::kPanelConvChain>(64, 256, &ch, st->gather, 6, two_warps ? 2 : 3, box);
     if (wide) {
