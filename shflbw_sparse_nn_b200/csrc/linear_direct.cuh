@@ -61,18 +61,20 @@ __global__ void __launch_bounds__(256) linear_direct(const DirectParams p) {
     int c0 = 0;
     do {
         const int n = cols - c0 < kDirectCols ? cols - c0 : kDirectCols;
-        // The value panels and the column ids are the layer's own: requested before the previous kernel is waited for.
+        // The value panels and the column ids are the layer's own: requested before the previous kernel is waited for.  (Not a
+        // word of arithmetic on the ids here: clamped as they are loaded, each load was waited for by itself, 4.9 us instead of
+        // 2.95 at 256 x 840, V = 128, 26 tokens.)
         const __half* const w = p.blk_val + (size_t)(row0 + c0) * V;
         for (int i = tid; i < n * (V / 8); i += 256) sm100::cp_async_16(w_smem + i * 16, w + i * 8, 16);
         sm100::cp_async_commit();
         int id[RUNS];
 #pragma unroll
-        for (int s = 0; s < RUNS; ++s)                        // (clamped: a corrupted id may give wrong numbers, never an address outside x)
-            id[s] = mine && s * 32 + lane < n ? (int)min((unsigned)__ldg(p.blk_idx + row0 + c0 + s * 32 + lane), (unsigned)p.K - 1u) : -1;
+        for (int s = 0; s < RUNS; ++s) id[s] = mine && s * 32 + lane < n ? __ldg(p.blk_idx + row0 + c0 + s * 32 + lane) : -1;
         if (c0 == 0) sm100::grid_dependency_wait();           // x may be the previous kernel's output
         unsigned short v[RUNS];                               // sixteen runs of 32 columns in flight
 #pragma unroll
-        for (int s = 0; s < RUNS; ++s) v[s] = id[s] >= 0 ? __ldcg(x + id[s]) : (unsigned short)0;
+        for (int s = 0; s < RUNS; ++s)                        // (clamped: a corrupted id may give wrong numbers, never an address outside x)
+            v[s] = id[s] >= 0 ? __ldcg(x + min(id[s], p.K - 1)) : (unsigned short)0;
 #pragma unroll
         for (int s = 0; s < RUNS; ++s)
             *(unsigned short*)(xs + warp * kDirectPitch + (s * 32 + lane) * 2) = v[s];

@@ -96,7 +96,8 @@ class _Ints:
 
 
 def test_ids_outside_the_layer_read_nothing_outside_x(monkeypatch):
-    """The ids lie in device memory: whatever stands there, the reads stay in x (the last column's, as the panel kernel's do)."""
+    """The ids lie in device memory: whatever stands there, the reads stay in x.  Beyond the last column they read that one, as
+    the panel kernel's do; negative ones read nothing."""
     monkeypatch.setenv("SHFLBW_LINEAR_DIRECT", "1")
     K, tokens, N = 96, 11, 16
     m = _matrix(32, K, (40, 96), True)
@@ -105,8 +106,11 @@ def test_ids_outside_the_layer_read_nothing_outside_x(monkeypatch):
     op = sb.SpmmBlockwiseOp().initialize(m, N, torch.zeros(K, N, device="cuda").half(), out[0])
     ids = torch.as_tensor(_Ints(op._state.blk_idx, 48 + 96), device="cuda")
     at = torch.tensor([0, 7, 39, 47, 48, 143], device="cuda")
-    for y, bad in zip(out, ([K, K + 5, 2 ** 31 - 1, -1, -2 ** 31, 1 << 20], [K - 1] * 6)):
-        ids[at] = torch.tensor(bad, dtype=torch.int32, device="cuda")
-        assert bw.linear_direct(m, tokens, x, None, N, y, torch.cuda.current_stream())
-        torch.cuda.synchronize()
-    assert torch.equal(*out) and not out[0].isnan().any()
+    for bad in ([K, K + 5, 2 ** 31 - 1, 1 << 20, K, K], [-1, -2 ** 31, -K, -2, -1, -1]):
+        if bad[0] < 0:
+            x[:, K - 1] = 0
+        for y, there in zip(out, (bad, [K - 1] * 6)):
+            ids[at] = torch.tensor(there, dtype=torch.int32, device="cuda")
+            assert bw.linear_direct(m, tokens, x, None, N, y, torch.cuda.current_stream())
+            torch.cuda.synchronize()
+        assert torch.equal(*out) and not out[0].isnan().any()
