@@ -323,16 +323,21 @@ int pick_tile(long long n_tokens, int row_blocks) {
 //   400x2312x1872, V = 16, 219: 6.3 and 5.9; 3712x280x1520, V = 128, 56: 6.9 and 5.9; 832x400x1520, V = 32, 39: 4.7 and 4.8;
 //   five sixths: 8576x728x1096, V = 128, 99: 15.5 and 14.0; 976x2488x1184, V = 16, 562: 13.2 and 12.3; 2912x352x416, V = 16, 123: 6.4 and 6.5;
 //   896x520x5536, V = 64, 182: 7.9 and 8.2.  Over 70 shapes on the 128 side 7 % less.
-// 16 rows and rows of B that are not whole sectors (N % 16 = 8; every second one is fetched in five sectors per box instead of four): from
-// 170 columns already at up to 19 rounds of 128 for 10 of 256 (3072x768x1000, 192 columns, 11 and 6 rounds: 14.7 and 13.5; 2880x3104x1208,
-// 415, 13 and 7: 24.0 and 23.2; 37 shapes 0.91 to 1.02, 4 % less; with whole sectors 3072x768x1024 10.9 and 12.0; 133 columns,
-// 9584x928x440: 14.4 and 15.3).
-int spmm_tile(int V, long long N, int row_blocks, long long padded_cols) {
+// 16 rows and rows of B that are not whole sectors (N % 16 = 8; every second one is fetched in five sectors per box instead of four, so
+// that the gather is more of an item): the 128-token side also where it saves fewer rounds.  128 over 256 tokens, means of 835 shapes by
+// rounds of 128 for one of 256 (up to 1.67 / 1.75 / 1.8 / 11:6 / 1.9): from 200 columns on 0.93 / 0.95 / 0.96 / 0.95 / 0.97, with C
+// 0.93 / 0.96 / 0.97 / 0.99 / 1.00; 165 to 199 columns 0.92 / 0.96 / 0.98 / 0.99 / 1.01; these with C, whose second epilogue a steady run of
+// rounds does not hide, up to seven rounds of 256 tokens 0.95 / 0.98 / 0.99 / 1.00 / 1.04, from eight on 0.99 / 1.02 / 1.08 / 1.12 / 1.09
+// (4096x3200x1400, 165 columns, 20 and 11 rounds: 20.3 and 24.3 us).  Below, with C, 1.1 to 1.2 from 1.75 on; whole sectors:
+// 3072x768x1024, 192 columns 10.9 and 12.0; 32 rows 0.96 to 1.04, with C 1.04 to 1.25.
+int spmm_tile(int V, long long N, int row_blocks, long long padded_cols, bool with_c) {
     const int tile = pick_tile(N, row_blocks);
     if (tile == 128 || tuned("SHFLBW_TILE") != kUnset) return tile;
     const long long r1 = rounds_of_items(N, 128, row_blocks), r2 = rounds_of_items(N, 256, row_blocks);
     if (r1 * 4 <= r2 * 6 && padded_cols >= (V == 128 ? 48ll : 100ll) * row_blocks) return 128;
-    if (V == 16 && N % 16 && r2 >= 4 && r1 * 20 <= r2 * 38 && padded_cols >= 170ll * row_blocks) return 128;
+    if (V == 16 && N % 16 && (padded_cols >= 200ll * row_blocks ? r1 * 20 <= r2 * 38
+                                                                 : padded_cols >= 170ll * row_blocks && r1 * 6 <= r2 * 11 && !(with_c && r2 > 7)))
+        return 128;
     return r1 * 6 <= r2 * 10 && V != 64 && padded_cols >= (V == 128 ? 64ll : 200ll) * row_blocks ? 128 : 256;
 }
 
@@ -664,7 +669,7 @@ static int plan_spmm(const shflbw_matrix_t* m, int N, const void* B, float alpha
     } else {
         PanelChoice ch;
         const long long padded_cols = m->kptr.empty() ? 0 : m->kptr.back();
-        const int blocks = out->num_row_blocks, tile = spmm_tile(m->brow, N, blocks, padded_cols);
+        const int blocks = out->num_row_blocks, tile = spmm_tile(m->brow, N, blocks, padded_cols, beta != 0.f);
         const bool sectors = N % 16 == 0 && !((uintptr_t)D & 31);
         const int swap = tuned("SHFLBW_SWAP");
         const bool wide = (swap == kUnset || swap == 0) && spmm_wide(m->brow, tile, N, sectors, beta != 0.f, padded_cols, blocks);

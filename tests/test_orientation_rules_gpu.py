@@ -186,3 +186,25 @@ def test_spmm_tile_by_rounds(monkeypatch, V, M, K, N, density, tile):
         torch.cuda.synchronize()
         got.append(d)
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("K,N,M,cols,beta,tile", (
+    (2816, 2392, 3728, 180, 1.0, 256), (2816, 2392, 3728, 180, 0.0, 256), (3200, 1400, 4096, 180, 1.0, 256),      # many rounds
+    (768, 1000, 3072, 180, 1.0, 128), (1776, 1288, 1856, 300, 1.0, 128), (1360, 2696, 1360, 180, 0.0, 256)))
+def test_tiles_of_16_rows_and_ragged_columns(monkeypatch, K, N, M, cols, beta, tile):
+    """Rows of B between sectors: 128-token items where the rounds that they save pay for their epilogues, C among them."""
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the rounds are of 148 SMs")
+    m = sb.BlockwiseSpMatrix().init_random(M, K, 16, 1, (cols + 0.5) / K, True, 7, values="uniform")
+    m.transform_and_sync_device()
+    b, c = ((torch.rand(r, N, device="cuda") * 2 - 1).half() for r in (K, M))
+    got = []
+    for forced in (None, "256", "128"):
+        if forced: monkeypatch.setenv("SHFLBW_TILE", forced)
+        d = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
+        op = sb.SpmmBlockwiseOp().initialize(m, N, b, 1.0, c, beta, d) if beta else sb.SpmmBlockwiseOp().initialize(m, N, b, d)
+        assert forced or op._state.tokens_per_cta == tile
+        op()
+        torch.cuda.synchronize()
+        got.append(d)
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
