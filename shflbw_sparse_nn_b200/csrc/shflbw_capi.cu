@@ -1019,19 +1019,19 @@ bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long item
 
 // Whether the panel kernel itself puts a permuted filter's positions in order, value by value: a pass less (2 us and a launch,
 // 2.2 us of the host's time), but every 32-byte sector of an F-vector is written once by each block that has a filter in it, and
-// the L2 takes some 80 of such partial sectors a clock.  So for small outputs, by the expected sectors that the busiest SM writes.
-// Device time with the pass and without: up to 2600 sectors 1 to 15 % less (40x11x11x192 -> 96 at stride 2, V = 32, 720: 6.4 and 5.7;
-// 31x16x16x64 -> 48, V = 16, 960: 7.7 and 6.6; 2x34x34x408 -> 128, V = 32: 9.6 and 8.7; 8x24x24x128 -> 448 at stride 2, V = 32, 2465: 7.4 and 7.0;
-// 28x28x256 -> 512, V = 64, 2560: 10.2 and 10.0), then up to 5 % more, for 3 us less of the host's time (5x27x27x256 -> 512 at stride 2, V = 32,
-// 2860: 8.1 and 8.5 of a call that takes 12.5 us with the pass and 9.5 without), from 5000 on up to twice as much.  Taller blocks are
-// fewer, and more is seen of each one's writes (V = 64, 3x34x34x512 -> 512 at stride 2, 3540: 9.9 and 11.4).
+// the L2 takes some 80 of such partial sectors a clock.  So for small outputs, by the expected sectors that the busiest SM writes; the
+// line rises with the share of the SMs that have items, since the pass is spread over all of them.  Scattered over the pass, means of 500
+// shapes of all heights in a graph (eager calls 0.01 to 0.05 less) by sectors, up to 1200 / 1800 / 2400 / 2900 / 3500 / 4600: items on up to a
+// quarter of the SMs 0.88 / 0.96 / 1.00 / 1.08 / 1.19 / 1.23; to a half 0.89 / 0.94 / 0.98 / 1.04 / 1.13 / 1.19; to three quarters 0.89 / 0.93 /
+// 0.94 / 1.02 / 1.04 / 1.13; to all 0.84 / 0.89 / 0.93 / 0.99 / 0.96 / 1.02; several rounds 0.81 / 0.86 / 0.90 / 0.94 / 0.94 / 1.01.  Among the 331
+// shapes that scatter by the line one takes 13 % longer, the others up to 9 in a graph and 2 eagerly.
 bool conv_scatters(const shflbw_matrix& f, long long positions, long long items) {
     if (const int e = tuned("SHFLBW_CONV_SCATTER"); e != kUnset) return e != 0;
     const long long sms = sm_count() > 0 ? sm_count() : 148;
     if (8 * items < sms) return false;                       // a few blocks keep the general form (2x12x12x128 -> 128: 6.35 us, 5.9 without the pass)
     const double sectors = f.F / 16.0, chunk = f.brow < 32 ? f.brow : 32;
     const double written = sectors * (1 - std::pow(1 - 1 / sectors, chunk)) * (f.F / chunk) * (double)positions;   // in all
-    return written / (double)items * (double)((items + sms - 1) / sms) <= (f.brow <= 32 ? 2900 : 2600);
+    return written / (double)items * (double)((items + sms - 1) / sms) <= 1500 + 1900 * (items < sms ? (double)items / (double)sms : 1.0);
 }
 
 // Launch plan of one NHWC SpConv call, without its scratch pointers: kernel choice, grid, and

@@ -41,3 +41,14 @@ def test_rule():
         f = sb.BlockwiseSpFilter().init_random(F, 1, 1, shape[3], V, 1, 0.1, True, 5, values="uniform")
         f.transform_and_sync_device()
         _call(f, shape, 2 if shape[0] == 5 else 1, None, launches)
+
+
+@pytest.mark.parametrize("shape,F,V,stride,launches", (
+    ((5, 12, 12, 32), 512, 64, 2, 3), ((11, 13, 13, 16), 320, 64, 2, 3),   # 24 and 35 items of 2450 sectors: the pass has all SMs
+    ((4, 13, 13, 416), 384, 64, 2, 2), ((5, 27, 27, 256), 512, 32, 2, 2)))  # 24 of 1750; 208 items, two rounds of 2858
+def test_few_items_scatter_less(shape, F, V, stride, launches):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the shares are of 148 SMs")
+    f = sb.BlockwiseSpFilter().init_random(F, 1, 1, shape[3], V, 1, 0.25, True, 5, values="uniform")
+    f.transform_and_sync_device()
+    _call(f, shape, stride, None, launches)
