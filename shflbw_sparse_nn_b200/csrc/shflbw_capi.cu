@@ -1007,14 +1007,24 @@ bool boxes_fit(const shflbw_spconv_state_t& st) {
 // 64 columns: 20.7, as planes 31.4; 14x14x512 -> 2048, 3x3, batch 16, 900: 29.0 and 33.2).
 // With filters in lanes (28.3 instead of 24.5 for 14x14x512 -> 2048, 460 columns) only at 64 rows from 1200 columns on, as
 // the chained layers (14x14x256 -> 1024, 1800 columns: 33.4, tokens 33.8).
-// Nor at 128 rows where the output is beyond 80 MB and of more than 640 filters: the last pass comes to planes that have left the
-// L2 (35x35x128 -> 1920, 1x1, batch 31, 146 MB: 112 and 142; 53x53x128 -> 768, 1x1, batch 24, 104 MB: 87 and 96; 28x28x128 -> 1280, 3x3, batch 64,
-// 128 MB: 106 and 111; but 42x42x256 -> 512, 3x3, batch 64, 116 MB: 170 and 161; 64 rows: 5 % less to 8 % more).
+// Nor where planes and output together are beyond the L2's 126 MB and of more than 640 filters: the last pass comes to planes that have
+// left it.  Planes over positions, means of 260 shapes by these megabytes, 80 to 100 / 126 / 150 / 200 / more: 64 rows 0.90 / 0.94 / 0.99 /
+// 1.00 / 1.02, 128 rows 0.95 / 0.98 / 1.01 / 1.06 / 1.08 (16x60x60 of 1920 filters, 1x1: 1.23); up to 640 filters, whose few
+// blocks are written sooner after one another, 0.91 / 0.92 / 0.95 / 0.95 / 0.93.
 bool conv_planes(const shflbw_matrix& f, int B, int Bp, int tile, long long items, bool padded_rows, long long padded_cols, int row_blocks,
-                 long long out_bytes) {
-    if (f.brow == 128 && f.F > 640 && out_bytes > 80000000) return false;
-    return f.row_permute && f.kval_logical.empty() && tile == 256 && (f.brow == 128 || items >= (sm_count() > 0 ? sm_count() : 148)) && 8 * (Bp - B) <= Bp &&
-           (padded_cols >= 64ll * row_blocks || !padded_rows);
+                 long long planes_and_out) {
+    if (f.F > 640 && planes_and_out > 126000000) return false;
+    return tile == 256 && (f.brow == 128 || items >= (sm_count() > 0 ? sm_count() : 148)) && 8 * (Bp - B) <= Bp && (padded_cols >= 64ll * row_blocks || !padded_rows);
+}
+// And whether it is for the number of its filters alone, whatever the padding of the batch, the tile and the SMs with items: the last pass
+// of positions loads the permutation in every block and holds an F-vector for each position, and gets slow.  Planes over positions,
+// means of 450 shapes with fewer than three items per SM, by filters, planes of up to 1.125 / 1.6 / 2 / 8 times the images: up to 512 filters
+// 0.96 / 0.98 / 1.04 / 1.13, 1024 0.95 / 0.97 / 0.98 / 1.09, 1536 0.91 / 0.92 / 0.97 / 1.05, 2304 0.89 / 0.88 / 0.91 / 0.99, more 0.82 / 0.82 / 0.81 / 0.87
+// (3x39x11x616 -> 3712, 1x1 at stride 2, 200 columns: 20.5 and 14.1 us; 8x8x8x544 -> 2944, V = 128, 290: 15.7 and 11.7).  From
+// three items per SM on 0.97 / 1.05 / 0.99 / 1.19 beyond 2304.
+bool conv_planes_by_filters(const shflbw_matrix& f, int B, int Bp, long long items, bool padded_rows, long long padded_cols, int row_blocks) {
+    return items < 3ll * (sm_count() > 0 ? sm_count() : 148) && (padded_cols >= 64ll * row_blocks || !padded_rows) &&
+           (f.F > 2304 || (f.F > 1024 && Bp <= 2 * B));
 }
 
 // Whether the panel kernel itself puts a permuted filter's positions in order, value by value: a pass less (2 us and a launch,
@@ -1092,11 +1102,12 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     // through the scattering kernel either).
     const bool across = f->row_permute && f->kval_logical.empty();        // filters leave their blocks
     const bool pass_fits = !across || (unperm_smem_bytes(f->F) <= 227 * 1024 && f->F <= 65536);
-    const bool planes = planes_possible && (ep != kUnset ? planes_fit && ep != 0
-                                               : !pass_fits || (planes_fit && conv_planes(*f, B, Bp, tile, items, ct.row_pix != Wo, padded_cols, row_blocks,
-                                                                                          2ll * B * Ho * Wo * f->F)));
+    const bool padded_rows = ct.row_pix != Wo, small = across && conv_scatters(*f, (long long)B * Ho * Wo, items);
+    const bool pays = across && (conv_planes(*f, B, Bp, tile, items, padded_rows, padded_cols, row_blocks, 2ll * (B + Bp) * Ho * Wo * f->F) ||
+                                 (!small && conv_planes_by_filters(*f, B, Bp, items, padded_rows, padded_cols, row_blocks)));
+    const bool planes = planes_possible && (ep != kUnset ? planes_fit && ep != 0 : !pass_fits || (planes_fit && pays));
     if (!planes && !pass_fits) return SHFLBW_ERR_UNSUPPORTED;
-    const bool scatter = !planes && across && conv_scatters(*f, (long long)B * Ho * Wo, items);
+    const bool scatter = !planes && small;
     PanelChoice ch;
     if (planes) {
         const int ring = chain_wide(f->brow, tile, items, padded_cols, row_blocks) ? wide_ring_of(false, padded_cols, row_blocks) : 0;

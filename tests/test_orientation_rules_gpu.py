@@ -208,3 +208,28 @@ def test_tiles_of_16_rows_and_ragged_columns(monkeypatch, K, N, M, cols, beta, t
         torch.cuda.synchronize()
         got.append(d)
     assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+
+
+@pytest.mark.parametrize("V,B,H,W,C,F,R,stride,cols,variant", (
+    (64, 3, 39, 11, 616, 3712, 1, 2, 197, 1), (128, 9, 5, 5, 64, 3840, 3, 1, 303, 1), (64, 18, 7, 7, 632, 3072, 3, 2, 267, 1),   # many filters:
+    (128, 27, 13, 13, 888, 2432, 1, 2, 356, 1), (64, 6, 9, 9, 176, 1088, 3, 1, 300, 1),                    # planes whatever the batch and the tile
+    (64, 3, 9, 9, 176, 1088, 3, 1, 300, 0), (64, 6, 9, 9, 176, 1024, 3, 1, 300, 0),                        # eight planes for three images; fewer filters
+    (64, 46, 46, 46, 328, 2112, 1, 2, 135, 0), (128, 58, 15, 8, 584, 3840, 1, 1, 40, 1), (64, 48, 58, 58, 64, 640, 1, 1, 40, 1)))   # beyond the L2; not; few filters
+def test_planes_by_filters_and_bytes(V, B, H, W, C, F, R, stride, cols, variant, monkeypatch):
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the item counts are of 148 SMs")
+    f = sb.BlockwiseSpFilter().init_random(F, R, R, C, V, 1, (cols + 0.5) / (R * R * C), True, 5, values="uniform")
+    f.transform_and_sync_device()
+    x = (torch.rand(B, H, W, C, device="cuda") * 2 - 1).half()
+    got = []
+    for planes in (None, "0", "1"):
+        if planes:
+            monkeypatch.setenv("SHFLBW_CONV_PLANES", planes)
+        y = torch.full((B, -(-H // stride), -(-W // stride), F), float("nan"), dtype=torch.float16, device="cuda")
+        op = sb.SpconvBlockwiseOp().initialize(f, B, H, W, stride, x, y, 0.25)
+        assert op._state.variant == (int(planes) if planes else variant)
+        op(torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        got.append(y)
+    f.device_status()
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
