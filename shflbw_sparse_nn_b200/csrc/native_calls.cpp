@@ -14,6 +14,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <climits>
 #include <cstring>
 
 #include <ATen/PythonTorchFunctionTLS.h>
@@ -163,7 +164,7 @@ PyObject* conv2d(PyObject*, PyObject* const* args, Py_ssize_t n) {
     const long long stride = PyLong_AsLongLong(args[3]), C = PyLong_AsLongLong(args[4]), F = PyLong_AsLongLong(args[5]);
     auto* f = (shflbw_matrix_t*)PyLong_AsVoidPtr(args[2]);
     if (PyErr_Occurred()) return nullptr;
-    if (!THPVariable_CheckExact(args[0])) Py_RETURN_NONE;
+    if (!THPVariable_CheckExact(args[0]) || stride < 1 || stride > INT_MAX) Py_RETURN_NONE;
     try {
         const at::Tensor x = THPVariable_Unpack(args[0]);
         at::Tensor bias, y;

@@ -122,3 +122,16 @@ def test_operators_take_every_stream_form(monkeypatch):
         ops[1]("no stream")
     with pytest.raises(Exception):
         bw.SpmmBlockwiseOp()(None)                                       # a state that no init has filled
+
+
+@pytest.mark.parametrize("stride", (0, -1, 2 ** 31, 2 ** 32 + 1))
+def test_a_stride_that_is_none_stays_with_python(stride):
+    """A division by it would end the process; as 32 bits it may be another one."""
+    conv = _conv()
+    x = torch.randn(2, 16, 6, 6, device="cuda").half().to(memory_format=torch.channels_last)
+    conv(x)                                                              # uploads the filter
+    conv.stride = stride
+    assert _raw(conv, x) is None
+    if stride <= 0:
+        with pytest.raises(Exception):                                   # ZeroDivisionError, an extent below zero
+            conv(x)
