@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import shflbw_sparse_nn_b200 as sb
+from shflbw_sparse_nn_b200 import blockwise as bw
 from gpu_util import dev
 from shflbw_sparse_nn_b200.nn import ShflBWConv2d, ShflBWLinear
 
@@ -97,6 +98,44 @@ def test_calls_of_different_kinds_back_to_back(permute):
     for _ in range(5):
         assert all(torch.equal(a, b) for a, b in zip(run(lambda: None), want))
     for m in (conv1, mat, layer, conv2, lin.spmat):
+        m.device_status()
+
+
+def test_few_tokens_between_kernels_that_start_each_other_early():
+    """SpMM -> one-launch linear layer -> SpMM on the same buffers every time: each reads what the kernel before has just written, and
+    writes what the one behind it was still reading a call ago."""
+    K, tokens = 4096, 64
+    first = sb.BlockwiseSpMatrix().init_random(tokens, K, 64, 1, 0.5, True, 41, values="uniform")     # one block: 32 stages on one SM
+    layer = sb.BlockwiseSpMatrix().init_random(1024, 96, 32, 1, 0.5, True, 42, values="uniform")
+    last = sb.BlockwiseSpMatrix().init_random(256, 1024, 64, 1, 0.3, True, 43, values="uniform")
+    for m in (first, layer, last):
+        m.transform_and_sync_device()
+    bias = dev(sb.uniform_half(44, 1024))
+    x = [dev(sb.uniform_half(50 + i, K * 96).reshape(K, 96)) for i in range(8)]
+    y1 = torch.zeros(tokens, 96, dtype=torch.float16, device="cuda")                                  # read on as 64 tokens of 96
+    y2 = torch.zeros(1024, tokens, dtype=torch.float16, device="cuda")
+    stream = torch.cuda.current_stream()
+
+    def run(wait):
+        out = [torch.zeros(256, tokens, dtype=torch.float16, device="cuda") for _ in x]
+        ops = [(sb.SpmmBlockwiseOp().initialize(first, 96, a, 0.0625, None, 0.0, y1),
+                sb.SpmmBlockwiseOp().initialize(last, tokens, y2, 0.0625, None, 0.0, y3)) for a, y3 in zip(x, out)]
+        torch.cuda.synchronize()
+        for before, behind in ops:
+            before(stream)
+            wait()
+            assert bw.linear_direct(layer, tokens, y1, bias, tokens, y2, stream)
+            wait()
+            behind(stream)
+            wait()
+        torch.cuda.synchronize()
+        return out
+
+    want = run(torch.cuda.synchronize)
+    assert all(torch.isfinite(w).all() and w.abs().max() > 0 for w in want) and not torch.equal(want[0], want[1])
+    for _ in range(5):
+        assert all(torch.equal(a, b) for a, b in zip(run(lambda: None), want))
+    for m in (first, layer, last):
         m.device_status()
 
 

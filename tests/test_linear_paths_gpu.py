@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import shflbw_sparse_nn_b200 as sb
+from shflbw_sparse_nn_b200 import blockwise as bw
 from gpu_util import epilogue_warps, operand_swap, tile
 from shflbw_sparse_nn_b200.nn import ShflBWLinear
 
@@ -88,3 +89,34 @@ def test_input_in_the_operands_order_is_copied_once(tokens):
     peak = torch.cuda.max_memory_allocated() - before
     assert torch.equal(y, want) and peak <= (K + M) * padded * 2 + 4096        # the operand, the result, rounding
     m.device_status()
+
+
+@pytest.mark.parametrize("direct", [0, 1])
+@pytest.mark.parametrize("V,K,tokens,offset,swap,ew,t,gather", [
+    (64, 320, 37, 0, 1, None, 128, None), (64, 328, 65, 0, 0, None, 128, None), (128, 320, 63, 0, 1, None, 128, None),
+    (64, 640, 300, 0, 1, None, 256, "0"), (128, 320, 300, 0, 0, None, 256, None), (32, 320, 1, 0, None, None, None, None),
+    (32, 203, 8, 0, None, None, None, None), (64, 203, 65, 0, 1, None, 256, None), (16, 77, 130, 0, None, None, None, None),   # K % 8 != 0: 2-byte loads,
+    (64, 203, 300, 0, 0, None, 256, None), (128, 1031, 65, 0, None, None, None, None),                     # one and several 64-token tiles
+    (64, 320, 65, 3, None, None, None, None), (32, 640, 130, 1, None, None, None, None), (16, 200, 300, 5, None, None, None, None),  # unaligned
+    (64, 203, 256 * 40 + 5, 0, 0, 16, 256, None), (64, 64, 256 * 40 + 5, 1, 0, 16, 256, None),             # sixteen epilogue warps
+])
+def test_both_routes_equal_the_operator_bit_for_bit(monkeypatch, V, K, tokens, offset, swap, ew, t, gather, direct):
+    """Few tokens go to the one-launch kernel by themselves: each case by it and by the transpose and the panel kernel."""
+    monkeypatch.setenv("SHFLBW_LINEAR_DIRECT", str(direct))
+    if gather is not None:
+        monkeypatch.setenv("SHFLBW_GATHER", gather)
+    m = sb.BlockwiseSpMatrix().init_random(512, K, V, 1, 0.3, True, 21, values="uniform")
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    b = (torch.rand(512, generator=g, device="cuda") * 2 - 1).half()
+    buf = torch.full((tokens * K + 2 * K + offset,), float("nan"), dtype=torch.float16, device="cuda")
+    x = buf[K + offset:][:tokens * K].view(tokens, K)        # amid NaN
+    x.copy_(torch.rand(tokens, K, generator=g, device="cuda") * 2 - 1)
+    lin = ShflBWLinear(m, b).cuda()
+    with operand_swap(swap), epilogue_warps(ew), tile(t):
+        y = lin(x)
+        want = _plain(m, x, b)
+    out = torch.empty((512, -(-tokens // 8) * 8), dtype=torch.float16, device="cuda")
+    assert bw.linear_direct(m, tokens, x, b, out.shape[1], out, torch.cuda.current_stream()) == bool(direct)
+    torch.cuda.synchronize()
+    m.device_status()
+    assert torch.equal(y, want) and (not direct or torch.equal(out[:, :tokens].t(), want))
