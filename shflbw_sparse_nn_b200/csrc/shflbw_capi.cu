@@ -356,14 +356,15 @@ int spmm_tile(int V, long long N, int row_blocks, long long padded_cols, bool wi
 // columns (V = 32, 40 columns: 9.45 and 8.95, 54: 4.3 and 3.9, 100: 4.0 and 4.6; V = 64 chained, 40: 4.07 and 3.99, 64: 4.4
 // and 4.6, 300: 5.5 and 6.3; V = 128, 40: 10.2 and 10.9, 300: 12.9 and 15.7).
 //   128 rows with tokens in lanes write the longest items of all.  Into NHWC, padding that fills the chip leaves no SM to
-// the passes around (10x10x24 -> 1792, batch 6, 98 -> 140 items: 10.0 and 11.3).  Chained, with a stage of columns and part of
+// the passes around (10x10x24 -> 1792, batch 6, 98 -> 140 items: 10.0 and 11.3); deep ones (is_deep) gain as much from the gather (38 shapes
+// of 207 to 870 columns whose padding does so, TMA over cp.async 0.89 to 1.06, mean 0.98).  Chained, with a stage of columns and part of
 // a second one, whose few copies the TMA gather's longer way to the first bytes does not repay, they gather by cp.async
 // (28x28x256 -> 256, 3x3, batch 64, 100 columns 12.2 and 12.1 without and 15.6 and 15.7 with a residual; 14x14x1024 -> 512,
 // batch 32, 6.4 and 7.0, 7.5 and 7.8; batch 8, 28x28x256 -> 256, 4.9 and 5.2), and up to three stages where there are fewer
 // items than SMs or the rows are padded (27x27x256 -> 256, 3x3, batch 100, 157 columns, with residual: 34.1 and 36.1).  Otherwise TMA: 16 columns 10.9 and 10.1, 48 14.4 and 13.1 with a residual, 200 13.8 and 12.9, 800 29.5 and
 // 26.2, 2000 59.8 and 49.3 (28x28x256 -> 256, batch 64).
 struct ConvTokens { int row_pix; int gather; };
-ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int V, int row_blocks, long long padded_cols, bool rows, bool chain) {
+ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int V, int row_blocks, long long padded_cols, bool chain) {
     const ConvTokens plain{Wo, shflbw::kGatherCpAsync};
     const int row_pix = tma_wanted() ? tma_row_pix(Wo, Wp, Bp, stride) : 0;
     const long long before = (long long)Ho * Wo * Bp, after = (long long)Ho * row_pix * Bp;
@@ -371,7 +372,7 @@ ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int V, int ro
     const int tile0 = pick_tile(before, row_blocks), tile1 = pick_tile(after, row_blocks);
     const long long rounds0 = rounds_of_items(before, tile0, row_blocks), rounds1 = rounds_of_items(after, tile1, row_blocks);
     const long long cost0 = rounds0 * (tile0 == 128 ? 2 : 3), cost1 = rounds1 * (tile1 == 128 ? 2 : 3);
-    if (V == 128 && !rows) {
+    if (V == 128 && !is_deep(padded_cols, row_blocks)) {
         const bool few = (after + tile1 - 1) / tile1 * row_blocks <= (sm_count() > 0 ? sm_count() : 148);
         if (chain && (few || row_pix != Wo ? tile1 == 256 || padded_cols > 64ll * row_blocks
                           : padded_cols > 64ll * row_blocks && padded_cols <= 128ll * row_blocks)) return plain;
@@ -379,7 +380,7 @@ ConvTokens conv_tokens(int Ho, int Wo, int Wp, int Bp, int stride, int V, int ro
             return plain;
     }
     const bool short_items = tile1 > tile0 && V <= 64 && padded_cols <= (V == 64 && chain ? 48ll : 64ll) * row_blocks;
-    const bool tight = !rows && V >= 64 && padded_cols > 32ll * row_blocks && padded_cols <= 128ll * row_blocks;
+    const bool tight = V >= 64 && padded_cols > 32ll * row_blocks && padded_cols <= 128ll * row_blocks;
     const bool roomy = cost1 <= cost0 || padded_cols <= 32ll * row_blocks || 10 * after <= 13 * before;
     const bool pays = short_items || (roomy && (tight ? 5 * cost1 <= 6 * cost0 : 4 * cost1 <= 5 * cost0));
     return pays ? ConvTokens{row_pix, shflbw::kGatherTma} : plain;
@@ -1090,8 +1091,7 @@ int plan_conv(const shflbw_matrix* f, int B, int Hin, int Win, int stride, const
     const int ep = tuned("SHFLBW_CONV_PLANES");
     // the input as the panel kernel sees it: a strided 1x1 filter's pixels are staged side by side
     const bool compact = f->R == 1 && f->S == 1;
-    const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, f->brow, row_blocks, padded_cols,
-                                      planes_possible && (ep != kUnset ? ep != 0 : is_deep(padded_cols, row_blocks)), false);
+    const ConvTokens ct = conv_tokens(Ho, Wo, compact ? Wo : Win + f->S - 1, Bp, compact ? 1 : stride, f->brow, row_blocks, padded_cols, false);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
     const int tile = pick_tile(counted, row_blocks);
     const long long items = (counted + tile - 1) / tile * row_blocks;
@@ -1391,8 +1391,7 @@ int shflbw_spconv_chain_init(shflbw_matrix_t* f, int B, int Hin, int Win, int st
     PanelChoice ch;
     const int row_blocks = f->F / f->brow;
     const long long padded_cols = f->kptr.empty() ? 0 : f->kptr.back();
-    const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, f->brow, row_blocks, padded_cols,
-                                      rows_in_lanes(f->brow, is_deep(padded_cols, row_blocks)), true);
+    const ConvTokens ct = conv_tokens(Ho, Wo, Win + f->S - 1, Bp, stride, f->brow, row_blocks, padded_cols, true);
     const long long counted = (long long)Ho * ct.row_pix * Bp;
     const int tile = pick_tile(counted, row_blocks);
     const long long items = (counted + tile - 1) / tile * row_blocks;
