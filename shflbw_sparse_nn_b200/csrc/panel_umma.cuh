@@ -10,12 +10,13 @@
 // memory: W[p][0..V) is a contiguous slice of the value panels, G[p][..] is row indices[p] of
 // the dense operand, gathered from L2.  Two orientations exist (template parameter MODE):
 //   tokens in lanes  tokens are the UMMA M dimension (128 TMEM lanes), the V rows of the block
-//                    the N dimension (32/64/128): TM instructions per 16 columns.  Used for
-//                    V = 32, for SpConv writing NHWC, and for blocks with few columns.
+//                    the N dimension (16/32/64/128): TM instructions per 16 columns.  V = 16 and
+//                    32, SpConv writing NHWC, and what the rules below keep from the other.
 //   rows in lanes    the V rows are M (64 or 128) and the T tokens N (128 or 256): ONE instruction
 //                    per 16 columns, 128 clk at 128 x 256, 80 clk at 64 x 256 (weight-stationary
-//                    form), and the accumulator holds one output row per lane.  Default for
-//                    SpMM and chained SpConv with V = 64 / 128 and >= 3 stages of columns.
+//                    form), and the accumulator holds one output row per lane.  V = 64 / 128:
+//                    SpMM by the layout of D, C and the depth (spmm_rows, spmm_wide), chained
+//                    SpConv where it is deep (chain_rows), planes of very deep 64-row filters.
 // The description below is written for the first orientation; the second differs in the
 // gathered tile's layout ([K group][T/64 swizzle atoms]), the MMA issue and the epilogue.
 //
@@ -177,8 +178,6 @@ struct PanelCfg {
     static constexpr int W_BYTES = KS * V * 2;
     static constexpr int STAGE_BYTES = G_BYTES + W_BYTES;
     static constexpr int PIPE_BYTES = STAGES * STAGE_BYTES;
-    // Each epilogue warp transposes 32 tokens x 32 output rows / filters through 2 KB so that
-    // its global stores are 16 bytes per lane and 64-byte runs.
     // Epilogue tiles (tokens in lanes only): each epilogue warp transposes 32 tokens x 32 output
     // rows / filters through 2 KB so that its global stores are 16 bytes per lane and 64-byte
     // runs.  With rows in lanes the stores go straight from registers.

@@ -539,8 +539,10 @@ void drop_device_copy(shflbw_matrix& m) {
 }  // namespace shflbw
 
 namespace {
-// Whether a linear layer on a few tokens goes to the one-launch kernel: where its blocks, of 8 tokens each, are resident at
-// once and read little.  Device time, two launches and one: 4096 x 4096, V = 64, density 0.1 on 1 / 8 / 16 / 37 / 64 tokens
+// Whether a linear layer on a few tokens goes to the one-launch kernel: where its blocks, of 8 tokens each, are few and read little.
+// Their registers (40 to 56 a thread) let four to six blocks of 256 threads be on an SM at once, shared memory often fewer, and the
+// limit is four; up to 8 tokens it is what shared memory lets in, eight at most, in two waves (66 shapes of 4 to 8 blocks an SM: 0.22 to 0.68
+// of the two launches' device time).  Device time, two launches and one: 4096 x 4096, V = 64, density 0.1 on 1 / 8 / 16 / 37 / 64 tokens
 // 5.4 / 5.7 / 5.1 / 5.5 / 5.4 and 2.9 / 3.4 / 4.1 / 5.0 / 9.2 us (64: 3.5 blocks an SM, of which 3 are resident); the host gains another
 // 2.2 us.  Over 160 shapes the two are equal near 270 KB an SM, of value panels and of the 32-byte sectors of x, less 20 KB for
 // every further pass over a block's columns (3712 x 7816, density 0.086, 18 tokens, 242 KB in two passes: 6.4 and 7.5;
